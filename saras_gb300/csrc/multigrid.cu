@@ -367,10 +367,11 @@ __device__ void smem_impose_bc(T *p, int X, int Y, int Z, const MgBC &bc, const 
 }
 
 // The coarsest-level solve on shared-memory arrays: p (zeroed by the caller)
-// and r in the padded layout of a level with core 0..X, 0..Y, 0..Z.
+// and r in the padded layout of a level with core 0..X, 0..Y, 0..Z.  done:
+// sweeps already in p, none of which met the tolerance.
 template <typename T>
 __device__ void coarse_gs(T *p, T *r, int X, int Y, int Z, const MgK &kk, const MgBC &bc, T tol, int maxCount, int tgtMode,
-                          long long *iters) {
+                          long long *iters, int done = 0) {
     __shared__ T red[32];
     __shared__ int stop;
     int sy = Z + 3, sx = (Y + 3) * (Z + 3);
@@ -406,8 +407,8 @@ __device__ void coarse_gs(T *p, T *r, int X, int Y, int Z, const MgK &kk, const 
         thresh = tol * red[0];
         __syncthreads();
     }
-    int iterCount = 0;
-    long long sweeps = 0;
+    int iterCount = done;
+    long long sweeps = done;
     int smax = X + Y + Z;
     while (true) {
         smem_impose_bc(p, X, Y, Z, bc, (const T *)nullptr, (const T *)nullptr, (const T *)nullptr);
@@ -588,6 +589,196 @@ __global__ void k_mg_gs_block(View3<double> pg, View3<const double> rg, MgK kk, 
     }
     smem_impose_bc(p, X, Y, Z, bc, wx, wy, wz);
     for (int t = threadIdx.x; t < n; t += blockDim.x) pg.p[t] = p[t];
+}
+
+// ---- several lexicographic sweeps in flight in one CTA
+// A hyperplane wavefront runs one sweep at a time: X + Y + Z + 1 dependent stages
+// a sweep, each a handful of points.  Here sweep m + 1 starts lam stages behind
+// sweep m, so a new sweep finishes every lam steps.  At step t sweep m updates
+// the points with i + j + k = t - lam m.  Its operands are the sequential
+// loop's, in place, for
+//   lower neighbours: sweep m, written one step before;
+//   upper neighbours: sweep m - 1, complete when lam >= 2, rewritten one step after;
+//   low ghosts (imposeBC before sweep m): the image plane of sweep m - 1 -- plane 1
+//     (mirror: complete when lam >= 2) or plane E - 1 (periodic: when lam >= E),
+//     not yet rewritten by sweep m;
+//   high ghosts: the image plane (E - 1 or 1) of sweep m - 1, which sweep m has
+//     rewritten by then: whoever rewrites it keeps its old value first (gx, gy,
+//     and a register along k).
+// A thread owns a (j, k)-free column (i, j) and the sweeps m = q mod Q, walking k
+// one point a step, so its addresses only step by one; Q lam >= Z + 1 keeps its
+// sweeps apart.  The arithmetic is mg_update's on the same operands: same bits.
+//
+// What bounds it: GB300 issues one FP64 instruction of a warp in 64 clocks on each
+// SM quarter whatever its live lanes (76 with all four busy; dependent or not),
+// so a step costs 64 clocks per FP64 operation of an update: they are what the
+// Arith forms below save (exact folding of powers of two: 9 operations on
+// equal power-of-two spacings and metrics, 12 otherwise, 16 as the expression is written).
+//
+// COARSE: the coarsest solve (poisson_d3.cc:190-247) -- sweeps from 0 until
+// max |r - Lp| < tol or maxCount + 1 of them.  Sweeps beyond the one that stops
+// would be in flight, so the stop is not tested on every point: one extra warp
+// evaluates the exact residual of sweep n at up to 32 interior points of one
+// hyperplane as their values pass by (lower neighbours two steps before sweep
+// n + 1 rewrites the point, the point one step before, upper neighbours with
+// it).  One of them at or above tol proves that the sweep does not stop; the
+// first sweep with none (its maximum may still lie elsewhere) is rerun up to the
+// sweep before and continued by coarse_gs, which tests every point.
+template <int ARITH>   // 0: equal spacings, power-of-two constants; 1: power-of-two constants; 2: any uniform mesh
+struct GsArith {
+    double cx2, cy2, cz2, c7, den, iden;   // 0: c7, den, iden over cx2
+    __device__ __forceinline__ double operator()(double E, double W, double N, double S, double U, double D, double r, bool planar) const {
+        const double ew = E + W, ud = U + D;
+        double t;
+        if (ARITH == 0) {
+            t = planar ? ew + ud : (ew + (N + S)) + ud;
+        } else if (ARITH == 1) {
+            t = cx2 * ew;
+            if (!planar) t = fma(cy2, N + S, t);
+            t = fma(cz2, ud, t);
+        } else {
+            t = cx2 * ew;
+            if (!planar) t = t + cy2 * (N + S);
+            t = t + cz2 * ud;
+        }
+        return div_rn(fma(-c7, r, t), den, iden);   // c7 is a power of two: c7 r is exact
+    }
+};
+
+struct GsPlan {
+    int lam, Q, threads;    // stages between sweeps, sweeps of a column apart, compute threads (a multiple of 32)
+    int rsmem;              // the right-hand side in shared memory too
+    size_t smem;
+};
+
+// `M` pipelined sweeps on P (core points, k fastest); `alarm` (COARSE): set to the
+// first sweep none of whose witness points is at or above tol.
+template <class A, bool PLANAR, bool RS, bool CHECK>
+__device__ __forceinline__ void gs_pipe_run(double *P, const double *R, long rsx, long rsy, double *gx, double *gy, int X, int Y, int Z,
+                                            const MgBC &bc, const A &ar, const MgK &kk, int lam, int Q, int M, double tol, int *alarm) {
+    const int W1 = Y + 1, Zn = Z + 1, nc = (X + 1) * W1;
+    const bool witness = CHECK && (int)threadIdx.x >= (int)blockDim.x - 32;
+    const int q = threadIdx.x / nc, col = threadIdx.x - q * nc, i = col / W1, j = col - i * W1;
+    const bool on = q < Q && !witness;
+    const int xs = bc.per[0] ? 1 : X - 1, ys = bc.per[1] ? 1 : Y - 1, zs = bc.per[2] ? 1 : Z - 1;   // planes the high ghosts image
+    const int il = i > 0 ? i - 1 : (bc.per[0] ? X - 1 : 1), jl = j > 0 ? j - 1 : (bc.per[1] ? Y - 1 : 1);
+    double *pc = P + col * Zn;
+    const double *pw = P + (il * W1 + j) * Zn, *pe = i < X ? P + (col + W1) * Zn : gx + j * Zn;
+    const double *ps = PLANAR ? P : P + (i * W1 + jl) * Zn, *pn = PLANAR ? P : j < Y ? P + (col + 1) * Zn : gy + i * Zn;
+    double *sx = on && i == xs ? gx + j * Zn : nullptr, *sy = on && !PLANAR && j == ys ? gy + i * Zn : nullptr;
+    const double *pr = RS ? R + col * Zn : R + i * rsx + j * rsy;
+    const int zl = bc.per[2] ? Z - 1 : 1, period = max(lam * Q, Zn);   // Q = M with lam Q < Z + 1: no second sweep
+    int k = -(i + j + lam * q), m = q;
+    double prev = 0.0, gz = 0.0, rv = on && q < M ? pr[0] : 0.0;
+    // witness points: interior, on the hyperplane sw
+    const int lane = threadIdx.x & 31, sw = (X + Y + Z) / 2;
+    int wo = -1;
+    double wr = 0.0, c2 = 0.0, wc = 0.0, lo0 = 0.0, lo1 = 0.0, lo2 = 0.0, acc = 0.0, zsum = 0.0;
+    int wi = 0, wj = 0, wk = 0, checked = 0, found = -1, tUp = sw + lam;   // step at which check `checked` reads its upper neighbours
+    if (witness) {
+        int seen = 0;
+        for (int a = 1; a < X && wo < 0; ++a)
+            for (int b = PLANAR ? 0 : 1; b < (PLANAR ? 1 : Y) && wo < 0; ++b) {
+                const int c = sw - a - b;
+                if (c < 1 || c >= Z) continue;
+                if (seen++ == lane) { wi = a; wj = b; wk = c; wo = (a * W1 + b) * Zn + c; }
+            }
+        if (wo >= 0) wr = RS ? R[wo] : R[wi * rsx + wj * rsy + wk];
+    }
+    const int steps = (M - 1) * lam + X + Y + Z + 1;
+    for (int t = 0; t < steps; ++t) {
+        if (on && k >= 0 && k <= Z && m < M) {
+            const double cold = pc[k];
+            const double U = k < Z ? pc[k + 1] : gz, D = k > 0 ? prev : pc[zl];
+            const double E = pe[k], W = pw[k], N = PLANAR ? 0.0 : pn[k], S = PLANAR ? 0.0 : ps[k];
+            const double v = ar(E, W, N, S, U, D, rv, PLANAR);
+            rv = pr[k < Z ? k + 1 : 0];   // the next step's
+            if (sx) sx[k] = cold;
+            if (sy) sy[k] = cold;
+            if (k == zs) gz = cold;
+            pc[k] = v;
+            prev = v;
+        }
+        if (++k == period) { k = 0; m += Q; }
+        if (CHECK && witness && checked < M - 1) {
+            if (t == tUp + 1) {   // the second half of check `checked`, and its vote
+                const double lap = acc + kk.lz * zsum;
+                const double v = fabs(wr - lap);
+                const bool alive = wo >= 0 && !(v < tol);
+                if (!__any_sync(0xffffffffu, alive) && found < 0) found = checked;
+                checked += 1;
+                tUp += lam;
+            }
+            if (wo >= 0) {
+                if (t == tUp) {
+                    c2 = 2.0 * wc;
+                    const double a = kk.lx * (P[wo + W1 * Zn] - c2 + lo0);
+                    acc = PLANAR ? a : a + kk.ly * (P[wo + Zn] - c2 + lo1);
+                    zsum = P[wo + 1] - c2 + lo2;
+                }
+                // lam = 2: the next check's lower neighbours are read with this check's upper ones
+                const int tLo = t >= tUp ? tUp + lam : tUp;
+                if (t == tLo - 2) { lo0 = P[wo - W1 * Zn]; lo1 = PLANAR ? 0.0 : P[wo - Zn]; lo2 = P[wo - 1]; }
+                if (t == tLo - 1) wc = P[wo];
+            }
+        }
+        if (CHECK && witness && lane == 0 && (t & 15) == 7 && found >= 0) *alarm = found;
+        __syncthreads();
+        if (CHECK && (t & 15) == 15 && *(volatile int *)alarm >= 0) break;   // written at t = 7 mod 16 only: every thread reads the same
+    }
+    if (CHECK && witness && lane == 0 && found >= 0) *alarm = found;
+    __syncthreads();
+}
+
+template <int ARITH, bool PLANAR, bool RS, bool COARSE>
+__global__ void __launch_bounds__(1024) k_gs_pipe(View3<double> pg, View3<const double> rg, MgK kk, MgBC bc, GsArith<ARITH> ar, int lam,
+                                                  int Q, int count, int zero, double tol, int maxCount, long long *iters) {
+    extern __shared__ unsigned char smraw[];
+    __shared__ int alarm;
+    const int X = bc.E[0], Y = bc.E[1], Z = bc.E[2], W1 = Y + 1, Zn = Z + 1, n = (X + 1) * W1 * Zn;
+    double *P = reinterpret_cast<double *>(smraw), *gx = P + n, *gy = gx + W1 * Zn, *R = gy + (PLANAR ? 0 : (X + 1) * Zn);
+    const long o0 = rg.off(0, 0, 0);
+    for (int t = threadIdx.x; t < n; t += blockDim.x) {
+        const int k = t % Zn, c = t / Zn, j = c % W1, i = c / W1;
+        P[t] = zero ? 0.0 : pg(i, j, k);
+        if (RS) R[t] = rg(i, j, k);
+    }
+    if (threadIdx.x == 0) alarm = -1;
+    __syncthreads();
+    const double *r = RS ? R : rg.p + o0;
+    gs_pipe_run<GsArith<ARITH>, PLANAR, RS, COARSE>(P, r, rg.sx, rg.sy, gx, gy, X, Y, Z, bc, ar, kk, lam, Q, count, tol, &alarm);
+    if (COARSE) {
+        const int stop = alarm;
+        if (stop >= 0) {
+            // the sweeps before the one in question, then one at a time with every point tested
+            for (int t = threadIdx.x; t < n; t += blockDim.x) P[t] = 0.0;
+            __syncthreads();
+            if (stop > 0)
+                gs_pipe_run<GsArith<ARITH>, PLANAR, RS, false>(P, r, rg.sx, rg.sy, gx, gy, X, Y, Z, bc, ar, kk, lam, Q, stop, tol, nullptr);
+            const int N = (X + 3) * (Y + 3) * (Z + 3), sy = Z + 3, sx = (Y + 3) * sy;
+            double *pp = R + (RS ? n : 0), *rr = pp + N;
+            for (int t = threadIdx.x; t < N; t += blockDim.x) { pp[t] = 0.0; rr[t] = rg.p[t]; }
+            __syncthreads();
+            for (int t = threadIdx.x; t < n; t += blockDim.x) {
+                const int k = t % Zn, c = t / Zn, j = c % W1, i = c / W1;
+                pp[(i + 1) * sx + (j + 1) * sy + k + 1] = P[t];
+            }
+            __syncthreads();
+            coarse_gs<double>(pp, rr, X, Y, Z, kk, bc, tol, maxCount, 0, iters, stop);
+            for (int t = threadIdx.x; t < N; t += blockDim.x) pg.p[t] = pp[t];
+            return;
+        }
+        if (threadIdx.x == 0 && iters) *iters += count;
+    }
+    // the core and the ghosts imposeBC leaves (2D: the y = 0 plane)
+    const int jn = PLANAR ? 1 : Y + 3, N = (X + 3) * jn * (Z + 3);
+    for (int t = threadIdx.x; t < N; t += blockDim.x) {
+        const int k = t % (Z + 3) - 1, c = t / (Z + 3), j = PLANAR ? 0 : c % jn - 1, i = c / jn - 1;
+        const int a = i < 0 ? (bc.per[0] ? X - 1 : 1) : i > X ? (bc.per[0] ? 1 : X - 1) : i;
+        const int b = j < 0 ? (bc.per[1] ? Y - 1 : 1) : j > Y ? (bc.per[1] ? 1 : Y - 1) : j;
+        const int d = k < 0 ? (bc.per[2] ? Z - 1 : 1) : k > Z ? (bc.per[2] ? 1 : Z - 1) : k;
+        pg(i, j, k) = P[(a * W1 + b) * Zn + d];
+    }
 }
 
 // Value that imposeBC (x planes, y planes, then z planes over full extents,
@@ -2350,11 +2541,117 @@ static double smooth_weight(const Ctx &c, int n, int count) {
     return 1.0 / lam;
 }
 
+// ---- the pipelined Gauss-Seidel kernel's launches
+static bool is_pow2(double x) {
+    int e;
+    return std::isfinite(x) && std::frexp(x, &e) == 0.5;
+}
+
+// Constants of a level's update in the folded forms of GsArith: 0, 1 or 2, or -1
+// (a stretched mesh, or a level whose c7 is no power of two).
+static int gs_arith(const Ctx &c, const Level &L, GsArith<2> &a) {
+    if (c.stretched) return -1;
+    double cx, cy = 0.0, cz, c7, den;
+    if (c.planar) {   // poisson_d2.cc:126-131 on a uniform mesh
+        cx = L.hz2 * c.m2[0];
+        cz = L.hx2 * c.m2[2];
+        c7 = 2.0 * L.hzhx;
+        den = 4.0 * (L.hz2 * c.m2[0] + L.hx2 * c.m2[2]);
+    } else {
+        cx = L.cx; cy = L.cy; cz = L.cz; c7 = L.c7; den = L.den;
+    }
+    if (!is_pow2(c7)) return -1;
+    a.cx2 = 2.0 * cx; a.cy2 = 2.0 * cy; a.cz2 = 2.0 * cz;
+    a.c7 = c7; a.den = den;
+    int form = is_pow2(cx) && is_pow2(cz) && (c.planar || is_pow2(cy)) ? 1 : 2;
+    if (form == 1 && cx == cz && (c.planar || cx == cy)) {
+        form = 0;
+        a.c7 = c7 / a.cx2;
+        a.den = den / a.cx2;
+    }
+    a.iden = 1.0 / a.den;
+    return form;
+}
+
+// The launch of `count` pipelined sweeps on level L (coarse: with the witness warp
+// and room for coarse_gs's padded arrays), or false where the block does not hold
+// them.  lam from its smallest value (2, or the interval count of a periodic
+// axis) up to Z + 1, by the estimated clocks a sweep (many sweeps) or in all
+// (a smoothing phase): a step costs about 76 clocks an FP64 operation and warp
+// on an SM quarter, and 90 around them.
+static bool gs_plan(const Ctx &c, const Level &L, const MgBC &bc, int form, int count, bool coarse, GsPlan &g) {
+    if (bc.dirichlet || form < 0) return false;
+    const int X = L.n[0], Y = c.planar ? 0 : L.n[1], Z = L.n[2];
+    const long nc = (long)(X + 1) * (Y + 1), n = nc * (Z + 1);
+    const size_t cap = 220 * 1024;
+    size_t smem = 8 * (size_t)(n + (long)(Y + 1) * (Z + 1) + (c.planar ? 0 : (long)(X + 1) * (Z + 1)));
+    if (coarse) smem += 8 * (size_t)(n + 2 * L.count);
+    if (smem > cap || nc > 992) return false;
+    g.rsmem = coarse || smem + 8 * (size_t)n <= cap;
+    g.smem = smem + (!coarse && g.rsmem ? 8 * (size_t)n : 0);
+    int lmin = 2;
+    for (int d = 0; d < 3; ++d)
+        if (bc.per[d]) lmin = std::max(lmin, L.n[d]);
+    const double ops = (form == 0 ? 9.0 : form == 1 ? 10.0 : 12.0) - (c.planar ? 2.0 : 0.0);
+    double best = 0.0;
+    g.Q = 0;
+    for (int lam = lmin; lam <= std::max(lmin, Z + 1); ++lam) {
+        const int Q = std::min((Z + 1 + lam - 1) / lam, count);
+        const long th = (nc * Q + 31) / 32 * 32;
+        if (th + (coarse ? 32 : 0) > 1024) continue;
+        const long q4 = (th / 32 + (coarse ? 1 : 0) + 3) / 4;
+        const double step = 90.0 + ops * (q4 > 1 ? 76.0 * q4 : 64.0);
+        const double cost = step * ((count - 1.0) * lam + X + Y + Z + 1);
+        if (g.Q == 0 || cost < best) { best = cost; g.lam = lam; g.Q = Q; g.threads = (int)th; }
+    }
+    return g.Q > 0;
+}
+
+template <int ARITH, bool COARSE>
+static cudaError_t gs_pipe_launch(Ctx &c, Level &L, const MgBC &bc, const GsArith<2> &a, const GsPlan &g, int count, bool zero) {
+    GsArith<ARITH> ar;
+    ar.cx2 = a.cx2; ar.cy2 = a.cy2; ar.cz2 = a.cz2; ar.c7 = a.c7; ar.den = a.den; ar.iden = a.iden;
+    void (*k)(View3<double>, View3<const double>, MgK, MgBC, GsArith<ARITH>, int, int, int, int, double, int, long long *);
+    if (COARSE || g.rsmem) k = c.planar ? k_gs_pipe<ARITH, true, true, COARSE> : k_gs_pipe<ARITH, false, true, COARSE>;
+    else k = c.planar ? k_gs_pipe<ARITH, true, false, false> : k_gs_pipe<ARITH, false, false, false>;
+    cudaError_t e = cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem);
+    if (e != cudaSuccess) return e;
+    k<<<1, g.threads + (COARSE ? 32 : 0), g.smem, c.stream>>>(lview<double>(L, L.pa()), lcview<double>(L, L.r), make_k(L), bc, ar, g.lam, g.Q,
+                                                              count, zero ? 1 : 0, c.p.mgTolerance, c.maxCount,
+                                                              (long long *)(c.dscal + 40));
+    return cudaGetLastError();
+}
+
+// `count` lexicographic sweeps of level l (coarse: the coarsest solve) in one
+// pipelined CTA; false in *ran where the kernel does not take the level.
+static int gs_pipe(Ctx &c, int l, int count, bool zero, bool coarse, bool *ran) {
+    Level &L = c.lv[l];
+    const MgBC bc = level_bc(c, l, false);
+    GsArith<2> a;
+    GsPlan g;
+    const int form = gs_arith(c, L, a);
+    *ran = count > 0 && gs_plan(c, L, bc, form, count, coarse, g);
+    if (!*ran) return SARAS_OK;
+    cudaError_t e;
+    if (coarse)
+        e = form == 0 ? gs_pipe_launch<0, true>(c, L, bc, a, g, count, zero)
+          : form == 1 ? gs_pipe_launch<1, true>(c, L, bc, a, g, count, zero) : gs_pipe_launch<2, true>(c, L, bc, a, g, count, zero);
+    else
+        e = form == 0 ? gs_pipe_launch<0, false>(c, L, bc, a, g, count, zero)
+          : form == 1 ? gs_pipe_launch<1, false>(c, L, bc, a, g, count, zero) : gs_pipe_launch<2, false>(c, L, bc, a, g, count, zero);
+    SARAS_CUDA_TRY(e);
+    count_launch(c);
+    return SARAS_OK;
+}
+
 // Gauss-Seidel smoothing of level l (reference mode with gsSmooth = 1): one
 // CTA from shared memory for levels up to kGsBlockSmem of iterate plus
 // right-hand side, else the cooperative grid kernel with one block an SM at
 // most (a stage has at most (X+1)(Y+1) points).
 static int gs_smooth(Ctx &c, int l, int count, bool zero_first) {
+    bool ran = false;
+    if (int s = gs_pipe(c, l, count, zero_first, false, &ran)) return s;
+    if (ran) return chk(c, "mg Gauss-Seidel");
     Level &L = c.lv[l];
     MgBC bc = level_bc(c, l, false);
     MgK kk = make_k(L);
@@ -2454,6 +2751,13 @@ static int coarse_solve(Ctx &c, bool tgt) {
     // V-cycle's own error reduction (about 0.1), so 1e-3 of the initial residual
     T tol = tgt ? (T)1.0e-3 : (T)c.p.mgTolerance;
     int maxc = tgt ? 500 : c.maxCount;
+    if constexpr (sizeof(T) == 8) {
+        if (!tgt) {   // sweeps from 0: at most maxCount + 1
+            bool ran = false;
+            if (int s = gs_pipe(c, c.depth, maxc + 1, true, true, &ran)) return s;
+            if (ran) return chk(c, "mg coarse");
+        }
+    }
     k_mg_coarse<T><<<1, kCoarseThreads, smem, c.stream>>>(lview<T>(L, A_<T>(L)), lcview<T>(L, R_<T>(L)), kk, bc, tol, maxc, tgt ? 1 : 0,
                                                (long long *)(c.dscal + 40));
     count_launch(c);
