@@ -158,19 +158,19 @@ struct Ctx {
     int coarseN = 0;          // coarsest core points solved by coarseM (0: Gauss-Seidel instead)
     double *coarseM64 = nullptr;   // coarsest-level solution operator (coarseN x coarseN, row-major)
     float *coarseM32 = nullptr;
-    // target-mode V-cycles replayed as CUDA graphs: [FP32?][zero start?]
-    // [FP32?][zero start?][timed?]: with profiling on, the timed instance holds
+    // V-cycles replayed as CUDA graphs: [0 target FP64, 1 target FP32, 2 reference]
+    // [zero start + 2 x level 0's buffer][timed?]: with profiling on, the timed instance holds
     // the profiling event nodes and replays one cycle in profEvery
-    cudaGraphExec_t vgraph[2][2][2] = {};
-    cudaGraph_t vgraphSrc[2][2][2] = {};      // kept for the event-node handles
-    std::vector<ProfNode> vgraphProf[2][2][2];   // profiling event nodes of each graph, in capture order
+    cudaGraphExec_t vgraph[3][4][2] = {};
+    cudaGraph_t vgraphSrc[3][4][2] = {};      // kept for the event-node handles
+    std::vector<ProfNode> vgraphProf[3][4][2];   // profiling event nodes of each graph, in capture order
     bool profCapturing = false;               // prof_begin / prof_end record graph event nodes
     bool profSuppress = false;                // prof_begin / prof_end record nothing (untimed capture)
     int profEvery = 1;
     long long profReplays = 0;
     std::vector<ProfNode> profCaptured;
-    long long vgraphLaunches[2][2][2] = {};
-    std::vector<int> vgraphState[2][2][2];
+    long long vgraphLaunches[3][4][2] = {};
+    std::vector<int> vgraphState[3][4][2], vgraphAfter[3][4][2];   // level buffers before and after the cycle
     int histCount = 0;
     bool ppInHist = false;    // Pp's buffer moved to pHist[0] by unet_begin_solve; the solve has not written Pp yet
     bool collecting = false;

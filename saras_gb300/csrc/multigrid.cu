@@ -41,6 +41,35 @@ namespace saras {
 
 __global__ void k_final_reduce(const double *part, int n, int op, double *out);
 
+// Programmatic dependent launch.  The level kernels of a V-cycle run back to
+// back, most of them microseconds long; launched with programmatic stream
+// serialisation (launch_pdl), a kernel may start before the previous one has
+// ended and waits in pdl_wait, before its first global access, until that grid has
+// completed and its writes are visible.  pdl_wait also lets the next kernel of the
+// stream start (once every block is past it): its blocks take the slots that the
+// last wave leaves and wait there, so the launch itself is off the critical path.
+// Launched the ordinary way, both instructions return at once.
+__device__ __forceinline__ void pdl_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <typename... P, typename... A>
+static cudaError_t launch_pdl(void (*k)(P...), dim3 g, dim3 b, size_t smem, cudaStream_t st, A &&...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = g;
+    cfg.blockDim = b;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
+}
+
+
 // max |a| over a whole array into *out (non-negative, atomic).
 __global__ void k_maxabs(const double *a, long n, double *out) {
     double m = 0;
@@ -207,6 +236,7 @@ __device__ __forceinline__ void put_scatter(const View3<T> &P, int i, int j, int
 // poisson.cc:258).  omega = 1 reproduces the reference exactly.
 template <typename T, bool ZERO>
 __global__ void k_mg_sweep(View3<T> out, View3<const T> in, View3<const T> r, MgK kk, MgBC bc, T omega) {
+    pdl_wait();
     int i, j, k;
     if (!core_pt(bc.E, i, j, k)) return;
     T v;
@@ -225,6 +255,7 @@ __global__ void k_mg_sweep(View3<T> out, View3<const T> in, View3<const T> r, Mg
 // computeResidual (poisson_d3.cc:90-111): tmp(core) = r - Lap(p).
 template <typename T>
 __global__ void k_mg_residual(View3<T> tmp, View3<const T> p, View3<const T> r, MgK kk, MgBC bc) {
+    pdl_wait();
     int i, j, k;
     if (!core_pt(bc.E, i, j, k)) return;
     T lap = mg_lap<T>(p(i + 1, j, k), p(i - 1, j, k), p(i, j + 1, k), p(i, j - 1, k), p(i, j, k + 1), p(i, j, k - 1), p(i, j, k), kk, i, j, k);
@@ -257,6 +288,7 @@ __device__ __forceinline__ T pad_val(const View3<const T> &t, int i, int j, int 
 // summation order.  bcf describes the fine level, Ec the coarse core.
 template <typename T>
 __global__ void k_mg_restrict(View3<T> rc, View3<const T> t, MgBC bcf, MgBC bcc) {
+    pdl_wait();
     int i, j, k;
     if (!core_pt(bcc.E, i, j, k)) return;
     int i2 = 2 * i, j2 = 2 * j, k2 = 2 * k;
@@ -285,6 +317,7 @@ __global__ void k_mg_restrict(View3<T> rc, View3<const T> t, MgBC bcf, MgBC bcc)
 // (poisson.cc:271); the saved data is the fine array itself, updated in place.
 template <typename T>
 __global__ void k_mg_prolong_add(View3<T> pf, View3<const T> pc, MgBC bc, int add) {
+    pdl_wait();
     int i, j, k;
     if (!core_pt(bc.E, i, j, k)) return;
     int i2 = i / 2, j2 = j / 2, k2 = k / 2;
@@ -538,6 +571,7 @@ __device__ void coarse_rbgs_warp(T *p, T *r, int X, int Y, int Z, const MgK &kk,
 template <typename T>
 __global__ void k_mg_coarse(View3<T> pg, View3<const T> rg, MgK kk, MgBC bc, T tol, int maxCount, int tgtMode,
                             long long *iters) {
+    pdl_wait();
     extern __shared__ unsigned char smraw[];
     int X = bc.E[0], Y = bc.E[1], Z = bc.E[2];
     int n = (X + 3) * (Y + 3) * (Z + 3);
@@ -567,6 +601,7 @@ __global__ void k_mg_coarse(View3<T> pg, View3<const T> rg, MgK kk, MgBC bc, T t
 constexpr size_t kGsBlockSmem = 200 * 1024;
 __global__ void k_mg_gs_block(View3<double> pg, View3<const double> rg, MgK kk, MgBC bc, int count, int zero,
                               const double *wx, const double *wy, const double *wz) {
+    pdl_wait();
     extern __shared__ unsigned char smraw[];
     const int X = bc.E[0], Y = bc.E[1], Z = bc.E[2];
     const int n = (X + 3) * (Y + 3) * (Z + 3), sy = Z + 3, sx = (Y + 3) * (Z + 3);
@@ -614,6 +649,10 @@ __global__ void k_mg_gs_block(View3<double> pg, View3<const double> rg, MgK kk, 
 // so a step costs 64 clocks per FP64 operation of an update: they are what the
 // Arith forms below save (exact folding of powers of two: 9 operations on
 // equal power-of-two spacings and metrics, 12 otherwise, 16 as the expression is written).
+// Measured, one sweep at a time -> pipelined: 217 sweeps of a 5^3 level 2.65 ms ->
+// 0.20 (mirror, lam 2) and 0.46 (periodic, general metrics, lam 4); 1001 of a 9^3
+// periodic level 24.9 -> 3.66 ms; four sweeps of a 17^3 level 0.27 -> 0.11 ms and of
+// a 65 x 65 2D level 1.66 -> 0.15 ms.
 //
 // COARSE: the coarsest solve (poisson_d3.cc:190-247) -- sweeps from 0 until
 // max |r - Lp| < tol or maxCount + 1 of them.  Sweeps beyond the one that stops
@@ -651,95 +690,157 @@ struct GsPlan {
     size_t smem;
 };
 
-// `M` pipelined sweeps on P (core points, k fastest); `alarm` (COARSE): set to the
-// first sweep none of whose witness points is at or above tol.
+// Doubles from one column to the next: Z + 1 is odd, and one more makes the
+// distance between the points that neighbouring columns update in one step (a
+// column less one point) odd, so a warp's accesses fall in different banks (a
+// 9^3 level's 1001 sweeps: 4.89 ms, packed columns 5.08).
+__host__ __device__ inline int gs_pitch(int Z) { return Z + 2; }
+
+// The CTA's step barrier, from the compute and the witness loops alike.
+__device__ __forceinline__ void gs_step_sync() { asm volatile("barrier.sync 0;" ::: "memory"); }
+
+// `M` pipelined sweeps on P (core points, columns gs_pitch apart); `alarm` (CHECK):
+// set to the first sweep none of whose witness points is at or above tol.  The
+// compute warps and the witness warp run loops of the same steps; *alarm is
+// written in step 7 of 16 and read after step 15, so that all leave together.
 template <class A, bool PLANAR, bool RS, bool CHECK>
 __device__ __forceinline__ void gs_pipe_run(double *P, const double *R, long rsx, long rsy, double *gx, double *gy, int X, int Y, int Z,
                                             const MgBC &bc, const A &ar, const MgK &kk, int lam, int Q, int M, double tol, int *alarm) {
-    const int W1 = Y + 1, Zn = Z + 1, nc = (X + 1) * W1;
-    const bool witness = CHECK && (int)threadIdx.x >= (int)blockDim.x - 32;
-    const int q = threadIdx.x / nc, col = threadIdx.x - q * nc, i = col / W1, j = col - i * W1;
-    const bool on = q < Q && !witness;
-    const int xs = bc.per[0] ? 1 : X - 1, ys = bc.per[1] ? 1 : Y - 1, zs = bc.per[2] ? 1 : Z - 1;   // planes the high ghosts image
-    const int il = i > 0 ? i - 1 : (bc.per[0] ? X - 1 : 1), jl = j > 0 ? j - 1 : (bc.per[1] ? Y - 1 : 1);
-    double *pc = P + col * Zn;
-    const double *pw = P + (il * W1 + j) * Zn, *pe = i < X ? P + (col + W1) * Zn : gx + j * Zn;
-    const double *ps = PLANAR ? P : P + (i * W1 + jl) * Zn, *pn = PLANAR ? P : j < Y ? P + (col + 1) * Zn : gy + i * Zn;
-    double *sx = on && i == xs ? gx + j * Zn : nullptr, *sy = on && !PLANAR && j == ys ? gy + i * Zn : nullptr;
-    const double *pr = RS ? R + col * Zn : R + i * rsx + j * rsy;
-    const int zl = bc.per[2] ? Z - 1 : 1, period = max(lam * Q, Zn);   // Q = M with lam Q < Z + 1: no second sweep
-    int k = -(i + j + lam * q), m = q;
-    double prev = 0.0, gz = 0.0, rv = on && q < M ? pr[0] : 0.0;
-    // witness points: interior, on the hyperplane sw
-    const int lane = threadIdx.x & 31, sw = (X + Y + Z) / 2;
-    int wo = -1;
-    double wr = 0.0, c2 = 0.0, wc = 0.0, lo0 = 0.0, lo1 = 0.0, lo2 = 0.0, acc = 0.0, zsum = 0.0;
-    int wi = 0, wj = 0, wk = 0, checked = 0, found = -1, tUp = sw + lam;   // step at which check `checked` reads its upper neighbours
-    if (witness) {
-        int seen = 0;
+    const int W1 = Y + 1, zp = gs_pitch(Z), nc = (X + 1) * W1;
+    const int steps = (M - 1) * lam + X + Y + Z + 1;
+    if (CHECK && threadIdx.x >= blockDim.x - 32) {
+        // the witness points: interior, on the hyperplane sw
+        const int lane = threadIdx.x & 31, sw = (X + Y + Z) / 2;
+        int wo = -1, seen = 0;
+        double wr = 0.0;
         for (int a = 1; a < X && wo < 0; ++a)
             for (int b = PLANAR ? 0 : 1; b < (PLANAR ? 1 : Y) && wo < 0; ++b) {
                 const int c = sw - a - b;
                 if (c < 1 || c >= Z) continue;
-                if (seen++ == lane) { wi = a; wj = b; wk = c; wo = (a * W1 + b) * Zn + c; }
+                if (seen++ == lane) {
+                    wo = (a * W1 + b) * zp + c;
+                    wr = RS ? R[wo] : R[a * rsx + b * rsy + c];
+                }
             }
-        if (wo >= 0) wr = RS ? R[wo] : R[wi * rsx + wj * rsy + wk];
-    }
-    const int steps = (M - 1) * lam + X + Y + Z + 1;
-    for (int t = 0; t < steps; ++t) {
-        if (on && k >= 0 && k <= Z && m < M) {
-            const double cold = pc[k];
-            const double U = k < Z ? pc[k + 1] : gz, D = k > 0 ? prev : pc[zl];
-            const double E = pe[k], W = pw[k], N = PLANAR ? 0.0 : pn[k], S = PLANAR ? 0.0 : ps[k];
-            const double v = ar(E, W, N, S, U, D, rv, PLANAR);
-            rv = pr[k < Z ? k + 1 : 0];   // the next step's
-            if (sx) sx[k] = cold;
-            if (sy) sy[k] = cold;
-            if (k == zs) gz = cold;
-            pc[k] = v;
-            prev = v;
-        }
-        if (++k == period) { k = 0; m += Q; }
-        if (CHECK && witness && checked < M - 1) {
-            if (t == tUp + 1) {   // the second half of check `checked`, and its vote
-                const double lap = acc + kk.lz * zsum;
-                const double v = fabs(wr - lap);
-                const bool alive = wo >= 0 && !(v < tol);
-                if (!__any_sync(0xffffffffu, alive) && found < 0) found = checked;
-                checked += 1;
-                tUp += lam;
-            }
-            if (wo >= 0) {
-                if (t == tUp) {
-                    c2 = 2.0 * wc;
-                    const double a = kk.lx * (P[wo + W1 * Zn] - c2 + lo0);
-                    acc = PLANAR ? a : a + kk.ly * (P[wo + Zn] - c2 + lo1);
-                    zsum = P[wo + 1] - c2 + lo2;
+        const bool has = wo >= 0;
+        const double *w = P + (has ? wo : 0);
+        double wc = 0.0, lo0 = 0.0, lo1 = 0.0, lo2 = 0.0, xterm = 0.0, ysum = 0.0, zsum = 0.0, zlo = 0.0;
+        int checked = 0, found = -1, tUp = sw + lam;   // step in which check `checked` reads its upper neighbours
+        for (int t = 0; t < steps; ++t) {
+            if (checked < M - 1) {
+                if (t == tUp + 1) {   // the second half of check `checked`, and its vote
+                    const double xy = PLANAR ? xterm : xterm + kk.ly * ysum;
+                    const double v = fabs(wr - (xy + kk.lz * (zsum + zlo)));
+                    if (!__any_sync(0xffffffffu, has && !(v < tol)) && found < 0) found = checked;
+                    checked += 1;
+                    tUp += lam;
+                }
+                if (t == tUp && has) {
+                    const double c2 = 2.0 * wc;
+                    xterm = kk.lx * (w[W1 * zp] - c2 + lo0);
+                    if (!PLANAR) ysum = w[zp] - c2 + lo1;
+                    zsum = w[1] - c2;
+                    zlo = lo2;
                 }
                 // lam = 2: the next check's lower neighbours are read with this check's upper ones
                 const int tLo = t >= tUp ? tUp + lam : tUp;
-                if (t == tLo - 2) { lo0 = P[wo - W1 * Zn]; lo1 = PLANAR ? 0.0 : P[wo - Zn]; lo2 = P[wo - 1]; }
-                if (t == tLo - 1) wc = P[wo];
+                if (t == tLo - 2 && has) { lo0 = w[-W1 * zp]; lo1 = PLANAR ? 0.0 : w[-zp]; lo2 = w[-1]; }
+                if (t == tLo - 1 && has) wc = w[0];
+            }
+            if ((t & 15) == 7 && lane == 0 && found >= 0) *alarm = found;
+            gs_step_sync();
+            if ((t & 15) == 15 && *(volatile int *)alarm >= 0) break;
+        }
+        if (lane == 0 && found >= 0) *alarm = found;
+        gs_step_sync();
+        return;
+    }
+    const int q = threadIdx.x / nc, col = threadIdx.x - q * nc, i = col / W1, j = col - i * W1;
+    const bool on = q < Q;
+    const int xs = bc.per[0] ? 1 : X - 1, ys = bc.per[1] ? 1 : Y - 1, zs = bc.per[2] ? 1 : Z - 1;   // planes the high ghosts image
+    const int il = i > 0 ? i - 1 : (bc.per[0] ? X - 1 : 1), jl = j > 0 ? j - 1 : (bc.per[1] ? Y - 1 : 1);
+    double *pc = P + col * zp;
+    const double *pw = P + (il * W1 + j) * zp, *pe = i < X ? P + (col + W1) * zp : gx + j * zp;
+    const double *ps = PLANAR ? P : P + (i * W1 + jl) * zp, *pn = PLANAR ? P : j < Y ? P + (col + 1) * zp : gy + i * zp;
+    double *sx = gx + j * zp, *sy = gy + i * zp;
+    const bool keepx = on && i == xs, keepy = on && !PLANAR && j == ys;
+    const double *pr = RS ? R + col * zp : R + i * rsx + j * rsy;
+    const int zl = bc.per[2] ? Z - 1 : 1, period = max(lam * Q, Z + 1);   // Q = M with lam Q < Z + 1: no second sweep
+    int k = on ? -(i + j + lam * q) : 0, m = q;
+    double prev = 0.0, gz = 0.0, rv = on && q < M ? pr[0] : 0.0;
+    auto any_step = [&]() {   // live lanes by their own k and m
+        const bool act = on && k >= 0 && k <= Z && m < M;
+        if (__any_sync(0xffffffffu, act)) {
+            const int kc = act ? k : 0;
+            const double cold = pc[kc], up = pc[kc < Z ? kc + 1 : Z], dn = pc[zl];
+            const double E = pe[kc], W = pw[kc], N = PLANAR ? 0.0 : pn[kc], S = PLANAR ? 0.0 : ps[kc];
+            const double U = kc < Z ? up : gz, D = kc > 0 ? prev : dn;
+            const double v = ar(E, W, N, S, U, D, rv, PLANAR);
+            const double rn = pr[kc < Z ? kc + 1 : 0];   // the next step's right-hand side
+            if (act && keepx) sx[kc] = cold;
+            if (act && keepy) sy[kc] = cold;
+            if (act) {
+                pc[kc] = v;
+                prev = v;
+                rv = rn;
+                gz = kc == zs ? cold : gz;
             }
         }
-        if (CHECK && witness && lane == 0 && (t & 15) == 7 && found >= 0) *alarm = found;
-        __syncthreads();
-        if (CHECK && (t & 15) == 15 && *(volatile int *)alarm >= 0) break;   // written at t = 7 mod 16 only: every thread reads the same
+        if (++k == period) { k = 0; m += Q; }
+    };
+    // Every sweep slot busy (the coarsest solve's hundreds of sweeps between the
+    // ramps): no tests of k and m (with them a 9^3 level's 1001 sweeps took 4.89 ms
+    // instead of 3.66, a 5^3 level's 217 took 248 us instead of 201).  A slot's idle steps (k = Z + 1) compute on and
+    // write the columns' spare double.
+    auto full_step = [&]() {
+        const int kn = k + 1 == period ? 0 : k + 1;
+        const double cold = pc[k], up = pc[k + 1], dn = pc[zl];
+        const double E = pe[k], W = pw[k], N = PLANAR ? 0.0 : pn[k], S = PLANAR ? 0.0 : ps[k];
+        const double U = k < Z ? up : gz, D = k > 0 ? prev : dn;
+        const double v = ar(E, W, N, S, U, D, rv, PLANAR);
+        rv = pr[k < Z ? k + 1 : 0];   // an idle step keeps the next sweep's first
+        if (keepx) sx[k] = cold;
+        if (keepy) sy[k] = cold;
+        if (on) pc[k] = v;
+        prev = v;
+        gz = k == zs ? cold : gz;
+        m += kn == 0 ? Q : 0;
+        k = kn;
+    };
+    // from fullLo (the last thread's first step) to fullHi (the first thread's
+    // last), in whole groups of 16 steps
+    const int fullLo = X + Y + lam * (Q - 1), fullHi = RS && period <= zp ? lam * (M - Q) + Z : 0;
+    for (int t0 = 0; t0 < steps; t0 += 16) {
+        const int n = min(16, steps - t0);
+        if (CHECK && t0 >= fullLo && t0 + 16 <= fullHi) {
+#pragma unroll 2
+            for (int e = 0; e < 16; ++e) {
+                full_step();
+                gs_step_sync();
+            }
+        } else {
+            for (int e = 0; e < n; ++e) {
+                any_step();
+                gs_step_sync();
+            }
+        }
+        if (CHECK && n == 16 && *(volatile int *)alarm >= 0) break;
     }
-    if (CHECK && witness && lane == 0 && found >= 0) *alarm = found;
-    __syncthreads();
+    gs_step_sync();
 }
 
 template <int ARITH, bool PLANAR, bool RS, bool COARSE>
 __global__ void __launch_bounds__(1024) k_gs_pipe(View3<double> pg, View3<const double> rg, MgK kk, MgBC bc, GsArith<ARITH> ar, int lam,
                                                   int Q, int count, int zero, double tol, int maxCount, long long *iters) {
+    pdl_wait();
     extern __shared__ unsigned char smraw[];
     __shared__ int alarm;
-    const int X = bc.E[0], Y = bc.E[1], Z = bc.E[2], W1 = Y + 1, Zn = Z + 1, n = (X + 1) * W1 * Zn;
-    double *P = reinterpret_cast<double *>(smraw), *gx = P + n, *gy = gx + W1 * Zn, *R = gy + (PLANAR ? 0 : (X + 1) * Zn);
+    const int X = bc.E[0], Y = bc.E[1], Z = bc.E[2], W1 = Y + 1, zp = gs_pitch(Z), n = (X + 1) * W1 * zp;
+    double *P = reinterpret_cast<double *>(smraw), *gx = P + n, *gy = gx + W1 * zp, *R = gy + (PLANAR ? 0 : (X + 1) * zp);
     const long o0 = rg.off(0, 0, 0);
     for (int t = threadIdx.x; t < n; t += blockDim.x) {
-        const int k = t % Zn, c = t / Zn, j = c % W1, i = c / W1;
+        const int k = t % zp, c = t / zp, j = c % W1, i = c / W1;
+        if (k > Z) continue;
         P[t] = zero ? 0.0 : pg(i, j, k);
         if (RS) R[t] = rg(i, j, k);
     }
@@ -760,8 +861,8 @@ __global__ void __launch_bounds__(1024) k_gs_pipe(View3<double> pg, View3<const 
             for (int t = threadIdx.x; t < N; t += blockDim.x) { pp[t] = 0.0; rr[t] = rg.p[t]; }
             __syncthreads();
             for (int t = threadIdx.x; t < n; t += blockDim.x) {
-                const int k = t % Zn, c = t / Zn, j = c % W1, i = c / W1;
-                pp[(i + 1) * sx + (j + 1) * sy + k + 1] = P[t];
+                const int k = t % zp, c = t / zp, j = c % W1, i = c / W1;
+                if (k <= Z) pp[(i + 1) * sx + (j + 1) * sy + k + 1] = P[t];
             }
             __syncthreads();
             coarse_gs<double>(pp, rr, X, Y, Z, kk, bc, tol, maxCount, 0, iters, stop);
@@ -777,7 +878,7 @@ __global__ void __launch_bounds__(1024) k_gs_pipe(View3<double> pg, View3<const 
         const int a = i < 0 ? (bc.per[0] ? X - 1 : 1) : i > X ? (bc.per[0] ? 1 : X - 1) : i;
         const int b = j < 0 ? (bc.per[1] ? Y - 1 : 1) : j > Y ? (bc.per[1] ? 1 : Y - 1) : j;
         const int d = k < 0 ? (bc.per[2] ? Z - 1 : 1) : k > Z ? (bc.per[2] ? 1 : Z - 1) : k;
-        pg(i, j, k) = P[(a * W1 + b) * Zn + d];
+        pg(i, j, k) = P[(a * W1 + b) * zp + d];
     }
 }
 
@@ -985,6 +1086,7 @@ __global__ void k_mg_error_sq(View3<const double> p, View3<const double> r, MgK 
 
 __global__ void k_mg_error(View3<const double> p, View3<const double> r, MgK kk, MgBC bc, int norm, double *maxv,
                            double *partNum, double *partDen) {
+    pdl_wait();
     __shared__ double s1[32], s2[32];
     int E0 = bc.E[0], E1 = bc.E[1], E2 = bc.E[2];
     long n = (long)(E0 + 1) * (E1 + 1) * (E2 + 1);
@@ -1055,30 +1157,6 @@ template <typename T>
 __device__ __noinline__ void scatter_slow(T *P, int sx, int sy, int i, int j, int k, T v, const MgBC &bc) {
     View3<T> V; V.p = P; V.sx = sx; V.sy = sy;
     put_scatter(V, i, j, k, v, bc);
-}
-
-// Programmatic dependent launch.  The target-mode level kernels run back to
-// back, each a few tens of microseconds at 257^3 and less below; launched with
-// programmatic stream serialisation (launch_pdl), the next kernel is launched
-// once every block of the previous one has exited, ahead of the grid's
-// completion, and waits in pdl_wait, before its first global access, until that
-// grid has completed and its writes are visible.  Launched the ordinary way,
-// pdl_wait returns at once.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
-template <typename... P, typename... A>
-static cudaError_t launch_pdl(void (*k)(P...), dim3 g, dim3 b, size_t smem, cudaStream_t st, A &&...args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = g;
-    cfg.blockDim = b;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
 }
 
 // The target-mode kernels march along x: a (32 k) x (8 j) thread tile walks
@@ -2582,9 +2660,9 @@ static int gs_arith(const Ctx &c, const Level &L, GsArith<2> &a) {
 static bool gs_plan(const Ctx &c, const Level &L, const MgBC &bc, int form, int count, bool coarse, GsPlan &g) {
     if (bc.dirichlet || form < 0) return false;
     const int X = L.n[0], Y = c.planar ? 0 : L.n[1], Z = L.n[2];
-    const long nc = (long)(X + 1) * (Y + 1), n = nc * (Z + 1);
+    const long nc = (long)(X + 1) * (Y + 1), zp = gs_pitch(Z), n = nc * zp;
     const size_t cap = 220 * 1024;
-    size_t smem = 8 * (size_t)(n + (long)(Y + 1) * (Z + 1) + (c.planar ? 0 : (long)(X + 1) * (Z + 1)));
+    size_t smem = 8 * (size_t)(n + (Y + 1) * zp + (c.planar ? 0 : (X + 1) * zp));
     if (coarse) smem += 8 * (size_t)(n + 2 * L.count);
     if (smem > cap || nc > 992) return false;
     g.rsmem = coarse || smem + 8 * (size_t)n <= cap;
@@ -2616,10 +2694,8 @@ static cudaError_t gs_pipe_launch(Ctx &c, Level &L, const MgBC &bc, const GsArit
     else k = c.planar ? k_gs_pipe<ARITH, true, false, false> : k_gs_pipe<ARITH, false, false, false>;
     cudaError_t e = cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem);
     if (e != cudaSuccess) return e;
-    k<<<1, g.threads + (COARSE ? 32 : 0), g.smem, c.stream>>>(lview<double>(L, L.pa()), lcview<double>(L, L.r), make_k(L), bc, ar, g.lam, g.Q,
-                                                              count, zero ? 1 : 0, c.p.mgTolerance, c.maxCount,
-                                                              (long long *)(c.dscal + 40));
-    return cudaGetLastError();
+    return launch_pdl(k, dim3(1), dim3(g.threads + (COARSE ? 32 : 0)), g.smem, c.stream, lview<double>(L, L.pa()), lcview<double>(L, L.r), make_k(L), bc,
+                      ar, g.lam, g.Q, count, zero ? 1 : 0, c.p.mgTolerance, c.maxCount, (long long *)(c.dscal + 40));
 }
 
 // `count` lexicographic sweeps of level l (coarse: the coarsest solve) in one
@@ -2661,7 +2737,7 @@ static int gs_smooth(Ctx &c, int l, int count, bool zero_first) {
     View3<const double> rv = lcview<double>(L, L.r);
     const size_t smem = 2 * sizeof(double) * (size_t)L.count;
     if (smem <= kGsBlockSmem) {
-        k_mg_gs_block<<<1, 512, smem, c.stream>>>(pv, rv, kk, bc, count, zero_first ? 1 : 0, wx, wy, wz);
+        SARAS_CUDA_TRY(launch_pdl(k_mg_gs_block, dim3(1), dim3(512), smem, c.stream, pv, rv, kk, bc, count, zero_first ? 1 : 0, wx, wy, wz));
         count_launch(c);
         return chk(c, "mg Gauss-Seidel");
     }
@@ -2721,9 +2797,9 @@ static int smooth(Ctx &c, int l, int count, bool zero_first, bool tgt) {
                 else SARAS_CUDA_TRY(launch_pdl(k_tgt_sweep<T, false>, gm, bm, 0, c.stream, B_<T>(L), A_<T>(L), R_<T>(L), sx, sy, bc, tk));
             } else SARAS_CUDA_TRY(launch_pdl(k_tgt_sweep<T, false>, gm, bm, 0, c.stream, B_<T>(L), A_<T>(L), R_<T>(L), sx, sy, bc, tk));
         } else if (n == 0 && zero_first)
-            k_mg_sweep<T, true><<<g, b, 0, c.stream>>>(lview<T>(L, B_<T>(L)), lcview<T>(L, A_<T>(L)), lcview<T>(L, R_<T>(L)), kk, bc, omega);
+            SARAS_CUDA_TRY(launch_pdl(k_mg_sweep<T, true>, g, b, 0, c.stream, lview<T>(L, B_<T>(L)), lcview<T>(L, A_<T>(L)), lcview<T>(L, R_<T>(L)), kk, bc, omega));
         else
-            k_mg_sweep<T, false><<<g, b, 0, c.stream>>>(lview<T>(L, B_<T>(L)), lcview<T>(L, A_<T>(L)), lcview<T>(L, R_<T>(L)), kk, bc, omega);
+            SARAS_CUDA_TRY(launch_pdl(k_mg_sweep<T, false>, g, b, 0, c.stream, lview<T>(L, B_<T>(L)), lcview<T>(L, A_<T>(L)), lcview<T>(L, R_<T>(L)), kk, bc, omega));
         count_launch(c);
         prof_end(c, pk, l, lb);
         flip<T>(L);
@@ -2758,8 +2834,8 @@ static int coarse_solve(Ctx &c, bool tgt) {
             if (ran) return chk(c, "mg coarse");
         }
     }
-    k_mg_coarse<T><<<1, kCoarseThreads, smem, c.stream>>>(lview<T>(L, A_<T>(L)), lcview<T>(L, R_<T>(L)), kk, bc, tol, maxc, tgt ? 1 : 0,
-                                               (long long *)(c.dscal + 40));
+    SARAS_CUDA_TRY(launch_pdl(k_mg_coarse<T>, dim3(1), dim3(kCoarseThreads), smem, c.stream, lview<T>(L, A_<T>(L)), lcview<T>(L, R_<T>(L)), kk, bc, tol,
+                              maxc, tgt ? 1 : 0, (long long *)(c.dscal + 40)));
     count_launch(c);
     return chk(c, "mg coarse");
 }
@@ -2798,13 +2874,13 @@ static int restrict_level(Ctx &c, int l, bool tgt) {
         prof_end(c, pk, l, sizeof(T) * pts * (1.0 + 1.0 / 8.0));
         return chk(c, "mg restrict");
     } else
-        k_mg_residual<T><<<g, b, 0, c.stream>>>(lview<T>(L, B_<T>(L)), lcview<T>(L, A_<T>(L)), lcview<T>(L, R_<T>(L)), kk, bcf);
+        SARAS_CUDA_TRY(launch_pdl(k_mg_residual<T>, g, b, 0, c.stream, lview<T>(L, B_<T>(L)), lcview<T>(L, A_<T>(L)), lcview<T>(L, R_<T>(L)), kk, bcf));
     count_launch(c);
     prof_end(c, pk, l, 3.0 * sizeof(T) * pts);
     dim3 g2, b2; core_dims(C, g2, b2);
     pk = sizeof(T) == 8 ? PK_MG_RESTRICT64 : PK_MG_RESTRICT32;
     prof_begin(c, pk, l);
-    k_mg_restrict<T><<<g2, b2, 0, c.stream>>>(lview<T>(C, R_<T>(C)), lcview<T>(L, B_<T>(L)), bcf, bcc);
+    SARAS_CUDA_TRY(launch_pdl(k_mg_restrict<T>, g2, b2, 0, c.stream, lview<T>(C, R_<T>(C)), lcview<T>(L, B_<T>(L)), bcf, bcc));
     count_launch(c);
     prof_end(c, pk, l, sizeof(T) * pts * (1.0 + 1.0 / 8.0));
     return chk(c, "mg restrict");
@@ -2824,7 +2900,7 @@ static int prolong_level(Ctx &c, int l, bool tgt, bool add) {
         SARAS_CUDA_TRY(launch_pdl(k_tgt_prolong_add<T>, gm, bm, 0, c.stream, A_<T>(L), A_<T>(C), sx, sy, (C.n[1] + 3) * (C.n[2] + 3),
                                   C.n[2] + 3, bc));
     } else {
-        k_mg_prolong_add<T><<<g, b, 0, c.stream>>>(lview<T>(L, A_<T>(L)), lcview<T>(C, A_<T>(C)), bc, add ? 1 : 0);
+        SARAS_CUDA_TRY(launch_pdl(k_mg_prolong_add<T>, g, b, 0, c.stream, lview<T>(L, A_<T>(L)), lcview<T>(C, A_<T>(C)), bc, add ? 1 : 0));
     }
     count_launch(c);
     prof_end(c, pk, l, sizeof(T) * pts * (2.0 + 1.0 / 8.0));
@@ -2899,14 +2975,13 @@ static int vcycle(Ctx &c, bool tgt, bool zero0) {
     return cycle_from<T>(c, 0, tgt, zero0, tgt ? std::max(1, c.p.coarseCycles) : 1);
 }
 
-// The target-mode V-cycle issues about ten kernels per level, most of them
-// microseconds long on the coarse levels, where the host's launch rate rather
-// than the GPU bounds the cycle.  It is captured once as a CUDA graph and
-// replayed: the kernels, their arguments and the level buffers they use are
-// the same every cycle, because every level's ping-pong flips an even number
-// of times per cycle (pre + post smoothing) and so returns to its starting
-// state.  The graph is rebuilt when the level states differ from the ones it
-// was captured with; with kernel profiling on, the cycle runs uncaptured.
+// A V-cycle issues about ten kernels per level, most of them microseconds long
+// on the coarse levels, where the host's launch rate rather than the GPU bounds
+// the cycle.  It is captured once as a CUDA graph and replayed: the kernels, their
+// arguments and the level buffers they use are the same every cycle that starts
+// from the same buffers (a level's ping-pong flips once a sweep; a cycle with an odd
+// number of sweeps alternates between two graphs).  A graph is rebuilt when the
+// level states differ from the ones it was captured with.
 static std::vector<int> level_state(const Ctx &c, bool timed) {
     std::vector<int> st;
     for (const Level &L : c.lv) { st.push_back(L.cur); st.push_back(L.cur32); }
@@ -2930,8 +3005,8 @@ static void vgraph_drop(Ctx &c, int a, int b, int t) {
 }
 
 void vgraph_reset(Ctx &c) {
-    for (int a = 0; a < 2; ++a)
-        for (int b = 0; b < 2; ++b)
+    for (int a = 0; a < 3; ++a)
+        for (int b = 0; b < 4; ++b)
             for (int t = 0; t < 2; ++t) vgraph_drop(c, a, b, t);
 }
 
@@ -2959,11 +3034,11 @@ static int map_prof_nodes(Ctx &c, cudaGraph_t g, std::vector<ProfNode> &out) {
     return SARAS_OK;
 }
 
-template <typename T>
-static int vcycle_tgt(Ctx &c, bool zero0) {
+// The launches of `run`, captured as graph (a, b) and replayed.
+template <typename F>
+static int graph_replay(Ctx &c, int a, int b, F run) {
     // with profiling on, one replay in profEvery runs the instance holding the
     // timing event nodes; the others run an instance captured without them
-    const int a = sizeof(T) == 4 ? 1 : 0, b = zero0 ? 1 : 0;
     const int t = any_profiling(c) && (c.profEvery <= 1 || c.profReplays++ % c.profEvery == 0) ? 1 : 0;
     std::vector<int> st = level_state(c, t == 1);
     if (c.vgraph[a][b][t] && c.vgraphState[a][b][t] != st) vgraph_drop(c, a, b, t);
@@ -2974,7 +3049,7 @@ static int vcycle_tgt(Ctx &c, bool zero0) {
         SARAS_CUDA_TRY(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeThreadLocal));
         c.profCapturing = true;
         c.profSuppress = t == 0;
-        int s = vcycle<T>(c, true, zero0);
+        int s = run();
         c.profCapturing = false;
         c.profSuppress = false;
         cudaGraph_t g = nullptr;
@@ -3000,17 +3075,21 @@ static int vcycle_tgt(Ctx &c, bool zero0) {
         c.vgraphLaunches[a][b][t] = c.launches - l0;
         c.launches = l0;
         c.vgraphState[a][b][t] = st;
-        if (level_state(c, t == 1) != st) {   // a cycle that does not restore the level states is never replayed:
-            vgraph_drop(c, a, b, t);          // back to the states before the capture, then run it directly
-            for (size_t q = 0; q < c.lv.size(); ++q) { c.lv[q].cur = st[2 * q]; c.lv[q].cur32 = st[2 * q + 1]; }
-            return vcycle<T>(c, true, zero0);
-        }
+        c.vgraphAfter[a][b][t] = level_state(c, t == 1);
     }
+    const std::vector<int> &after = c.vgraphAfter[a][b][t];   // the buffers a cycle with an odd number of sweeps leaves the iterates in
+    for (size_t q = 0; q < c.lv.size(); ++q) { c.lv[q].cur = after[2 * q]; c.lv[q].cur32 = after[2 * q + 1]; }
     int s = prof_graph_replay(c, c.vgraph[a][b][t], c.vgraphProf[a][b][t]);
     if (s) { c.err = "V-cycle graph: profiling events"; return s; }
     SARAS_CUDA_TRY(cudaGraphLaunch(c.vgraph[a][b][t], c.stream));
     c.launches += c.vgraphLaunches[a][b][t];
     return SARAS_OK;
+}
+
+template <typename T>
+static int vcycle_tgt(Ctx &c, bool zero0) {
+    const int buf = sizeof(T) == 4 ? c.lv[0].cur32 : c.lv[0].cur;
+    return graph_replay(c, sizeof(T) == 4 ? 1 : 0, (zero0 ? 1 : 0) + 2 * buf, [&]() { return vcycle<T>(c, true, zero0); });
 }
 
 static int read_scalars(Ctx &c, int first, int count) {
@@ -3021,22 +3100,18 @@ static int read_scalars(Ctx &c, int first, int count) {
 
 static int grid_blocks(long n) { return (int)std::max<long>(1, std::min<long>((n + 255) / 256, 152L * 8)); }
 
-int mg_compute_error(Ctx &c, int norm, double *err) {
+// computeError's launches: the maximum (or the squared sums) of the residual over
+// the level-0 core into dscal[22] (24, 25).
+static int error_launches(Ctx &c, int norm) {
     Level &L = c.lv[0];
     MgBC bc = level_bc(c, 0, false);
     MgK kk = make_k(L);
     long n = (long)(L.n[0] + 1) * (L.n[1] + 1) * (L.n[2] + 1);
-    int nb = std::min(grid_blocks(n), c.redCap);
-    SARAS_CUDA_TRY(cudaMemsetAsync(c.dscal + 22, 0, sizeof(double), c.stream));
-    // denominator max|residualData(0)| over the padded array (poisson_d3.cc:437)
-    SARAS_CUDA_TRY(cudaMemsetAsync(c.dscal + 21, 0, sizeof(double), c.stream));
     if (norm == 1) {
-        k_maxabs<<<grid_blocks(L.count), 256, 0, c.stream>>>(L.r, L.count, c.dscal + 21);
-        count_launch(c);
-    }
-    if (norm == 1) {
-        k_mg_error<<<nb, 256, 0, c.stream>>>(lcview<double>(L, L.pa()), lcview<double>(L, L.r), kk, bc, norm, c.dscal + 22, c.red,
-                                             c.red + c.redCap);
+        SARAS_CUDA_TRY(cudaMemsetAsync(c.dscal + 22, 0, sizeof(double), c.stream));
+        int nb = std::min(grid_blocks(n), c.redCap);
+        SARAS_CUDA_TRY(launch_pdl(k_mg_error, dim3(nb), dim3(256), 0, c.stream, lcview<double>(L, L.pa()), lcview<double>(L, L.r), kk, bc, norm,
+                                  c.dscal + 22, c.red, c.red + c.redCap));
         count_launch(c);
     } else {
         long nch = (n + kChunk - 1) / kChunk;
@@ -3047,19 +3122,40 @@ int mg_compute_error(Ctx &c, int norm, double *err) {
         k_seq_sum<<<1, 32, 0, c.stream>>>(c.red + c.redCap, nch, c.dscal + 25);
         count_launch(c, 3);
     }
-    int s = chk(c, "computeError");
-    if (s) return s;
-    if ((s = read_scalars(c, 21, 5))) return s;
-    double e = 0;
+    SARAS_CUDA_TRY(cudaMemcpyAsync(c.hscal + 21, c.dscal + 21, sizeof(double) * 5, cudaMemcpyDeviceToHost, c.stream));
+    return chk(c, "computeError");
+}
+
+// The denominator max|residualData(0)| over the padded array (poisson_d3.cc:437) into dscal[21].
+static int error_denominator(Ctx &c) {
+    Level &L = c.lv[0];
+    SARAS_CUDA_TRY(cudaMemsetAsync(c.dscal + 21, 0, sizeof(double), c.stream));
+    k_maxabs<<<grid_blocks(L.count), 256, 0, c.stream>>>(L.r, L.count, c.dscal + 21);
+    count_launch(c);
+    return chk(c, "computeError");
+}
+
+// The value computeError returns, from the scalars error_launches has read.
+static double error_value(const Ctx &c, int norm) {
     if (norm == 1) {
         double num = c.hscal[22], den = c.hscal[21];
-        e = den ? num / den : num;
-    } else if (norm == 2) {
-        double cnt = (double)n;
-        double num = c.hscal[24], den = c.hscal[25];
-        e = den ? std::sqrt(num / cnt) / std::sqrt(den / cnt) : std::sqrt(num / cnt);
+        return den ? num / den : num;
     }
-    *err = e;
+    if (norm == 2) {
+        const Level &L = c.lv[0];
+        double cnt = (double)((long)(L.n[0] + 1) * (L.n[1] + 1) * (L.n[2] + 1));
+        double num = c.hscal[24], den = c.hscal[25];
+        return den ? std::sqrt(num / cnt) / std::sqrt(den / cnt) : std::sqrt(num / cnt);
+    }
+    return 0;
+}
+
+int mg_compute_error(Ctx &c, int norm, double *err) {
+    int s;
+    if (norm == 1 && (s = error_denominator(c))) return s;
+    if ((s = error_launches(c, norm))) return s;
+    SARAS_CUDA_TRY(cudaStreamSynchronize(c.stream));
+    *err = error_value(c, norm);
     return SARAS_OK;
 }
 
@@ -3082,8 +3178,9 @@ static int mg_solve_reference(Ctx &c, int *cycles, double *residual) {
         k_mg_sub_mean<<<grid_blocks(L0.count), 256, 0, c.stream>>>(L0.r, L0.count, c.dscal + 20, (double)L0.count, c.dscal + 27);
         count_launch(c, 3);
     }
-    // pressureData(0)(core) = Pp(core) (+ face ghosts)
-    L0.cur = 0;
+    // pressureData(0)(core) = Pp(core) (+ face ghosts); every level from its first
+    // buffer, so that the solves replay the same cycle graphs
+    for (Level &L : c.lv) L.cur = 0;
     dim3 g, b; core_dims(L0, g, b);
     k_mg_init_p<double><<<g, b, 0, c.stream>>>(lview<double>(L0, L0.pa()), lcview<double>(L0, c.f[SARAS_FIELD_PP]), bc0);
     count_launch(c);
@@ -3096,12 +3193,20 @@ static int mg_solve_reference(Ctx &c, int *cycles, double *residual) {
         count_launch(c, 2);
     }
     if ((s = chk(c, "mg load"))) return s;
+    // the residual's denominator does not change over the solve
+    if (c.p.resType == 1 && (s = error_denominator(c))) return s;
     double prev = 0.0, res = 0.0;
     int cyc = 0;
     for (int i = 0; i < c.p.vcCount; ++i) {
-        if ((s = vcycle<double>(c, false, false))) return s;
+        // one V-cycle, its error and the copy of the error to the host, as one graph
+        s = graph_replay(c, 2, 2 * L0.cur, [&]() {
+            const int e = vcycle<double>(c, false, false);
+            return e ? e : error_launches(c, c.p.resType);
+        });
+        if (s) return s;
         cyc += 1;
-        if ((s = mg_compute_error(c, c.p.resType, &res))) return s;
+        SARAS_CUDA_TRY(cudaStreamSynchronize(c.stream));
+        res = error_value(c, c.p.resType);
         if (!std::isfinite(res)) { c.err = "multigrid residual is not finite"; return SARAS_NOT_FINITE; }
         if (!c.p.testPoisson) {
             if (std::fabs(prev - res) < c.p.mgTolerance) break;
