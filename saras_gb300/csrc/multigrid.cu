@@ -231,35 +231,92 @@ __device__ __forceinline__ void put_scatter(const View3<T> &P, int i, int j, int
     }
 }
 
+// The update of mg_update on a uniform mesh with its constants folded; the same
+// bits.  Multiplying by a power of two commutes with rounding, so (cx (E + W)) 2 is
+// cx2 (E + W), a product with a power-of-two constant can ride in a fused
+// multiply-add, and with cx2 = cy2 = cz2 all of them move into the other
+// constants.  c7 is always a power of two.
+template <int ARITH>   // 0: equal spacings, power-of-two constants; 1: power-of-two constants; 2: any uniform mesh
+struct GsArith {
+    double cx2, cy2, cz2, c7, den, iden;   // 0: c7, den, iden over cx2
+    __device__ __forceinline__ double operator()(double E, double W, double N, double S, double U, double D, double r, bool planar) const {
+        const double ew = E + W, ud = U + D;
+        double t;
+        if (ARITH == 0) {
+            t = planar ? ew + ud : (ew + (N + S)) + ud;
+        } else if (ARITH == 1) {
+            t = cx2 * ew;
+            if (!planar) t = fma(cy2, N + S, t);
+            t = fma(cz2, ud, t);
+        } else {
+            t = cx2 * ew;
+            if (!planar) t = t + cy2 * (N + S);
+            t = t + cz2 * ud;
+        }
+        return div_rn(fma(-c7, r, t), den, iden);   // c7 is a power of two: c7 r is exact
+    }
+    __device__ __forceinline__ double from_zero(double r) const { return div_rn(fma(-c7, r, 0.0), den, iden); }
+};
+
+// The reference-mode level kernels take one thread a point, the (j, k) plane
+// numbered k fastest over blockIdx.x and the planes over blockIdx.y: rows of
+// 2^m + 1 points leave no warp with a single live lane (a 64 x 4 block's third
+// block of a 129-point row cost the FP64 pipe, which bounds these kernels, a
+// quarter more warps).
+__device__ __forceinline__ bool plane_pt(const int E[3], int &i, int &j, int &k) {
+    const int W = E[2] + 1, t = blockIdx.x * blockDim.x + threadIdx.x;
+    j = t / W;
+    k = t - j * W;
+    i = blockIdx.y;
+    return j <= E[1];
+}
+
 // One Jacobi sweep (poisson_d3.cc:153-168).  zero_guess: the incoming iterate
 // is identically 0 (pressureData = 0 before smoothing a coarse level,
-// poisson.cc:258).  omega = 1 reproduces the reference exactly.
-template <typename T, bool ZERO>
-__global__ void k_mg_sweep(View3<T> out, View3<const T> in, View3<const T> r, MgK kk, MgBC bc, T omega) {
+// poisson.cc:258).  ARITH: the folded forms of GsArith on uniform meshes (the
+// same bits with 9, 10 or 12 FP64 operations a point instead of 16), or -1: the
+// expression with the metrics read at each point.
+template <int ARITH, bool ZERO>
+__global__ void __launch_bounds__(256) k_mg_sweep(View3<double> out, View3<const double> in, View3<const double> r, MgK kk, MgBC bc,
+                                                  GsArith<ARITH < 0 ? 2 : ARITH> ar) {
     pdl_wait();
     int i, j, k;
-    if (!core_pt(bc.E, i, j, k)) return;
-    T v;
-    if (ZERO) {
-        v = mg_update<T>((T)0, (T)0, (T)0, (T)0, (T)0, (T)0, r(i, j, k), kk, i, j, k);
-        if (omega != (T)1.0) v = omega * v;
-    } else {
-        T C = in(i, j, k);
-        v = mg_update<T>(in(i + 1, j, k), in(i - 1, j, k), in(i, j + 1, k), in(i, j - 1, k), in(i, j, k + 1), in(i, j, k - 1),
-                         r(i, j, k), kk, i, j, k);
-        if (omega != (T)1.0) v = C + omega * (v - C);
+    if (!plane_pt(bc.E, i, j, k)) return;
+    double E = 0.0, W = 0.0, N = 0.0, S = 0.0, U = 0.0, D = 0.0;
+    if (!ZERO) {
+        E = in(i + 1, j, k); W = in(i - 1, j, k); U = in(i, j, k + 1); D = in(i, j, k - 1);
+        N = in(i, j + 1, k); S = in(i, j - 1, k);
     }
+    double v;
+    if (ARITH < 0) v = mg_update<double>(E, W, N, S, U, D, r(i, j, k), kk, i, j, k);
+    else if (ZERO) v = ar.from_zero(r(i, j, k));
+    else v = ar(E, W, N, S, U, D, r(i, j, k), false);
     put_scatter(out, i, j, k, v, bc);
 }
 
+// Laplacian of a uniform level in the folded forms of mg_lap, as r - lap (rounded
+// as the two expressions are): FORM 0: equal power-of-two factors (9 FP64
+// operations), 1: power-of-two factors (10), 2: any (12); -1: mg_lap.  2 C and, by
+// a power of two, l (E - 2C + W) are exact, so a fused multiply-add rounds where the
+// separate sum does.
+template <int FORM>
+__device__ __forceinline__ double mg_res(double E, double W, double N, double S, double U, double D, double C, double r, const MgK &k, int x, int y,
+                                         int z) {
+    if (FORM < 0) return r - mg_lap<double>(E, W, N, S, U, D, C, k, x, y, z);
+    const double tx = fma(-2.0, C, E) + W, ty = fma(-2.0, C, N) + S, tz = fma(-2.0, C, U) + D;
+    if (FORM == 0) return fma(-k.lx, (tx + ty) + tz, r);
+    if (FORM == 1) return r - fma(k.lz, tz, fma(k.ly, ty, k.lx * tx));
+    return r - (k.lx * tx + k.ly * ty + k.lz * tz);
+}
+
 // computeResidual (poisson_d3.cc:90-111): tmp(core) = r - Lap(p).
-template <typename T>
-__global__ void k_mg_residual(View3<T> tmp, View3<const T> p, View3<const T> r, MgK kk, MgBC bc) {
+template <int FORM>
+__global__ void __launch_bounds__(256) k_mg_residual(View3<double> tmp, View3<const double> p, View3<const double> r, MgK kk, MgBC bc) {
     pdl_wait();
     int i, j, k;
-    if (!core_pt(bc.E, i, j, k)) return;
-    T lap = mg_lap<T>(p(i + 1, j, k), p(i - 1, j, k), p(i, j + 1, k), p(i, j - 1, k), p(i, j, k + 1), p(i, j, k - 1), p(i, j, k), kk, i, j, k);
-    tmp(i, j, k) = r(i, j, k) - lap;
+    if (!plane_pt(bc.E, i, j, k)) return;
+    tmp(i, j, k) = mg_res<FORM>(p(i + 1, j, k), p(i - 1, j, k), p(i, j + 1, k), p(i, j - 1, k), p(i, j, k + 1), p(i, j, k - 1), p(i, j, k), r(i, j, k),
+                                kk, i, j, k);
 }
 
 // Value of the residual array at a possibly-ghost index after updatePads
@@ -285,13 +342,16 @@ __device__ __forceinline__ T pad_val(const View3<const T> &t, int i, int j, int 
 }
 
 // coarsen (poisson_d3.cc:250-298): 27-point full weighting in the reference's
-// summation order.  bcf describes the fine level, Ec the coarse core.
+// summation order.  bcf describes the fine level, bcc the coarse one.  The three
+// fine indices of each axis are resolved once (updatePads: periodic images along x
+// and y, otherwise 0) and the 27 loads issued together, without a branch each (a
+// few loads in flight at a time took 10 us on the smallest levels).
 template <typename T>
-__global__ void k_mg_restrict(View3<T> rc, View3<const T> t, MgBC bcf, MgBC bcc) {
+__global__ void __launch_bounds__(64) k_mg_restrict(View3<T> rc, View3<const T> t, MgBC bcf, MgBC bcc) {
     pdl_wait();
     int i, j, k;
-    if (!core_pt(bcc.E, i, j, k)) return;
-    int i2 = 2 * i, j2 = 2 * j, k2 = 2 * k;
+    if (!plane_pt(bcc.E, i, j, k)) return;
+    const int i2 = 2 * i, j2 = 2 * j, k2 = 2 * k;
     if (bcf.planar) {   // poisson_d2.cc:207-225: 9-point full weighting in the y = 0 plane
         const bool in2 = i2 > 0 && k2 > 0 && i2 < bcf.E[0] && k2 < bcf.E[2];
         auto Q = [&](int a, int c) -> T { return in2 ? t(a, 0, c) : pad_val(t, a, 0, c, bcf); };
@@ -300,17 +360,39 @@ __global__ void k_mg_restrict(View3<T> rc, View3<const T> t, MgBC bcf, MgBC bcc)
         rc(i, 0, k) = facePoints + vertPoints + t(i2, 0, k2) * (T)0.25;
         return;
     }
-    bool interior = i2 > 0 && j2 > 0 && k2 > 0 && i2 < bcf.E[0] && j2 < bcf.E[1] && k2 < bcf.E[2];
-    auto T_ = [&](int a, int b, int c) -> T { return interior ? t(a, b, c) : pad_val(t, a, b, c, bcf); };
-    T facePoints = (T_(i2 + 1, j2, k2) + T_(i2 - 1, j2, k2) + T_(i2, j2 + 1, k2) + T_(i2, j2 - 1, k2) +
-                    T_(i2, j2, k2 + 1) + T_(i2, j2, k2 - 1)) * (T)0.0625;
-    T edgePoints = (T_(i2 + 1, j2 + 1, k2) + T_(i2 + 1, j2 - 1, k2) + T_(i2 - 1, j2 - 1, k2) + T_(i2 - 1, j2 + 1, k2) +
-                    T_(i2, j2 + 1, k2 + 1) + T_(i2, j2 - 1, k2 + 1) + T_(i2, j2 - 1, k2 - 1) + T_(i2, j2 + 1, k2 - 1) +
-                    T_(i2 + 1, j2, k2 + 1) + T_(i2 + 1, j2, k2 - 1) + T_(i2 - 1, j2, k2 - 1) + T_(i2 - 1, j2, k2 + 1)) * (T)0.03125;
-    T vertPoints = (T_(i2 + 1, j2 + 1, k2 + 1) + T_(i2 + 1, j2 + 1, k2 - 1) + T_(i2 + 1, j2 - 1, k2 + 1) +
-                    T_(i2 - 1, j2 + 1, k2 + 1) + T_(i2 + 1, j2 - 1, k2 - 1) + T_(i2 - 1, j2 + 1, k2 - 1) +
-                    T_(i2 - 1, j2 - 1, k2 + 1) + T_(i2 - 1, j2 - 1, k2 - 1)) * (T)0.015625;
-    rc(i, j, k) = facePoints + edgePoints + vertPoints + t(i2, j2, k2) * (T)0.125;
+    const int c[3] = {i2, j2, k2};
+    long o[3][3];
+    bool in[3][3];
+    const long st[3] = {t.sx, t.sy, 1};
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const int E = bcf.E[d];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            int q = c[d] - 1 + a;
+            const bool core = q >= 0 && q <= E;
+            in[d][a] = core || (d < 2 && bcf.per[d]);
+            if (!core) q = in[d][a] ? (q < 0 ? E - 1 : 1) : c[d];
+            o[d][a] = (long)(q + 1) * st[d];
+        }
+    }
+    T v[3][3][3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int b = 0; b < 3; ++b)
+#pragma unroll
+            for (int e = 0; e < 3; ++e) {
+                const T x = t.p[o[0][a] + o[1][b] + o[2][e]];
+                v[a][b][e] = in[0][a] && in[1][b] && in[2][e] ? x : (T)0;
+            }
+    auto T_ = [&](int a, int b, int e) -> T { return v[a + 1][b + 1][e + 1]; };
+    T facePoints = (T_(1, 0, 0) + T_(-1, 0, 0) + T_(0, 1, 0) + T_(0, -1, 0) + T_(0, 0, 1) + T_(0, 0, -1)) * (T)0.0625;
+    T edgePoints = (T_(1, 1, 0) + T_(1, -1, 0) + T_(-1, -1, 0) + T_(-1, 1, 0) + T_(0, 1, 1) + T_(0, -1, 1) + T_(0, -1, -1) + T_(0, 1, -1) +
+                    T_(1, 0, 1) + T_(1, 0, -1) + T_(-1, 0, -1) + T_(-1, 0, 1)) * (T)0.03125;
+    T vertPoints = (T_(1, 1, 1) + T_(1, 1, -1) + T_(1, -1, 1) + T_(-1, 1, 1) + T_(1, -1, -1) + T_(-1, 1, -1) + T_(-1, -1, 1) + T_(-1, -1, -1)) *
+                   (T)0.015625;
+    rc(i, j, k) = facePoints + edgePoints + vertPoints + T_(0, 0, 0) * (T)0.125;
 }
 
 // prolong (poisson_d3.cc:301-388) followed by pressureData += smoothedPres
@@ -319,7 +401,7 @@ template <typename T>
 __global__ void k_mg_prolong_add(View3<T> pf, View3<const T> pc, MgBC bc, int add) {
     pdl_wait();
     int i, j, k;
-    if (!core_pt(bc.E, i, j, k)) return;
+    if (!plane_pt(bc.E, i, j, k)) return;
     int i2 = i / 2, j2 = j / 2, k2 = k / 2;
     bool io = i & 1, jo = j & 1, ko = k & 1;
     T v;
@@ -663,27 +745,6 @@ __global__ void k_mg_gs_block(View3<double> pg, View3<const double> rg, MgK kk, 
 // it).  One of them at or above tol proves that the sweep does not stop; the
 // first sweep with none (its maximum may still lie elsewhere) is rerun up to the
 // sweep before and continued by coarse_gs, which tests every point.
-template <int ARITH>   // 0: equal spacings, power-of-two constants; 1: power-of-two constants; 2: any uniform mesh
-struct GsArith {
-    double cx2, cy2, cz2, c7, den, iden;   // 0: c7, den, iden over cx2
-    __device__ __forceinline__ double operator()(double E, double W, double N, double S, double U, double D, double r, bool planar) const {
-        const double ew = E + W, ud = U + D;
-        double t;
-        if (ARITH == 0) {
-            t = planar ? ew + ud : (ew + (N + S)) + ud;
-        } else if (ARITH == 1) {
-            t = cx2 * ew;
-            if (!planar) t = fma(cy2, N + S, t);
-            t = fma(cz2, ud, t);
-        } else {
-            t = cx2 * ew;
-            if (!planar) t = t + cy2 * (N + S);
-            t = t + cz2 * ud;
-        }
-        return div_rn(fma(-c7, r, t), den, iden);   // c7 is a power of two: c7 r is exact
-    }
-};
-
 struct GsPlan {
     int lam, Q, threads;    // stages between sweeps, sweeps of a column apart, compute threads (a multiple of 32)
     int rsmem;              // the right-hand side in shared memory too
@@ -1084,32 +1145,17 @@ __global__ void k_mg_error_sq(View3<const double> p, View3<const double> r, MgK 
     partDen[c] = sd;
 }
 
-__global__ void k_mg_error(View3<const double> p, View3<const double> r, MgK kk, MgBC bc, int norm, double *maxv,
-                           double *partNum, double *partDen) {
+template <int FORM>
+__global__ void __launch_bounds__(256) k_mg_error(View3<const double> p, View3<const double> r, MgK kk, MgBC bc, double *maxv) {
     pdl_wait();
-    __shared__ double s1[32], s2[32];
-    int E0 = bc.E[0], E1 = bc.E[1], E2 = bc.E[2];
-    long n = (long)(E0 + 1) * (E1 + 1) * (E2 + 1);
-    double m = 0, sn = 0, sd = 0;
-    for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x) {
-        int k = (int)(t % (E2 + 1)), j = (int)((t / (E2 + 1)) % (E1 + 1)), i = (int)(t / ((long)(E2 + 1) * (E1 + 1)));
-        double lap = mg_lap<double>(p(i + 1, j, k), p(i - 1, j, k), p(i, j + 1, k), p(i, j - 1, k), p(i, j, k + 1), p(i, j, k - 1),
-                                    p(i, j, k), kk, i, j, k);
-        double v = fabs(lap - r(i, j, k));
-        if (v != v) v = INFINITY;
-        m = fmax(m, v);
-        sn += v * v;
-        sd += r(i, j, k) * r(i, j, k);
+    int i, j, k;
+    unsigned long long m = 0ull;
+    if (plane_pt(bc.E, i, j, k)) {
+        // |lap - r| = |r - lap|; a NaN's bits stay above every number's
+        m = abs_bits(mg_res<FORM>(p(i + 1, j, k), p(i - 1, j, k), p(i, j + 1, k), p(i, j - 1, k), p(i, j, k + 1), p(i, j, k - 1), p(i, j, k), r(i, j, k),
+                                  kk, i, j, k));
     }
-    if (norm == 1) { block_max_to(m, maxv); return; }
-    sn = warp_sum(sn); sd = warp_sum(sd);
-    if ((threadIdx.x & 31) == 0) { s1[threadIdx.x >> 5] = sn; s2[threadIdx.x >> 5] = sd; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double A = 0, B = 0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) { A += s1[w]; B += s2[w]; }
-        partNum[blockIdx.x] = A; partDen[blockIdx.x] = B;
-    }
+    block_max_bits_to(m, maxv);
 }
 
 // ---- target-mode level kernels
@@ -2254,6 +2300,14 @@ static View3<const T> lcview(const Level &L, const T *p) {
     return v;
 }
 
+// Launch shape of the kernels on plane_pt: small blocks on small levels, to spread them.
+static void plane_dims(const Level &L, dim3 &g, dim3 &b) {
+    const int pts = (L.n[1] + 1) * (L.n[2] + 1);
+    const int bs = (long)pts * (L.n[0] + 1) >= (1l << 17) ? 256 : 64;
+    b = dim3(bs, 1, 1);
+    g = dim3((pts + bs - 1) / bs, L.n[0] + 1, 1);
+}
+
 static void core_dims(const Level &L, dim3 &g, dim3 &b) {
     int nz = L.n[2] + 1, ny = L.n[1] + 1, nx = L.n[0] + 1;
     b = nz >= 64 ? dim3(64, 4, 1) : nz >= 32 ? dim3(32, 8, 1) : dim3(16, 8, 2);
@@ -2762,14 +2816,44 @@ static int gs_status(Ctx &c) {
     return SARAS_OK;
 }
 
+// ---- the reference mode's level launches in the folded forms
+template <int ARITH, bool ZERO>
+static cudaError_t ref_sweep_form(Ctx &c, Level &L, const MgBC &bc, const GsArith<2> &a) {
+    GsArith<ARITH < 0 ? 2 : ARITH> ar;
+    ar.cx2 = a.cx2; ar.cy2 = a.cy2; ar.cz2 = a.cz2; ar.c7 = a.c7; ar.den = a.den; ar.iden = a.iden;
+    dim3 g, b; plane_dims(L, g, b);
+    return launch_pdl(k_mg_sweep<ARITH, ZERO>, g, b, 0, c.stream, lview<double>(L, L.pb()), lcview<double>(L, L.pa()), lcview<double>(L, L.r), make_k(L),
+                      bc, ar);
+}
+template <bool ZERO>
+static cudaError_t ref_sweep(Ctx &c, Level &L, const MgBC &bc) {
+    GsArith<2> a = {};
+    switch (c.planar ? -1 : gs_arith(c, L, a)) {
+    case 0: return ref_sweep_form<0, ZERO>(c, L, bc, a);
+    case 1: return ref_sweep_form<1, ZERO>(c, L, bc, a);
+    case 2: return ref_sweep_form<2, ZERO>(c, L, bc, a);
+    default: return ref_sweep_form<-1, ZERO>(c, L, bc, a);
+    }
+}
+
+// Form of a level's Laplacian in mg_res.
+static int lap_form(const Ctx &c, const Level &L) {
+    if (c.stretched || c.planar) return -1;
+    if (!is_pow2(L.lx) || !is_pow2(L.ly) || !is_pow2(L.lz)) return 2;
+    return L.lx == L.ly && L.ly == L.lz ? 0 : 1;
+}
+static cudaError_t ref_residual(Ctx &c, Level &L, const MgBC &bc) {
+    const int f = lap_form(c, L);
+    dim3 g, b; plane_dims(L, g, b);
+    auto k = f == 0 ? k_mg_residual<0> : f == 1 ? k_mg_residual<1> : f == 2 ? k_mg_residual<2> : k_mg_residual<-1>;
+    return launch_pdl(k, g, b, 0, c.stream, lview<double>(L, L.pb()), lcview<double>(L, L.pa()), lcview<double>(L, L.r), make_k(L), bc);
+}
+
 template <typename T>
 static int smooth(Ctx &c, int l, int count, bool zero_first, bool tgt) {
     if (!tgt && c.p.gsSmooth && sizeof(T) == 8) return gs_smooth(c, l, count, zero_first);
     Level &L = c.lv[l];
     MgBC bc = level_bc(c, l, tgt);
-    MgK kk = make_k(L);
-    dim3 g, b; core_dims(L, g, b);
-    T omega = tgt ? (T)c.p.jacobiWeight : (T)1.0;
     int pk = sizeof(T) == 8 ? PK_MG_SMOOTH64 : PK_MG_SMOOTH32;
     double bytes = 3.0 * sizeof(T) * (double)(L.n[0] + 1) * (L.n[1] + 1) * (L.n[2] + 1);
     int sx = (L.n[1] + 3) * (L.n[2] + 3), sy = L.n[2] + 3;
@@ -2797,9 +2881,9 @@ static int smooth(Ctx &c, int l, int count, bool zero_first, bool tgt) {
                 else SARAS_CUDA_TRY(launch_pdl(k_tgt_sweep<T, false>, gm, bm, 0, c.stream, B_<T>(L), A_<T>(L), R_<T>(L), sx, sy, bc, tk));
             } else SARAS_CUDA_TRY(launch_pdl(k_tgt_sweep<T, false>, gm, bm, 0, c.stream, B_<T>(L), A_<T>(L), R_<T>(L), sx, sy, bc, tk));
         } else if (n == 0 && zero_first)
-            SARAS_CUDA_TRY(launch_pdl(k_mg_sweep<T, true>, g, b, 0, c.stream, lview<T>(L, B_<T>(L)), lcview<T>(L, A_<T>(L)), lcview<T>(L, R_<T>(L)), kk, bc, omega));
+            SARAS_CUDA_TRY(ref_sweep<true>(c, L, bc));
         else
-            SARAS_CUDA_TRY(launch_pdl(k_mg_sweep<T, false>, g, b, 0, c.stream, lview<T>(L, B_<T>(L)), lcview<T>(L, A_<T>(L)), lcview<T>(L, R_<T>(L)), kk, bc, omega));
+            SARAS_CUDA_TRY(ref_sweep<false>(c, L, bc));
         count_launch(c);
         prof_end(c, pk, l, lb);
         flip<T>(L);
@@ -2844,8 +2928,6 @@ template <typename T>
 static int restrict_level(Ctx &c, int l, bool tgt) {
     Level &L = c.lv[l], &C = c.lv[l + 1];
     MgBC bcf = level_bc(c, l, tgt), bcc = level_bc(c, l + 1, tgt);
-    MgK kk = make_k(L);
-    dim3 g, b; core_dims(L, g, b);
     int pk = sizeof(T) == 8 ? PK_MG_RESID64 : PK_MG_RESID32;
     double pts = (double)(L.n[0] + 1) * (L.n[1] + 1) * (L.n[2] + 1);
     prof_begin(c, pk, l);
@@ -2874,13 +2956,13 @@ static int restrict_level(Ctx &c, int l, bool tgt) {
         prof_end(c, pk, l, sizeof(T) * pts * (1.0 + 1.0 / 8.0));
         return chk(c, "mg restrict");
     } else
-        SARAS_CUDA_TRY(launch_pdl(k_mg_residual<T>, g, b, 0, c.stream, lview<T>(L, B_<T>(L)), lcview<T>(L, A_<T>(L)), lcview<T>(L, R_<T>(L)), kk, bcf));
+        SARAS_CUDA_TRY(ref_residual(c, L, bcf));
     count_launch(c);
     prof_end(c, pk, l, 3.0 * sizeof(T) * pts);
-    dim3 g2, b2; core_dims(C, g2, b2);
+    const int cpts = (C.n[1] + 1) * (C.n[2] + 1);
     pk = sizeof(T) == 8 ? PK_MG_RESTRICT64 : PK_MG_RESTRICT32;
     prof_begin(c, pk, l);
-    SARAS_CUDA_TRY(launch_pdl(k_mg_restrict<T>, g2, b2, 0, c.stream, lview<T>(C, R_<T>(C)), lcview<T>(L, B_<T>(L)), bcf, bcc));
+    SARAS_CUDA_TRY(launch_pdl(k_mg_restrict<T>, dim3((cpts + 63) / 64, C.n[0] + 1, 1), dim3(64), 0, c.stream, lview<T>(C, R_<T>(C)), lcview<T>(L, B_<T>(L)), bcf, bcc));
     count_launch(c);
     prof_end(c, pk, l, sizeof(T) * pts * (1.0 + 1.0 / 8.0));
     return chk(c, "mg restrict");
@@ -2890,7 +2972,7 @@ template <typename T>
 static int prolong_level(Ctx &c, int l, bool tgt, bool add) {
     Level &L = c.lv[l], &C = c.lv[l + 1];
     MgBC bc = level_bc(c, l, tgt);
-    dim3 g, b; core_dims(L, g, b);
+    dim3 g, b; plane_dims(L, g, b);
     int pk = sizeof(T) == 8 ? PK_MG_PROLONG64 : PK_MG_PROLONG32;
     double pts = (double)(L.n[0] + 1) * (L.n[1] + 1) * (L.n[2] + 1);
     prof_begin(c, pk, l);
@@ -3109,9 +3191,10 @@ static int error_launches(Ctx &c, int norm) {
     long n = (long)(L.n[0] + 1) * (L.n[1] + 1) * (L.n[2] + 1);
     if (norm == 1) {
         SARAS_CUDA_TRY(cudaMemsetAsync(c.dscal + 22, 0, sizeof(double), c.stream));
-        int nb = std::min(grid_blocks(n), c.redCap);
-        SARAS_CUDA_TRY(launch_pdl(k_mg_error, dim3(nb), dim3(256), 0, c.stream, lcview<double>(L, L.pa()), lcview<double>(L, L.r), kk, bc, norm,
-                                  c.dscal + 22, c.red, c.red + c.redCap));
+        const int f = lap_form(c, L);
+        dim3 g, b; plane_dims(L, g, b);
+        auto k = f == 0 ? k_mg_error<0> : f == 1 ? k_mg_error<1> : f == 2 ? k_mg_error<2> : k_mg_error<-1>;
+        SARAS_CUDA_TRY(launch_pdl(k, g, b, 0, c.stream, lcview<double>(L, L.pa()), lcview<double>(L, L.r), kk, bc, c.dscal + 22));
         count_launch(c);
     } else {
         long nch = (n + kChunk - 1) / kChunk;
@@ -3138,7 +3221,7 @@ static int error_denominator(Ctx &c) {
 // The value computeError returns, from the scalars error_launches has read.
 static double error_value(const Ctx &c, int norm) {
     if (norm == 1) {
-        double num = c.hscal[22], den = c.hscal[21];
+        const double num = std::isnan(c.hscal[22]) ? INFINITY : c.hscal[22], den = c.hscal[21];
         return den ? num / den : num;
     }
     if (norm == 2) {
@@ -3666,7 +3749,7 @@ int mg_test_prolong(Ctx &c, double *err) {
     SARAS_CUDA_TRY(cudaMemcpyAsync(L1.pa(), h1.data(), L1.count * 8, cudaMemcpyHostToDevice, c.stream));
     SARAS_CUDA_TRY(cudaMemsetAsync(L0.pa(), 0, L0.count * 8, c.stream));
     MgBC bc = level_bc(c, 0, false);
-    dim3 g, b; core_dims(L0, g, b);
+    dim3 g, b; plane_dims(L0, g, b);
     k_mg_prolong_add<double><<<g, b, 0, c.stream>>>(lview<double>(L0, L0.pa()), lcview<double>(L1, L1.pa()), bc, 0);
     count_launch(c);
     std::vector<double> out(L0.count);
