@@ -140,6 +140,7 @@ struct Ctx {
     size_t probeBytes = 0;
     double *hscal = nullptr;        // pinned host mirror
     int *dflag = nullptr;
+    double *gsFace = nullptr;       // planes kept by the wavefront of blocks (Gauss-Seidel on large levels)
     // stats
     long long launches = 0;
     long long coarseIters = 0;

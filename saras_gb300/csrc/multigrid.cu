@@ -967,75 +967,140 @@ __device__ __forceinline__ double mg_ghost_value(const View3<const double> &p, i
         if (bc.dirichlet) sign = -sign;
         q[d] = q[d] < 0 ? 1 : E - 1;
     }
-    return sign * __ldcg(&p(q[0], q[1], q[2]));
+    return sign * p(q[0], q[1], q[2]);
 }
 
-// Grid-wide barrier for the cooperative Gauss-Seidel kernel: block arrivals
-// are counted on *count (zeroed before the launch); the b-th barrier waits
-// for b * gridDim.x arrivals.  The wait is bounded: after kGsSpinLimit polls
-// (about a second) the block records the failure in *err and every block
-// leaves the kernel at its next barrier.
-constexpr long long kGsSpinLimit = 1ll << 24;
-__device__ __forceinline__ bool gs_grid_sync(unsigned *count, unsigned target, int *err) {
-    __shared__ int ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        atomicAdd(count, 1u);
-        long long spins = 0;
-        int good = 1;
-        while (*(volatile unsigned *)count < target) {
-            if (*(volatile int *)err) { good = 0; break; }
-            if (++spins > kGsSpinLimit) { atomicExch(err, 1); good = 0; break; }
-            __nanosleep(64);
-        }
-        __threadfence();
-        ok = good;
-    }
-    __syncthreads();
-    return ok != 0;
+// ---- levels beyond one CTA: a wavefront of blocks
+// The level is cut into blocks of about eight points an axis; the blocks with
+// bi + bj + bk = b depend on those of stage b - 1 (this sweep) and of stage b + 1 of
+// the sweep before, as single points do, so one launch runs a whole stage, and with
+// it stage b - lam m of every sweep m of the phase: lam = 2 launches from sweep to
+// sweep, or a periodic axis's block count (its first block reads the last one's
+// plane E - 1 of the sweep before).  A block loads its points and a one-point halo
+// into shared memory -- below, points of this sweep or (imposeBC) the image plane of
+// the state before it; above, the state before it, where a periodic axis's plane 1
+// has been rewritten by then and is kept aside by its first block (face) -- and
+// runs its own wavefront of ni + nj + nk - 2 steps in place.  The operands are the
+// sequential loop's: same bits.
+//
+// What bounds it: 22 to 25 dependent steps of 9 to 16 FP64 operations a block (about
+// 9 us) and 3 us of launch, load and store around them, (blocks an axis) x 3 - 2 times
+// plus lam a further sweep.  Four sweeps of a 65^3 level, periodic: 46 launches,
+// 0.64 ms; of a 33^3 level 0.30 ms periodic, 0.22 with mirror walls.  A wavefront of
+// single points with a grid barrier a stage took 2.7, 1.2 and 1.2 ms.  (0.88 and
+// 0.42 ms with one load in flight a thread, kGsLoads = 1.)
+struct GsBlocks {
+    int T[3], nb[3], lam;   // block size (the last one of an axis: one point more), blocks, stages between sweeps
+    int stages;             // of one sweep
+};
+
+constexpr int kGsLoads = 6, kGsThreads = 256;   // every thread loads; the columns' threads (at most 96) compute and store
+
+// Value of the ghost (i, j, k) beyond axis d before a sweep: its image point's
+// value v, negated or replaced by a wall in the Dirichlet check.
+__device__ __forceinline__ double gs_ghost(double v, int d, int i, int j, int k, const MgBC &bc, const double *wx, const double *wy, const double *wz) {
+    if (bc.per[d] || !bc.dirichlet) return v;
+    if (bc.zeroBC) return -v;
+    if (d == 0) return wx[(j + 1) * (bc.E[2] + 3) + k + 1];
+    if (d == 1) return wy[(i + 1) * (bc.E[2] + 3) + k + 1];
+    return wz[(i + 1) * (bc.E[1] + 3) + j + 1];
 }
 
-// Levels too large for one CTA's shared memory: a cooperative launch over
-// gridDim.x co-resident blocks, the stages separated by grid barriers.  The
-// iterate is read past L1 (ld.global.cg), so a block never sees a line that
-// another block has updated since.  `count` sweeps, each preceded by the
-// ghost fill, and a final ghost fill.
-__global__ void __launch_bounds__(256) k_mg_gs_grid(View3<double> p, View3<const double> r, MgK kk, MgBC bc, int count,
-                                                    unsigned *sync, int *err, const double *wx, const double *wy,
-                                                    const double *wz) {
-    const int X = bc.E[0], Y = bc.E[1], Z = bc.E[2];
-    const long tid = blockIdx.x * (long)blockDim.x + threadIdx.x, nt = (long)gridDim.x * blockDim.x;
-    const View3<const double> pc{p.p, {p.n[0], p.n[1], p.n[2]}, p.sx, p.sy};
-    // ghost points: two full x planes, two y planes (x core), two z planes (x, y core)
-    const long fx = (long)(Y + 3) * (Z + 3), fy = (long)(X + 1) * (Z + 3), fz = (long)(X + 1) * (Y + 1);
-    const long ng = 2 * (fx + fy + fz);
-    unsigned target = 0;
-    for (int it = 0;; ++it) {
-        for (long t = tid; t < ng; t += nt) {
-            int i, j, k;
-            long u = t;
-            if (u < 2 * fx) { i = u < fx ? -1 : X + 1; u %= fx; j = (int)(u / (Z + 3)) - 1; k = (int)(u % (Z + 3)) - 1; }
-            else if ((u -= 2 * fx) < 2 * fy) { j = u < fy ? -1 : Y + 1; u %= fy; i = (int)(u / (Z + 3)); k = (int)(u % (Z + 3)) - 1; }
-            else { u -= 2 * fy; k = u < fz ? -1 : Z + 1; u %= fz; i = (int)(u / (Y + 1)); j = (int)(u % (Y + 1)); }
-            p(i, j, k) = mg_ghost_value(pc, i, j, k, bc, wx, wy, wz);   // reads the core past L1
+template <int ARITH>
+__global__ void __launch_bounds__(kGsThreads) k_gs_blocks(View3<double> p, View3<const double> r, MgK kk, MgBC bc, GsArith<ARITH < 0 ? 2 : ARITH> ar, GsBlocks g,
+                                                   int stage, double *face, const double *wx, const double *wy, const double *wz) {
+    pdl_wait();
+    const int bi = blockIdx.x / g.nb[1], bj = blockIdx.x - bi * g.nb[1], bk = stage - g.lam * (int)blockIdx.y - bi - bj;
+    if (bk < 0 || bk >= g.nb[2]) return;
+    extern __shared__ double gs_sm[];
+    const int X = bc.E[0], Y = bc.E[1], Z = bc.E[2], planar = bc.planar;
+    const int lo[3] = {bi * g.T[0], bj * g.T[1], bk * g.T[2]};
+    const int ni = bi == g.nb[0] - 1 ? X + 1 - lo[0] : g.T[0], nj = bj == g.nb[1] - 1 ? Y + 1 - lo[1] : g.T[1],
+              nk = bk == g.nb[2] - 1 ? Z + 1 - lo[2] : g.T[2];
+    const int sj = (nk + 3) & ~1, si = (nj + 2) * sj;   // an even pitch: neighbouring columns of a step in different banks
+    double *fx = face, *fy = fx + (long)(Y + 1) * (Z + 1), *fz = fy + (long)(X + 1) * (Z + 1);
+    // points and halo, kGsLoads of a thread's loads in flight together
+    const int cells = (ni + 2) * (nj + 2) * (nk + 2);
+    for (int t0 = threadIdx.x; t0 < cells; t0 += kGsLoads * blockDim.x) {
+        double v[kGsLoads];
+        int o[kGsLoads];
+        int pt[kGsLoads];   // 1 + plane-1 flags of a point of the block, 0: halo or nothing
+#pragma unroll
+        for (int u = 0; u < kGsLoads; ++u) {
+            const int t = t0 + u * blockDim.x;
+            const int c = t / (nk + 2), dk = t - c * (nk + 2) - 1, di = c / (nj + 2) - 1, dj = c - (di + 1) * (nj + 2) - 1;
+            const int hi = di < 0 || di >= ni, hj = dj < 0 || dj >= nj, hk = dk < 0 || dk >= nk;
+            o[u] = -1;
+            pt[u] = 0;
+            if (t >= cells || hi + hj + hk > 1 || (planar && hj)) continue;
+            const int i = lo[0] + di, j = lo[1] + dj, k = lo[2] + dk;
+            const double *q = &p(i, j, k);
+            if (i < 0) q = &p(bc.per[0] ? X - 1 : 1, j, k);
+            if (i > X) q = bc.per[0] ? (bi == 0 ? &p(1, j, k) : fx + (long)j * (Z + 1) + k) : &p(X - 1, j, k);
+            if (j < 0) q = &p(i, bc.per[1] ? Y - 1 : 1, k);
+            if (j > Y) q = bc.per[1] ? (bj == 0 ? &p(i, 1, k) : fy + (long)i * (Z + 1) + k) : &p(i, Y - 1, k);
+            if (k < 0) q = &p(i, j, bc.per[2] ? Z - 1 : 1);
+            if (k > Z) q = bc.per[2] ? (bk == 0 ? &p(i, j, 1) : fz + (long)i * (Y + 1) + j) : &p(i, j, Z - 1);
+            v[u] = *q;
+            o[u] = (di + 1) * si + (dj + 1) * sj + dk + 1;
+            if (hi + hj + hk == 0) pt[u] = 1 + (i == 1 && bc.per[0] ? 2 : 0) + (j == 1 && bc.per[1] ? 4 : 0) + (k == 1 && bc.per[2] ? 8 : 0);
         }
-        if (it == count) break;
-        target += gridDim.x;
-        if (!gs_grid_sync(sync, target, err)) return;
-        for (int s = 0; s <= X + Y + Z; ++s) {
-            const int ilo = max(0, s - Y - Z), ihi = min(X, s), jlo = max(0, s - X - Z), jhi = min(Y, s);
-            const long nj = jhi - jlo + 1, m = (long)(ihi - ilo + 1) * nj;
-            for (long t = tid; t < m; t += nt) {
-                const int i = ilo + (int)(t / nj), j = jlo + (int)(t % nj), k = s - i - j;
-                if (k < 0 || k > Z) continue;
-                p(i, j, k) = mg_update<double>(__ldcg(&p(i + 1, j, k)), __ldcg(&p(i - 1, j, k)), __ldcg(&p(i, j + 1, k)),
-                                               __ldcg(&p(i, j - 1, k)), __ldcg(&p(i, j, k + 1)), __ldcg(&p(i, j, k - 1)), r(i, j, k), kk, i, j, k);
+#pragma unroll
+        for (int u = 0; u < kGsLoads; ++u) {
+            if (o[u] < 0) continue;
+            if (bc.dirichlet || pt[u] > 1) {
+                const int t = t0 + u * blockDim.x;
+                const int c = t / (nk + 2), di = c / (nj + 2) - 1, i = lo[0] + di, j = lo[1] + c - (di + 1) * (nj + 2) - 1, k = lo[2] + t - c * (nk + 2) - 1;
+                if (i < 0 || i > X) v[u] = gs_ghost(v[u], 0, i, j, k, bc, wx, wy, wz);
+                if (j < 0 || j > Y) v[u] = gs_ghost(v[u], 1, i, j, k, bc, wx, wy, wz);
+                if (k < 0 || k > Z) v[u] = gs_ghost(v[u], 2, i, j, k, bc, wx, wy, wz);
+                // plane 1 of a periodic axis, for its last block (another one, in a later launch)
+                if (pt[u] & 2) fx[(long)j * (Z + 1) + k] = v[u];
+                if (pt[u] & 4) fy[(long)i * (Z + 1) + k] = v[u];
+                if (pt[u] & 8) fz[(long)i * (Y + 1) + j] = v[u];
             }
-            target += gridDim.x;
-            if (!gs_grid_sync(sync, target, err)) return;
+            gs_sm[o[u]] = v[u];
         }
     }
+    const int i = threadIdx.x / nj, j = threadIdx.x - i * nj, gi = lo[0] + i, gj = lo[1] + j;
+    const bool on = i < ni;
+    double *c = gs_sm + (i + 1) * si + (j + 1) * sj + 1;
+    const double *pr = &r(on ? gi : lo[0], on ? gj : lo[1], lo[2]);
+    double rv = pr[0];
+    __syncthreads();
+    const int live = (ni * nj + 31) & ~31;
+    if ((int)threadIdx.x >= live) return;   // the step barriers are the remaining warps'
+    for (int t = 0; t < ni + nj + nk - 2; ++t) {
+        const int k = t - i - j;
+        if (on && k >= 0 && k < nk) {
+            const double E = c[k + si], W = c[k - si], N = planar ? 0.0 : c[k + sj], S = planar ? 0.0 : c[k - sj], U = c[k + 1], D = c[k - 1];
+            const double v = ARITH < 0 ? mg_update<double>(E, W, N, S, U, D, rv, kk, gi, gj, lo[2] + k) : ar(E, W, N, S, U, D, rv, planar);
+            rv = pr[k + 1 < nk ? k + 1 : 0];
+            c[k] = v;
+        }
+        __syncthreads();
+    }
+    for (int t = threadIdx.x; t < ni * nj * nk; t += live) {
+        const int q = t / nk, dk = t - q * nk, di = q / nj, dj = q - di * nj;
+        p(lo[0] + di, lo[1] + dj, lo[2] + dk) = gs_sm[(di + 1) * si + (dj + 1) * sj + dk + 1];
+    }
+}
+
+// The ghosts imposeBC leaves on a level (2D: the y = 0 plane's): a thread a padded
+// point of two x planes, two y planes (x core) and two z planes (x, y core).
+__global__ void __launch_bounds__(256) k_mg_ghosts(View3<double> p, MgBC bc, const double *wx, const double *wy, const double *wz) {
+    pdl_wait();
+    const int X = bc.E[0], Y = bc.E[1], Z = bc.E[2];
+    const View3<const double> pc{p.p, {p.n[0], p.n[1], p.n[2]}, p.sx, p.sy};
+    const long fx = (long)(Y + 3) * (Z + 3), fy = (long)(X + 1) * (Z + 3), fz = (long)(X + 1) * (Y + 1);
+    long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    if (t >= 2 * (fx + fy + fz)) return;
+    int i, j, k;
+    if (t < 2 * fx) { i = t < fx ? -1 : X + 1; t %= fx; j = (int)(t / (Z + 3)) - 1; k = (int)(t % (Z + 3)) - 1; }
+    else if ((t -= 2 * fx) < 2 * fy) { j = t < fy ? -1 : Y + 1; t %= fy; i = (int)(t / (Z + 3)); k = (int)(t % (Z + 3)) - 1; }
+    else { t -= 2 * fy; k = t < fz ? -1 : Z + 1; t %= fz; i = (int)(t / (Y + 1)); j = (int)(t % (Y + 1)); }
+    if (bc.planar && j != 0) return;
+    p(i, j, k) = mg_ghost_value(pc, i, j, k, bc, wx, wy, wz);   // resolved from the core, which this launch does not write
 }
 
 // ------------------------------------------------------------------ FP64 drivers
@@ -2508,6 +2573,12 @@ static void plane_launch(Ctx &c, int mode, float *out, const float *in, const fl
     }
 }
 
+// Doubles of the planes a periodic axis's first block keeps for its last one (k_gs_blocks).
+static size_t gs_face_count(const Level &L) {
+    const size_t x = L.n[0] + 1, y = L.n[1] + 1, z = L.n[2] + 1;
+    return y * z + x * z + x * y;
+}
+
 int mg_setup(Ctx &c) {
     const saras_params &p = c.p;
     c.depth = p.vcDepth;
@@ -2574,6 +2645,7 @@ int mg_setup(Ctx &c) {
     SARAS_CUDA_TRY(cudaDeviceGetAttribute(&c.numSMs, cudaDevAttrMultiProcessorCount, c.dev));
     SARAS_CUDA_TRY(cudaFuncSetAttribute(k_mg_gs_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGsBlockSmem));
     SARAS_CUDA_TRY(cudaMemsetAsync(c.dflag, 0, 3 * sizeof(int), c.stream));
+    if (p.gsSmooth) SARAS_CUDA_TRY(cudaMalloc(&c.gsFace, sizeof(double) * gs_face_count(c.lv[0])));
     if (int e = plane_setup(c)) return e;
     c.tailLt = c.planar ? 0 : tail_level(c);   // target modes only (3D)
     if (c.tailLt > 0) {
@@ -2621,6 +2693,8 @@ void mg_free(Ctx &c) {
         cudaFree(L.a); cudaFree(L.b); cudaFree(L.r); cudaFree(L.a32); cudaFree(L.b32); cudaFree(L.r32); cudaFree(L.metBlock);
     }
     for (long long *&q : c.fx) { cudaFree(q); q = nullptr; }
+    cudaFree(c.gsFace);
+    c.gsFace = nullptr;
     c.lv.clear();
     cudaFree(c.wallX); cudaFree(c.wallY); cudaFree(c.wallZ);
     c.wallX = c.wallY = c.wallZ = nullptr;
@@ -2774,10 +2848,10 @@ static int gs_pipe(Ctx &c, int l, int count, bool zero, bool coarse, bool *ran) 
     return SARAS_OK;
 }
 
-// Gauss-Seidel smoothing of level l (reference mode with gsSmooth = 1): one
-// CTA from shared memory for levels up to kGsBlockSmem of iterate plus
-// right-hand side, else the cooperative grid kernel with one block an SM at
-// most (a stage has at most (X+1)(Y+1) points).
+// Gauss-Seidel smoothing of level l (reference mode with gsSmooth = 1): the
+// pipelined CTA where it holds the level, one CTA a sweep (k_mg_gs_block) for the
+// small levels it does not take (stretched meshes, the Dirichlet check), else the
+// wavefront of blocks.
 static int gs_smooth(Ctx &c, int l, int count, bool zero_first) {
     bool ran = false;
     if (int s = gs_pipe(c, l, count, zero_first, false, &ran)) return s;
@@ -2796,24 +2870,37 @@ static int gs_smooth(Ctx &c, int l, int count, bool zero_first) {
         return chk(c, "mg Gauss-Seidel");
     }
     if (zero_first) SARAS_CUDA_TRY(cudaMemsetAsync(L.pa(), 0, sizeof(double) * (size_t)L.count, c.stream));
-    SARAS_CUDA_TRY(cudaMemsetAsync(c.dflag, 0, sizeof(int), c.stream));   // barrier arrivals
-    const long pairs = (long)(L.n[0] + 1) * (L.n[1] + 1);
-    int blocks = (int)std::max<long>(1, std::min<long>((pairs + 255) / 256, c.numSMs));
-    unsigned *sync = reinterpret_cast<unsigned *>(c.dflag);
-    int *err = c.dflag + 1;
-    void *args[] = {&pv, &rv, &kk, &bc, &count, &sync, &err, &wx, &wy, &wz};
-    SARAS_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)k_mg_gs_grid, dim3(blocks), dim3(256), args, 0, c.stream));
+    GsBlocks g;
+    const int T = c.planar ? 32 : 8;
+    long cells = 1;
+    g.lam = 2;
+    g.stages = -2;
+    for (int d = 0; d < 3; ++d) {
+        g.T[d] = T;
+        g.nb[d] = std::max(1, L.n[d] / T);   // 2^m + 1 points: whole blocks, the last one point longer
+        g.stages += g.nb[d];
+        if (bc.per[d]) g.lam = std::max(g.lam, g.nb[d]);
+        const int most = std::min(T, L.n[d]) + 1;
+        cells *= d == 2 ? (most + 3) & ~1 : most + 2;
+    }
+    GsArith<2> a = {};
+    const int form = bc.dirichlet && c.planar ? -1 : gs_arith(c, L, a);
+    cudaError_t e = cudaSuccess;
+    for (int st = 0; st < g.stages + g.lam * (count - 1) && e == cudaSuccess; ++st) {
+        const dim3 grid(g.nb[0] * g.nb[1], count, 1);
+        auto go = [&](auto k, auto ar) {
+            ar.cx2 = a.cx2; ar.cy2 = a.cy2; ar.cz2 = a.cz2; ar.c7 = a.c7; ar.den = a.den; ar.iden = a.iden;
+            return launch_pdl(k, grid, dim3(kGsThreads), 8 * (size_t)cells, c.stream, pv, rv, kk, bc, ar, g, st, c.gsFace, wx, wy, wz);
+        };
+        e = form == 0 ? go(k_gs_blocks<0>, GsArith<0>()) : form == 1 ? go(k_gs_blocks<1>, GsArith<1>())
+          : form == 2 ? go(k_gs_blocks<2>, GsArith<2>()) : go(k_gs_blocks<-1>, GsArith<2>());
+        count_launch(c);
+    }
+    SARAS_CUDA_TRY(e);
+    const long ng = 2 * ((long)(L.n[1] + 3) * (L.n[2] + 3) + (long)(L.n[0] + 1) * (L.n[2] + 3) + (long)(L.n[0] + 1) * (L.n[1] + 1));
+    SARAS_CUDA_TRY(launch_pdl(k_mg_ghosts, dim3((unsigned)((ng + 255) / 256)), dim3(256), 0, c.stream, pv, bc, wx, wy, wz));
     count_launch(c);
     return chk(c, "mg Gauss-Seidel");
-}
-
-// Status of the Gauss-Seidel grid barriers since the last reset (synchronises).
-static int gs_status(Ctx &c) {
-    int e = 0;
-    SARAS_CUDA_TRY(cudaMemcpyAsync(&e, c.dflag + 1, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
-    SARAS_CUDA_TRY(cudaStreamSynchronize(c.stream));
-    if (e) { c.err = "Gauss-Seidel smoothing: a grid barrier wait timed out"; return SARAS_CUDA_ERROR; }
-    return SARAS_OK;
 }
 
 // ---- the reference mode's level launches in the folded forms
@@ -3296,7 +3383,6 @@ static int mg_solve_reference(Ctx &c, int *cycles, double *residual) {
             prev = res;
         }
     }
-    if (c.p.gsSmooth && (s = gs_status(c))) return s;
     // inFn.F = pressureData(0) over the padded array (poisson.cc:151)
     k_mg_output<<<grid_blocks(L0.count), 256, 0, c.stream>>>(lview<double>(L0, c.f[SARAS_FIELD_PP]), lcview<double>(L0, L0.pa()), bc0,
                                                              c.wallX, c.wallY, c.wallZ);
@@ -3720,9 +3806,7 @@ int mg_get_level(Ctx &c, int level, int which, double *host) {
 int mg_smooth_level(Ctx &c, int level, int count) {
     if (level < 0 || level > c.depth) return SARAS_BAD_ARG;
     if (level == c.depth && count < 0) return coarse_solve<double>(c, false);
-    int s = smooth<double>(c, level, count, false, false);
-    if (!s && c.p.gsSmooth) s = gs_status(c);
-    return s;
+    return smooth<double>(c, level, count, false, false);
 }
 
 int mg_restrict_level(Ctx &c, int level) {

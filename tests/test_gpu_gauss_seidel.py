@@ -17,6 +17,7 @@ NNN, PPP, PPN, NPN, PNP = (0, 0, 0), (1, 1, 1), (1, 1, 0), (0, 1, 0), (1, 0, 1)
 # grid indices, depth, periodic axes, length of the box
 GRIDS = [((3, 3, 3), 2, NNN, 1.0), ((3, 3, 3), 2, PPP, 2.0), ((4, 4, 4), 2, NNN, 1.0), ((4, 4, 4), 2, PPP, 6.28), ((5, 4, 3), 2, PPN, 1.0),
          ((3, 4, 5), 2, PNP, 3.0), ((4, 5, 3), 2, NPN, 0.7), ((5, 5, 4), 2, PPN, 2.0), ((5, 5, 5), 2, PPP, 1.0), ((5, 5, 5), 2, NNN, 1.0),
+         ((6, 5, 5), 3, NPN, 1.0), ((5, 6, 6), 3, PPP, 2.0),
          ((4, 0, 4), 2, NNN, 1.0), ((6, 0, 5), 3, NNN, 1.0), ((5, 0, 6), 2, (1, 0, 0), 1.5), ((7, 0, 7), 4, NNN, 1.0)]
 
 
@@ -42,8 +43,6 @@ def test_smoothing_sweeps(ind, depth, per, length):
     g, o = Solver(p), Oracle(p)
     rng = np.random.default_rng(7)
     for level in range(depth + 1):
-        if 2 ** (max(ind) - level) > 128:
-            continue
         for count in (1, 2, 4, 7):
             a, r = rng.standard_normal(g.level_dims(level)), rng.standard_normal(g.level_dims(level))
             for s in (g, o):
@@ -56,6 +55,32 @@ def test_smoothing_sweeps(ind, depth, per, length):
             if level < depth:
                 o.mg_restrict(level)
                 assert np.array_equal(core(g.get_level(level + 1, 1), not ind[1]), core(o.get_level(level + 1, 1), not ind[1])), (level, count)
+
+
+@pytest.mark.parametrize("make", ["ldc_d", "tgv_d", "rbc_d", "dirichlet", "2d257"])
+def test_block_wavefront(make):
+    """Levels beyond one CTA: stretched meshes, the Dirichlet check's walls and negated images, a large 2D level."""
+    if make == "2d257":
+        p = case((8, 0, 8), 6, NNN, 1.0)
+    elif make == "dirichlet":
+        p = case((5, 5, 5), 1, NNN, 1.0)
+        p.testPoisson = 1
+    else:
+        p = C.CASES[make](ind=(6, 5, 5) if make == "rbc_d" else 5, depth=1 if make != "rbc_d" else 2)
+        p.gsSmooth = 1
+        p.vcDepth = 2
+    g, o = Solver(p), Oracle(p)
+    rng = np.random.default_rng(19)
+    for level in (0, 1):
+        for count in (1, 3, 4):
+            a, r = rng.standard_normal(g.level_dims(level)), rng.standard_normal(g.level_dims(level))
+            if make == "dirichlet":          # the walls' values come with a solve
+                a[0], a[-1], a[:, 0], a[:, -1], a[:, :, 0], a[:, :, -1] = 0, 0, 0, 0, 0, 0
+            for s in (g, o):
+                s.set_level(level, 1, r)
+                s.set_level(level, 0, a)
+                s.mg_smooth(level, count)
+            assert np.array_equal(core(g.get_level(level, 0), p.yInd == 0), core(o.get_level(level, 0), p.yInd == 0)), (level, count)
 
 
 @pytest.mark.parametrize("tol", [1e-12, 1e-2, 0.3, 10.0])
