@@ -43,6 +43,11 @@ struct UC {                 // stencil constants of one field
     // xi_x of the gradient (sfield.cc:155-171) and the staggered xi_x of the
     // divergence (vfield.cc:299-320)
     const double *m1p[3], *mxp[3], *m2p[3], *gcp[3], *gsp[3];
+    // uniform meshes: the factors of each derivative folded.  1/dXi, 0.5 and the
+    // slice counts are powers of two, so moving them into the metric's factor
+    // changes no rounding: k2 = m2h ih2, k1[n] = m1 ih / 2 / (1, 2, 4 slices),
+    // kg = gm ih
+    double k2[3], k1[3][3], kg[3];
     int var, half;          // half: iScheme 1 (the 0.5 of calcDerivative2xx)
     int planar;             // 2D: the y terms are left out (vfield.cc, sfield.cc under PLANAR)
 };
@@ -57,6 +62,9 @@ static UC make_uc(const Ctx &c, int field) {
         u.m1[d] = c.m1[d];
         u.m2h[d] = (c.p.iScheme == 1) ? 0.5 * c.m2[d] : c.m2[d];
         u.gm[d] = c.m1[d];
+        u.k2[d] = u.m2h[d] * u.ih2[d];
+        for (int n = 0; n < 3; ++n) u.k1[d][n] = u.m1[d] * 0.5 * u.ih[d] / double(1 << n);
+        u.kg[d] = u.gm[d] * u.ih[d];
         const int st = f.stag[d] ? 1 : 0;
         u.m1p[d] = c.met[d][st][0];
         u.mxp[d] = c.met[d][st][1];
@@ -86,22 +94,29 @@ __device__ __forceinline__ void nbr(const View3<T> &F, int d, int i, int j, int 
 __device__ __forceinline__ double d2_at(const View3<const double> &F, int d, int i, int j, int k, const UC &u) {
     double fm, fp, f0 = F(i, j, k);
     nbr(F, d, i, j, k, fm, fp);
+    if (!u.var) return u.k2[d] * (fma(-2.0, f0, fm) + fp);   // 2 f0 is exact
     double out = (fm - 2.0 * f0 + fp) * u.ih2[d];
-    if (!u.var) return u.m2h[d] * out;
     const double tmp = ((fp - fm) * 0.5) * u.ih[d];
     const double x2 = at_axis(u.m2p[d], d, i, j, k);
     return at_axis(u.mxp[d], d, i, j, k) * tmp + (u.half ? 0.5 * x2 * out : x2 * out);
 }
 // derivative::calcDerivative1_x (derivative.cc:121-126): x_Metric*(central12n(F)*ihx)
+// divided by N, the slice count its factor was summed over (exact)
+template <int N>
 __device__ __forceinline__ double d1_at(const View3<const double> &F, int d, int i, int j, int k, const UC &u) {
     double fm, fp;
     nbr(F, d, i, j, k, fm, fp);
+    if (!u.var) return u.k1[d][N >> 1] * (fp - fm);
     double t = ((fp - fm) * 0.5) * u.ih[d];
-    return (u.var ? at_axis(u.m1p[d], d, i, j, k) : u.m1[d]) * t;
+    return (at_axis(u.m1p[d], d, i, j, k) * t) * (1.0 / N);
 }
-// gradient metric (collocated xi_x along axis C) and divergence metric (staggered xi_x along d)
-__device__ __forceinline__ double grad_m(const UC &u, int C, int i, int j, int k) { return u.var ? at_axis(u.gcp[C], C, i, j, k) : u.gm[C]; }
-__device__ __forceinline__ double div_m(const UC &u, int d, int i, int j, int k) { return u.var ? at_axis(u.gsp[d], d, i, j, k) : u.gm[d]; }
+// gradient (collocated xi_x along axis C) and divergence (staggered xi_x along d) of a difference x
+__device__ __forceinline__ double grad_of(const UC &u, int C, double x, int i, int j, int k) {
+    return u.var ? (at_axis(u.gcp[C], C, i, j, k) * x) * u.ih[C] : u.kg[C] * x;
+}
+__device__ __forceinline__ double div_of(const UC &u, int d, double x, int i, int j, int k) {
+    return u.var ? (at_axis(u.gsp[d], d, i, j, k) * x) * u.ih[d] : u.kg[d] * x;
+}
 
 // Interpolation slices (field.cc:309-575): interTemp(core) accumulated in
 // slice order.  T = 0,1,2: target Vx, Vy, Vz;  T = 3: vertex field (P, T).
@@ -165,9 +180,9 @@ struct Vel {
 // sfield.cc:113-142).  Division by the slice count (1, 2 or 4) is exact.
 template <int T>
 __device__ __forceinline__ double nlin_update(double H, const View3<const double> &F, const Vel &V, int i, int j, int k, const UC &u) {
-    H = H - (interp<T, 0>(V.v[0], i, j, k) * d1_at(F, 0, i, j, k, u)) * (1.0 / Slices<T, 0>::n);
-    if (!u.planar) H = H - (interp<T, 1>(V.v[1], i, j, k) * d1_at(F, 1, i, j, k, u)) * (1.0 / Slices<T, 1>::n);
-    H = H - (interp<T, 2>(V.v[2], i, j, k) * d1_at(F, 2, i, j, k, u)) * (1.0 / Slices<T, 2>::n);
+    H = H - interp<T, 0>(V.v[0], i, j, k) * d1_at<Slices<T, 0>::n>(F, 0, i, j, k, u);
+    if (!u.planar) H = H - interp<T, 1>(V.v[1], i, j, k) * d1_at<Slices<T, 1>::n>(F, 1, i, j, k, u);
+    H = H - interp<T, 2>(V.v[2], i, j, k) * d1_at<Slices<T, 2>::n>(F, 2, i, j, k, u);
     return H;
 }
 
@@ -180,16 +195,21 @@ __device__ __forceinline__ double diff_sum(const View3<const double> &F, int i, 
 struct Box {
     int lo[3], ext[3];
 };
+// One thread a point, the (j, k) plane numbered k fastest over blockIdx.x and the
+// planes over blockIdx.y.  Rows of 2^m + 1 (+ 2) points cut into 64-wide blocks left
+// up to half the warps with a few live lanes, which the FP64 pipe that bounds
+// these kernels charges in full (35-point rows: 70 warps a plane instead of 39).
 __device__ __forceinline__ bool box_point(const Box &b, int &i, int &j, int &k) {
-    k = b.lo[2] + blockIdx.x * blockDim.x + threadIdx.x;
-    j = b.lo[1] + blockIdx.y * blockDim.y + threadIdx.y;
-    i = b.lo[0] + blockIdx.z * blockDim.z + threadIdx.z;
-    return k < b.lo[2] + b.ext[2] && j < b.lo[1] + b.ext[1] && i < b.lo[0] + b.ext[0];
+    const int W = b.ext[2], t = blockIdx.x * blockDim.x + threadIdx.x, q = t / W;
+    k = b.lo[2] + (t - q * W);
+    j = b.lo[1] + q;
+    i = b.lo[0] + blockIdx.y;
+    return q < b.ext[1];
 }
 static void box_launch_dims(const Box &b, dim3 &grid, dim3 &block) {
-    block = dim3(64, 4, 1);
-    if (b.ext[2] <= 32) block = dim3(32, 8, 1);
-    grid = dim3((b.ext[2] + block.x - 1) / block.x, (b.ext[1] + block.y - 1) / block.y, b.ext[0]);
+    const long pts = (long)b.ext[1] * b.ext[2];
+    block = dim3(pts * b.ext[0] >= (1l << 17) ? 256 : 64, 1, 1);   // small boxes in small blocks, to spread them
+    grid = dim3((unsigned)((pts + block.x - 1) / block.x), b.ext[0], 1);
 }
 static Box core_box(const FieldInfo &f) { Box b; for (int d = 0; d < 3; ++d) { b.lo[d] = 0; b.ext[d] = f.n[d]; } return b; }
 static Box full_box(const FieldInfo &f) { Box b; for (int d = 0; d < 3; ++d) { b.lo[d] = -1; b.ext[d] = f.n[d] + 2; } return b; }
@@ -235,7 +255,7 @@ __global__ void k_gradient(View3<double> G, View3<const double> S, Box b, UC u) 
     int i, j, k;
     if (!box_point(b, i, j, k)) return;
     double sp = C == 0 ? S(i + 1, j, k) : C == 1 ? S(i, j + 1, k) : S(i, j, k + 1);
-    G(i, j, k) = (grad_m(u, C, i, j, k) * (sp - S(i, j, k))) * u.ih[C];
+    G(i, j, k) = grad_of(u, C, sp - S(i, j, k), i, j, k);
 }
 
 // vfield::divergence (vfield.cc:299-320), then optionally mgRHS *= 1/dt
@@ -262,9 +282,9 @@ __global__ void k_divergence(View3<double> D, Vel V, Box full, UC u, double scal
             D(i, j, k) = fma(fk.k[0], dx, fma(fk.k[1], dy, fk.k[2] * dz));
             return;
         }
-        double tx = (div_m(u, 0, i, j, k) * dx) * u.ih[0];
-        double ty = (div_m(u, 1, i, j, k) * dy) * u.ih[1];
-        double tz = (div_m(u, 2, i, j, k) * dz) * u.ih[2];
+        double tx = div_of(u, 0, dx, i, j, k);
+        double ty = div_of(u, 1, dy, i, j, k);
+        double tz = div_of(u, 2, dz, i, j, k);
         out = u.planar ? tx + tz : tx + ty + tz;
     }
     if (do_scale) out = out * scale;
@@ -347,8 +367,7 @@ __global__ void k_rhs(RhsArgs a) {
         h = h + a.Fb * t;
     }
     double sp = C == 0 ? a.P(i + 1, j, k) : C == 1 ? a.P(i, j + 1, k) : a.P(i, j, k + 1);
-    double g = (grad_m(u, C, i, j, k) * (sp - a.P(i, j, k))) * u.ih[C];
-    h = h - g;
+    h = h - grad_of(u, C, sp - a.P(i, j, k), i, j, k);
     h = h * a.dt;
     h = h + a.F(i, j, k);
     a.H(i, j, k) = h;
@@ -736,11 +755,11 @@ __global__ void k_cn(CnArgs a) {
                     L = (a.mx[i] * (V(i + 1, j, k) - 2.0 * v0 + V(i - 1, j, k))) * a.ihx2 +
                         (a.my[j] * (V(i, j + 1, k) - 2.0 * v0 + V(i, j - 1, k))) * a.ihy2 +
                         (a.mz[k] * (V(i, j, k + 1) - 2.0 * v0 + V(i, j, k - 1))) * a.ihz2;
-                else
-                    L = (a.lx * (V(i + 1, j, k) - 2.0 * v0 + V(i - 1, j, k))) +
-                        (a.ly * (V(i, j + 1, k) - 2.0 * v0 + V(i, j - 1, k))) +
-                        (a.lz * (V(i, j, k + 1) - 2.0 * v0 + V(i, j, k - 1)));
-                double val = v0 - L * 0.5 * a.dt * a.resCoef;
+                else   // 2 v0 is exact
+                    L = (a.lx * (fma(-2.0, v0, V(i + 1, j, k)) + V(i - 1, j, k))) +
+                        (a.ly * (fma(-2.0, v0, V(i, j + 1, k)) + V(i, j - 1, k))) +
+                        (a.lz * (fma(-2.0, v0, V(i, j, k + 1)) + V(i, j, k - 1)));
+                double val = v0 - L * (0.5 * a.dt) * a.resCoef;   // L 0.5 dt: the half exact either way
                 res = fabs(val - a.rhs(i, j, k));
                 if (res != res) res = INFINITY;   // a NaN residual never converges
             }
@@ -1064,8 +1083,7 @@ __global__ void k_project(View3<double> out, View3<const double> in, View3<const
         if (x >= 0 && y >= 0 && z >= 0 && x < in.n[0] && y < in.n[1] && z < in.n[2]) {
             double sp = C == 0 ? Pp(x + 1, y, z) : C == 1 ? Pp(x, y + 1, z) : Pp(x, y, z + 1);
             if (FAST) return fma(-fastDt, sp - Pp(x, y, z), v);
-            double g = (grad_m(u, C, x, y, z) * (sp - Pp(x, y, z))) * u.ih[C];
-            v = v - g * dt;
+            v = v - grad_of(u, C, sp - Pp(x, y, z), x, y, z) * dt;
         }
         return v;
     };
@@ -1157,9 +1175,9 @@ __global__ void k_diag(Vel V, View3<const double> T, int has_t, int nP0, int nP1
         e += (u.planar ? a * a + c * c : a * a + b * b + c * c) * dvp;
         if (has_t) w += ((V.v[2](i, j, k) + V.v[2](i, j, k - 1)) / 2.0) * T(i, j, k) * dvp;
         if (i < nc0 && j < nc1 && k < nc2) {
-            double tx = (div_m(u, 0, i, j, k) * (V.v[0](i, j, k) - V.v[0](i - 1, j, k))) * u.ih[0];
-            double ty = (div_m(u, 1, i, j, k) * (V.v[1](i, j, k) - V.v[1](i, j - 1, k))) * u.ih[1];
-            double tz = (div_m(u, 2, i, j, k) * (V.v[2](i, j, k) - V.v[2](i, j, k - 1))) * u.ih[2];
+            double tx = div_of(u, 0, V.v[0](i, j, k) - V.v[0](i - 1, j, k), i, j, k);
+            double ty = div_of(u, 1, V.v[1](i, j, k) - V.v[1](i, j - 1, k), i, j, k);
+            double tz = div_of(u, 2, V.v[2](i, j, k) - V.v[2](i, j, k - 1), i, j, k);
             dmax = fmax(dmax, u.planar ? tx + tz : tx + ty + tz);
         }
     }
