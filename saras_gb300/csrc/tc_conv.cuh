@@ -10,9 +10,14 @@
 // domain) and the B tile (N x 16 packed weights) sit in shared memory in the
 // canonical K-major layout without swizzle: 8x8 "core matrices" of 128 bytes,
 // K-adjacent core matrices 128 B apart (leading byte offset), M/N-adjacent
-// ones 256 B apart (stride byte offset).  A four-stage ring overlaps the
-// gathers with the MMAs; tcgen05.commit arrives on a per-stage mbarrier that
-// releases the stage for reuse.  The accumulator (128 lanes x N FP32 columns)
+// ones 256 B apart (stride byte offset).  A four-stage ring of three K steps a
+// stage overlaps the gathers with the MMAs (a barrier and a wait a K step bounded the
+// kernel); tcgen05.commit arrives on a per-stage mbarrier that
+// releases the stage for reuse.  The gathers' index work is a table lookup and a
+// mask a tap (each voxel's position against the faces is one set of bits), and a warp
+// gathers whole 32-byte sectors of consecutive voxels through L1, where the next
+// taps find them: 50 us for 16 -> 16 channels on 65^3 voxels (237 MB of taps), 65
+// with one K step a barrier and half-sector gathers past L1.  The accumulator (128 lanes x N FP32 columns)
 // is read back with tcgen05.ld: warp w reads lanes 32w..32w+31, i.e. thread t
 // of the CTA reads the N channels of voxel t, matching channels-last storage.
 //
@@ -29,6 +34,10 @@ namespace saras {
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, int src_bytes) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
+}
+// The same through L1: neighbouring taps read the same lines.
+__device__ __forceinline__ void cp_async16_l1(uint32_t dst, const void *src, int src_bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
@@ -98,19 +107,31 @@ struct ConvArgs {
     int *err;
 };
 
-constexpr int kConvStages = 4;
+constexpr int kConvStages = 4, kConvK = 3;   // stages of the ring, K steps a stage (27 x channel chunks is a multiple)
 constexpr int kConvTileBytesA = 128 * 16 * 2;
 
 template <int N>
-__host__ __device__ constexpr int conv_smem_bytes() { return kConvStages * (kConvTileBytesA + N * 32) + 128; }
+__host__ __device__ constexpr int conv_smem_bytes() { return kConvStages * kConvK * (kConvTileBytesA + N * 32) + 128; }
 template <int N>
 __host__ __device__ constexpr uint32_t conv_tmem_cols() { return N <= 32 ? 32u : N <= 64 ? 64u : 128u; }
+
+// Faces a voxel lies on (x low, x high, y low, y high, z low, z high; bit 6: no
+// voxel), and the faces a tap's neighbour would cross: the neighbour exists when the
+// two sets share no bit.
+__device__ __forceinline__ int conv_faces(int x, int y, int z, int W, int H, int D) {
+    return (x == 0) | (x == W - 1) << 1 | (y == 0) << 2 | (y == H - 1) << 3 | (z == 0) << 4 | (z == D - 1) << 5;
+}
+__device__ __forceinline__ int conv_crosses(int tap) {
+    const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
+    return 64 | (dx < 0) | (dx > 0) << 1 | (dy < 0) << 2 | (dy > 0) << 3 | (dz < 0) << 4 | (dz > 0) << 5;
+}
 
 template <int N>
 __global__ void __launch_bounds__(128) k_conv3d_tc(ConvArgs a) {
     static_assert(N % 16 == 0 && N >= 16 && N <= 128, "N");
     extern __shared__ __align__(128) uint8_t smem[];
-    constexpr int SB = kConvTileBytesA + N * 32;
+    __shared__ int tapOff[27], tapMask[27];
+    constexpr int SB = kConvK * (kConvTileBytesA + N * 32);
     uint64_t *mbar = reinterpret_cast<uint64_t *>(smem + kConvStages * SB);
     uint32_t *tslot = reinterpret_cast<uint32_t *>(mbar + kConvStages);
     const int tid = threadIdx.x, warp = tid >> 5;
@@ -122,36 +143,52 @@ __global__ void __launch_bounds__(128) k_conv3d_tc(ConvArgs a) {
         for (int s = 0; s < kConvStages; ++s) mbar_init(&mbar[s], 1);
         fence_mbar_init();
     }
+    if (tid >= 32 && tid < 59) {
+        const int tap = tid - 32;
+        tapOff[tap] = ((tap / 9 - 1) * a.H + (tap / 3) % 3 - 1) * a.W + tap % 3 - 1;
+        tapMask[tap] = conv_crosses(tap);
+    }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t taddr = *tslot;
 
-    // this thread's output voxel
+    // this thread's output voxel (epilogue), and the two rows it gathers half of: a pair of
+    // neighbouring threads fetches a voxel's 32 bytes, a warp 16 consecutive voxels
     const int v = blockIdx.x * 128 + tid;
     const bool valid = v < a.nvox;
-    int z = 0, y = 0, x = 0;
-    if (valid) { x = v % a.W; int t = v / a.W; y = t % a.H; z = t / a.H; }
+    int gv[2], faces[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        gv[u] = blockIdx.x * 128 + (tid >> 1) + 64 * u;
+        const int x = gv[u] % a.W, t = gv[u] / a.W, y = t % a.H, z = t / a.H;
+        faces[u] = gv[u] < a.nvox ? conv_faces(x, y, z, a.W, a.H, a.D) : 64;
+    }
+    const int half = (tid & 1) * 8;
+    const uint32_t rowA = (uint32_t)(tid >> 4) * 256 + ((tid >> 1) & 7) * 16 + (tid & 1) * 128;   // row tid / 2; row + 64: 2048 further
     const int nch0 = a.c0 >> 4, nch = (a.c0 + a.c1) >> 4;
-    const int nsteps = 27 * nch;
+    const int nsteps = 27 * nch / kConvK;
+    int tap = 0, ch = 0;   // of the next K step to load
 
-    auto load_step = [&](int s, int st) {
-        int tap = s / nch, ch = s - tap * nch;
-        int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
-        const __nv_bfloat16 *src;
-        int cs, co;
-        if (ch < nch0) { src = a.in0; cs = a.c0; co = ch << 4; }
-        else { src = a.in1; cs = a.c1; co = (ch - nch0) << 4; }
-        int zz = z + dz, yy = y + dy, xx = x + dx;
-        bool ok = valid && zz >= 0 && zz < a.D && yy >= 0 && yy < a.H && xx >= 0 && xx < a.W;
-        long sv = ok ? ((long)(zz * a.H + yy) * a.W + xx) : 0;
-        const __nv_bfloat16 *g = src + sv * cs + co;
-        uint32_t dA = su32(smem + st * SB) + (tid >> 3) * 256 + (tid & 7) * 16;
-        cp_async16(dA, g, ok ? 16 : 0);
-        cp_async16(dA + 128, g + 8, ok ? 16 : 0);
-        const uint8_t *wsrc = reinterpret_cast<const uint8_t *>(a.wpk) + (long)s * N * 32;
-        uint32_t dB = su32(smem + st * SB + kConvTileBytesA);
-        for (int q = tid; q < N * 2; q += 128) cp_async16(dB + q * 16, wsrc + q * 16, 16);
+    auto load_step = [&](int s, int st) {   // stages in order
+        const uint32_t base = su32(smem + st * SB);
+#pragma unroll
+        for (int e = 0; e < kConvK; ++e) {
+            const __nv_bfloat16 *src;
+            int cs, co;
+            if (ch < nch0) { src = a.in0; cs = a.c0; co = ch << 4; }
+            else { src = a.in1; cs = a.c1; co = (ch - nch0) << 4; }
+            const int off = tapOff[tap], mask = tapMask[tap];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const bool in = (faces[u] & mask) == 0;
+                cp_async16_l1(base + e * kConvTileBytesA + rowA + u * 2048, src + (in ? (long)(gv[u] + off) * cs + co + half : 0), in ? 16 : 0);
+            }
+            if (++ch == nch) { ch = 0; ++tap; }
+        }
+        const uint8_t *wsrc = reinterpret_cast<const uint8_t *>(a.wpk) + (long)s * kConvK * N * 32;
+        const uint32_t dB = base + kConvK * kConvTileBytesA;
+        for (int q = tid; q < kConvK * N * 2; q += 128) cp_async16(dB + q * 16, wsrc + q * 16, 16);
     };
 
     bool ok = true;
@@ -168,8 +205,10 @@ __global__ void __launch_bounds__(128) k_conv3d_tc(ConvArgs a) {
         fence_async_smem();
         if (tid == 0 && ok) {
             tc_fence_after();
-            uint32_t aAddr = su32(smem + st * SB), bAddr = aAddr + kConvTileBytesA;
-            tc_mma_bf16(taddr, smem_desc(aAddr, 128, 256), smem_desc(bAddr, 128, 256), IDESC, s > 0 ? 1u : 0u);
+            const uint32_t aAddr = su32(smem + st * SB), bAddr = aAddr + kConvK * kConvTileBytesA;
+#pragma unroll
+            for (int e = 0; e < kConvK; ++e)
+                tc_mma_bf16(taddr, smem_desc(aAddr + e * kConvTileBytesA, 128, 256), smem_desc(bAddr + e * N * 32, 128, 256), IDESC, s + e > 0 ? 1u : 0u);
             tc_commit(&mbar[st]);
         }
         const int ns = s + kConvStages - 1;
@@ -242,9 +281,7 @@ __global__ void __launch_bounds__(128) k_conv3d_tc(ConvArgs a) {
 // is one 16-byte cp.async straight from global memory.  Core matrices adjacent
 // along M (or N) are 128 B apart (the stride byte offset of a no-swizzle
 // MN-major descriptor), the two 8-voxel halves of a K step of 16 voxels
-// 16 x 128 B (A) or N / 8 x 128 B (B) apart (its leading byte offset; a first
-// build with the two exchanged read past the tile, into the reserve below, and
-// produced wrong sums, not a fault).  Each CTA reduces a chunk of voxels for one M tile
+// 16 x 128 B (A) or N / 8 x 128 B (B) apart (its leading byte offset).  Each CTA reduces a chunk of voxels for one M tile
 // into its tensor-memory accumulator and adds it to the FP32 dW with atomics;
 // the CTAs of M tile 0 also add their chunk's sum of dY to db.
 struct DwArgs {
@@ -254,27 +291,32 @@ struct DwArgs {
     float *dw;                        // [N][27][c0 + c1]
     float *db;                        // [N], or null
     int D, H, W, nvox;
-    int chunk;                        // voxels a CTA reduces (a multiple of 16)
+    int chunk;                        // voxels a CTA reduces (a multiple of kDwK)
     int *err;
 };
 
-constexpr int kDwStages = 4;
-constexpr int kDwTileA = 128 * 16 * 2;
-// Reserve: the ring is followed by 32 KB that no operand occupies, so that even
-// a descriptor read with its two byte offsets exchanged (15 x 2048 B past a
-// stage at most) stays inside the CTA's shared memory.
-constexpr int kDwReserve = 32768;
+// A stage holds kDwK voxels: kDwK / 16 K steps to a barrier.  Two neighbouring threads
+// stage one voxel's row of each of the M tile's eight pairs of channel groups (one
+// tap, 16 channels, a 32-byte sector; a warp 16 consecutive voxels), with the
+// tap's offset and face mask of each pair fixed for the whole loop and the voxel's
+// position advanced by carries.
+// (One K step of 16 voxels a barrier, two 64-bit divisions a row, half-sector gathers
+// and a serial sum for db took 162 us for 16 -> 16 channels on 65^3 voxels; this
+// takes 52, the gathers through L2 and L1 its bound.)
+constexpr int kDwStages = 4, kDwK = 64;
+constexpr int kDwTileA = 128 * 16 * 2;   // one K step
 template <int N>
-__host__ __device__ constexpr int dw_stage_bytes() { return kDwTileA + N * 32; }
+__host__ __device__ constexpr int dw_stage_bytes() { return kDwK / 16 * (kDwTileA + N * 32); }
 template <int N>
-__host__ __device__ constexpr int dw_smem_bytes() { return kDwStages * dw_stage_bytes<N>() + kDwReserve + 128; }
+__host__ __device__ constexpr int dw_smem_bytes() { return kDwStages * dw_stage_bytes<N>() + 128; }
 
 template <int N>
 __global__ void __launch_bounds__(128) k_conv_dw_tc(DwArgs a) {
     static_assert(N % 16 == 0 && N >= 16 && N <= 128, "N");
     extern __shared__ __align__(128) uint8_t smem[];
-    constexpr int SB = dw_stage_bytes<N>();
-    uint64_t *mbar = reinterpret_cast<uint64_t *>(smem + kDwStages * SB + kDwReserve);
+    __shared__ float sdb[N];
+    constexpr int SB = dw_stage_bytes<N>(), KS = kDwK / 16;
+    uint64_t *mbar = reinterpret_cast<uint64_t *>(smem + kDwStages * SB);
     uint32_t *tslot = reinterpret_cast<uint32_t *>(mbar + kDwStages);
     const int tid = threadIdx.x, warp = tid >> 5;
     constexpr uint32_t NCOLS = conv_tmem_cols<N>();
@@ -283,49 +325,60 @@ __global__ void __launch_bounds__(128) k_conv_dw_tc(DwArgs a) {
     const int mt = blockIdx.y;
     const long v0 = (long)blockIdx.x * a.chunk;
     const long v1 = min(v0 + (long)a.chunk, (long)a.nvox);
-    const int nsteps = v1 > v0 ? (int)((v1 - v0 + 15) / 16) : 0;
+    const int nsteps = v1 > v0 ? (int)((v1 - v0 + kDwK - 1) / kDwK) : 0;
 
     if (warp == 0) { tmem_alloc(tslot, NCOLS); tmem_relinquish(); }
     if (tid == 0) {
         for (int s = 0; s < kDwStages; ++s) mbar_init(&mbar[s], 1);
         fence_mbar_init();
     }
+    if (tid < N) sdb[tid] = 0.0f;
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t taddr = *tslot;
 
-    auto load_step = [&](int s, int st) {
-        const uint32_t base = su32(smem + st * SB);
-        const long vb = v0 + (long)s * 16;
+    // this thread's voxel row and its half of a pair of channel groups, eight pairs
+    const int vr = tid >> 1, r = vr & 15, half = tid & 1;
+    long v = v0 + vr;   // of the next stage to load (stages in order)
+    int x, y, z;
+    {
+        const int w = (int)min(v, (long)a.nvox - 1);   // a row past the chunk loads nothing
+        x = w % a.W;
+        const int t = w / a.W;
+        y = t % a.H;
+        z = t / a.H;
+    }
+    const int ax = kDwK % a.W, ay = (kDwK / a.W) % a.H, az = kDwK / (a.W * a.H);   // a stage's advance
+    const __nv_bfloat16 *src[8];
+    int cs[8], crosses[8];
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {   // A: 16 M groups x 16 voxel rows, two rows a thread
-            const int cidx = tid + h * 128, mg = cidx >> 4, r = cidx & 15;
-            const int m0 = mt * 128 + mg * 8;
-            const long v = vb + r;
-            const __nv_bfloat16 *src = a.in0;
-            bool ok = m0 < mtot && v < v1;
-            if (ok) {
-                const int tap = m0 / cin, c = m0 - tap * cin;
-                const int x = (int)(v % a.W);
-                const long t = v / a.W;
-                const int y = (int)(t % a.H), z = (int)(t / a.H);
-                const int zz = z + tap / 9 - 1, yy = y + (tap / 3) % 3 - 1, xx = x + tap % 3 - 1;
-                ok = zz >= 0 && zz < a.D && yy >= 0 && yy < a.H && xx >= 0 && xx < a.W;
-                if (ok) {
-                    const long sv = ((long)zz * a.H + yy) * a.W + xx;
-                    src = c < a.c0 ? a.in0 + sv * a.c0 + c : a.in1 + sv * a.c1 + (c - a.c0);
-                }
-            }
-            cp_async16(base + mg * 128 + (r & 7) * 16 + (r >> 3) * 2048, src, ok ? 16 : 0);
+    for (int h = 0; h < 8; ++h) {
+        const int m0 = mt * 128 + h * 16;
+        const int tap = min(m0 / cin, 26), c = m0 - (m0 / cin) * cin;
+        const long off = (long)((tap / 9 - 1) * a.H + (tap / 3) % 3 - 1) * a.W + tap % 3 - 1;
+        crosses[h] = m0 < mtot ? conv_crosses(tap) : -1;   // -1: past the last row, always zero
+        cs[h] = c < a.c0 ? a.c0 : a.c1;
+        src[h] = (c < a.c0 ? a.in0 + c : a.in1 + (c - a.c0)) + off * cs[h] + half * 8;   // only dereferenced at voxels whose neighbour exists
+    }
+    auto load_step = [&](int, int st) {
+        const uint32_t base = su32(smem + st * SB) + (vr >> 4) * kDwTileA + (r & 7) * 16 + (r >> 3) * 2048;
+        const int faces = v < v1 ? conv_faces(x, y, z, a.W, a.H, a.D) | 128 : 64 | 128;
+#pragma unroll
+        for (int h = 0; h < 8; ++h) {
+            const bool in = (faces & crosses[h]) == 0;
+            cp_async16_l1(base + h * 256 + half * 128, in ? src[h] + v * cs[h] : a.in0, in ? 16 : 0);
         }
-        for (int cidx = tid; cidx < N * 2; cidx += 128) {   // B: N / 8 groups x 16 voxel rows
-            const int ng = cidx >> 4, r = cidx & 15;
-            const long v = vb + r;
-            const bool ok = v < v1;
-            cp_async16(base + kDwTileA + ng * 128 + (r & 7) * 16 + (r >> 3) * (N / 8) * 128, ok ? a.dy + v * N + ng * 8 : a.dy,
-                       ok ? 16 : 0);
-        }
+        const uint32_t bb = su32(smem + st * SB) + KS * kDwTileA + (vr >> 4) * (N * 32) + (r & 7) * 16 + (r >> 3) * (N / 8) * 128;
+        const bool ok = v < v1;
+#pragma unroll
+        for (int ng = half; ng < N / 8; ng += 2) cp_async16(bb + ng * 128, ok ? a.dy + v * N + ng * 8 : a.dy, ok ? 16 : 0);
+        v += kDwK;
+        x += ax;
+        if (x >= a.W) { x -= a.W; ++y; }
+        y += ay;
+        if (y >= a.H) { y -= a.H; ++z; }
+        z += az;
     };
 
     bool ok = true;
@@ -342,10 +395,13 @@ __global__ void __launch_bounds__(128) k_conv_dw_tc(DwArgs a) {
         fence_async_smem();
         if (tid == 0 && ok) {
             tc_fence_after();
-            const uint32_t aAddr = su32(smem + st * SB), bAddr = aAddr + kDwTileA;
+            const uint32_t aAddr = su32(smem + st * SB), bAddr = aAddr + KS * kDwTileA;
             // no-swizzle MN-major: the stride byte offset steps between core
             // matrices along M / N, the leading byte offset along K
-            tc_mma_bf16(taddr, smem_desc(aAddr, 2048, 128), smem_desc(bAddr, (N / 8) * 128, 128), IDESC, s > 0 ? 1u : 0u);
+#pragma unroll
+            for (int e = 0; e < KS; ++e)
+                tc_mma_bf16(taddr, smem_desc(aAddr + e * kDwTileA, 2048, 128), smem_desc(bAddr + e * N * 32, (N / 8) * 128, 128), IDESC,
+                            s + e > 0 ? 1u : 0u);
             tc_commit(&mbar[st]);
         }
         const int ns = s + kDwStages - 1;
@@ -378,10 +434,25 @@ __global__ void __launch_bounds__(128) k_conv_dw_tc(DwArgs a) {
             }
         }
     }
-    if (a.db && mt == 0 && tid < N) {
-        float sum = 0.0f;
-        for (long v = v0; v < v1; ++v) sum += __bfloat162float(a.dy[v * N + tid]);
-        atomicAdd(&a.db[tid], sum);
+    if (a.db && mt == 0) {   // the chunk's sum of dY: a thread 8 channels of every (1024 / N)-th voxel
+        const int ng = tid % (N / 8), rows = 128 / (N / 8);
+        float sum[8] = {};
+        if (tid < rows * (N / 8)) {
+#pragma unroll 4
+            for (long w = v0 + tid / (N / 8); w < v1; w += rows) {
+                const uint4 q = *reinterpret_cast<const uint4 *>(a.dy + w * N + ng * 8);
+                const __nv_bfloat162 *p = reinterpret_cast<const __nv_bfloat162 *>(&q);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    sum[2 * e] += __low2float(p[e]);
+                    sum[2 * e + 1] += __high2float(p[e]);
+                }
+            }
+#pragma unroll
+            for (int e = 0; e < 8; ++e) atomicAdd(&sdb[ng * 8 + e], sum[e]);
+        }
+        __syncthreads();
+        if (tid < N) atomicAdd(&a.db[tid], sdb[tid]);
     }
     tc_fence_before();
     __syncthreads();

@@ -36,16 +36,31 @@ struct Grid3 {
 
 __device__ __forceinline__ float fw1(int d) { return d == 0 ? 0.5f : 0.25f; }
 
+// Eight consecutive channels (16 bytes; channel counts are multiples of 16) as floats and back.
+__device__ __forceinline__ void ld8(const bf16 *p, float (&v)[8]) {
+    const uint4 q = *reinterpret_cast<const uint4 *>(p);
+    const __nv_bfloat162 *h = reinterpret_cast<const __nv_bfloat162 *>(&q);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) { v[2 * e] = __low2float(h[e]); v[2 * e + 1] = __high2float(h[e]); }
+}
+__device__ __forceinline__ void st8(bf16 *p, const float (&v)[8]) {
+    uint4 q;
+    __nv_bfloat162 *h = reinterpret_cast<__nv_bfloat162 *>(&q);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) h[e] = __nv_bfloat162(__float2bfloat16(v[2 * e]), __float2bfloat16(v[2 * e + 1]));
+    *reinterpret_cast<uint4 *>(p) = q;
+}
+
 // Full-weighting restriction of a channels-last tensor (vertex grids, coarse
 // point i sits on fine point 2i; zero outside the fine grid), times `scale`.
-__global__ void k_pool_down(const bf16 *__restrict__ in, bf16 *__restrict__ out, int C, Grid3 f, Grid3 c, float scale) {
-    long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    long total = c.n() * C;
-    if (t >= total) return;
-    int ch = (int)(t % C);
-    long v = t / C;
-    int x = (int)(v % c.W), y = (int)((v / c.W) % c.H), z = (int)(v / ((long)c.W * c.H));
-    float s = 0.0f;
+// This kernel, the prolongation and the masked sum take eight channels a thread: one
+// channel a thread spent its time on indices (prolongation to 65^3 x 32 channels
+// 40 us for 20 MB, now 17; the loss 28 us, now 8).
+__global__ void __launch_bounds__(256) k_pool_down(const bf16 *__restrict__ in, bf16 *__restrict__ out, int C, Grid3 f, Grid3 c, float scale) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, C8 = C >> 3;
+    if (t >= (int)c.n() * C8) return;
+    const int v = t / C8, ch = (t - v * C8) * 8, q = v / c.W, x = v - q * c.W, z = q / c.H, y = q - z * c.H;
+    float s[8] = {};
     for (int dz = -1; dz <= 1; ++dz) {
         int zz = 2 * z + dz;
         if (zz < 0 || zz >= f.D) continue;
@@ -55,36 +70,66 @@ __global__ void k_pool_down(const bf16 *__restrict__ in, bf16 *__restrict__ out,
             for (int dx = -1; dx <= 1; ++dx) {
                 int xx = 2 * x + dx;
                 if (xx < 0 || xx >= f.W) continue;
-                s += fw1(dz) * fw1(dy) * fw1(dx) * __bfloat162float(in[(((long)zz * f.H + yy) * f.W + xx) * C + ch]);
+                float w[8];
+                ld8(in + (((long)zz * f.H + yy) * f.W + xx) * C + ch, w);
+                const float k = fw1(dz) * fw1(dy) * fw1(dx);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) s[e] += k * w[e];
             }
         }
     }
-    out[t] = __float2bfloat16(s * scale);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) s[e] = s[e] * scale;
+    st8(out + (long)v * C + ch, s);
 }
 
 // Trilinear vertex prolongation of a channels-last tensor, times `scale`.
-__global__ void k_pool_up(const bf16 *__restrict__ in, bf16 *__restrict__ out, int C, Grid3 c, Grid3 f, float scale) {
-    long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    long total = f.n() * C;
-    if (t >= total) return;
-    int ch = (int)(t % C);
-    long v = t / C;
-    int x = (int)(v % f.W), y = (int)((v / f.W) % f.H), z = (int)(v / ((long)f.W * f.H));
+__global__ void __launch_bounds__(256) k_pool_up(const bf16 *__restrict__ in, bf16 *__restrict__ out, int C, Grid3 c, Grid3 f, float scale) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, C8 = C >> 3;
+    if (t >= (int)f.n() * C8) return;
+    const int v = t / C8, ch = (t - v * C8) * 8, q = v / f.W, x = v - q * f.W, z = q / f.H, y = q - z * f.H;
     int x0 = x >> 1, y0 = y >> 1, z0 = z >> 1;
     int x1 = min(x0 + (x & 1), c.W - 1), y1 = min(y0 + (y & 1), c.H - 1), z1 = min(z0 + (z & 1), c.D - 1);
-    auto at = [&](int a, int b, int d) { return __bfloat162float(in[(((long)a * c.H + b) * c.W + d) * C + ch]); };
-    float s = at(z0, y0, x0) + at(z0, y0, x1) + at(z0, y1, x0) + at(z0, y1, x1) + at(z1, y0, x0) + at(z1, y0, x1) +
-              at(z1, y1, x0) + at(z1, y1, x1);
-    out[t] = __float2bfloat16(0.125f * s * scale);
+    float s[8], w[8];
+    auto at = [&](int a, int b, int d) { ld8(in + (((long)a * c.H + b) * c.W + d) * C + ch, w); };
+    auto add = [&]() {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s[e] = s[e] + w[e];
+    };
+    ld8(in + (((long)z0 * c.H + y0) * c.W + x0) * C + ch, s);
+    at(z0, y0, x1); add();
+    at(z0, y1, x0); add();
+    at(z0, y1, x1); add();
+    at(z1, y0, x0); add();
+    at(z1, y0, x1); add();
+    at(z1, y1, x0); add();
+    at(z1, y1, x1); add();
+#pragma unroll
+    for (int e = 0; e < 8; ++e) s[e] = 0.125f * s[e] * scale;
+    st8(out + (long)v * C + ch, s);
 }
 
 // out = (a + b) where mask > 0, else 0  (b and mask optional).
-__global__ void k_add_mask(const bf16 *a, const bf16 *b, const bf16 *mask, bf16 *out, long n) {
-    long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(256) k_add_mask(const bf16 *a, const bf16 *b, const bf16 *mask, bf16 *out, long n) {
+    const long t = (blockIdx.x * (long)blockDim.x + threadIdx.x) * 8;
     if (t >= n) return;
-    float v = __bfloat162float(a[t]) + (b ? __bfloat162float(b[t]) : 0.0f);
-    if (mask && !(__bfloat162float(mask[t]) > 0.0f)) v = 0.0f;
-    out[t] = __float2bfloat16(v);
+    float v[8], w[8];
+    ld8(a + t, v);
+    if (b) {
+        ld8(b + t, w);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = v[e] + w[e];
+    } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = v[e] + 0.0f;
+    }
+    if (mask) {
+        ld8(mask + t, w);
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+            if (!(w[e] > 0.0f)) v[e] = 0.0f;
+    }
+    st8(out + t, v);
 }
 
 // Pack FP32 master weights W[cout][27][cin] into the per-K-step tensor-core
@@ -230,11 +275,12 @@ __global__ void k_features(const double *rb0, const double *rb1, const double *r
 
 // Expand 3-channel FP32 features into the 16-channel BF16 network input.
 __global__ void k_expand(const float *feat, bf16 *x0, long nv) {
-    long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-    if (t >= nv * 16) return;
-    long v = t / 16;
-    int c = (int)(t % 16);
-    x0[t] = __float2bfloat16(c < 3 ? feat[v * 3 + c] : 0.0f);
+    const long v = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    if (v >= nv) return;
+    float w[8] = {feat[v * 3], feat[v * 3 + 1], feat[v * 3 + 2], 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    st8(x0 + v * 16, w);
+    w[0] = w[1] = w[2] = 0.0f;
+    st8(x0 + v * 16 + 8, w);
 }
 
 // Loss 0.5 * mean (d - d*)^2 and the output gradient (channel 0 of a 16-channel BF16 tensor).
@@ -246,8 +292,10 @@ __global__ void k_loss(const float *d, const float *dstar, bf16 *gout, long nv, 
         float r = d[v] - dstar[v];
         e = 0.5 * (double)r * r;
         float gr = r / (float)nv;
-#pragma unroll
-        for (int c = 0; c < 16; ++c) gout[v * 16 + c] = __float2bfloat16(c == 0 ? gr : 0.0f);
+        float w[8] = {gr, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+        st8(gout + v * 16, w);
+        w[0] = 0.0f;
+        st8(gout + v * 16 + 8, w);
     }
     e = warp_sum(e);
     if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = e;
@@ -451,22 +499,27 @@ static int ucheck(Ctx &c, const char *what) {
 }
 
 template <int N>
-static void launch_conv_n(const ConvArgs &a, cudaStream_t s) {
+static cudaError_t launch_conv_n(const ConvArgs &a, cudaStream_t s) {
+    cudaError_t e = cudaFuncSetAttribute(k_conv3d_tc<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, conv_smem_bytes<N>());
+    if (e != cudaSuccess) return e;
     int blocks = (a.nvox + 127) / 128;
     k_conv3d_tc<N><<<blocks, 128, conv_smem_bytes<N>(), s>>>(a);
+    return cudaGetLastError();
 }
 
 static int launch_conv(Ctx &c, int N, const ConvArgs &a) {
+    cudaError_t e;
     switch (N) {
-    case 16: launch_conv_n<16>(a, c.stream); break;
-    case 32: launch_conv_n<32>(a, c.stream); break;
-    case 48: launch_conv_n<48>(a, c.stream); break;
-    case 64: launch_conv_n<64>(a, c.stream); break;
-    case 96: launch_conv_n<96>(a, c.stream); break;
+    case 16: e = launch_conv_n<16>(a, c.stream); break;
+    case 32: e = launch_conv_n<32>(a, c.stream); break;
+    case 48: e = launch_conv_n<48>(a, c.stream); break;
+    case 64: e = launch_conv_n<64>(a, c.stream); break;
+    case 96: e = launch_conv_n<96>(a, c.stream); break;
     default: c.err = "unsupported convolution width"; return SARAS_BAD_ARG;
     }
     count_launch(c);
-    return ucheck(c, "k_conv3d_tc");
+    if (e != cudaSuccess) { c.err = std::string("k_conv3d_tc: ") + cudaGetErrorString(e); return SARAS_CUDA_ERROR; }
+    return SARAS_OK;
 }
 
 // Activation / gradient slot indices.
@@ -603,7 +656,7 @@ static ConvArgs conv_args(UNet *u, const Grid3 &g) {
 }
 
 static int pool(Ctx &c, const bf16 *in, bf16 *out, int C, const Grid3 &from, const Grid3 &to, bool down, float scale) {
-    long total = to.n() * C;
+    long total = to.n() * (C / 8);
     int blocks = (int)((total + 255) / 256);
     if (down) k_pool_down<<<blocks, 256, 0, c.stream>>>(in, out, C, from, to, scale);
     else k_pool_up<<<blocks, 256, 0, c.stream>>>(in, out, C, from, to, scale);
@@ -647,21 +700,17 @@ static int unet_forward(Ctx &c) {
 }
 
 static int add_mask(Ctx &c, const bf16 *a, const bf16 *b, const bf16 *mask, bf16 *out, long n) {
-    k_add_mask<<<(int)((n + 255) / 256), 256, 0, c.stream>>>(a, b, mask, out, n);
+    k_add_mask<<<(int)((n / 8 + 255) / 256), 256, 0, c.stream>>>(a, b, mask, out, n);
     count_launch(c);
     return ucheck(c, "add_mask");
 }
 
 // Weight and bias gradients of layer li on the tensor cores (k_conv_dw_tc):
-// voxel chunks sized for about four CTAs an SM over all M tiles.
+// voxel chunks sized for about three CTAs an SM over all M tiles.
 template <int N>
 static cudaError_t launch_dw_n(const DwArgs &a, int mtiles, cudaStream_t st) {
-    static bool attr = false;
-    if (!attr) {
-        cudaError_t e = cudaFuncSetAttribute(k_conv_dw_tc<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, dw_smem_bytes<N>());
-        if (e != cudaSuccess) return e;
-        attr = true;
-    }
+    cudaError_t e = cudaFuncSetAttribute(k_conv_dw_tc<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, dw_smem_bytes<N>());
+    if (e != cudaSuccess) return e;
     const long nch = (a.nvox + a.chunk - 1) / a.chunk;
     k_conv_dw_tc<N><<<dim3((unsigned)nch, (unsigned)mtiles), 128, dw_smem_bytes<N>(), st>>>(a);
     return cudaGetLastError();
@@ -670,8 +719,8 @@ static cudaError_t launch_dw_n(const DwArgs &a, int mtiles, cudaStream_t st) {
 static int launch_dw(Ctx &c, int N, DwArgs a) {
     const int cin = a.c0 + a.c1;
     const int mtiles = (27 * cin + 127) / 128;
-    const long want = std::max(1L, 4L * 152 / mtiles);   // voxel chunks
-    a.chunk = (int)std::max(16L, (((long)a.nvox + want - 1) / want + 15) / 16 * 16);
+    const long want = std::max(1L, 3L * 152 / mtiles);   // voxel chunks
+    a.chunk = (int)std::max((long)kDwK, (((long)a.nvox + want - 1) / want + kDwK - 1) / kDwK * kDwK);
     cudaError_t e;
     switch (N) {
     case 16: e = launch_dw_n<16>(a, mtiles, c.stream); break;
@@ -987,7 +1036,7 @@ int unet_guess(Ctx &c, const double *b, double *dst, int mode, long long *fxdst,
     if (use_net) {
         long n = u->g[0].n();
         if ((s = features(c, u->feat, nullptr))) return s;
-        k_expand<<<(int)((n * 16 + 255) / 256), 256, 0, c.stream>>>(u->feat, u->x0, n);
+        k_expand<<<(int)((n + 255) / 256), 256, 0, c.stream>>>(u->feat, u->x0, n);
         count_launch(c);
         if ((s = unet_forward(c))) return s;
         // two low-pass passes (out -> feat -> out; feat is free after the forward pass)
@@ -1060,7 +1109,7 @@ int unet_train(Ctx &c, int iters, double lr, double *loss) {
     for (int it = 0; it < iters; ++it) {
         if ((s = pack_all(c))) return s;
         const float *smp = u->samples[it % u->nsamples];
-        k_expand<<<(int)((n1 * 16 + 255) / 256), 256, 0, c.stream>>>(smp, u->x0, n1);
+        k_expand<<<(int)((n1 + 255) / 256), 256, 0, c.stream>>>(smp, u->x0, n1);
         count_launch(c);
         if ((s = unet_forward(c))) return s;
         k_loss<<<nb, 256, 0, c.stream>>>(u->out, smp + 3 * n1, u->grd[A_X0], n1, u->part);
@@ -1114,7 +1163,7 @@ int unet_grad_check(Ctx &c, const float *feat, const float *target, const float 
     SARAS_CUDA_TRY(cudaMemcpyAsync(u->feat + 3 * n1, target, sizeof(float) * n1, cudaMemcpyHostToDevice, c.stream));
     SARAS_CUDA_TRY(cudaMemsetAsync(u->err, 0, sizeof(int), c.stream));
     if ((s = pack_all(c))) return s;
-    k_expand<<<(int)((n1 * 16 + 255) / 256), 256, 0, c.stream>>>(u->feat, u->x0, n1);
+    k_expand<<<(int)((n1 + 255) / 256), 256, 0, c.stream>>>(u->feat, u->x0, n1);
     count_launch(c);
     if ((s = unet_forward(c))) return s;
     k_loss<<<nb, 256, 0, c.stream>>>(u->out, u->feat + 3 * n1, u->grd[A_X0], n1, u->part);
