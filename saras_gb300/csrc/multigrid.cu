@@ -1248,22 +1248,6 @@ static TgK<T> make_tgk(const Level &L, double omega) {
     return k;
 }
 
-// Face-ghost images of core point (i, j, k) in the target modes (put_scatter
-// without the Dirichlet cases: mirror 1 -> -1, E-1 -> E+1; periodic E-1 -> -1,
-// 1 -> E+1), inline: no device call in the caller.
-template <typename T>
-__device__ __forceinline__ void tgt_images(T *P, int sx, int sy, int i, int j, int k, T v, const MgBC &bc) {
-    const long o = (long)(i + 1) * sx + (long)(j + 1) * sy + (k + 1);
-    const int q[3] = {i, j, k};
-    const long st[3] = {sx, sy, 1};
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        int E = bc.E[d];
-        if (q[d] == 1) P[o + (long)((bc.per[d] ? E + 1 : -1) - 1) * st[d]] = v;
-        if (q[d] == E - 1) P[o + (long)((bc.per[d] ? -1 : E + 1) - (E - 1)) * st[d]] = v;
-    }
-}
-
 template <typename T>
 __device__ __noinline__ void scatter_slow(T *P, int sx, int sy, int i, int j, int k, T v, const MgBC &bc) {
     View3<T> V; V.p = P; V.sx = sx; V.sy = sy;
@@ -2127,7 +2111,7 @@ constexpr int kTailMaxLevels = 8;
 // the tail.
 constexpr int kTailIntervals = 8;
 constexpr int kTailMaxSweeps = 16;
-constexpr int kTailThreads = 1024;
+constexpr int kTailThreads = 768;   // a thread a point of the largest tail level (9^3)
 
 template <typename T>
 struct TailArgs {
@@ -2146,36 +2130,6 @@ struct TailArgs {
     long long *iters;
 };
 
-template <typename T>
-__device__ __forceinline__ int tail_count(const MgBC &b) { return (b.E[0] + 3) * (b.E[1] + 3) * (b.E[2] + 3); }
-
-// The core points (i, j, k) of an (X1 x Y1 x Z1)-point level, k fastest, that
-// thread t visits at t, t + nt, ...: the first point by division, the others
-// by adding the stride nt in mixed radix (one carry per digit at most, since
-// each digit of the stride is below its radix), so the loop body is free of
-// integer divisions.
-template <typename F>
-__device__ __forceinline__ void tail_for(int X1, int Y1, int Z1, F f) {
-    const int nt = blockDim.x, n = X1 * Y1 * Z1, YZ = Y1 * Z1;
-    int t = threadIdx.x;
-    if (t >= n) return;
-    int i = t / YZ, r = t - i * YZ, j = r / Z1, k = r - j * Z1;
-    const int di = nt / YZ, rr = nt - di * YZ, dj = rr / Z1, dk = rr - dj * Z1;
-    for (; t < n; t += nt) {
-        f(i, j, k);
-        k += dk;
-        if (k >= Z1) { k -= Z1; ++j; }
-        j += dj;
-        if (j >= Y1) { j -= Y1; ++i; }
-        i += di;
-    }
-}
-
-template <typename T>
-__device__ __forceinline__ bool near_face(int i, int j, int k, const MgBC &bc) {
-    return i <= 1 || j <= 1 || k <= 1 || i >= bc.E[0] - 1 || j >= bc.E[1] - 1 || k >= bc.E[2] - 1;
-}
-
 // The sweep constants at weight w from those at weight 1.
 template <typename T>
 __device__ __forceinline__ TgK<T> tgk_weight(const TgK<T> &c1, T w) {
@@ -2185,163 +2139,185 @@ __device__ __forceinline__ TgK<T> tgk_weight(const TgK<T> &c1, T w) {
     return c;
 }
 
-template <typename T, bool ZERO>
-__device__ void tail_sweep(T *out, const T *in, const T *r, const MgBC &bc, const TgK<T> &c) {
-    const int E1 = bc.E[1], E2 = bc.E[2], sy = E2 + 3, sx = (E1 + 3) * sy;
-    tail_for(bc.E[0] + 1, E1 + 1, E2 + 1, [&](int i, int j, int k) {
-        int o = (i + 1) * sx + (j + 1) * sy + (k + 1);
-        T v;
-        if (ZERO) v = c.ar * r[o];
-        else v = fma(c.ax, in[o - sx] + in[o + sx], fma(c.ay, in[o + sy] + in[o - sy], fma(c.az, in[o + 1] + in[o - 1], fma(c.ar, r[o], c.om1 * in[o]))));
-        out[o] = v;
-        if (near_face<T>(i, j, k, bc)) tgt_images(out, sx, sy, i, j, k, v, bc);
-    });
-    __syncthreads();
+// A thread's point of a tail level: its position, its offset in the level's compact
+// core arrays (k fastest) and its neighbours' offsets, through their images at a
+// face.  Found once a level and direction; a sweep is then eight loads, its
+// arithmetic and one store.
+struct TailPt {
+    bool on;
+    int i, j, k, o, e, w, n, s, u, d;
+};
+__device__ __forceinline__ int tail_points(const MgBC &b) { return (b.E[0] + 1) * (b.E[1] + 1) * (b.E[2] + 1); }
+__device__ __forceinline__ TailPt tail_pt(const MgBC &b) {
+    TailPt p;
+    const int W = b.E[2] + 1, P = (b.E[1] + 1) * W, t = threadIdx.x;
+    p.on = t < tail_points(b);
+    p.o = p.on ? t : 0;
+    p.i = p.o / P;
+    const int r = p.o - p.i * P;
+    p.j = r / W;
+    p.k = r - p.j * W;
+    p.e = p.o + (pad_img(p.i + 1, b.E[0], b.per[0]) - p.i) * P;
+    p.w = p.o + (pad_img(p.i - 1, b.E[0], b.per[0]) - p.i) * P;
+    p.n = p.o + (pad_img(p.j + 1, b.E[1], b.per[1]) - p.j) * W;
+    p.s = p.o + (pad_img(p.j - 1, b.E[1], b.per[1]) - p.j) * W;
+    p.u = p.o + pad_img(p.k + 1, b.E[2], b.per[2]) - p.k;
+    p.d = p.o + pad_img(p.k - 1, b.E[2], b.per[2]) - p.k;
+    return p;
 }
 
+// What bounds it: the dependent steps of one CTA, about a dozen a level, each a
+// barrier, shared-memory loads and (FP64) a few pipe turns.  With padded arrays in
+// thread-private pointer tables, ghost copies and index arithmetic in every step it took
+// the FP32 tail took 24.5 us on 9^3 and 5^3, and a 65^3 mixed step (three cycles)
+// 634 us; in this form 608, a 257^3 step (four) 4.32 ms instead of 4.35 (the FP64
+// tail's time is its pipe's: unchanged).
 template <typename T>
-__global__ void __launch_bounds__(kTailThreads) k_mg_tail(TailArgs<T> a) {
-    pdl_wait();
+__global__ void __launch_bounds__(kTailThreads) k_mg_tail(const __grid_constant__ TailArgs<T> a) {
     extern __shared__ unsigned char smraw[];
-    T *base = reinterpret_cast<T *>(smraw);
-    T *P[kTailMaxLevels], *Q[kTailMaxLevels], *R[kTailMaxLevels];
-    {
-        T *q = base;
-        for (int l = 0; l < a.nl; ++l) {
-            int n = tail_count<T>(a.bc[l]);
-            P[l] = q; Q[l] = q + n; R[l] = q + 2 * n;
-            q += 3 * n;
-        }
-    }
+    T *const base = reinterpret_cast<T *>(smraw);
     const int tid = threadIdx.x, nt = blockDim.x;
-    for (int t = tid; t < tail_count<T>(a.bc[0]); t += nt) R[0][t] = a.rin[t];
+    // level l's array `which` (0, 1: the iterates; 2: the right-hand side); the iterate is array (sweeps so far) mod 2
+    auto arr = [&](int l, int which) -> T * {
+        int o = 0;
+        for (int m = 0; m < l; ++m) o += 3 * tail_points(a.bc[m]);
+        return base + o + which * tail_points(a.bc[l]);
+    };
+    TailPt p = tail_pt(a.bc[0]);
+    const int pad0 = (a.bc[0].E[1] + 3) * (a.bc[0].E[2] + 3), pad1 = a.bc[0].E[2] + 3;
+    const long og = (long)(p.i + 1) * pad0 + (p.j + 1) * pad1 + (p.k + 1);
+    pdl_wait();
+    T r = a.rin[og];
+    if (p.on) arr(0, 2)[p.o] = r;
     __syncthreads();
     for (int l = 0; l + 1 < a.nl; ++l) {
         const MgBC &bc = a.bc[l];
-        int E1 = bc.E[1], E2 = bc.E[2], sy = E2 + 3, sx = (E1 + 3) * sy;
+        if (l > 0) {
+            p = tail_pt(bc);
+            r = arr(l, 2)[p.o];
+        }
         // pre-smoothing from zero (the first sweep ignores its input)
         for (int n = 0; n < a.pre; ++n) {
-            const TgK<T> cw = tgk_weight(a.tk[l], a.wpre[n]);
-            if (n == 0) tail_sweep<T, true>(Q[l], P[l], R[l], bc, cw);
-            else tail_sweep<T, false>(Q[l], P[l], R[l], bc, cw);
-            T *x = P[l]; P[l] = Q[l]; Q[l] = x;
+            const TgK<T> c = tgk_weight(a.tk[l], a.wpre[n]);
+            const T *in = arr(l, n & 1);
+            T *out = arr(l, (n & 1) ^ 1);
+            T v;
+            if (n == 0) v = c.ar * r;
+            else v = fma(c.ax, in[p.w] + in[p.e], fma(c.ay, in[p.n] + in[p.s], fma(c.az, in[p.u] + in[p.d], fma(c.ar, r, c.om1 * in[p.o]))));
+            if (p.on) out[p.o] = v;
+            __syncthreads();
         }
-        // residual into Q (core), then full-weighting restriction (k_tgt_restrict's
+        // residual into the other array, then full-weighting restriction (k_tgt_restrict's
         // separable form; fine positions outside the core at their images)
         const TgK<T> &c = a.tr[l];
-        {
-            const T *p = P[l], *rr = R[l];
-            T *qq = Q[l];
-            tail_for(bc.E[0] + 1, E1 + 1, E2 + 1, [&](int i, int j, int k) {
-                int o = (i + 1) * sx + (j + 1) * sy + (k + 1);
-                T lap = fma(c.lx, p[o - sx] + p[o + sx], fma(c.ly, p[o + sy] + p[o - sy], fma(c.lz, p[o + 1] + p[o - 1], c.lc * p[o])));
-                qq[o] = rr[o] - lap;
-            });
-        }
+        const T *in = arr(l, a.pre & 1);
+        T *res = arr(l, (a.pre & 1) ^ 1);
+        const T lap = fma(c.lx, in[p.w] + in[p.e], fma(c.ly, in[p.n] + in[p.s], fma(c.lz, in[p.u] + in[p.d], c.lc * in[p.o])));
+        if (p.on) res[p.o] = r - lap;
         __syncthreads();
-        const MgBC &bcc = a.bc[l + 1];
-        int C1 = bcc.E[1], C2 = bcc.E[2], csy = C2 + 3, csx = (C1 + 3) * csy;
-        {
-            const T *qf = Q[l];
-            T *rc = R[l + 1];
-            tail_for(bcc.E[0] + 1, C1 + 1, C2 + 1, [&](int I, int J, int K) {
-                int oj[3], ok[3];
+        const TailPt q = tail_pt(a.bc[l + 1]);
+        if (q.on) {
+            const int W = bc.E[2] + 1, P = (bc.E[1] + 1) * W;
+            int oj[3], ok[3];
 #pragma unroll
-                for (int q = 0; q < 3; ++q) {
-                    oj[q] = (pad_img(2 * J - 1 + q, E1, bc.per[1]) + 1) * sy;
-                    ok[q] = pad_img(2 * K - 1 + q, E2, bc.per[2]) + 1;
-                }
-                T acc = (T)0;
+            for (int e = 0; e < 3; ++e) {
+                oj[e] = pad_img(2 * q.j - 1 + e, bc.E[1], bc.per[1]) * W;
+                ok[e] = pad_img(2 * q.k - 1 + e, bc.E[2], bc.per[2]);
+            }
+            T acc = (T)0;
 #pragma unroll
-                for (int q = 0; q < 3; ++q) {
-                    const T *pl = qf + (pad_img(2 * I - 1 + q, bc.E[0], bc.per[0]) + 1) * sx;
-                    T row[3];
+            for (int e = 0; e < 3; ++e) {
+                const T *pl = res + pad_img(2 * q.i - 1 + e, bc.E[0], bc.per[0]) * P;
+                T row[3];
 #pragma unroll
-                    for (int w = 0; w < 3; ++w) {
-                        const T *pr = pl + oj[w];
-                        row[w] = pr[ok[0]] + (T)2 * pr[ok[1]] + pr[ok[2]];
-                    }
-                    T sp = row[0] + (T)2 * row[1] + row[2];
-                    acc += q == 1 ? (T)2 * sp : sp;
-                }
-                rc[(I + 1) * csx + (J + 1) * csy + (K + 1)] = acc * (T)0.015625;
-            });
+                for (int w = 0; w < 3; ++w) row[w] = pl[oj[w] + ok[0]] + (T)2 * pl[oj[w] + ok[1]] + pl[oj[w] + ok[2]];
+                const T sp = row[0] + (T)2 * row[1] + row[2];
+                acc += e == 1 ? (T)2 * sp : sp;
+            }
+            arr(l + 1, 2)[q.o] = acc * (T)0.015625;
         }
         __syncthreads();
     }
-    // coarsest level: e = M r with the precomputed solution operator (one warp
-    // per row, the core right-hand side gathered into a compact vector first),
-    // else Gauss-Seidel to tol
+    // coarsest level: e = M r with the precomputed solution operator (a warp four
+    // rows at a time, their loads together), else Gauss-Seidel to tol
     {
-        int L = a.nl - 1;
+        const int L = a.nl - 1;
         const MgBC &bc = a.bc[L];
-        for (int t = tid; t < tail_count<T>(bc); t += nt) P[L][t] = (T)0;
+        T *e = arr(L, 0), *rl = arr(L, 2);
         if (a.M) {
-            int Y = bc.E[1], Z = bc.E[2], sy = Z + 3, sx = (Y + 3) * sy;
-            T *rv = Q[L];
-            const T *rl = R[L];
-            tail_for(bc.E[0] + 1, Y + 1, Z + 1, [&](int i, int j, int k) {
-                rv[(i * (Y + 1) + j) * (Z + 1) + k] = rl[(i + 1) * sx + (j + 1) * sy + (k + 1)];
-            });
-            __syncthreads();
-            int lane = tid & 31;
-            for (int row = tid >> 5; row < a.nM; row += nt >> 5) {
-                const T *m = a.M + (long)row * a.nM;
-                T s = (T)0;
-                for (int q = lane; q < a.nM; q += 32) s = fma(m[q], rv[q], s);
-                s = warp_sum(s);
-                if (lane == 0) {
-                    int k = row % (Z + 1), j = (row / (Z + 1)) % (Y + 1), i = row / ((Z + 1) * (Y + 1));
-                    P[L][(i + 1) * sx + (j + 1) * sy + (k + 1)] = s;
+            const int lane = tid & 31, nw = nt >> 5;
+            for (int row0 = tid >> 5; row0 < a.nM; row0 += 4 * nw) {
+                T s[4] = {(T)0, (T)0, (T)0, (T)0};
+                for (int q = lane; q < a.nM; q += 32) {
+                    const T x = rl[q];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (row0 + u * nw < a.nM) s[u] = fma(a.M[(long)(row0 + u * nw) * a.nM + q], x, s[u]);
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    s[u] = warp_sum(s[u]);
+                    if (lane == 0 && row0 + u * nw < a.nM) e[row0 + u * nw] = s[u];
                 }
             }
+        } else {   // padded copies after the levels' arrays
+            const int X = bc.E[0], Y = bc.E[1], Z = bc.E[2], N = (X + 3) * (Y + 3) * (Z + 3), sy = Z + 3, sx = (Y + 3) * sy;
+            T *pp = arr(L, 3), *pr = pp + N;
+            const TailPt q = tail_pt(bc);
+            const int o = (q.i + 1) * sx + (q.j + 1) * sy + q.k + 1;
+            for (int t = tid; t < N; t += nt) pp[t] = pr[t] = (T)0;
             __syncthreads();
-        } else {
+            if (q.on) pr[o] = rl[q.o];
             __syncthreads();
-            if (tid < 32) coarse_rbgs_warp(P[L], R[L], bc.E[0], bc.E[1], bc.E[2], a.kkc, bc, a.tol, a.maxc, a.iters);
+            if (tid < 32) coarse_rbgs_warp(pp, pr, X, Y, Z, a.kkc, bc, a.tol, a.maxc, a.iters);
             __syncthreads();
+            if (q.on) e[q.o] = pp[o];
         }
+        __syncthreads();
     }
     // back up: prolongation + add, post-smoothing
     for (int l = a.nl - 2; l >= 0; --l) {
         const MgBC &bc = a.bc[l], &bcc = a.bc[l + 1];
-        int E1 = bc.E[1], E2 = bc.E[2], sy = E2 + 3, sx = (E1 + 3) * sy;
-        T *pf = P[l];
-        View3<const T> C; C.p = P[l + 1]; C.sy = bcc.E[2] + 3; C.sx = (bcc.E[1] + 3) * C.sy;
-        tail_for(bc.E[0] + 1, E1 + 1, E2 + 1, [&](int i, int j, int k) {
-            int i2 = i / 2, j2 = j / 2, k2 = k / 2;
-            bool io = i & 1, jo = j & 1, ko = k & 1;
+        p = tail_pt(bc);
+        r = arr(l, 2)[p.o];
+        const int sy = bcc.E[2] + 1, sx = (bcc.E[1] + 1) * sy;
+        {
+            const T *c = arr(l + 1, l + 1 == a.nl - 1 ? 0 : (a.pre + a.post) & 1) + (p.i >> 1) * sx + (p.j >> 1) * sy + (p.k >> 1);
+            const bool io = p.i & 1, jo = p.j & 1, ko = p.k & 1;
             T v;
             if (io) {
                 if (jo) {
-                    if (ko) v = (C(i2, j2, k2) + C(i2 + 1, j2, k2) + C(i2, j2 + 1, k2) + C(i2, j2, k2 + 1) + C(i2 + 1, j2 + 1, k2) +
-                                 C(i2 + 1, j2, k2 + 1) + C(i2, j2 + 1, k2 + 1) + C(i2 + 1, j2 + 1, k2 + 1)) * (T)0.125;
-                    else v = (C(i2, j2, k2) + C(i2, j2 + 1, k2) + C(i2 + 1, j2, k2) + C(i2 + 1, j2 + 1, k2)) * (T)0.25;
+                    if (ko) v = (c[0] + c[sx] + c[sy] + c[1] + c[sx + sy] + c[sx + 1] + c[sy + 1] + c[sx + sy + 1]) * (T)0.125;
+                    else v = (c[0] + c[sy] + c[sx] + c[sx + sy]) * (T)0.25;
                 } else {
-                    if (ko) v = (C(i2, j2, k2) + C(i2, j2, k2 + 1) + C(i2 + 1, j2, k2) + C(i2 + 1, j2, k2 + 1)) * (T)0.25;
-                    else v = (C(i2, j2, k2) + C(i2 + 1, j2, k2)) * (T)0.5;
+                    if (ko) v = (c[0] + c[1] + c[sx] + c[sx + 1]) * (T)0.25;
+                    else v = (c[0] + c[sx]) * (T)0.5;
                 }
             } else {
                 if (jo) {
-                    if (ko) v = (C(i2, j2, k2) + C(i2, j2, k2 + 1) + C(i2, j2 + 1, k2) + C(i2, j2 + 1, k2 + 1)) * (T)0.25;
-                    else v = (C(i2, j2, k2) + C(i2, j2 + 1, k2)) * (T)0.5;
+                    if (ko) v = (c[0] + c[1] + c[sy] + c[sy + 1]) * (T)0.25;
+                    else v = (c[0] + c[sy]) * (T)0.5;
                 } else {
-                    if (ko) v = (C(i2, j2, k2) + C(i2, j2, k2 + 1)) * (T)0.5;
-                    else v = C(i2, j2, k2);
+                    if (ko) v = (c[0] + c[1]) * (T)0.5;
+                    else v = c[0];
                 }
             }
-            int o = (i + 1) * sx + (j + 1) * sy + (k + 1);
-            v = v + pf[o];
-            pf[o] = v;
-            if (near_face<T>(i, j, k, bc)) tgt_images(pf, sx, sy, i, j, k, v, bc);
-        });
+            if (p.on) {
+                T *f = arr(l, a.pre & 1) + p.o;
+                *f = v + *f;
+            }
+        }
         __syncthreads();
         for (int m = 0; m < a.post; ++m) {
-            tail_sweep<T, false>(Q[l], P[l], R[l], bc, tgk_weight(a.tk[l], a.wpost[m]));
-            T *x = P[l]; P[l] = Q[l]; Q[l] = x;
+            const TgK<T> c = tgk_weight(a.tk[l], a.wpost[m]);
+            const T *in = arr(l, (a.pre + m) & 1);
+            T *out = arr(l, (a.pre + m + 1) & 1);
+            const T v = fma(c.ax, in[p.w] + in[p.e], fma(c.ay, in[p.n] + in[p.s], fma(c.az, in[p.u] + in[p.d], fma(c.ar, r, c.om1 * in[p.o]))));
+            if (p.on) out[p.o] = v;
+            __syncthreads();
         }
     }
-    for (int t = tid; t < tail_count<T>(a.bc[0]); t += nt) a.pout[t] = P[0][t];
+    if (p.on) a.pout[og] = arr(0, (a.pre + a.post) & 1)[p.o];   // the core: the level kernels read images by index
 }
 
 // ------------------------------------------------------------------ host
@@ -3093,8 +3069,9 @@ static int tail_run(Ctx &c, int Lt) {
         a.bc[q] = level_bc(c, Lt + q, true);
         a.tk[q] = make_tgk<T>(L, 1.0);
         a.tr[q] = make_tgk<T>(L, 1.0);
-        smem += 3 * sizeof(T) * (size_t)L.count;
+        smem += 3 * sizeof(T) * (size_t)(L.n[0] + 1) * (L.n[1] + 1) * (L.n[2] + 1);
     }
+    if (!c.coarseN) smem += 2 * sizeof(T) * (size_t)c.lv[c.depth].count;
     a.kkc = make_k(c.lv[c.depth]);
     a.M = nullptr;
     a.nM = c.coarseN;
