@@ -747,27 +747,26 @@ __global__ void k_mg_gs_block(View3<double> pg, View3<const double> rg, MgK kk, 
 // sweep before and continued by coarse_gs, which tests every point.
 struct GsPlan {
     int lam, Q, threads;    // stages between sweeps, sweeps of a column apart, compute threads (a multiple of 32)
+    // Doubles from one column to the next: Z + 1 points and, in the coarsest solve,
+    // the idle steps of a period (full_step writes there); even, so that the
+    // points that neighbouring columns update in one step (a column less one
+    // point apart) fall in different banks (a 9^3 level's 1001 sweeps: 4.89 ms, packed 5.08).
+    int zp;
     int rsmem;              // the right-hand side in shared memory too
     size_t smem;
 };
 
-// Doubles from one column to the next: Z + 1 is odd, and one more makes the
-// distance between the points that neighbouring columns update in one step (a
-// column less one point) odd, so a warp's accesses fall in different banks (a
-// 9^3 level's 1001 sweeps: 4.89 ms, packed columns 5.08).
-__host__ __device__ inline int gs_pitch(int Z) { return Z + 2; }
-
 // The CTA's step barrier, from the compute and the witness loops alike.
 __device__ __forceinline__ void gs_step_sync() { asm volatile("barrier.sync 0;" ::: "memory"); }
 
-// `M` pipelined sweeps on P (core points, columns gs_pitch apart); `alarm` (CHECK):
+// `M` pipelined sweeps on P (core points, columns zp apart); `alarm` (CHECK):
 // set to the first sweep none of whose witness points is at or above tol.  The
 // compute warps and the witness warp run loops of the same steps; *alarm is
 // written in step 7 of 16 and read after step 15, so that all leave together.
 template <class A, bool PLANAR, bool RS, bool CHECK>
 __device__ __forceinline__ void gs_pipe_run(double *P, const double *R, long rsx, long rsy, double *gx, double *gy, int X, int Y, int Z,
-                                            const MgBC &bc, const A &ar, const MgK &kk, int lam, int Q, int M, double tol, int *alarm) {
-    const int W1 = Y + 1, zp = gs_pitch(Z), nc = (X + 1) * W1;
+                                            const MgBC &bc, const A &ar, const MgK &kk, int lam, int Q, int zp, int M, double tol, int *alarm) {
+    const int W1 = Y + 1, nc = (X + 1) * W1;
     const int steps = (M - 1) * lam + X + Y + Z + 1;
     if (CHECK && threadIdx.x >= blockDim.x - 32) {
         // the witness points: interior, on the hyperplane sw
@@ -892,11 +891,11 @@ __device__ __forceinline__ void gs_pipe_run(double *P, const double *R, long rsx
 
 template <int ARITH, bool PLANAR, bool RS, bool COARSE>
 __global__ void __launch_bounds__(1024) k_gs_pipe(View3<double> pg, View3<const double> rg, MgK kk, MgBC bc, GsArith<ARITH> ar, int lam,
-                                                  int Q, int count, int zero, double tol, int maxCount, long long *iters) {
+                                                  int Q, int zp, int count, int zero, double tol, int maxCount, long long *iters) {
     pdl_wait();
     extern __shared__ unsigned char smraw[];
     __shared__ int alarm;
-    const int X = bc.E[0], Y = bc.E[1], Z = bc.E[2], W1 = Y + 1, zp = gs_pitch(Z), n = (X + 1) * W1 * zp;
+    const int X = bc.E[0], Y = bc.E[1], Z = bc.E[2], W1 = Y + 1, n = (X + 1) * W1 * zp;
     double *P = reinterpret_cast<double *>(smraw), *gx = P + n, *gy = gx + W1 * zp, *R = gy + (PLANAR ? 0 : (X + 1) * zp);
     const long o0 = rg.off(0, 0, 0);
     for (int t = threadIdx.x; t < n; t += blockDim.x) {
@@ -908,7 +907,7 @@ __global__ void __launch_bounds__(1024) k_gs_pipe(View3<double> pg, View3<const 
     if (threadIdx.x == 0) alarm = -1;
     __syncthreads();
     const double *r = RS ? R : rg.p + o0;
-    gs_pipe_run<GsArith<ARITH>, PLANAR, RS, COARSE>(P, r, rg.sx, rg.sy, gx, gy, X, Y, Z, bc, ar, kk, lam, Q, count, tol, &alarm);
+    gs_pipe_run<GsArith<ARITH>, PLANAR, RS, COARSE>(P, r, rg.sx, rg.sy, gx, gy, X, Y, Z, bc, ar, kk, lam, Q, zp, count, tol, &alarm);
     if (COARSE) {
         const int stop = alarm;
         if (stop >= 0) {
@@ -916,7 +915,7 @@ __global__ void __launch_bounds__(1024) k_gs_pipe(View3<double> pg, View3<const 
             for (int t = threadIdx.x; t < n; t += blockDim.x) P[t] = 0.0;
             __syncthreads();
             if (stop > 0)
-                gs_pipe_run<GsArith<ARITH>, PLANAR, RS, false>(P, r, rg.sx, rg.sy, gx, gy, X, Y, Z, bc, ar, kk, lam, Q, stop, tol, nullptr);
+                gs_pipe_run<GsArith<ARITH>, PLANAR, RS, false>(P, r, rg.sx, rg.sy, gx, gy, X, Y, Z, bc, ar, kk, lam, Q, zp, stop, tol, nullptr);
             const int N = (X + 3) * (Y + 3) * (Z + 3), sy = Z + 3, sx = (Y + 3) * sy;
             double *pp = R + (RS ? n : 0), *rr = pp + N;
             for (int t = threadIdx.x; t < N; t += blockDim.x) { pp[t] = 0.0; rr[t] = rg.p[t]; }
@@ -2168,7 +2167,7 @@ __device__ __forceinline__ TailPt tail_pt(const MgBC &b) {
 
 // What bounds it: the dependent steps of one CTA, about a dozen a level, each a
 // barrier, shared-memory loads and (FP64) a few pipe turns.  With padded arrays in
-// thread-private pointer tables, ghost copies and index arithmetic in every step it took
+// thread-private pointer tables, ghost copies and index arithmetic in every step
 // the FP32 tail took 24.5 us on 9^3 and 5^3, and a 65^3 mixed step (three cycles)
 // 634 us; in this form 608, a 257^3 step (four) 4.32 ms instead of 4.35 (the FP64
 // tail's time is its pipe's: unchanged).
@@ -2764,13 +2763,9 @@ static int gs_arith(const Ctx &c, const Level &L, GsArith<2> &a) {
 static bool gs_plan(const Ctx &c, const Level &L, const MgBC &bc, int form, int count, bool coarse, GsPlan &g) {
     if (bc.dirichlet || form < 0) return false;
     const int X = L.n[0], Y = c.planar ? 0 : L.n[1], Z = L.n[2];
-    const long nc = (long)(X + 1) * (Y + 1), zp = gs_pitch(Z), n = nc * zp;
+    const long nc = (long)(X + 1) * (Y + 1);
     const size_t cap = 220 * 1024;
-    size_t smem = 8 * (size_t)(n + (Y + 1) * zp + (c.planar ? 0 : (X + 1) * zp));
-    if (coarse) smem += 8 * (size_t)(n + 2 * L.count);
-    if (smem > cap || nc > 992) return false;
-    g.rsmem = coarse || smem + 8 * (size_t)n <= cap;
-    g.smem = smem + (!coarse && g.rsmem ? 8 * (size_t)n : 0);
+    if (nc > 992) return false;
     int lmin = 2;
     for (int d = 0; d < 3; ++d)
         if (bc.per[d]) lmin = std::max(lmin, L.n[d]);
@@ -2781,10 +2776,21 @@ static bool gs_plan(const Ctx &c, const Level &L, const MgBC &bc, int form, int 
         const int Q = std::min((Z + 1 + lam - 1) / lam, count);
         const long th = (nc * Q + 31) / 32 * 32;
         if (th + (coarse ? 32 : 0) > 1024) continue;
+        const long zp = (std::max(Z + 2, coarse ? lam * Q : 0) + 1) & ~1, n = nc * zp;
+        size_t smem = 8 * (size_t)(n + (Y + 1) * zp + (c.planar ? 0 : (X + 1) * zp));
+        if (coarse) smem += 8 * (size_t)(n + 2 * L.count);
+        if (smem > cap) continue;
         const long q4 = (th / 32 + (coarse ? 1 : 0) + 3) / 4;
         const double step = 90.0 + ops * (q4 > 1 ? 76.0 * q4 : 64.0);
         const double cost = step * ((count - 1.0) * lam + X + Y + Z + 1);
-        if (g.Q == 0 || cost < best) { best = cost; g.lam = lam; g.Q = Q; g.threads = (int)th; }
+        if (g.Q && cost >= best) continue;
+        best = cost;
+        g.lam = lam;
+        g.Q = Q;
+        g.zp = (int)zp;
+        g.threads = (int)th;
+        g.rsmem = coarse || smem + 8 * (size_t)n <= cap;
+        g.smem = smem + (!coarse && g.rsmem ? 8 * (size_t)n : 0);
     }
     return g.Q > 0;
 }
@@ -2793,13 +2799,13 @@ template <int ARITH, bool COARSE>
 static cudaError_t gs_pipe_launch(Ctx &c, Level &L, const MgBC &bc, const GsArith<2> &a, const GsPlan &g, int count, bool zero) {
     GsArith<ARITH> ar;
     ar.cx2 = a.cx2; ar.cy2 = a.cy2; ar.cz2 = a.cz2; ar.c7 = a.c7; ar.den = a.den; ar.iden = a.iden;
-    void (*k)(View3<double>, View3<const double>, MgK, MgBC, GsArith<ARITH>, int, int, int, int, double, int, long long *);
+    void (*k)(View3<double>, View3<const double>, MgK, MgBC, GsArith<ARITH>, int, int, int, int, int, double, int, long long *);
     if (COARSE || g.rsmem) k = c.planar ? k_gs_pipe<ARITH, true, true, COARSE> : k_gs_pipe<ARITH, false, true, COARSE>;
     else k = c.planar ? k_gs_pipe<ARITH, true, false, false> : k_gs_pipe<ARITH, false, false, false>;
     cudaError_t e = cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem);
     if (e != cudaSuccess) return e;
     return launch_pdl(k, dim3(1), dim3(g.threads + (COARSE ? 32 : 0)), g.smem, c.stream, lview<double>(L, L.pa()), lcview<double>(L, L.r), make_k(L), bc,
-                      ar, g.lam, g.Q, count, zero ? 1 : 0, c.p.mgTolerance, c.maxCount, (long long *)(c.dscal + 40));
+                      ar, g.lam, g.Q, g.zp, count, zero ? 1 : 0, c.p.mgTolerance, c.maxCount, (long long *)(c.dscal + 40));
 }
 
 // `count` lexicographic sweeps of level l (coarse: the coarsest solve) in one
