@@ -302,14 +302,14 @@ __global__ void k_divergence(View3<double> D, Vel V, Box full, UC u, double scal
 struct DivDf {
     fpair k[3];
 };
-constexpr int kProjMarch = 8;   // points per thread along i (divergence, projection)
+constexpr int kProjMarch = 8;   // points per thread along i at most (divergence, projection)
 
-__global__ void __launch_bounds__(256) k_divergence_df(View3<double> D, Vel V, Box full, DivDf q) {
+__global__ void __launch_bounds__(256) k_divergence_df(View3<double> D, Vel V, Box full, DivDf q, int march) {
     int k = full.lo[2] + blockIdx.x * 32 + threadIdx.x;
     int j = full.lo[1] + blockIdx.y * 8 + threadIdx.y;
-    int i0 = full.lo[0] + blockIdx.z * kProjMarch;
+    int i0 = full.lo[0] + blockIdx.z * march;
     if (k >= full.lo[2] + full.ext[2] || j >= full.lo[1] + full.ext[1]) return;
-    int iend = min(i0 + kProjMarch, full.lo[0] + full.ext[0]);
+    int iend = min(i0 + march, full.lo[0] + full.ext[0]);
     bool jk = j >= 0 && k >= 0 && j < D.n[1] && k < D.n[2];
     double xm = 0.0;
     bool have = false;   // xm holds Vx(i-1)
@@ -445,6 +445,7 @@ struct Rhs3Args {
     const double *T;           // buoyancy: T, in P's layout
     float *n0h[3], *n0l[3];    // A of each component, component layouts
     int nu[3];                 // union of the cores
+    int march;                 // planes a CTA marches: kRhs3March, fewer on small grids (march_planes)
     int edgeK;                 // nu[2] - 1 when it is a multiple of 32 (the tiles then end below it), else -1
     int buoyancy;
     Rhs3K q[3];
@@ -560,8 +561,8 @@ __global__ void __launch_bounds__(256, 5) k_rhs_df3(Rhs3Args a) {
         rhs3_point<2, ISO>(a, G, i, j, k);
         return;
     }
-    const int k0 = blockIdx.x * 32, j0 = blockIdx.y * 8, i0 = blockIdx.z * kRhs3March;
-    const int iend = min(i0 + kRhs3March, a.nu[0]);
+    const int k0 = blockIdx.x * 32, j0 = blockIdx.y * 8, i0 = blockIdx.z * a.march;
+    const int iend = min(i0 + a.march, a.nu[0]);
     int js[2], ks[2];
     bool lt[2];
 #pragma unroll
@@ -601,6 +602,17 @@ __global__ void __launch_bounds__(256, 5) k_rhs_df3(Rhs3Args a) {
         rhs3_point<1, ISO>(a, G, i, j, k);
         rhs3_point<2, ISO>(a, G, i, j, k);
     }
+}
+
+// Planes a CTA of a marching kernel takes along i: `most`, halved (down to 2) while
+// the grid of `tiles` (j, k) tiles would give the SMs fewer than three CTAs each.  A
+// marching CTA waits for each plane's loads in turn, so a grid of less than a wave
+// lasts as long as its longest march: at 65^3 the right-hand side took 80 us
+// in 135 CTAs of 16 planes, 36 in 459 of 4, which load half as many halo planes again.
+static int march_planes(const Ctx &c, long tiles, int planes, int most) {
+    int m = most;
+    while (m > 2 && tiles * ((planes + m - 1) / m) < 3L * c.numSMs) m /= 2;
+    return m;
 }
 
 // The constants of every component have the isotropic form rhs3_point's ISO
@@ -665,6 +677,13 @@ __global__ void k_bc_apply(View3<double> out, View3<const double> in, BcProgram 
 // took 0.187 ms a Jacobi solve and 0.279 ms a projection, against 0.191 and
 // 0.289 with 64 and 0.192 and 0.289 with 1024).
 constexpr int kShellBlocks = 256;
+// Blocks a slab on a box: no more than hold its largest face's points (a 65^3
+// field's 1536 blocks, most of them empty, took a shell kernel 8 us).
+static int shell_blocks(const Box &b) {
+    long most = 1;
+    for (int d = 0; d < 3; ++d) most = std::max(most, (long)b.ext[(d + 1) % 3] * b.ext[(d + 2) % 3]);
+    return (int)std::min<long>(kShellBlocks, (most + 255) / 256);
+}
 
 // k_bc_apply in place (copy_bulk = 0) over the non-bulk points only, as six
 // disjoint slabs (blockIdx.y: along axis d = slab / 2 the points below / above
@@ -1100,7 +1119,7 @@ __global__ void k_project(View3<double> out, View3<const double> in, View3<const
 // resolves the program on the remaining points of the full box.
 template <int C>
 __global__ void __launch_bounds__(256) k_project_bulk(View3<double> out, View3<const double> in, View3<const double> Pp, BcProgram prog,
-                                                      double fastDt) {
+                                                      double fastDt, int march) {
     // one thread per (j, k) column of the bulk, numbered k fastest over the
     // whole bulk plane (256 a block, blockIdx.y the segment): 32-wide tiles
     // would leave warps with one active lane on rows of 2^m + 1 points, which
@@ -1108,9 +1127,9 @@ __global__ void __launch_bounds__(256) k_project_bulk(View3<double> out, View3<c
     const int W = prog.bhi[2] - prog.blo[2] + 1, t = blockIdx.x * 256 + threadIdx.x, jj = t / W;
     int k = prog.blo[2] + (t - jj * W);
     int j = prog.blo[1] + jj;
-    int i0 = prog.blo[0] + blockIdx.y * kProjMarch;
+    int i0 = prog.blo[0] + blockIdx.y * march;
     if (j > prog.bhi[1]) return;
-    int iend = min(i0 + kProjMarch - 1, prog.bhi[0]);
+    int iend = min(i0 + march - 1, prog.bhi[0]);
     bool jk = j < in.n[1] && k < in.n[2];
     double pc = Pp(i0, j, k);
     for (int i = i0; i <= iend; ++i) {
@@ -1489,7 +1508,7 @@ static int apply_program(Ctx &c, int field, const BcProgram &prog) {
         // Programs of fields without a scratch partner only copy from core
         // points that no op targets (syncData), so they run in place, on the
         // non-bulk points alone.
-        k_bc_apply_shell<<<dim3(kShellBlocks, 6), 256, 0, c.stream>>>(mview(c, field), cview(c, field), prog, fb);
+        k_bc_apply_shell<<<dim3(shell_blocks(fb), 6), 256, 0, c.stream>>>(mview(c, field), cview(c, field), prog, fb);
         count_launch(c);
     }
     return check_launch(c, "k_bc_apply");
@@ -1588,8 +1607,10 @@ int vfield_divergence(Ctx &c, double *dst, bool scale_dt) {
     if (c.p.fastKernels == 2 && !(scale_dt && c.p.testPoisson)) {
         DivDf q;
         for (int d = 0; d < 3; ++d) { q.k[d].h = (float)fk.k[d]; q.k[d].l = (float)(fk.k[d] - (double)q.k[d].h); }
-        dim3 gd((fb.ext[2] + 31) / 32, (fb.ext[1] + 7) / 8, (fb.ext[0] + kProjMarch - 1) / kProjMarch);
-        k_divergence_df<<<gd, dim3(32, 8), 0, c.stream>>>(D, make_vel(c), fb, q);
+        dim3 gd((fb.ext[2] + 31) / 32, (fb.ext[1] + 7) / 8, 1);
+        const int march = march_planes(c, (long)gd.x * gd.y, fb.ext[0], kProjMarch);
+        gd.z = (fb.ext[0] + march - 1) / march;
+        k_divergence_df<<<gd, dim3(32, 8), 0, c.stream>>>(D, make_vel(c), fb, q, march);
     } else {
         k_divergence<<<g, bl, 0, c.stream>>>(D, make_vel(c), fb, u, 1.0 / c.dt, scale_dt ? 1 : 0,
                                              (scale_dt && c.p.testPoisson) ? 1 : 0, c.p.fastKernels != 0, fk);
@@ -1745,8 +1766,9 @@ int compute_rhs(Ctx &c) {
                 a3.buoyancy = a.buoyancy;
                 // rows of 32 m + 1 points: m tiles of 32 and one block column for the last point
                 a3.edgeK = (a3.nu[2] > 32 && (a3.nu[2] - 1) % 32 == 0) ? a3.nu[2] - 1 : -1;
-                dim3 gr(a3.edgeK >= 0 ? a3.edgeK / 32 + 1 : (a3.nu[2] + 31) / 32, (a3.nu[1] + 7) / 8,
-                        (a3.nu[0] + kRhs3March - 1) / kRhs3March);
+                dim3 gr(a3.edgeK >= 0 ? a3.edgeK / 32 + 1 : (a3.nu[2] + 31) / 32, (a3.nu[1] + 7) / 8, 1);
+                a3.march = march_planes(c, (long)gr.x * gr.y, a3.nu[0], kRhs3March);
+                gr.z = (a3.nu[0] + a3.march - 1) / a3.march;
                 if (rhs3_iso(a3)) k_rhs_df3<true><<<gr, dim3(32, 8, 1), 0, c.stream>>>(a3);
                 else k_rhs_df3<false><<<gr, dim3(32, 8, 1), 0, c.stream>>>(a3);
                 count_launch(c);
@@ -1824,7 +1846,7 @@ static int cn_solve_delta(Ctx &c, int comp, int field, const CnFast &fa, double 
     // N0): its non-bulk points from their boundary-program sources, in place.
     d.dh = d.oh = n0h;
     d.dl = d.ol = n0l;
-    k_cn_delta_shell<false, true><<<dim3(kShellBlocks, 6), 256, 0, c.stream>>>(d);
+    k_cn_delta_shell<false, true><<<dim3(shell_blocks(d.full), 6), 256, 0, c.stream>>>(d);
     count_launch(c);
     // The iterates: A (read only), then alternately P and Q.
     float *const bufs[3][2] = {{n0h, n0l}, {dA, dAl}, {dB, dBl}};
@@ -1844,10 +1866,10 @@ static int cn_solve_delta(Ctx &c, int comp, int field, const CnFast &fa, double 
         prof_begin(c, PK_CN, 0);
         if (vout) {
             k_cn_delta<true><<<gm, bm, 0, c.stream>>>(d);
-            k_cn_delta_shell<true, false><<<dim3(kShellBlocks, 6), 256, 0, c.stream>>>(d);
+            k_cn_delta_shell<true, false><<<dim3(shell_blocks(d.full), 6), 256, 0, c.stream>>>(d);
         } else {
             k_cn_delta<false><<<gm, bm, 0, c.stream>>>(d);
-            k_cn_delta_shell<false, false><<<dim3(kShellBlocks, 6), 256, 0, c.stream>>>(d);
+            k_cn_delta_shell<false, false><<<dim3(shell_blocks(d.full), 6), 256, 0, c.stream>>>(d);
         }
         count_launch(c, 2);
         prof_end(c, PK_CN, 0, vout ? bytes * 4.0 / 3.0 : bytes);
@@ -2031,12 +2053,13 @@ int project(Ctx &c, bool with_bc) {
         int wb = with_bc ? 1 : 0;
         if (c.p.fastKernels && with_bc) {
             const BcProgram &pg = f.full;
-            dim3 gb((unsigned)(((long)(pg.bhi[2] - pg.blo[2] + 1) * (pg.bhi[1] - pg.blo[1] + 1) + 255) / 256),
-                    (pg.bhi[0] - pg.blo[0] + 1 + kProjMarch - 1) / kProjMarch);
-            dim3 gs(kShellBlocks, 6);
-            if (q == 0) { k_project_bulk<0><<<gb, 256, 0, c.stream>>>(out, in, Pp, pg, fdt); k_project_shell<0><<<gs, 256, 0, c.stream>>>(out, in, Pp, pg, fb, fdt); }
-            if (q == 1) { k_project_bulk<1><<<gb, 256, 0, c.stream>>>(out, in, Pp, pg, fdt); k_project_shell<1><<<gs, 256, 0, c.stream>>>(out, in, Pp, pg, fb, fdt); }
-            if (q == 2) { k_project_bulk<2><<<gb, 256, 0, c.stream>>>(out, in, Pp, pg, fdt); k_project_shell<2><<<gs, 256, 0, c.stream>>>(out, in, Pp, pg, fb, fdt); }
+            dim3 gb((unsigned)(((long)(pg.bhi[2] - pg.blo[2] + 1) * (pg.bhi[1] - pg.blo[1] + 1) + 255) / 256), 1);
+            const int march = march_planes(c, gb.x, pg.bhi[0] - pg.blo[0] + 1, kProjMarch);
+            gb.y = (pg.bhi[0] - pg.blo[0] + 1 + march - 1) / march;
+            dim3 gs(shell_blocks(fb), 6);
+            if (q == 0) { k_project_bulk<0><<<gb, 256, 0, c.stream>>>(out, in, Pp, pg, fdt, march); k_project_shell<0><<<gs, 256, 0, c.stream>>>(out, in, Pp, pg, fb, fdt); }
+            if (q == 1) { k_project_bulk<1><<<gb, 256, 0, c.stream>>>(out, in, Pp, pg, fdt, march); k_project_shell<1><<<gs, 256, 0, c.stream>>>(out, in, Pp, pg, fb, fdt); }
+            if (q == 2) { k_project_bulk<2><<<gb, 256, 0, c.stream>>>(out, in, Pp, pg, fdt, march); k_project_shell<2><<<gs, 256, 0, c.stream>>>(out, in, Pp, pg, fb, fdt); }
             count_launch(c);
         } else if (c.p.fastKernels) {
             if (q == 0) k_project<0, true><<<g, bl, 0, c.stream>>>(out, in, Pp, f.full, fb, u, c.dt, wb, fdt);
