@@ -1281,10 +1281,32 @@ static void col_dims(const Level &L, dim3 &g, dim3 &b) {
     b = dim3(kColBlock, 1, 1);
     g = dim3((unsigned)((cols + kColBlock - 1) / kColBlock), (L.n[0] + 1 + kIch - 1) / kIch, 1);
 }
+// Planes a thread of an FP64 launch marches: kIch, and kShort where columns of kIch
+// leave fewer than four blocks a SM.  A warp's FP64 instructions follow one
+// another at the pipe's rate of one in 64 clocks, so a level that does not fill
+// the SMs takes as long as one thread's planes: a 33^3 sweep 8.5 us in
+// columns of eight, 4.5 of two (17^3 8.3 -> 4.4, its restriction 12.6 -> 6.2); a plain 257^3
+// step 15.35 -> 14.63 ms.
+constexpr int kShort = 2;
+static bool short_march(const Ctx &c, const Level &L) {
+    const long cols = (long)(L.n[1] + 1) * (L.n[2] + 1);
+    return (cols + kColBlock - 1) / kColBlock * ((L.n[0] + kIch) / kIch) < 4L * c.numSMs;
+}
+// Launch shape of a level's target-mode kernels; the planes of a march returned.
 template <typename T>
-static void level_dims(const Level &L, dim3 &g, dim3 &b) {
-    if (sizeof(T) == 8) col_dims(L, g, b);
-    else march_dims(L, g, b);
+static int level_dims(const Ctx &c, const Level &L, dim3 &g, dim3 &b) {
+    if (sizeof(T) == 4) { march_dims(L, g, b); return kIch; }
+    col_dims(L, g, b);
+    if (!short_march(c, L)) return kIch;
+    g.y = (L.n[0] + kShort) / kShort;
+    return kShort;
+}
+// f(integral_constant of a march length of level_dims<T>)
+template <typename T, typename F>
+static auto with_march(int ch, F f) {
+    if constexpr (sizeof(T) == 8)
+        if (ch == kShort) return f(std::integral_constant<int, kShort>());
+    return f(std::integral_constant<int, kIch>());
 }
 // The (j, k) column and plane segment of this thread under the launch shape
 // of level_dims (COL: columns); false outside the core.
@@ -1339,26 +1361,26 @@ __device__ __forceinline__ long nbr_x(int i, int d, int sx, const MgBC &bc) {
 // 32 the compiler picks unbounded (46.5 us against 49.0 a level-0 sweep at
 // 257^3; 4 and 5 blocks measured 48.7 and 47.4).  FP64 sweeps wait on the
 // FP64 pipe instead; five blocks leave them the registers they took unbounded.
-template <typename T, bool ZERO>
+template <typename T, bool ZERO, int CH>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 6 : 5) k_tgt_sweep(T *__restrict__ out, const T *__restrict__ in, const T *__restrict__ r,
                                                    int sx, int sy, MgBC bc, TgK<T> c) {
     pdl_wait();
     int j, k, seg;
     if (!col_of<sizeof(T) == 8>(bc, j, k, seg)) return;
-    const int i0 = seg * kIch;
-    int n = min(kIch, bc.E[0] - i0 + 1);
+    const int i0 = seg * CH;
+    int n = min(CH, bc.E[0] - i0 + 1);
     const NbrJK nb = nbr_jk(j, k, sy, bc);
     const long o0 = (long)(i0 + 1) * sx + (long)(j + 1) * sy + (k + 1);
     T cm = (T)0, cc = (T)0;
     if (!ZERO) { cm = in[o0 + nbr_x(i0, -1, sx, bc)]; cc = in[o0]; }
-    // a full column segment (its planes i0 + 1 .. i0 + kIch are core planes):
+    // a full column segment (its planes i0 + 1 .. i0 + CH are core planes):
     // every load of the segment issued before the first store (the loads are
     // independent of the stores, and issuing them together keeps enough bytes
     // in flight for HBM), then the updates
-    if (n == kIch && i0 + kIch <= bc.E[0]) {
-        T nc[kIch + 1], ns[kIch], ud[kIch], rr[kIch];
+    if (n == CH && i0 + CH <= bc.E[0]) {
+        T nc[CH + 1], ns[CH], ud[CH], rr[CH];
 #pragma unroll
-        for (int q = 0; q < kIch; ++q) {
+        for (int q = 0; q < CH; ++q) {
             long o = o0 + (long)q * sx;
             nc[q + 1] = ZERO ? (T)0 : in[o + sx];
             ns[q] = ZERO ? (T)0 : in[o + nb.yp] + in[o + nb.ym];
@@ -1367,7 +1389,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 6 : 5) k_tgt_sweep(T *__
         }
         nc[0] = cc;
 #pragma unroll
-        for (int q = 0; q < kIch; ++q) {
+        for (int q = 0; q < CH; ++q) {
             T v;
             if (ZERO) v = c.ar * rr[q];
             else v = fma(c.ax, cm + nc[q + 1], fma(c.ay, ns[q], fma(c.az, ud[q], fma(c.ar, rr[q], c.om1 * nc[q]))));
@@ -1445,14 +1467,14 @@ __global__ void __launch_bounds__(256, 6) k_tgt_sweep2z(T *__restrict__ out, con
 // is written).  A thread owns a fine (j, k)
 // column and marches fine planes in pairs: the coarse plane m interpolated to
 // (j, k) serves fine plane 2m and, averaged with plane m+1, fine plane 2m+1.
-template <typename T>
+template <typename T, int CH>
 __global__ void __launch_bounds__(256) k_tgt_prolong_add(T *__restrict__ pf, const T *__restrict__ pc, int sxf, int syf, int sxc, int syc,
                                                          MgBC bc) {
     pdl_wait();
     int j, k, seg;
     if (!col_of<sizeof(T) == 8>(bc, j, k, seg)) return;
-    const int i0 = seg * kIch;   // kIch is even
-    int iend = min(i0 + kIch - 1, bc.E[0]);
+    const int i0 = seg * CH;   // CH is even
+    int iend = min(i0 + CH - 1, bc.E[0]);
     int k2 = k >> 1, j2 = j >> 1;
     bool ko = k & 1, jo = j & 1;
     auto A = [&](int m) -> T {   // coarse plane m at (j, k)
@@ -1463,16 +1485,16 @@ __global__ void __launch_bounds__(256) k_tgt_prolong_add(T *__restrict__ pf, con
         return (T)0.5 * (v0 + v1);
     };
     long o = (long)(i0 + 1) * sxf + (long)(j + 1) * syf + (k + 1);
-    if (iend - i0 + 1 == kIch) {
+    if (iend - i0 + 1 == CH) {
         // a full segment: every load issued before the first store (the coarse
-        // plane i0 / 2 + kIch / 2 is at most the coarse core's last plane)
-        T a[kIch / 2 + 1], v[kIch];
+        // plane i0 / 2 + CH / 2 is at most the coarse core's last plane)
+        T a[CH / 2 + 1], v[CH];
 #pragma unroll
-        for (int q = 0; q <= kIch / 2; ++q) a[q] = A((i0 >> 1) + q);
+        for (int q = 0; q <= CH / 2; ++q) a[q] = A((i0 >> 1) + q);
 #pragma unroll
-        for (int q = 0; q < kIch; ++q) v[q] = pf[o + q * (long)sxf];
+        for (int q = 0; q < CH; ++q) v[q] = pf[o + q * (long)sxf];
 #pragma unroll
-        for (int q = 0; q < kIch; ++q) pf[o + q * (long)sxf] = v[q] + ((q & 1) ? (T)0.5 * (a[q >> 1] + a[(q >> 1) + 1]) : a[q >> 1]);
+        for (int q = 0; q < CH; ++q) pf[o + q * (long)sxf] = v[q] + ((q & 1) ? (T)0.5 * (a[q >> 1] + a[(q >> 1) + 1]) : a[q >> 1]);
         return;
     }
     T am = A(i0 >> 1);
@@ -1487,23 +1509,23 @@ __global__ void __launch_bounds__(256) k_tgt_prolong_add(T *__restrict__ pf, con
 }
 
 // r_out = b - Lap(p) over the core; optional max |r| (FP64 accumulation).
-template <typename T, typename OT, bool MAXRED>
+template <typename T, typename OT, bool MAXRED, int CH>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 6 : 5) k_tgt_residual(OT *__restrict__ out, const T *__restrict__ p, const T *__restrict__ b,
                                                       int sx, int sy, MgBC bc, TgK<T> c, double *maxres) {
     pdl_wait();
     int j, k, seg;
     const bool on = col_of<sizeof(T) == 8>(bc, j, k, seg);
-    const int i0 = seg * kIch;
+    const int i0 = seg * CH;
     unsigned long long m = 0ull;
-    if (!MAXRED && on && i0 + kIch <= bc.E[0]) {
+    if (!MAXRED && on && i0 + CH <= bc.E[0]) {
         // a full column segment (as in k_tgt_sweep): every load before the first store
         const NbrJK nb = nbr_jk(j, k, sy, bc);
         const long o0 = (long)(i0 + 1) * sx + (long)(j + 1) * sy + (k + 1);
-        T nc[kIch + 1], ns[kIch], ud[kIch], rr[kIch];
+        T nc[CH + 1], ns[CH], ud[CH], rr[CH];
         T cm = p[o0 + nbr_x(i0, -1, sx, bc)];
         nc[0] = p[o0];
 #pragma unroll
-        for (int q = 0; q < kIch; ++q) {
+        for (int q = 0; q < CH; ++q) {
             long o = o0 + (long)q * sx;
             nc[q + 1] = p[o + sx];
             ns[q] = p[o + nb.yp] + p[o + nb.ym];
@@ -1511,7 +1533,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 6 : 5) k_tgt_residual(OT
             rr[q] = b[o];
         }
 #pragma unroll
-        for (int q = 0; q < kIch; ++q) {
+        for (int q = 0; q < CH; ++q) {
             T lap = fma(c.lx, cm + nc[q + 1], fma(c.ly, ns[q], fma(c.lz, ud[q], c.lc * nc[q])));
             out[o0 + (long)q * sx] = (OT)(rr[q] - lap);
             cm = nc[q];
@@ -1519,7 +1541,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 6 : 5) k_tgt_residual(OT
         return;
     }
     if (on) {
-        int iend = min(i0 + kIch - 1, bc.E[0]);
+        int iend = min(i0 + CH - 1, bc.E[0]);
         const NbrJK nb = nbr_jk(j, k, sy, bc);
         long o = (long)(i0 + 1) * sx + (long)(j + 1) * sy + (k + 1);
         T cm = p[o + nbr_x(i0, -1, sx, bc)], cc = p[o];
@@ -1730,13 +1752,13 @@ constexpr int rr_ch() { return sizeof(T) == 8 ? 4 : 8; }
 // with the compiler's unbounded choice of 32 registers).
 
 
-template <typename T>
+template <typename T, int CH>
 __global__ void __launch_bounds__(256, 4) k_tgt_restrict(T *__restrict__ rc, const T *__restrict__ r, int sx, int sy, int csx, int csy,
                                                        MgBC bcf) {
     pdl_wait();
     const int E0 = bcf.E[0], E1 = bcf.E[1], E2 = bcf.E[2];
     const int W = E2 / 2 + 1, t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int J = t / W, K = t - J * W, I0 = blockIdx.y * rr_ch<T>();
+    const int J = t / W, K = t - J * W, I0 = blockIdx.y * CH;
     if (J > E1 / 2) return;
     long oj[3];
     int ok[3];
@@ -1755,7 +1777,7 @@ __global__ void __launch_bounds__(256, 4) k_tgt_restrict(T *__restrict__ rc, con
         }
         return row[0] + (T)2 * row[1] + row[2];
     };
-    const int Iend = min(I0 + rr_ch<T>() - 1, E0 / 2);
+    const int Iend = min(I0 + CH - 1, E0 / 2);
     T lo = plane(2 * I0 - 1);
 #pragma unroll 2
     for (int I = I0; I <= Iend; ++I) {
@@ -2926,7 +2948,13 @@ static int smooth(Ctx &c, int l, int count, bool zero_first, bool tgt) {
     int pk = sizeof(T) == 8 ? PK_MG_SMOOTH64 : PK_MG_SMOOTH32;
     double bytes = 3.0 * sizeof(T) * (double)(L.n[0] + 1) * (L.n[1] + 1) * (L.n[2] + 1);
     int sx = (L.n[1] + 3) * (L.n[2] + 3), sy = L.n[2] + 3;
-    dim3 gm, bm; level_dims<T>(L, gm, bm);
+    dim3 gm, bm;
+    const int ch = level_dims<T>(c, L, gm, bm);
+    auto sweep = [&](auto zero, const TgK<T> &tk) {
+        return with_march<T>(ch, [&](auto m) {
+            return launch_pdl(k_tgt_sweep<T, decltype(zero)::value, decltype(m)::value>, gm, bm, 0, c.stream, B_<T>(L), A_<T>(L), R_<T>(L), sx, sy, bc, tk);
+        });
+    };
     for (int n = 0; n < count; ++n) {
         TgK<T> tk = make_tgk<T>(L, tgt ? smooth_weight(c, n, count) : c.p.jacobiWeight);
         prof_begin(c, pk, l);
@@ -2944,11 +2972,11 @@ static int smooth(Ctx &c, int l, int count, bool zero_first, bool tgt) {
                     continue;
                 }
             }
-            if (n == 0 && zero_first) SARAS_CUDA_TRY(launch_pdl(k_tgt_sweep<T, true>, gm, bm, 0, c.stream, B_<T>(L), A_<T>(L), R_<T>(L), sx, sy, bc, tk));
+            if (n == 0 && zero_first) SARAS_CUDA_TRY(sweep(std::true_type(), tk));
             else if constexpr (sizeof(T) == 4) {
                 if (l == 0 && c.planeOk) plane_launch(c, 0, B_<T>(L), A_<T>(L), R_<T>(L), bc, tk);
-                else SARAS_CUDA_TRY(launch_pdl(k_tgt_sweep<T, false>, gm, bm, 0, c.stream, B_<T>(L), A_<T>(L), R_<T>(L), sx, sy, bc, tk));
-            } else SARAS_CUDA_TRY(launch_pdl(k_tgt_sweep<T, false>, gm, bm, 0, c.stream, B_<T>(L), A_<T>(L), R_<T>(L), sx, sy, bc, tk));
+                else SARAS_CUDA_TRY(sweep(std::false_type(), tk));
+            } else SARAS_CUDA_TRY(sweep(std::false_type(), tk));
         } else if (n == 0 && zero_first)
             SARAS_CUDA_TRY(ref_sweep<true>(c, L, bc));
         else
@@ -3002,7 +3030,8 @@ static int restrict_level(Ctx &c, int l, bool tgt) {
     prof_begin(c, pk, l);
     if (tgt) {
         int sx = (L.n[1] + 3) * (L.n[2] + 3), sy = L.n[2] + 3;
-        dim3 gm, bm; level_dims<T>(L, gm, bm);
+        dim3 gm, bm;
+        const int ch = level_dims<T>(c, L, gm, bm);
         bool planed = false;
         if constexpr (sizeof(T) == 4) {
             if (l == 0 && c.planeOk) {
@@ -3011,16 +3040,19 @@ static int restrict_level(Ctx &c, int l, bool tgt) {
             }
         }
         if (!planed)
-            SARAS_CUDA_TRY(launch_pdl(k_tgt_residual<T, T, false>, gm, bm, 0, c.stream, B_<T>(L), A_<T>(L), R_<T>(L), sx, sy, bcf,
-                                      make_tgk<T>(L, 1.0), (double *)nullptr));
+            SARAS_CUDA_TRY(with_march<T>(ch, [&](auto m) {
+                return launch_pdl(k_tgt_residual<T, T, false, decltype(m)::value>, gm, bm, 0, c.stream, B_<T>(L), A_<T>(L), R_<T>(L), sx, sy, bcf,
+                                  make_tgk<T>(L, 1.0), (double *)nullptr);
+            }));
         count_launch(c);
         prof_end(c, pk, l, 3.0 * sizeof(T) * pts);
         pk = sizeof(T) == 8 ? PK_MG_RESTRICT64 : PK_MG_RESTRICT32;
         prof_begin(c, pk, l);
         int csx = (C.n[1] + 3) * (C.n[2] + 3), csy = C.n[2] + 3;
         long ccols = (long)(C.n[1] + 1) * (C.n[2] + 1);
-        dim3 gr((unsigned)((ccols + 255) / 256), (C.n[0] + 1 + rr_ch<T>() - 1) / rr_ch<T>(), 1);
-        SARAS_CUDA_TRY(launch_pdl(k_tgt_restrict<T>, gr, dim3(256, 1, 1), 0, c.stream, R_<T>(C), B_<T>(L), sx, sy, csx, csy, bcf));
+        const int rch = ch == kIch ? rr_ch<T>() : 1;   // coarse planes of a march
+        dim3 gr((unsigned)((ccols + 255) / 256), (C.n[0] + 1 + rch - 1) / rch, 1);
+        SARAS_CUDA_TRY(launch_pdl(ch == kIch ? k_tgt_restrict<T, rr_ch<T>()> : k_tgt_restrict<T, 1>, gr, dim3(256, 1, 1), 0, c.stream, R_<T>(C), B_<T>(L), sx, sy, csx, csy, bcf));
         count_launch(c);
         prof_end(c, pk, l, sizeof(T) * pts * (1.0 + 1.0 / 8.0));
         return chk(c, "mg restrict");
@@ -3046,10 +3078,13 @@ static int prolong_level(Ctx &c, int l, bool tgt, bool add) {
     double pts = (double)(L.n[0] + 1) * (L.n[1] + 1) * (L.n[2] + 1);
     prof_begin(c, pk, l);
     if (tgt && add) {   // the core only: target-mode kernels read face neighbours at their images
-        dim3 gm, bm; level_dims<T>(L, gm, bm);
+        dim3 gm, bm;
+        const int ch = level_dims<T>(c, L, gm, bm);
         int sx = (L.n[1] + 3) * (L.n[2] + 3), sy = L.n[2] + 3;
-        SARAS_CUDA_TRY(launch_pdl(k_tgt_prolong_add<T>, gm, bm, 0, c.stream, A_<T>(L), A_<T>(C), sx, sy, (C.n[1] + 3) * (C.n[2] + 3),
-                                  C.n[2] + 3, bc));
+        SARAS_CUDA_TRY(with_march<T>(ch, [&](auto m) {
+            return launch_pdl(k_tgt_prolong_add<T, decltype(m)::value>, gm, bm, 0, c.stream, A_<T>(L), A_<T>(C), sx, sy,
+                              (C.n[1] + 3) * (C.n[2] + 3), C.n[2] + 3, bc);
+        }));
     } else {
         SARAS_CUDA_TRY(launch_pdl(k_mg_prolong_add<T>, g, b, 0, c.stream, lview<T>(L, A_<T>(L)), lcview<T>(C, A_<T>(C)), bc, add ? 1 : 0));
     }
@@ -3656,10 +3691,12 @@ static int mg_solve_target_run(Ctx &c, int *cycles, double *residual, saras_step
         }
         prof_begin(c, PK_REFINE_RESID, 0);
         if (c.mgMode == SARAS_MG_MIXED) {
-            k_tgt_residual<double, float, true><<<gk0, bk0, 0, c.stream>>>(L0.r32, L0.pa(), L0.r, sx0, sy0, bc0, t0, c.dscal + 32);
+            k_tgt_residual<double, float, true, kIch><<<gk0, bk0, 0, c.stream>>>(L0.r32, L0.pa(), L0.r, sx0, sy0, bc0, t0, c.dscal + 32);
             prof_end(c, PK_REFINE_RESID, 0, (8.0 + 8.0 + 4.0) * (double)ncore);
         } else {
-            k_tgt_residual<double, double, true><<<gk0, bk0, 0, c.stream>>>(nullptr, L0.pa(), L0.r, sx0, sy0, bc0, t0, c.dscal + 32);
+            dim3 gr, br;
+            const int ch = level_dims<double>(c, L0, gr, br);
+            (ch == kIch ? k_tgt_residual<double, double, true, kIch> : k_tgt_residual<double, double, true, kShort>)<<<gr, br, 0, c.stream>>>(nullptr, L0.pa(), L0.r, sx0, sy0, bc0, t0, c.dscal + 32);
             prof_end(c, PK_REFINE_RESID, 0, (8.0 + 8.0) * (double)ncore);
         }
         count_launch(c);
