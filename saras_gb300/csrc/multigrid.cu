@@ -7,6 +7,7 @@
 //                          coarsest Gauss-Seidel to mgTolerance / maxCount).
 //   SARAS_MG_PLAIN_TARGET  FP64 V-cycles on the compatible system until
 //                          max|b-Ap| <= target * max|b|.
+//                          (an isotropic level 0 in 64-bit fixed point, k_fx_sweep).
 //   SARAS_MG_MIXED         FP32 V-cycles as the inner solver of an
 //                          iterative-refinement loop to the same target; the
 //                          outer residual is FP64, or exact 64-bit fixed point
@@ -1832,30 +1833,194 @@ __device__ __forceinline__ long long round53(long long p) {
     return p < 0 ? -(long long)a : (long long)a;
 }
 
-__global__ void __launch_bounds__(256) k_fx_refine(const long long *__restrict__ pin, const long long *__restrict__ bfx,
-                                                   float *__restrict__ r32, int sx, int sy, MgBC bc, float rscale,
-                                                   unsigned long long *maxr) {
+// A column segment's B-free stencil sums in one go: every load issued before the first
+// store, as in k_tgt_sweep.  f(offset, centre, sum of the six neighbours - 6 centre - B).
+template <int CH, typename F>
+__device__ __forceinline__ void fx_column(const long long *__restrict__ pin, const long long *__restrict__ bfx, int sx, int sy, const MgBC &bc, int j,
+                                          int k, int seg, F f) {
+    const int i0 = seg * CH;
+    const NbrJK nb = nbr_jk(j, k, sy, bc);
+    long o = (long)(i0 + 1) * sx + (long)(j + 1) * sy + (k + 1);
+    long long cm = pin[o + nbr_x(i0, -1, sx, bc)], cc = pin[o];
+    if (i0 + CH <= bc.E[0]) {
+        long long nc[CH + 1], t[CH];
+        nc[0] = cc;
+#pragma unroll
+        for (int q = 0; q < CH; ++q) {
+            const long p = o + (long)q * sx;
+            nc[q + 1] = pin[p + sx];
+            t[q] = (pin[p + nb.yp] + pin[p + nb.ym]) + (pin[p + nb.zp] + pin[p + nb.zm]) - bfx[p];
+        }
+#pragma unroll
+        for (int q = 0; q < CH; ++q) {
+            f(o + (long)q * sx, nc[q], (cm + nc[q + 1]) + t[q] - 6 * nc[q]);
+            cm = nc[q];
+        }
+        return;
+    }
+    for (int i = i0; i <= bc.E[0]; ++i, o += sx) {   // the last segment
+        const long long cp = pin[o + nbr_x(i, 1, sx, bc)];
+        f(o, cc, (cm + cp) + (pin[o + nb.yp] + pin[o + nb.ym]) + (pin[o + nb.zp] + pin[o + nb.zm]) - bfx[o] - 6 * cc);
+        cm = cc;
+        cc = cp;
+    }
+}
+
+__global__ void __launch_bounds__(256, 3) k_fx_refine(const long long *__restrict__ pin, const long long *__restrict__ bfx,
+                                                      float *__restrict__ r32, int sx, int sy, MgBC bc, float rscale,
+                                                      unsigned long long *maxr) {
     int j, k, seg;
     const bool on = col_of<true>(bc, j, k, seg);
-    const int i0 = seg * kIch;
     unsigned long long m = 0;
-    if (on) {
-        int iend = min(i0 + kIch - 1, bc.E[0]);
-        const NbrJK nb = nbr_jk(j, k, sy, bc);
-        long o = (long)(i0 + 1) * sx + (long)(j + 1) * sy + (k + 1);
-        long long cm = pin[o + nbr_x(i0, -1, sx, bc)], cc = pin[o];
-        for (int i = i0; i <= iend; ++i, o += sx) {
-            long long cp = pin[o + (i < bc.E[0] ? (long)sx : nbr_x(i, 1, sx, bc))];
-            long long nsum = (cm + cp) + (pin[o + nb.yp] + pin[o + nb.ym]) + (pin[o + nb.zp] + pin[o + nb.zm]);
-            long long r = bfx[o] - (nsum - 6 * cc);
-            if (r32) r32[o] = fx2f(r) * rscale;
-            unsigned long long a = (unsigned long long)(r < 0 ? -r : r);
+    if (on)
+        fx_column<kIch>(pin, bfx, sx, sy, bc, j, k, seg, [&](long o, long long, long long d) {
+            if (r32) r32[o] = fx2f(-d) * rscale;
+            const unsigned long long a = (unsigned long long)(d < 0 ? -d : d);
             m = a > m ? a : m;
-            cm = cc;
-            cc = cp;
+        });
+    block_max_bits_to(m, reinterpret_cast<double *>(maxr));
+}
+
+// ---- fixed-point V-cycle on level 0 (SARAS_MG_PLAIN_TARGET, isotropic level 0)
+// The same integers P and B carry the plain mode's finest level: with d = sum of the
+// six neighbours - 6 P - B (exact), the damped Jacobi sweep of weight w is
+// P + d w / 6, one 64 x 64 -> 128 bit multiplication by w / 6 in units of 2^-64; the
+// residual for the level below is -d, exact, where an FP64 residual loses the
+// digits that the stencil cancels; the correction comes back rounded to P's
+// last bit.  With 2^57 <= max|P| < 2^58 that bit is finer than FP64's for every value
+// above max|P| / 32; what the solve returns is rounded to FP64 by its last sweep.  The
+// exact residual left after 25 cycles, relative to max|b| (Taylor-Green 33^3 / 65^3 /
+// 129^3): 2.0e-15 / 8.7e-15 / 3.8e-14, with FP64 levels 4.2e-15 / 2.8e-14 / 9.9e-14.  An FP64 sweep is bound by the FP64 pipe (one warp instruction in
+// 64 clocks on an SM quarter), the integer one by HBM: at
+// 257^3 a sweep 265 -> 76 us, residual 265 -> 70, its maximum 298 -> 62, restriction
+// 134 -> 32, prolongation 182 -> 93; a step 14.6 -> 9.0 ms.
+// Level 0's arrays hold the integers themselves (pa, pb, r), so the mode takes no more
+// memory.  flag: a value beyond +-2^59, where sums of seven terms could pass 2^63.
+__device__ __forceinline__ bool fx_far(long long p) { return p > (1LL << 59) || p < -(1LL << 59); }
+
+// ROUND: the sweep whose output the solve may return (round53).
+template <bool ROUND, int CH>
+__global__ void __launch_bounds__(256, 3) k_fx_sweep(long long *__restrict__ out, const long long *__restrict__ in, const long long *__restrict__ bfx,
+                                                     int sx, int sy, MgBC bc, long long w6, int *flag) {
+    pdl_wait();
+    int j, k, seg;
+    if (!col_of<true>(bc, j, k, seg)) return;
+    bool bad = false;
+    fx_column<CH>(in, bfx, sx, sy, bc, j, k, seg, [&](long o, long long cc, long long d) {
+        long long v = cc + __mul64hi(d, w6);
+        if (ROUND) v = round53(v);
+        bad |= fx_far(v);
+        out[o] = v;
+    });
+    if (bad) atomicExch(flag, 1);
+}
+
+// -d over the core: the residual in units of l 2^-s.
+template <int CH>
+__global__ void __launch_bounds__(256, 3) k_fx_residual(long long *__restrict__ out, const long long *__restrict__ in, const long long *__restrict__ bfx,
+                                                        int sx, int sy, MgBC bc) {
+    pdl_wait();
+    int j, k, seg;
+    if (!col_of<true>(bc, j, k, seg)) return;
+    fx_column<CH>(in, bfx, sx, sy, bc, j, k, seg, [&](long o, long long, long long d) { out[o] = -d; });
+}
+
+// Full weighting of the integer residual (k_tgt_restrict's stencil): exact sums in a
+// plane, the planes' sum in units of four (residuals up to 2^58 stay inside 63 bits),
+// then one conversion: scale[0] = l 2^-s / 16.
+template <int CH>
+__global__ void __launch_bounds__(256, 4) k_fx_restrict(double *__restrict__ rc, const long long *__restrict__ r, int sx, int sy, int csx, int csy,
+                                                        MgBC bcf, const double *__restrict__ scale) {
+    pdl_wait();
+    const int E0 = bcf.E[0], E1 = bcf.E[1], E2 = bcf.E[2];
+    const int W = E2 / 2 + 1, t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int J = t / W, K = t - J * W, I0 = blockIdx.y * CH;
+    if (J > E1 / 2) return;
+    long oj[3];
+    int ok[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        oj[a] = (long)(pad_img(2 * J - 1 + a, E1, bcf.per[1]) + 1) * sy;
+        ok[a] = pad_img(2 * K - 1 + a, E2, bcf.per[2]) + 1;
+    }
+    auto plane = [&](int i) -> long long {
+        const long long *q = r + (long)(pad_img(i, E0, bcf.per[0]) + 1) * sx;
+        long long row[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            const long long *qa = q + oj[a];
+            row[a] = qa[ok[0]] + 2 * qa[ok[1]] + qa[ok[2]];
+        }
+        return (row[0] + 2 * row[1] + row[2] + 2) >> 2;
+    };
+    const double mul = scale[0];
+    const int Iend = min(I0 + CH - 1, E0 / 2);
+    long long lo = plane(2 * I0 - 1);
+#pragma unroll 2
+    for (int I = I0; I <= Iend; ++I) {
+        const long long mid = plane(2 * I), hi = plane(2 * I + 1);
+        rc[(long)(I + 1) * csx + (long)(J + 1) * csy + (K + 1)] = __ll2double_rn(lo + 2 * mid + hi) * mul;
+        lo = hi;
+    }
+}
+
+// k_tgt_prolong_add on the integers: the coarse FP64 correction in units of 2^-(s + 1)
+// (scale[1] holds s), its trilinear interpolant exact in units of 2^-(s + 4), rounded
+// once.
+template <bool ROUND, int CH>
+__global__ void __launch_bounds__(256, 3) k_fx_prolong_add(long long *__restrict__ pf, const double *__restrict__ pc, int sxf, int syf, int sxc,
+                                                           int syc, MgBC bc, const double *__restrict__ scale, int *flag) {
+    pdl_wait();
+    int j, k, seg;
+    if (!col_of<true>(bc, j, k, seg)) return;
+    const int s1 = (int)scale[1] + 1;
+    const int i0 = seg * CH;   // CH is even
+    const int iend = min(i0 + CH - 1, bc.E[0]);
+    const int k2 = k >> 1, j2 = j >> 1;
+    const int k1 = k & 1, j1 = (j & 1) ? syc : 0;   // offsets of the second coarse neighbours (the point itself where it has none)
+    bool bad = false;
+    auto fx = [&](double v) -> long long {
+        const long long q = d2fx(v, s1, bad);
+        bad |= fx_far(q);
+        return q;
+    };
+    auto A = [&](int m) -> long long {   // coarse plane m at (j, k), times 4
+        const double *q = pc + (long)(m + 1) * sxc + (long)(j2 + 1) * syc + (k2 + 1);
+        const long long a = fx(q[0]);
+        long long v = k1 ? a + fx(q[1]) : 2 * a;
+        if (!j1) return 2 * v;
+        const long long b = fx(q[syc]);
+        return v + (k1 ? b + fx(q[syc + 1]) : 2 * b);
+    };
+    auto put = [&](long o, long long p, long long e8) {   // e8: eight times the correction in units of 2^-(s + 1)
+        long long v = p + ((e8 + 8) >> 4);
+        if (ROUND) v = round53(v);
+        bad |= fx_far(v);
+        pf[o] = v;
+    };
+    long o = (long)(i0 + 1) * sxf + (long)(j + 1) * syf + (k + 1);
+    if (iend - i0 + 1 == CH) {
+        // a full segment: the loads of the fine column issued before the first store (the
+        // coarse plane i0 / 2 + CH / 2 is at most the coarse core's last plane)
+        long long a[CH / 2 + 1], v[CH];
+#pragma unroll
+        for (int q = 0; q < CH; ++q) v[q] = pf[o + q * (long)sxf];
+#pragma unroll
+        for (int q = 0; q <= CH / 2; ++q) a[q] = A((i0 >> 1) + q);
+#pragma unroll
+        for (int q = 0; q < CH; ++q) put(o + q * (long)sxf, v[q], (q & 1) ? a[q >> 1] + a[(q >> 1) + 1] : 2 * a[q >> 1]);
+    } else {
+        long long am = A(i0 >> 1);
+        for (int i = i0; i <= iend; i += 2, o += 2 * (long)sxf) {
+            put(o, pf[o], 2 * am);
+            if (i + 1 <= iend) {
+                const long long ap = A((i >> 1) + 1);
+                put(o + sxf, pf[o + sxf], am + ap);
+                am = ap;
+            }
         }
     }
-    block_max_bits_to(m, reinterpret_cast<double *>(maxr));
+    if (bad) atomicExch(flag, 1);
 }
 
 // The iterate advanced by the FP32 correction e of the inner V-cycles,
@@ -3134,6 +3299,74 @@ static int tail_run(Ctx &c, int Lt) {
     return chk(c, "mg tail");
 }
 
+// Level 0 of a fixed-point V-cycle (k_fx_sweep and its companions): smooth,
+// restrict_level and prolong_level on the integers in pa, pb and r.
+static long long *fx_of(double *p) { return reinterpret_cast<long long *>(p); }
+static int *fx_flag(Ctx &c) { return reinterpret_cast<int *>(c.dscal + 35); }
+static const double *fx_scale(Ctx &c) { return c.dscal + 36; }
+
+static int fx_smooth(Ctx &c, int count, bool last) {
+    Level &L = c.lv[0];
+    MgBC bc = level_bc(c, 0, true);
+    const double bytes = 3.0 * 8.0 * (double)(L.n[0] + 1) * (L.n[1] + 1) * (L.n[2] + 1);
+    const int sx = (L.n[1] + 3) * (L.n[2] + 3), sy = L.n[2] + 3;
+    dim3 g, b;
+    const int ch = level_dims<double>(c, L, g, b);
+    for (int n = 0; n < count; ++n) {
+        const long long w6 = std::llround(std::ldexp(smooth_weight(c, n, count) / 6.0, 64));
+        prof_begin(c, PK_MG_SMOOTH64, 0);
+        SARAS_CUDA_TRY(with_march<double>(ch, [&](auto m) {
+            constexpr int CH = decltype(m)::value;
+            return launch_pdl(last && n == count - 1 ? k_fx_sweep<true, CH> : k_fx_sweep<false, CH>, g, b, 0, c.stream, fx_of(L.pb()), fx_of(L.pa()),
+                              fx_of(L.r), sx, sy, bc, w6, fx_flag(c));
+        }));
+        count_launch(c);
+        prof_end(c, PK_MG_SMOOTH64, 0, bytes);
+        flip<double>(L);
+    }
+    return chk(c, "fixed-point smooth");
+}
+
+static int fx_restrict(Ctx &c) {
+    Level &L = c.lv[0], &C = c.lv[1];
+    MgBC bc = level_bc(c, 0, true);
+    const double pts = (double)(L.n[0] + 1) * (L.n[1] + 1) * (L.n[2] + 1);
+    const int sx = (L.n[1] + 3) * (L.n[2] + 3), sy = L.n[2] + 3, csx = (C.n[1] + 3) * (C.n[2] + 3), csy = C.n[2] + 3;
+    dim3 g, b;
+    const int ch = level_dims<double>(c, L, g, b);
+    prof_begin(c, PK_MG_RESID64, 0);
+    SARAS_CUDA_TRY(with_march<double>(ch, [&](auto m) {
+        return launch_pdl(k_fx_residual<decltype(m)::value>, g, b, 0, c.stream, fx_of(L.pb()), fx_of(L.pa()), fx_of(L.r), sx, sy, bc);
+    }));
+    prof_end(c, PK_MG_RESID64, 0, 3.0 * 8.0 * pts);
+    const long ccols = (long)(C.n[1] + 1) * (C.n[2] + 1);
+    const int rch = ch == kIch ? rr_ch<double>() : 1;
+    dim3 gr((unsigned)((ccols + 255) / 256), (C.n[0] + 1 + rch - 1) / rch, 1);
+    prof_begin(c, PK_MG_RESTRICT64, 0);
+    SARAS_CUDA_TRY(launch_pdl(ch == kIch ? k_fx_restrict<rr_ch<double>()> : k_fx_restrict<1>, gr, dim3(256, 1, 1), 0, c.stream, C.r, fx_of(L.pb()), sx,
+                              sy, csx, csy, bc, fx_scale(c)));
+    prof_end(c, PK_MG_RESTRICT64, 0, 8.0 * pts * (1.0 + 1.0 / 8.0));
+    count_launch(c, 2);
+    return chk(c, "fixed-point restrict");
+}
+
+static int fx_prolong(Ctx &c, bool last) {
+    Level &L = c.lv[0], &C = c.lv[1];
+    MgBC bc = level_bc(c, 0, true);
+    const double pts = (double)(L.n[0] + 1) * (L.n[1] + 1) * (L.n[2] + 1);
+    dim3 g, b;
+    const int ch = level_dims<double>(c, L, g, b);
+    prof_begin(c, PK_MG_PROLONG64, 0);
+    SARAS_CUDA_TRY(with_march<double>(ch, [&](auto m) {
+        constexpr int CH = decltype(m)::value;
+        return launch_pdl(last ? k_fx_prolong_add<true, CH> : k_fx_prolong_add<false, CH>, g, b, 0, c.stream, fx_of(L.pa()), C.pa(),
+                          (L.n[1] + 3) * (L.n[2] + 3), L.n[2] + 3, (C.n[1] + 3) * (C.n[2] + 3), C.n[2] + 3, bc, fx_scale(c), fx_flag(c));
+    }));
+    prof_end(c, PK_MG_PROLONG64, 0, 8.0 * pts * (2.0 + 1.0 / 8.0));
+    count_launch(c);
+    return chk(c, "fixed-point prolong");
+}
+
 // poisson::vCycle (poisson.cc:219-280) on level arrays of precision T.
 // zero0: the level-0 iterate starts at 0 (inner FP32 solve of the mixed mode).
 // A cycle from level l down (pre-smoothing, from zero when zero, restriction)
@@ -3148,13 +3381,14 @@ static int cycle_from(Ctx &c, int l, bool tgt, bool zero, int gamma) {
     if (l == c.depth) return coarse_solve<T>(c, tgt);
     const int pre = l > 0 ? coarse_sweeps(c, tgt, true) : c.p.preSmooth;
     const int post = l > 0 ? coarse_sweeps(c, tgt, false) : c.p.postSmooth;
-    if ((s = smooth<T>(c, l, pre, zero, tgt))) return s;
-    if ((s = restrict_level<T>(c, l, tgt))) return s;
+    const bool fx = sizeof(T) == 8 && l == 0 && c.fxPlain;   // level 0 on integers (plain_fixed)
+    if ((s = fx ? fx_smooth(c, pre, false) : smooth<T>(c, l, pre, zero, tgt))) return s;
+    if ((s = fx ? fx_restrict(c) : restrict_level<T>(c, l, tgt))) return s;
     const int g = l == 0 ? gamma : 1;
     for (int q = 0; q < g; ++q)
         if ((s = cycle_from<T>(c, l + 1, tgt, q == 0, 1))) return s;
-    if ((s = prolong_level<T>(c, l, tgt, true))) return s;
-    return smooth<T>(c, l, post, false, tgt);
+    if ((s = fx ? fx_prolong(c, post == 0) : prolong_level<T>(c, l, tgt, true))) return s;
+    return fx ? fx_smooth(c, post, true) : smooth<T>(c, l, post, false, tgt);
 }
 
 template <typename T>
@@ -3276,7 +3510,9 @@ static int graph_replay(Ctx &c, int a, int b, F run) {
 template <typename T>
 static int vcycle_tgt(Ctx &c, bool zero0) {
     const int buf = sizeof(T) == 4 ? c.lv[0].cur32 : c.lv[0].cur;
-    return graph_replay(c, sizeof(T) == 4 ? 1 : 0, (zero0 ? 1 : 0) + 2 * buf, [&]() { return vcycle<T>(c, true, zero0); });
+    // FP64 cycles never start from zero: that slot holds the fixed-point cycle's graph
+    return graph_replay(c, sizeof(T) == 4 ? 1 : 0, (zero0 || (sizeof(T) == 8 && c.fxPlain) ? 1 : 0) + 2 * buf,
+                        [&]() { return vcycle<T>(c, true, zero0); });
 }
 
 static int read_scalars(Ctx &c, int first, int count) {
@@ -3627,6 +3863,75 @@ static int mixed_fixed(Ctx &c, const double *pp0, double mean, double bmax, doub
     return fp64_start();
 }
 
+// The plain mode's solve with level 0 in fixed point (k_fx_sweep): V-cycles until the
+// exact residual meets the target.  done: the result is in Pp; otherwise (no scale to
+// take from the previous Pp, or values out of range) nothing the FP64 path reads has changed.
+static int plain_fixed(Ctx &c, const double *pp0, double mean, double bmax, double pmax, double target, double &r, int &cyc, bool &done,
+                       saras_step_stats *st) {
+    done = false;
+    Level &L0 = c.lv[0];
+    const double l = L0.lx;
+    // the previous Pp sets the scale (2^57 <= max|P| < 2^58); B has to fit it (|B| < 2^59)
+    if (!(pmax > 0.0) || !std::isfinite(pmax) || !(bmax / l <= 2.0 * pmax)) return SARAS_OK;
+    const int sc = 57 - std::ilogb(pmax);
+    if (sc < -900 || sc > 900) return SARAS_OK;
+    for (int n = 0; n < std::max(c.p.preSmooth, c.p.postSmooth); ++n)   // w / 6 in 63 bits
+        for (int count : {c.p.preSmooth, c.p.postSmooth})
+            if (n < count && !(std::fabs(smooth_weight(c, n, count)) < 2.9)) return SARAS_OK;
+    MgBC bc0 = level_bc(c, 0, true);
+    const int sx = (L0.n[1] + 3) * (L0.n[2] + 3), sy = L0.n[2] + 3;
+    dim3 gk, bk; col_dims(L0, gk, bk);
+    dim3 gc, bcd; core_dims(L0, gc, bcd);
+    unsigned long long *dmax = reinterpret_cast<unsigned long long *>(c.dscal + 34);
+    const double inv2s = std::ldexp(1.0, -sc), rs = l * inv2s;
+    SARAS_CUDA_TRY(cudaMemsetAsync(c.dscal + 34, 0, sizeof(double) * 2, c.stream));
+    c.hscal[36] = rs * 0.0625;
+    c.hscal[37] = (double)sc;
+    SARAS_CUDA_TRY(cudaMemcpyAsync(c.dscal + 36, c.hscal + 36, 2 * sizeof(double), cudaMemcpyHostToDevice, c.stream));
+    L0.cur = 0;
+    k_fx_rhs<<<gk, bk, 0, c.stream>>>(fx_of(L0.r), nullptr, c.f[SARAS_FIELD_MGRHS], sx, sy, bc0, mean, std::ldexp(1.0, sc) / l, fx_flag(c));
+    k_fx_init<<<gc, bcd, 0, c.stream>>>(fx_of(L0.pa()), lcview<double>(L0, pp0), bc0, sc, fx_flag(c));
+    count_launch(c, 2);
+    bool bad = false;
+    auto residual = [&]() -> int {
+        SARAS_CUDA_TRY(cudaMemsetAsync(c.dscal + 34, 0, sizeof(double), c.stream));
+        prof_begin(c, PK_REFINE_RESID, 0);
+        k_fx_refine<<<gk, bk, 0, c.stream>>>(fx_of(L0.pa()), fx_of(L0.r), nullptr, sx, sy, bc0, 0.0f, dmax);
+        prof_end(c, PK_REFINE_RESID, 0, 16.0 * (double)L0.count);
+        count_launch(c);
+        if (int e = chk(c, "fixed-point residual")) return e;
+        if (int e = read_scalars(c, 34, 2)) return e;
+        unsigned long long mx;
+        int fl;
+        std::memcpy(&mx, &c.hscal[34], sizeof mx);
+        std::memcpy(&fl, &c.hscal[35], sizeof fl);
+        bad = fl != 0 || mx > (1ull << 58);   // k_fx_restrict sums 16 of them in a plane
+        r = (double)mx * rs;
+        return SARAS_OK;
+    };
+    int s = residual();
+    if (s) return s;
+    if (!bad && st) { st->guess_residual = bmax > 0 ? r / bmax : r; st->guess_source = 0; }
+    while (!bad && r > target && cyc < c.mgMaxCycles) {
+        c.fxPlain = true;
+        s = vcycle_tgt<double>(c, false);
+        c.fxPlain = false;
+        if (s) return s;
+        cyc += 1;
+        if ((s = residual())) return s;
+    }
+    if (bad) {
+        cyc = 0;
+        L0.cur = 0;
+        return SARAS_OK;
+    }
+    dim3 bo(64, 4, 1), go((L0.n[2] + 3 + 63) / 64, (L0.n[1] + 3 + 3) / 4, L0.n[0] + 3);
+    k_fx_output<<<go, bo, 0, c.stream>>>(c.f[SARAS_FIELD_PP], fx_of(L0.pa()), bc0, inv2s);
+    count_launch(c);
+    done = true;
+    return chk(c, "fixed-point output");
+}
+
 // Target modes: plain FP64 V-cycles or FP32 V-cycles inside FP64 refinement.
 static int mg_solve_target_run(Ctx &c, int *cycles, double *residual, saras_step_stats *st) {
     int s;
@@ -3654,7 +3959,11 @@ static int mg_solve_target_run(Ctx &c, int *cycles, double *residual, saras_step
     dim3 gk0, bk0; col_dims(L0, gk0, bk0);
     int nparts = (int)(gk0.x * gk0.y);
     if (nparts > c.redCap) { c.err = "reduction buffer too small"; return SARAS_TOO_LARGE; }
-    k_tgt_stats<<<gk0, bk0, 0, c.stream>>>(lcview<double>(L0, rhs), fixedPath ? pp0 : nullptr, bc0, c.red, c.dscal + 31, c.dscal + 32,
+    // the plain mode's levels are FP64 but for an isotropic level 0, in fixed point unless a
+    // guess or training reads b from level-0 r
+    const bool fixedPlain = c.mgMode == SARAS_MG_PLAIN_TARGET && L0.lx == L0.ly && L0.ly == L0.lz && c.depth > 0 && c.tailLt != 0 && !wantGuess &&
+                            !c.collecting && !c.unet && !c.ppInHist;
+    k_tgt_stats<<<gk0, bk0, 0, c.stream>>>(lcview<double>(L0, rhs), fixedPath || fixedPlain ? pp0 : nullptr, bc0, c.red, c.dscal + 31, c.dscal + 32,
                                            c.dscal + 33);
     k_final_reduce<<<1, 256, 0, c.stream>>>(c.red, nparts, 0, c.dscal + 30);
     count_launch(c, 2);
@@ -3672,7 +3981,13 @@ static int mg_solve_target_run(Ctx &c, int *cycles, double *residual, saras_step
         bmax = (std::isnan(up) || std::isnan(dn)) ? up + dn : std::max(up, dn);
     }
     L0.cur = 0;
-    if (!fixedPath) {
+    double r = 0;
+    int source = 0, cyc = 0, steps = 0, built = 0;
+    bool fixedDone = false;
+    if (fixedPlain) {
+        if ((s = plain_fixed(c, pp0, mean, bmax, pmax, c.mgTarget * bmax, r, cyc, fixedDone, st))) return s;
+    }
+    if (!fixedPath && !fixedDone) {
         dim3 g, b; core_dims(L0, g, b);
         k_tgt_rhs<<<gk0, bk0, 0, c.stream>>>(L0.r, rhs, sx0, sy0, bc0, mean);
         k_mg_init_p<double><<<g, b, 0, c.stream>>>(lview<double>(L0, L0.pa()), lcview<double>(L0, pp0), bc0);
@@ -3707,9 +4022,6 @@ static int mg_solve_target_run(Ctx &c, int *cycles, double *residual, saras_step
         *out = c.hscal[32];
         return SARAS_OK;
     };
-    double r = 0;
-    int source = 0, cyc = 0, steps = 0, built = 0;
-    bool fixedDone = false;
     if (fixedPath) {
         if ((s = mixed_fixed(c, pp0, mean, bmax, pmax, target, wantGuess, r, source, cyc, steps, fixedDone, st))) return s;
     }
