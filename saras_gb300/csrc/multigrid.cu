@@ -2291,13 +2291,15 @@ __global__ void __launch_bounds__(256) k_tgt_rhs(double *__restrict__ b, const d
 // (k_tgt_sweep, k_tgt_residual, k_mg_restrict, k_mg_prolong_add), and writes
 // the level-Lt iterate with its face-ghost images to global memory.
 constexpr int kTailMaxLevels = 8;
-// The tail's first level: 9^3 at most.  One CTA runs a 17^3 level's Chebyshev
-// sweeps instruction-bound on one SM; graph-replayed kernels on all SMs ran
-// the 257^3 steps 0.7% (mixed) and 3% (plain FP64) faster with 17^3 outside
-// the tail.
+// The tail's first level: 9^3 at most, a point a thread (FP64 sweeps of a 17^3 level are
+// bound by one SM's pipe: with it in the tail the plain FP64 257^3 step was 3% slower).
 constexpr int kTailIntervals = 8;
 constexpr int kTailMaxSweeps = 16;
 constexpr int kTailThreads = 768;   // a thread a point of the largest tail level (9^3)
+// FP32 tails take one level more (BIG, at most 17^3): a thread owns up to kTailSeg points
+// of a column in registers, so a sweep reads four shared-memory neighbours a point.
+constexpr int kTailBigIntervals = 16, kTailSeg = 6;
+constexpr int kTailBigThreads = 896;   // 17 x 17 columns of three segments
 
 template <typename T>
 struct TailArgs {
@@ -2314,6 +2316,7 @@ struct TailArgs {
     const T *rin;                    // level-Lt right-hand side (padded)
     T *pout;                         // level-Lt iterate (padded)
     long long *iters;
+    TgK<float> bpre[kTailMaxSweeps], bpost[kTailMaxSweeps];   // BIG: the first level's sweep constants, as its own kernels'
 };
 
 // The sweep constants at weight w from those at weight 1.
@@ -2358,49 +2361,28 @@ __device__ __forceinline__ TailPt tail_pt(const MgBC &b) {
 // the FP32 tail took 24.5 us on 9^3 and 5^3, and a 65^3 mixed step (three cycles)
 // 634 us; in this form 608, a 257^3 step (four) 4.32 ms instead of 4.35 (the FP64
 // tail's time is its pipe's: unchanged).
-template <typename T>
-__global__ void __launch_bounds__(kTailThreads) k_mg_tail(const __grid_constant__ TailArgs<T> a) {
+//
+// BIG: level 0 of the tail is the 17^3 one, with its own kernels' arithmetic (bit for bit).
+// One CTA runs a 17^3 sweep in about 0.6 us where a launch on all SMs takes 4.3: the 65^3
+// mixed step goes from 501 to 475 us, the 257^3 step from 4.17 to 4.15 ms, the 257 x 257 x
+// 129 convection step from 5.26 to 5.22.  (FP64 would hold it at the pipe's rate, 12 us a sweep.)
+template <typename T, bool BIG>
+__global__ void __launch_bounds__(BIG ? kTailBigThreads : kTailThreads) k_mg_tail(const __grid_constant__ TailArgs<T> a) {
     extern __shared__ unsigned char smraw[];
     T *const base = reinterpret_cast<T *>(smraw);
     const int tid = threadIdx.x, nt = blockDim.x;
-    // level l's array `which` (0, 1: the iterates; 2: the right-hand side); the iterate is array (sweeps so far) mod 2
+    constexpr int l0 = BIG ? 1 : 0;
+    // level l's array `which` (0, 1: the iterates; 2: the right-hand side, in registers for
+    // the BIG level); the iterate is array (sweeps so far) mod 2
     auto arr = [&](int l, int which) -> T * {
         int o = 0;
-        for (int m = 0; m < l; ++m) o += 3 * tail_points(a.bc[m]);
+        for (int m = 0; m < l; ++m) o += (BIG && m == 0 ? 2 : 3) * tail_points(a.bc[m]);
         return base + o + which * tail_points(a.bc[l]);
     };
-    TailPt p = tail_pt(a.bc[0]);
-    const int pad0 = (a.bc[0].E[1] + 3) * (a.bc[0].E[2] + 3), pad1 = a.bc[0].E[2] + 3;
-    const long og = (long)(p.i + 1) * pad0 + (p.j + 1) * pad1 + (p.k + 1);
-    pdl_wait();
-    T r = a.rin[og];
-    if (p.on) arr(0, 2)[p.o] = r;
-    __syncthreads();
-    for (int l = 0; l + 1 < a.nl; ++l) {
+    // full weighting of the residual res of level l into level l + 1's right-hand side
+    // (k_tgt_restrict's separable form; fine positions outside the core at their images)
+    auto restrict_to = [&](int l, const T *res) {
         const MgBC &bc = a.bc[l];
-        if (l > 0) {
-            p = tail_pt(bc);
-            r = arr(l, 2)[p.o];
-        }
-        // pre-smoothing from zero (the first sweep ignores its input)
-        for (int n = 0; n < a.pre; ++n) {
-            const TgK<T> c = tgk_weight(a.tk[l], a.wpre[n]);
-            const T *in = arr(l, n & 1);
-            T *out = arr(l, (n & 1) ^ 1);
-            T v;
-            if (n == 0) v = c.ar * r;
-            else v = fma(c.ax, in[p.w] + in[p.e], fma(c.ay, in[p.n] + in[p.s], fma(c.az, in[p.u] + in[p.d], fma(c.ar, r, c.om1 * in[p.o]))));
-            if (p.on) out[p.o] = v;
-            __syncthreads();
-        }
-        // residual into the other array, then full-weighting restriction (k_tgt_restrict's
-        // separable form; fine positions outside the core at their images)
-        const TgK<T> &c = a.tr[l];
-        const T *in = arr(l, a.pre & 1);
-        T *res = arr(l, (a.pre & 1) ^ 1);
-        const T lap = fma(c.lx, in[p.w] + in[p.e], fma(c.ly, in[p.n] + in[p.s], fma(c.lz, in[p.u] + in[p.d], c.lc * in[p.o])));
-        if (p.on) res[p.o] = r - lap;
-        __syncthreads();
         const TailPt q = tail_pt(a.bc[l + 1]);
         if (q.on) {
             const int W = bc.E[2] + 1, P = (bc.E[1] + 1) * W;
@@ -2422,6 +2404,117 @@ __global__ void __launch_bounds__(kTailThreads) k_mg_tail(const __grid_constant_
             }
             arr(l + 1, 2)[q.o] = acc * (T)0.015625;
         }
+    };
+    // the BIG level: this thread's column, its segment's planes, their values and right-hand sides
+    constexpr int NB = BIG ? kTailSeg : 1;
+    T bv[NB] = {}, br[NB] = {};
+    int bn = 0, bi = 0, bj = 0, bk = 0, bo = 0, bP = 0, bw = 0, be = 0, by0 = 0, by1 = 0, bz0 = 0, bz1 = 0;
+    long bg = 0, bgs = 0;
+    if constexpr (BIG) {
+        const MgBC &bc = a.bc[0];
+        const int W = bc.E[2] + 1;
+        bP = (bc.E[1] + 1) * W;
+        const int seg = tid / bP, c = tid - seg * bP;
+        bj = c / W;
+        bk = c - bj * W;
+        bi = seg * kTailSeg;
+        bn = max(0, min(kTailSeg, bc.E[0] + 1 - bi));
+        if (bn == 0) bi = 0;
+        bo = bi * bP + c;
+        bw = bo + (pad_img(bi - 1, bc.E[0], bc.per[0]) - bi) * bP;
+        be = bo + (pad_img(bi + bn, bc.E[0], bc.per[0]) - bi) * bP;
+        by1 = (pad_img(bj + 1, bc.E[1], bc.per[1]) - bj) * W;
+        by0 = (pad_img(bj - 1, bc.E[1], bc.per[1]) - bj) * W;
+        bz1 = pad_img(bk + 1, bc.E[2], bc.per[2]) - bk;
+        bz0 = pad_img(bk - 1, bc.E[2], bc.per[2]) - bk;
+        bgs = (long)(bc.E[1] + 3) * (bc.E[2] + 3);
+        bg = (long)(bi + 1) * bgs + (long)(bj + 1) * (bc.E[2] + 3) + (bk + 1);
+    }
+    // f(plane of the segment, west + east, north + south, up + down) at every point of it, from
+    // the level's array in
+    auto big_points = [&](const T *in, auto f) {
+        const T west = bn > 0 ? in[bw] : (T)0, east = bn > 0 ? in[be] : (T)0;
+        T cm = west;
+#pragma unroll
+        for (int q = 0; q < NB; ++q) {
+            if (q >= bn) break;
+            const T *x = in + bo + q * bP;
+            const T cc = bv[q], cp = q + 1 < NB && q + 1 < bn ? bv[q + 1 < NB ? q + 1 : q] : east;
+            f(q, cm + cp, x[by1] + x[by0], x[bz1] + x[bz0]);
+            cm = cc;
+        }
+    };
+    auto big_sweep = [&](int from, const TgK<T> &c) {
+        T *out = arr(0, from ^ 1);
+        T nv[NB];
+        big_points(arr(0, from), [&](int q, T we, T ns, T ud) {
+            nv[q] = fma(c.ax, we, fma(c.ay, ns, fma(c.az, ud, fma(c.ar, br[q], c.om1 * bv[q]))));
+        });
+#pragma unroll
+        for (int q = 0; q < NB; ++q) {
+            if (q >= bn) break;
+            bv[q] = nv[q];
+            out[bo + q * bP] = nv[q];
+        }
+        __syncthreads();
+    };
+    if constexpr (BIG) {
+        pdl_wait();
+#pragma unroll
+        for (int q = 0; q < NB; ++q) br[q] = q < bn ? a.rin[bg + q * bgs] : (T)0;
+        const TgK<T> c0 = a.bpre[0];
+        T *out = arr(0, 1);
+#pragma unroll
+        for (int q = 0; q < NB; ++q) {   // the first sweep, from zero
+            bv[q] = c0.ar * br[q];
+            if (q < bn) out[bo + q * bP] = bv[q];
+        }
+        __syncthreads();
+        for (int n = 1; n < a.pre; ++n) big_sweep(n & 1, a.bpre[n]);
+        const TgK<T> &c = a.tr[0];
+        T *res = arr(0, (a.pre & 1) ^ 1);
+        big_points(arr(0, a.pre & 1), [&](int q, T we, T ns, T ud) {
+            res[bo + q * bP] = br[q] - fma(c.lx, we, fma(c.ly, ns, fma(c.lz, ud, c.lc * bv[q])));
+        });
+        __syncthreads();
+        restrict_to(0, res);
+        __syncthreads();
+    }
+    TailPt p = tail_pt(a.bc[l0]);
+    const int pad0 = (a.bc[0].E[1] + 3) * (a.bc[0].E[2] + 3), pad1 = a.bc[0].E[2] + 3;
+    const long og = (long)(p.i + 1) * pad0 + (p.j + 1) * pad1 + (p.k + 1);
+    T r = (T)0;
+    if constexpr (!BIG) {
+        pdl_wait();
+        r = a.rin[og];
+        if (p.on) arr(0, 2)[p.o] = r;
+        __syncthreads();
+    }
+    for (int l = l0; l + 1 < a.nl; ++l) {
+        const MgBC &bc = a.bc[l];
+        if (l > 0) {
+            p = tail_pt(bc);
+            r = arr(l, 2)[p.o];
+        }
+        // pre-smoothing from zero (the first sweep ignores its input)
+        for (int n = 0; n < a.pre; ++n) {
+            const TgK<T> c = tgk_weight(a.tk[l], a.wpre[n]);
+            const T *in = arr(l, n & 1);
+            T *out = arr(l, (n & 1) ^ 1);
+            T v;
+            if (n == 0) v = c.ar * r;
+            else v = fma(c.ax, in[p.w] + in[p.e], fma(c.ay, in[p.n] + in[p.s], fma(c.az, in[p.u] + in[p.d], fma(c.ar, r, c.om1 * in[p.o]))));
+            if (p.on) out[p.o] = v;
+            __syncthreads();
+        }
+        // residual into the other array, then the restriction
+        const TgK<T> &c = a.tr[l];
+        const T *in = arr(l, a.pre & 1);
+        T *res = arr(l, (a.pre & 1) ^ 1);
+        const T lap = fma(c.lx, in[p.w] + in[p.e], fma(c.ly, in[p.n] + in[p.s], fma(c.lz, in[p.u] + in[p.d], c.lc * in[p.o])));
+        if (p.on) res[p.o] = r - lap;
+        __syncthreads();
+        restrict_to(l, res);
         __syncthreads();
     }
     // coarsest level: e = M r with the precomputed solution operator (a warp four
@@ -2462,7 +2555,7 @@ __global__ void __launch_bounds__(kTailThreads) k_mg_tail(const __grid_constant_
         __syncthreads();
     }
     // back up: prolongation + add, post-smoothing
-    for (int l = a.nl - 2; l >= 0; --l) {
+    for (int l = a.nl - 2; l >= l0; --l) {
         const MgBC &bc = a.bc[l], &bcc = a.bc[l + 1];
         p = tail_pt(bc);
         r = arr(l, 2)[p.o];
@@ -2503,7 +2596,40 @@ __global__ void __launch_bounds__(kTailThreads) k_mg_tail(const __grid_constant_
             __syncthreads();
         }
     }
-    if (p.on) a.pout[og] = arr(0, (a.pre + a.post) & 1)[p.o];   // the core: the level kernels read images by index
+    // the core: the level kernels read images by index
+    if constexpr (BIG) {
+        // k_tgt_prolong_add's arithmetic
+        const MgBC &bcc = a.bc[1];
+        const int sy = bcc.E[2] + 1, sx = (bcc.E[1] + 1) * sy;
+        const T *c = arr(1, a.nl == 2 ? 0 : (a.pre + a.post) & 1) + (bj >> 1) * sy + (bk >> 1);
+        const bool jo = bj & 1, ko = bk & 1;
+        auto A = [&](int m) -> T {
+            const T *x = c + m * sx;
+            const T v0 = ko ? (T)0.5 * (x[0] + x[1]) : x[0];
+            if (!jo) return v0;
+            const T v1 = ko ? (T)0.5 * (x[sy] + x[sy + 1]) : x[sy];
+            return (T)0.5 * (v0 + v1);
+        };
+        T *f = arr(0, a.pre & 1);
+        if (bn > 0) {   // kTailSeg is even: a segment starts on a coarse plane
+            T am = A(bi >> 1);
+#pragma unroll
+            for (int q = 0; q < NB; ++q) {
+                if (q >= bn) break;
+                if (q & 1) {
+                    const T ap = A((bi + q + 1) >> 1);
+                    bv[q] = bv[q] + (T)0.5 * (am + ap);
+                    am = ap;
+                } else bv[q] = bv[q] + am;
+                f[bo + q * bP] = bv[q];
+            }
+        }
+        __syncthreads();
+        for (int m = 0; m < a.post; ++m) big_sweep((a.pre + m) & 1, a.bpost[m]);
+#pragma unroll
+        for (int q = 0; q < NB; ++q)
+            if (q < bn) a.pout[bg + q * bgs] = bv[q];
+    } else if (p.on) a.pout[og] = arr(0, (a.pre + a.post) & 1)[p.o];
 }
 
 // ------------------------------------------------------------------ host
@@ -2811,8 +2937,15 @@ int mg_setup(Ctx &c) {
     if (int e = plane_setup(c)) return e;
     c.tailLt = c.planar ? 0 : tail_level(c);   // target modes only (3D)
     if (c.tailLt > 0) {
-        SARAS_CUDA_TRY(cudaFuncSetAttribute(k_mg_tail<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-        SARAS_CUDA_TRY(cudaFuncSetAttribute(k_mg_tail<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        SARAS_CUDA_TRY(cudaFuncSetAttribute(k_mg_tail<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        SARAS_CUDA_TRY(cudaFuncSetAttribute(k_mg_tail<float, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        SARAS_CUDA_TRY(cudaFuncSetAttribute(k_mg_tail<float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+        // the level above in the FP32 tail: every visit of it has to start from zero (level 1
+        // is visited again, with its iterate, when coarseCycles > 1)
+        const int lb = c.tailLt - 1;
+        c.tailBig = lb >= (p.coarseCycles > 1 ? 2 : 1) && c.depth - lb + 1 <= kTailMaxLevels &&
+                    std::max(c.lv[lb].n[0], std::max(c.lv[lb].n[1], c.lv[lb].n[2])) <= kTailBigIntervals &&
+                    (p.coarseSmooth > 0 ? p.coarseSmooth : p.preSmooth) >= 1;
         // the tail's coarsest solve as a matrix-vector product when the level is small
         const Level &Lc = c.lv[c.depth];
         long nc = (long)(Lc.n[0] + 1) * (Lc.n[1] + 1) * (Lc.n[2] + 1);
@@ -3266,7 +3399,7 @@ static int coarse_sweeps(const Ctx &c, bool tgt, bool pre) {
 }
 
 template <typename T>
-static int tail_run(Ctx &c, int Lt) {
+static int tail_run(Ctx &c, int Lt, bool big) {
     TailArgs<T> a;
     a.nl = c.depth - Lt + 1;
     size_t smem = 0;
@@ -3276,6 +3409,14 @@ static int tail_run(Ctx &c, int Lt) {
         a.tk[q] = make_tgk<T>(L, 1.0);
         a.tr[q] = make_tgk<T>(L, 1.0);
         smem += 3 * sizeof(T) * (size_t)(L.n[0] + 1) * (L.n[1] + 1) * (L.n[2] + 1);
+    }
+    if (big) {
+        const Level &L = c.lv[Lt];
+        smem -= sizeof(T) * (size_t)(L.n[0] + 1) * (L.n[1] + 1) * (L.n[2] + 1);   // its right-hand side is in registers
+        for (int n = 0; n < kTailMaxSweeps; ++n) {
+            a.bpre[n] = make_tgk<float>(L, smooth_weight(c, n, coarse_sweeps(c, true, true)));
+            a.bpost[n] = make_tgk<float>(L, smooth_weight(c, n, coarse_sweeps(c, true, false)));
+        }
     }
     if (!c.coarseN) smem += 2 * sizeof(T) * (size_t)c.lv[c.depth].count;
     a.kkc = make_k(c.lv[c.depth]);
@@ -3294,7 +3435,14 @@ static int tail_run(Ctx &c, int Lt) {
     a.rin = R_<T>(c.lv[Lt]);
     a.pout = A_<T>(c.lv[Lt]);
     a.iters = (long long *)(c.dscal + 40);
-    SARAS_CUDA_TRY(launch_pdl(k_mg_tail<T>, dim3(1), dim3(kTailThreads), smem, c.stream, a));
+    if constexpr (sizeof(T) == 4) {
+        if (big) {
+            SARAS_CUDA_TRY(launch_pdl(k_mg_tail<T, true>, dim3(1), dim3(kTailBigThreads), smem, c.stream, a));
+            count_launch(c);
+            return chk(c, "mg tail");
+        }
+    }
+    SARAS_CUDA_TRY(launch_pdl(k_mg_tail<T, false>, dim3(1), dim3(kTailThreads), smem, c.stream, a));
     count_launch(c);
     return chk(c, "mg tail");
 }
@@ -3377,7 +3525,8 @@ template <typename T>
 static int cycle_from(Ctx &c, int l, bool tgt, bool zero, int gamma) {
     int s;
     int Lt = tgt ? c.tailLt : -1;   // target modes: levels Lt.. run as one fused kernel
-    if (l == Lt) return tail_run<T>(c, Lt);
+    if (sizeof(T) == 4 && tgt && l > 0 && l == Lt - 1 && zero && c.tailBig) return tail_run<T>(c, l, true);
+    if (l == Lt) return tail_run<T>(c, Lt, false);
     if (l == c.depth) return coarse_solve<T>(c, tgt);
     const int pre = l > 0 ? coarse_sweeps(c, tgt, true) : c.p.preSmooth;
     const int post = l > 0 ? coarse_sweeps(c, tgt, false) : c.p.postSmooth;
