@@ -1830,7 +1830,10 @@ int compute_trhs(Ctx &c) {
 // semantics of cn_solve: each sweep also reports the residual of its input,
 // and the input of the first sweep whose input residual is below the
 // tolerance is the answer.
-static int cn_solve_delta(Ctx &c, int comp, int field, const CnFast &fa, double Dn, double bytes, int *iters, double *maxerr) {
+// stage 0: the whole solve; 1: its launches up to the speculative final sweep's,
+// without waiting; 2: the rest, with that sweep's residual in hscal[comp] already
+// (cn_together: the components' residuals come in one copy).
+static int cn_solve_delta(Ctx &c, int comp, int field, const CnFast &fa, double Dn, double bytes, int *iters, double *maxerr, int stage) {
     const FieldInfo &f = c.info[field];
     View3<double> V = mview(c, field);
     long n = V.size();
@@ -1840,7 +1843,7 @@ static int cn_solve_delta(Ctx &c, int comp, int field, const CnFast &fa, double 
     float *n0h = c.cnp + (size_t)2 * comp * N, *n0l = n0h + N;
     float *dA = c.cnp + (size_t)8 * N, *dAl = dA + N, *dB = dAl + N, *dBl = dB + N;
     CnDf fd = cn_df_consts(fa);
-    if (!c.n0Fresh[comp]) {   // N0 not already written by the right-hand-side kernel
+    if (stage != 2 && !c.n0Fresh[comp]) {   // N0 not already written by the right-hand-side kernel
         dim3 g, bl; box_launch_dims(fa.full, g, bl);
         k_cn_pack<<<g, bl, 0, c.stream>>>(cview(c, field), fa.rhs, f.full, fa.full, fd, n0h, n0l);
         count_launch(c);
@@ -1853,15 +1856,17 @@ static int cn_solve_delta(Ctx &c, int comp, int field, const CnFast &fa, double 
     d.prog = f.full;
     d.full = fa.full;
     d.f = fd;
-    d.resMax = c.dscal;
+    d.resMax = c.dscal + comp;
     d.vout = nullptr;
     d.withResidual = 0;
     // The first iterate from D = 0 is A = N0 / Dn itself (on the bulk, written with
     // N0): its non-bulk points from their boundary-program sources, in place.
     d.dh = d.oh = n0h;
     d.dl = d.ol = n0l;
-    k_cn_delta_shell<false, true><<<dim3(shell_blocks(d.full), 6), 256, 0, c.stream>>>(d);
-    count_launch(c);
+    if (stage != 2) {
+        k_cn_delta_shell<false, true><<<dim3(shell_blocks(d.full), 6), 256, 0, c.stream>>>(d);
+        count_launch(c);
+    }
     // The iterates: A (read only), then alternately P and Q.
     float *const bufs[3][2] = {{n0h, n0l}, {dA, dAl}, {dB, dBl}};
     int cur = 0, nxt = 1;
@@ -1891,9 +1896,9 @@ static int cn_solve_delta(Ctx &c, int comp, int field, const CnFast &fa, double 
     auto read_res = [&](double &r) -> int {
         int s = check_launch(c, "cn");
         if (s) return s;
-        SARAS_CUDA_TRY(cudaMemcpyAsync(c.hscal, c.dscal, sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+        SARAS_CUDA_TRY(cudaMemcpyAsync(c.hscal + comp, d.resMax, sizeof(double), cudaMemcpyDeviceToHost, c.stream));
         SARAS_CUDA_TRY(cudaStreamSynchronize(c.stream));
-        r = c.hscal[0] * Dn;
+        r = c.hscal[comp] * Dn;
         return SARAS_OK;
     };
     // The Jacobi map contracts the max norm of successive corrections by
@@ -1919,10 +1924,15 @@ static int cn_solve_delta(Ctx &c, int comp, int field, const CnFast &fa, double 
             advance();
             sweeps += 1;
         }
-        SARAS_CUDA_TRY(cudaMemsetAsync(c.dscal, 0, sizeof(double), c.stream));
-        launch(1, c.scratch[slot]);
-        int s = read_res(res);
-        if (s) return s;
+        if (stage != 2) {
+            SARAS_CUDA_TRY(cudaMemsetAsync(d.resMax, 0, sizeof(double), c.stream));
+            launch(1, c.scratch[slot]);
+            if (stage == 1) return check_launch(c, "cn");
+            int s = read_res(res);
+            if (s) return s;
+        } else {
+            res = c.hscal[comp] * Dn;
+        }
         if (!std::isfinite(res)) {
             c.err = "Jacobi residual is not finite";
             status = SARAS_NOT_FINITE;
@@ -1940,7 +1950,7 @@ static int cn_solve_delta(Ctx &c, int comp, int field, const CnFast &fa, double 
     }
     if (status == SARAS_OK && spec >= 0) {
         while (true) {
-            SARAS_CUDA_TRY(cudaMemsetAsync(c.dscal, 0, sizeof(double), c.stream));
+            SARAS_CUDA_TRY(cudaMemsetAsync(d.resMax, 0, sizeof(double), c.stream));
             launch(1, nullptr);
             int s = read_res(res);
             if (s) return s;
@@ -1972,7 +1982,7 @@ static int cn_solve_delta(Ctx &c, int comp, int field, const CnFast &fa, double 
     return status;
 }
 
-int cn_solve(Ctx &c, int comp, int *iters, double *maxerr) {
+static int cn_solve_stage(Ctx &c, int comp, int *iters, double *maxerr, int stage) {
     if (comp < 0 || comp > 3) return SARAS_BAD_ARG;
     if (comp == 3 && !c.scalar) return SARAS_BAD_ARG;
     if (comp == 1 && c.planar) { c.err = "the 2D solver has no Vy equation"; return SARAS_BAD_ARG; }
@@ -1986,7 +1996,7 @@ int cn_solve(Ctx &c, int comp, int *iters, double *maxerr) {
     double bytes = 3.0 * 8.0 * (double)make_view<double>(nullptr, f.n[0], f.n[1], f.n[2]).size();
     bool fast = c.p.fastKernels != 0;
     const double resScale = fast ? a.Dn : 1.0;
-    if (c.p.fastKernels == 2) return cn_solve_delta(c, comp, field, fa, a.Dn, bytes, iters, maxerr);
+    if (c.p.fastKernels == 2) return cn_solve_delta(c, comp, field, fa, a.Dn, bytes, iters, maxerr, stage);
     auto launch = [&](int withRes) {
         if (fast) {
             fa.in = cview(c, field);
@@ -2037,6 +2047,27 @@ int cn_solve(Ctx &c, int comp, int *iters, double *maxerr) {
     }
     if (iters) *iters = sweeps;
     if (maxerr) *maxerr = res;
+    return SARAS_OK;
+}
+
+int cn_solve(Ctx &c, int comp, int *iters, double *maxerr) { return cn_solve_stage(c, comp, iters, maxerr, 0); }
+
+// fastKernels = 2: the velocity components' launches up to their speculative final
+// sweeps (each reads its own A and writes its own field's partner) with one copy of
+// the three residuals and one wait instead of three: 65^3 step 537 -> 507 us.  Only
+// when no component takes more sweeps than those two: further ones share the D buffers.
+static int cn_together(Ctx &c, bool *begun) {
+    *begun = false;
+    if (c.p.fastKernels != 2) return SARAS_OK;
+    for (int q = 0; q < 3; ++q)
+        if (c.cnSweeps[q] > 2) return SARAS_OK;
+    for (int q = 0; q < 3; ++q) {
+        if (c.planar && q == 1) continue;
+        if (int e = cn_solve_stage(c, q, nullptr, nullptr, 1)) return e;
+    }
+    SARAS_CUDA_TRY(cudaMemcpyAsync(c.hscal, c.dscal, 3 * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+    SARAS_CUDA_TRY(cudaStreamSynchronize(c.stream));
+    *begun = true;
     return SARAS_OK;
 }
 
@@ -2254,11 +2285,13 @@ int time_advance(Ctx &c, saras_step_stats *st) {
     saras_step_stats local;
     std::memset(&local, 0, sizeof(local));
     int s = compute_rhs(c);
+    bool begun = false;
+    if (!s) s = cn_together(c, &begun);
     if (s) { for (int &q : c.n0Fresh) q = 0; return s; }
     for (int q = 0; q < 3; ++q) {
         if (c.planar && q == 1) continue;   // hydro_d2.cc:242-244: solveVx, solveVz
         int it = 0; double e = 0;
-        s = cn_solve(c, q, &it, &e);
+        s = cn_solve_stage(c, q, &it, &e, begun ? 2 : 0);
         local.cn_iters[q] = it;
         if (s) { for (int &r : c.n0Fresh) r = 0; local.status = s; if (st) *st = local; return s; }
     }
@@ -2310,6 +2343,7 @@ int time_advance(Ctx &c, saras_step_stats *st) {
 namespace saras {
 
 constexpr long kNoAllocMaxPoints = 4L << 20;   // 4 Mi doubles (32 MiB): padded field arrays up to this size
+constexpr long kCnBatchPoints = 128L << 10;   // at most kNoAllocMaxPoints / 4
 static __device__ __align__(256) double g_cn_scratch[kNoAllocMaxPoints + 32];
 // Device address of g_cn_scratch, per device ordinal.  Atomic: two host
 // threads making their first call on a device at the same time both look the
@@ -2380,7 +2414,7 @@ extern "C" int saras_cn_solve_noalloc(const saras_params *p, int component, doub
         }
         g_cn_scratch_dev[dev].store(scratch, std::memory_order_release);
     }
-    double *resSlot = scratch + kNoAllocMaxPoints;
+    double *const resSlots = scratch + kNoAllocMaxPoints;   // one per sweep of a batch
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
 
     // grid constants (grid.cc:84-86, 405-421; hydro.cc:223-241)
@@ -2464,7 +2498,7 @@ extern "C" int saras_cn_solve_noalloc(const saras_params *p, int component, doub
     a.lx = m2[0] * (1.0 / (dXi[0] * dXi[0]));
     a.ly = m2[1] * (1.0 / (dXi[1] * dXi[1]));
     a.lz = m2[2] * (1.0 / (dXi[2] * dXi[2]));
-    a.resMax = resSlot;
+    a.resMax = resSlots;
     dim3 g, bl; box_launch_dims(fb, g, bl);
 
     // the fused multiply-add form when the parameters ask for it, as cn_solve does
@@ -2478,45 +2512,61 @@ extern "C" int saras_cn_solve_noalloc(const saras_params *p, int component, doub
         fa.resMax = a.resMax;
     }
     const double resScale = fast ? a.Dn : 1.0;
-    double *cur = v, *nxt = scratch;
+    // The iterates go round a ring: iterate n is in buffer n mod ring, buffer 0 being v
+    // and the others fields in the fixed array.  Sweep n + 1 writes the next iterate and,
+    // from the first on, the residual of iterate n; ring - 1 sweeps run between waits,
+    // their residuals are read in one copy and tested in order, and sweeps beyond the
+    // accepted iterate are thrown away.  A wait costs as much as several sweeps of a
+    // small field (33^3: a solve 106 -> 81 us), but less than one of a large field, which
+    // waits after each sweep.
+    constexpr int kRing = 5;
+    const int ring = points <= kCnBatchPoints ? kRing : 2;
+    const int batch = ring - 1;
+    auto buf = [&](int n) { return n % ring == 0 ? v : scratch + (long)(n % ring - 1) * points; };
     auto view_of = [&](double *ptr) { return make_view<double>(ptr, f.n[0], f.n[1], f.n[2]); };
-    auto launch = [&](int withRes) {
-        View3<double> in = view_of(cur), out = view_of(nxt);
+    auto launch = [&](int n, double *slot) {   // iterate n -> n + 1; slot: iterate n's residual
+        View3<double> in = view_of(buf(n)), out = view_of(buf(n + 1));
         View3<const double> cin;
         cin.p = in.p; cin.n[0] = in.n[0]; cin.n[1] = in.n[1]; cin.n[2] = in.n[2]; cin.sx = in.sx; cin.sy = in.sy;
         if (fast) {
-            fa.in = cin; fa.out = out; fa.withResidual = withRes;
+            fa.in = cin; fa.out = out; fa.withResidual = slot ? 1 : 0; fa.resMax = slot;
             // fastKernels 1 and 2 both run this fused multiply-add form: the
             // split-FP64 form of fastKernels = 2 keeps N0 and the correction
             // as float pairs, 12 more floats a point than the fixed array holds
             k_cn_fast<<<g, bl, 0, st>>>(fa);
         } else {
-            a.in = cin; a.out = out; a.withResidual = withRes;
+            a.in = cin; a.out = out; a.withResidual = slot ? 1 : 0; a.resMax = slot;
             k_cn<<<g, bl, 0, st>>>(a);
         }
         return cudaGetLastError();
     };
-    cudaError_t e = launch(0);
+    cudaError_t e = launch(0, nullptr);
     if (e != cudaSuccess) { set_error(cudaGetErrorString(e)); return SARAS_CUDA_ERROR; }
-    std::swap(cur, nxt);
-    int sweeps = 1, failed = 0;
-    double res = 0.0;
+    int sweeps = 1, failed = 0, done = 1;   // iterate under test; iterates computed
+    double res = 0.0, got[kRing];
     int status = SARAS_OK;
-    while (true) {
-        if ((e = cudaMemsetAsync(resSlot, 0, sizeof(double), st)) != cudaSuccess) break;
-        if ((e = launch(1)) != cudaSuccess) break;
-        if ((e = cudaMemcpyAsync(&res, resSlot, sizeof(double), cudaMemcpyDeviceToHost, st)) != cudaSuccess) break;
+    bool more = true;
+    while (more) {
+        const int n = batch;
+        if ((e = cudaMemsetAsync(resSlots, 0, sizeof(double) * n, st)) != cudaSuccess) break;
+        for (int q = 0; q < n && e == cudaSuccess; ++q) e = launch(done++, resSlots + q);
+        if (e != cudaSuccess) break;
+        if ((e = cudaMemcpyAsync(got, resSlots, sizeof(double) * n, cudaMemcpyDeviceToHost, st)) != cudaSuccess) break;
         if ((e = cudaStreamSynchronize(st)) != cudaSuccess) break;
-        res *= resScale;
-        if (!std::isfinite(res)) { set_error("Jacobi residual is not finite"); status = SARAS_NOT_FINITE; break; }
-        if (res < p->cnTolerance) break;
-        failed += 1;
-        if (failed > maxIterations) { status = SARAS_NOT_CONVERGED; break; }
-        std::swap(cur, nxt);
-        sweeps += 1;
+        for (int q = 0; q < n; ++q) {
+            res = got[q] * resScale;
+            more = false;
+            if (!std::isfinite(res)) { set_error("Jacobi residual is not finite"); status = SARAS_NOT_FINITE; break; }
+            if (res < p->cnTolerance) break;
+            failed += 1;
+            if (failed > maxIterations) { status = SARAS_NOT_CONVERGED; break; }
+            more = true;
+            sweeps += 1;
+        }
     }
     if (e != cudaSuccess) { set_error(cudaGetErrorString(e)); return SARAS_CUDA_ERROR; }
-    // the answer is `cur`; bring it into the caller's array if it sits in the scratch
+    // the answer is iterate `sweeps`; bring it into the caller's array if it sits in the scratch
+    const double *cur = buf(sweeps);
     if (cur != v) {
         if ((e = cudaMemcpyAsync(v, cur, sizeof(double) * points, cudaMemcpyDeviceToDevice, st)) != cudaSuccess ||
             (e = cudaStreamSynchronize(st)) != cudaSuccess) {
