@@ -150,7 +150,7 @@ struct Ctx {
     void *unet = nullptr;
     double *pHist[3] = {nullptr, nullptr, nullptr};   // Pp of the three previous steps (newest first)
     long long *fx[3] = {nullptr, nullptr, nullptr};   // level-0 fixed-point iterate ping-pong + rhs (mixed mode)
-    bool fxPlain = false;   // the V-cycle being issued runs level 0 on integers (plain_fixed)
+    int fxPlain = 0;   // levels that the V-cycle being issued runs on integers (plain_fixed)
     float *cnp = nullptr;      // split-FP64 Jacobi solve: N0 of each component and the D ping-pong (float pairs)
     long cnpCount = 0;
     int n0Fresh[4] = {0, 0, 0, 0};   // N0 of component q written by this step's right-hand side

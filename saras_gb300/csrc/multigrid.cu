@@ -7,7 +7,8 @@
 //                          coarsest Gauss-Seidel to mgTolerance / maxCount).
 //   SARAS_MG_PLAIN_TARGET  FP64 V-cycles on the compatible system until
 //                          max|b-Ap| <= target * max|b|.
-//                          (an isotropic level 0 in 64-bit fixed point, k_fx_sweep).
+//                          (levels above the tail in 64-bit fixed point when
+//                          the stencil is isotropic, k_fx_sweep).
 //   SARAS_MG_MIXED         FP32 V-cycles as the inner solver of an
 //                          iterative-refinement loop to the same target; the
 //                          outer residual is FP64, or exact 64-bit fixed point
@@ -1881,8 +1882,8 @@ __global__ void __launch_bounds__(256, 3) k_fx_refine(const long long *__restric
     block_max_bits_to(m, reinterpret_cast<double *>(maxr));
 }
 
-// ---- fixed-point V-cycle on level 0 (SARAS_MG_PLAIN_TARGET, isotropic level 0)
-// The same integers P and B carry the plain mode's finest level: with d = sum of the
+// ---- fixed-point V-cycle (SARAS_MG_PLAIN_TARGET, isotropic levels)
+// The same integers P and B carry the plain mode's levels above the tail: with d = sum of the
 // six neighbours - 6 P - B (exact), the damped Jacobi sweep of weight w is
 // P + d w / 6, one 64 x 64 -> 128 bit multiplication by w / 6 in units of 2^-64; the
 // residual for the level below is -d, exact, where an FP64 residual loses the
@@ -1893,19 +1894,28 @@ __global__ void __launch_bounds__(256, 3) k_fx_refine(const long long *__restric
 // 129^3): 2.0e-15 / 8.7e-15 / 3.8e-14, with FP64 levels 4.2e-15 / 2.8e-14 / 9.9e-14.  An FP64 sweep is bound by the FP64 pipe (one warp instruction in
 // 64 clocks on an SM quarter), the integer one by HBM: at
 // 257^3 a sweep 265 -> 76 us, residual 265 -> 70, its maximum 298 -> 62, restriction
-// 134 -> 32, prolongation 182 -> 93; a step 14.6 -> 9.0 ms.
-// Level 0's arrays hold the integers themselves (pa, pb, r), so the mode takes no more
-// memory.  flag: a value beyond +-2^59, where sums of seven terms could pass 2^63.
+// 134 -> 32, prolongation 182 -> 55; a step 14.6 -> 9.0 ms with level 0 alone, 6.2 with
+// every level above the tail (129^3: sweep 37 -> 13 us).
+// The levels' arrays hold the integers themselves (pa, pb, r), so the mode takes no more
+// memory.  flag: P beyond +-2^59 or B beyond +-2^60, above which a sum could pass 2^63.
 __device__ __forceinline__ bool fx_far(long long p) { return p > (1LL << 59) || p < -(1LL << 59); }
 
-// ROUND: the sweep whose output the solve may return (round53).
-template <bool ROUND, int CH>
+// ROUND: the sweep whose output the solve may return (round53).  ZERO: from P = 0.
+template <bool ROUND, bool ZERO, int CH>
 __global__ void __launch_bounds__(256, 3) k_fx_sweep(long long *__restrict__ out, const long long *__restrict__ in, const long long *__restrict__ bfx,
                                                      int sx, int sy, MgBC bc, long long w6, int *flag) {
     pdl_wait();
     int j, k, seg;
     if (!col_of<true>(bc, j, k, seg)) return;
     bool bad = false;
+    if (ZERO) {
+        const int i0 = seg * CH;
+        const long o = (long)(i0 + 1) * sx + (long)(j + 1) * sy + (k + 1);
+#pragma unroll
+        for (int q = 0; q < CH; ++q)
+            if (i0 + q <= bc.E[0]) out[o + (long)q * sx] = __mul64hi(-bfx[o + (long)q * sx], w6);
+        return;
+    }
     fx_column<CH>(in, bfx, sx, sy, bc, j, k, seg, [&](long o, long long cc, long long d) {
         long long v = cc + __mul64hi(d, w6);
         if (ROUND) v = round53(v);
@@ -1927,10 +1937,12 @@ __global__ void __launch_bounds__(256, 3) k_fx_residual(long long *__restrict__ 
 
 // Full weighting of the integer residual (k_tgt_restrict's stencil): exact sums in a
 // plane, the planes' sum in units of four (residuals up to 2^58 stay inside 63 bits),
-// then one conversion: scale[0] = l 2^-s / 16.
-template <int CH>
-__global__ void __launch_bounds__(256, 4) k_fx_restrict(double *__restrict__ rc, const long long *__restrict__ r, int sx, int sy, int csx, int csy,
-                                                        MgBC bcf, const double *__restrict__ scale) {
+// then one conversion (scale[0] = l 2^-s / 16), or, to a level in fixed point, the
+// shift sh: B = 4 R there (a quarter of l), and twice that below level 0, whose unit is
+// two of the others'.
+template <typename TC, int CH>
+__global__ void __launch_bounds__(256, 4) k_fx_restrict(TC *__restrict__ rc, const long long *__restrict__ r, int sx, int sy, int csx, int csy,
+                                                        MgBC bcf, const double *__restrict__ scale, int sh, int *flag) {
     pdl_wait();
     const int E0 = bcf.E[0], E1 = bcf.E[1], E2 = bcf.E[2];
     const int W = E2 / 2 + 1, t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1953,47 +1965,56 @@ __global__ void __launch_bounds__(256, 4) k_fx_restrict(double *__restrict__ rc,
         }
         return (row[0] + 2 * row[1] + row[2] + 2) >> 2;
     };
-    const double mul = scale[0];
+    const double mul = std::is_same<TC, double>::value ? scale[0] : 0.0;
+    bool bad = false;
     const int Iend = min(I0 + CH - 1, E0 / 2);
     long long lo = plane(2 * I0 - 1);
 #pragma unroll 2
     for (int I = I0; I <= Iend; ++I) {
         const long long mid = plane(2 * I), hi = plane(2 * I + 1);
-        rc[(long)(I + 1) * csx + (long)(J + 1) * csy + (K + 1)] = __ll2double_rn(lo + 2 * mid + hi) * mul;
+        const long o = (long)(I + 1) * csx + (long)(J + 1) * csy + (K + 1);
+        if constexpr (std::is_same<TC, double>::value) rc[o] = __ll2double_rn(lo + 2 * mid + hi) * mul;
+        else {
+            rc[o] = (lo + 2 * mid + hi + (1LL << (sh - 1))) >> sh;
+            bad |= rc[o] > (1LL << 60) || rc[o] < -(1LL << 60);
+        }
         lo = hi;
     }
+    if (bad) atomicExch(flag, 1);
 }
 
-// k_tgt_prolong_add on the integers: the coarse FP64 correction in units of 2^-(s + 1)
-// (scale[1] holds s), its trilinear interpolant exact in units of 2^-(s + 4), rounded
-// once.
-template <bool ROUND, int CH>
-__global__ void __launch_bounds__(256, 3) k_fx_prolong_add(long long *__restrict__ pf, const double *__restrict__ pc, int sxf, int syf, int sxc,
-                                                           int syc, MgBC bc, const double *__restrict__ scale, int *flag) {
+// k_tgt_prolong_add on the integers: an FP64 coarse correction in units of 2^-(s + 1)
+// (scale[1] holds s), one in fixed point in its own; the trilinear interpolant, eight of
+// them exact, rounded once by the shift sh.
+template <bool ROUND, typename TC, int CH>
+__global__ void __launch_bounds__(256, 3) k_fx_prolong_add(long long *__restrict__ pf, const TC *__restrict__ pc, int sxf, int syf, int sxc,
+                                                           int syc, MgBC bc, const double *__restrict__ scale, int sh, int *flag) {
     pdl_wait();
     int j, k, seg;
     if (!col_of<true>(bc, j, k, seg)) return;
-    const int s1 = (int)scale[1] + 1;
+    const int s1 = std::is_same<TC, double>::value ? (int)scale[1] + 1 : 0;
     const int i0 = seg * CH;   // CH is even
     const int iend = min(i0 + CH - 1, bc.E[0]);
     const int k2 = k >> 1, j2 = j >> 1;
     const int k1 = k & 1, j1 = (j & 1) ? syc : 0;   // offsets of the second coarse neighbours (the point itself where it has none)
     bool bad = false;
-    auto fx = [&](double v) -> long long {
-        const long long q = d2fx(v, s1, bad);
-        bad |= fx_far(q);
-        return q;
+    auto fx = [&](TC v) -> long long {
+        if constexpr (std::is_same<TC, double>::value) {
+            const long long q = d2fx(v, s1, bad);
+            bad |= fx_far(q);
+            return q;
+        } else return v;
     };
     auto A = [&](int m) -> long long {   // coarse plane m at (j, k), times 4
-        const double *q = pc + (long)(m + 1) * sxc + (long)(j2 + 1) * syc + (k2 + 1);
+        const TC *q = pc + (long)(m + 1) * sxc + (long)(j2 + 1) * syc + (k2 + 1);
         const long long a = fx(q[0]);
         long long v = k1 ? a + fx(q[1]) : 2 * a;
         if (!j1) return 2 * v;
         const long long b = fx(q[syc]);
         return v + (k1 ? b + fx(q[syc + 1]) : 2 * b);
     };
-    auto put = [&](long o, long long p, long long e8) {   // e8: eight times the correction in units of 2^-(s + 1)
-        long long v = p + ((e8 + 8) >> 4);
+    auto put = [&](long o, long long p, long long e8) {   // e8: eight times the correction in the coarse unit
+        long long v = p + ((e8 + (1LL << (sh - 1))) >> sh);
         if (ROUND) v = round53(v);
         bad |= fx_far(v);
         pf[o] = v;
@@ -3447,70 +3468,81 @@ static int tail_run(Ctx &c, int Lt, bool big) {
     return chk(c, "mg tail");
 }
 
-// Level 0 of a fixed-point V-cycle (k_fx_sweep and its companions): smooth,
+// A level of a fixed-point V-cycle (k_fx_sweep and its companions): smooth,
 // restrict_level and prolong_level on the integers in pa, pb and r.
 static long long *fx_of(double *p) { return reinterpret_cast<long long *>(p); }
 static int *fx_flag(Ctx &c) { return reinterpret_cast<int *>(c.dscal + 35); }
 static const double *fx_scale(Ctx &c) { return c.dscal + 36; }
+static bool fx_level(const Ctx &c, int l) { return l < c.fxPlain; }
 
-static int fx_smooth(Ctx &c, int count, bool last) {
-    Level &L = c.lv[0];
-    MgBC bc = level_bc(c, 0, true);
+static int fx_smooth(Ctx &c, int l, int count, bool zero, bool last) {
+    Level &L = c.lv[l];
+    MgBC bc = level_bc(c, l, true);
     const double bytes = 3.0 * 8.0 * (double)(L.n[0] + 1) * (L.n[1] + 1) * (L.n[2] + 1);
     const int sx = (L.n[1] + 3) * (L.n[2] + 3), sy = L.n[2] + 3;
     dim3 g, b;
     const int ch = level_dims<double>(c, L, g, b);
     for (int n = 0; n < count; ++n) {
         const long long w6 = std::llround(std::ldexp(smooth_weight(c, n, count) / 6.0, 64));
-        prof_begin(c, PK_MG_SMOOTH64, 0);
+        prof_begin(c, PK_MG_SMOOTH64, l);
         SARAS_CUDA_TRY(with_march<double>(ch, [&](auto m) {
             constexpr int CH = decltype(m)::value;
-            return launch_pdl(last && n == count - 1 ? k_fx_sweep<true, CH> : k_fx_sweep<false, CH>, g, b, 0, c.stream, fx_of(L.pb()), fx_of(L.pa()),
-                              fx_of(L.r), sx, sy, bc, w6, fx_flag(c));
+            return launch_pdl(zero && n == 0               ? k_fx_sweep<false, true, CH>
+                              : last && n == count - 1 ? k_fx_sweep<true, false, CH>
+                                                       : k_fx_sweep<false, false, CH>,
+                              g, b, 0, c.stream, fx_of(L.pb()), fx_of(L.pa()), fx_of(L.r), sx, sy, bc, w6, fx_flag(c));
         }));
         count_launch(c);
-        prof_end(c, PK_MG_SMOOTH64, 0, bytes);
+        prof_end(c, PK_MG_SMOOTH64, l, zero && n == 0 ? bytes * 2.0 / 3.0 : bytes);
         flip<double>(L);
     }
     return chk(c, "fixed-point smooth");
 }
 
-static int fx_restrict(Ctx &c) {
-    Level &L = c.lv[0], &C = c.lv[1];
-    MgBC bc = level_bc(c, 0, true);
+static int fx_restrict(Ctx &c, int l) {
+    Level &L = c.lv[l], &C = c.lv[l + 1];
+    MgBC bc = level_bc(c, l, true);
     const double pts = (double)(L.n[0] + 1) * (L.n[1] + 1) * (L.n[2] + 1);
     const int sx = (L.n[1] + 3) * (L.n[2] + 3), sy = L.n[2] + 3, csx = (C.n[1] + 3) * (C.n[2] + 3), csy = C.n[2] + 3;
     dim3 g, b;
     const int ch = level_dims<double>(c, L, g, b);
-    prof_begin(c, PK_MG_RESID64, 0);
+    prof_begin(c, PK_MG_RESID64, l);
     SARAS_CUDA_TRY(with_march<double>(ch, [&](auto m) {
         return launch_pdl(k_fx_residual<decltype(m)::value>, g, b, 0, c.stream, fx_of(L.pb()), fx_of(L.pa()), fx_of(L.r), sx, sy, bc);
     }));
-    prof_end(c, PK_MG_RESID64, 0, 3.0 * 8.0 * pts);
+    prof_end(c, PK_MG_RESID64, l, 3.0 * 8.0 * pts);
     const long ccols = (long)(C.n[1] + 1) * (C.n[2] + 1);
     const int rch = ch == kIch ? rr_ch<double>() : 1;
     dim3 gr((unsigned)((ccols + 255) / 256), (C.n[0] + 1 + rch - 1) / rch, 1);
-    prof_begin(c, PK_MG_RESTRICT64, 0);
-    SARAS_CUDA_TRY(launch_pdl(ch == kIch ? k_fx_restrict<rr_ch<double>()> : k_fx_restrict<1>, gr, dim3(256, 1, 1), 0, c.stream, C.r, fx_of(L.pb()), sx,
-                              sy, csx, csy, bc, fx_scale(c)));
-    prof_end(c, PK_MG_RESTRICT64, 0, 8.0 * pts * (1.0 + 1.0 / 8.0));
+    prof_begin(c, PK_MG_RESTRICT64, l);
+    auto run = [&](auto k, auto *rc) {
+        return launch_pdl(k, gr, dim3(256, 1, 1), 0, c.stream, rc, fx_of(L.pb()), sx, sy, csx, csy, bc, fx_scale(c), l == 0 ? 1 : 2, fx_flag(c));
+    };
+    constexpr int kCh = rr_ch<double>();
+    if (fx_level(c, l + 1)) SARAS_CUDA_TRY(run(ch == kIch ? k_fx_restrict<long long, kCh> : k_fx_restrict<long long, 1>, fx_of(C.r)));
+    else SARAS_CUDA_TRY(run(ch == kIch ? k_fx_restrict<double, kCh> : k_fx_restrict<double, 1>, C.r));
+    prof_end(c, PK_MG_RESTRICT64, l, 8.0 * pts * (1.0 + 1.0 / 8.0));
     count_launch(c, 2);
     return chk(c, "fixed-point restrict");
 }
 
-static int fx_prolong(Ctx &c, bool last) {
-    Level &L = c.lv[0], &C = c.lv[1];
-    MgBC bc = level_bc(c, 0, true);
+static int fx_prolong(Ctx &c, int l, bool last) {
+    Level &L = c.lv[l], &C = c.lv[l + 1];
+    MgBC bc = level_bc(c, l, true);
     const double pts = (double)(L.n[0] + 1) * (L.n[1] + 1) * (L.n[2] + 1);
     dim3 g, b;
     const int ch = level_dims<double>(c, L, g, b);
-    prof_begin(c, PK_MG_PROLONG64, 0);
+    prof_begin(c, PK_MG_PROLONG64, l);
     SARAS_CUDA_TRY(with_march<double>(ch, [&](auto m) {
         constexpr int CH = decltype(m)::value;
-        return launch_pdl(last ? k_fx_prolong_add<true, CH> : k_fx_prolong_add<false, CH>, g, b, 0, c.stream, fx_of(L.pa()), C.pa(),
-                          (L.n[1] + 3) * (L.n[2] + 3), L.n[2] + 3, (C.n[1] + 3) * (C.n[2] + 3), C.n[2] + 3, bc, fx_scale(c), fx_flag(c));
+        auto run = [&](auto k, auto *pc) {
+            return launch_pdl(k, g, b, 0, c.stream, fx_of(L.pa()), pc, (L.n[1] + 3) * (L.n[2] + 3), L.n[2] + 3, (C.n[1] + 3) * (C.n[2] + 3), C.n[2] + 3,
+                              bc, fx_scale(c), l > 0 && fx_level(c, l + 1) ? 3 : 4, fx_flag(c));
+        };
+        if (fx_level(c, l + 1)) return run(last ? k_fx_prolong_add<true, long long, CH> : k_fx_prolong_add<false, long long, CH>, fx_of(C.pa()));
+        return run(last ? k_fx_prolong_add<true, double, CH> : k_fx_prolong_add<false, double, CH>, C.pa());
     }));
-    prof_end(c, PK_MG_PROLONG64, 0, 8.0 * pts * (2.0 + 1.0 / 8.0));
+    prof_end(c, PK_MG_PROLONG64, l, 8.0 * pts * (2.0 + 1.0 / 8.0));
     count_launch(c);
     return chk(c, "fixed-point prolong");
 }
@@ -3530,14 +3562,14 @@ static int cycle_from(Ctx &c, int l, bool tgt, bool zero, int gamma) {
     if (l == c.depth) return coarse_solve<T>(c, tgt);
     const int pre = l > 0 ? coarse_sweeps(c, tgt, true) : c.p.preSmooth;
     const int post = l > 0 ? coarse_sweeps(c, tgt, false) : c.p.postSmooth;
-    const bool fx = sizeof(T) == 8 && l == 0 && c.fxPlain;   // level 0 on integers (plain_fixed)
-    if ((s = fx ? fx_smooth(c, pre, false) : smooth<T>(c, l, pre, zero, tgt))) return s;
-    if ((s = fx ? fx_restrict(c) : restrict_level<T>(c, l, tgt))) return s;
+    const bool fx = sizeof(T) == 8 && tgt && fx_level(c, l);   // the level on integers (plain_fixed)
+    if ((s = fx ? fx_smooth(c, l, pre, l > 0 && zero, false) : smooth<T>(c, l, pre, zero, tgt))) return s;
+    if ((s = fx ? fx_restrict(c, l) : restrict_level<T>(c, l, tgt))) return s;
     const int g = l == 0 ? gamma : 1;
     for (int q = 0; q < g; ++q)
         if ((s = cycle_from<T>(c, l + 1, tgt, q == 0, 1))) return s;
-    if ((s = fx ? fx_prolong(c, post == 0) : prolong_level<T>(c, l, tgt, true))) return s;
-    return fx ? fx_smooth(c, post, true) : smooth<T>(c, l, post, false, tgt);
+    if ((s = fx ? fx_prolong(c, l, l == 0 && post == 0) : prolong_level<T>(c, l, tgt, true))) return s;
+    return fx ? fx_smooth(c, l, post, false, l == 0) : smooth<T>(c, l, post, false, tgt);
 }
 
 template <typename T>
@@ -3660,7 +3692,7 @@ template <typename T>
 static int vcycle_tgt(Ctx &c, bool zero0) {
     const int buf = sizeof(T) == 4 ? c.lv[0].cur32 : c.lv[0].cur;
     // FP64 cycles never start from zero: that slot holds the fixed-point cycle's graph
-    return graph_replay(c, sizeof(T) == 4 ? 1 : 0, (zero0 || (sizeof(T) == 8 && c.fxPlain) ? 1 : 0) + 2 * buf,
+    return graph_replay(c, sizeof(T) == 4 ? 1 : 0, (zero0 || (sizeof(T) == 8 && c.fxPlain > 0) ? 1 : 0) + 2 * buf,
                         [&]() { return vcycle<T>(c, true, zero0); });
 }
 
@@ -4012,7 +4044,7 @@ static int mixed_fixed(Ctx &c, const double *pp0, double mean, double bmax, doub
     return fp64_start();
 }
 
-// The plain mode's solve with level 0 in fixed point (k_fx_sweep): V-cycles until the
+// The plain mode's solve in fixed point (k_fx_sweep): V-cycles until the
 // exact residual meets the target.  done: the result is in Pp; otherwise (no scale to
 // take from the previous Pp, or values out of range) nothing the FP64 path reads has changed.
 static int plain_fixed(Ctx &c, const double *pp0, double mean, double bmax, double pmax, double target, double &r, int &cyc, bool &done,
@@ -4020,13 +4052,16 @@ static int plain_fixed(Ctx &c, const double *pp0, double mean, double bmax, doub
     done = false;
     Level &L0 = c.lv[0];
     const double l = L0.lx;
-    // the previous Pp sets the scale (2^57 <= max|P| < 2^58); B has to fit it (|B| < 2^59)
-    if (!(pmax > 0.0) || !std::isfinite(pmax) || !(bmax / l <= 2.0 * pmax)) return SARAS_OK;
+    // the previous Pp sets the scale (2^57 <= max|P| < 2^58); B has to fit it (|B| < 2^60)
+    if (!(pmax > 0.0) || !std::isfinite(pmax) || !(bmax / l <= 4.0 * pmax)) return SARAS_OK;
     const int sc = 57 - std::ilogb(pmax);
     if (sc < -900 || sc > 900) return SARAS_OK;
-    for (int n = 0; n < std::max(c.p.preSmooth, c.p.postSmooth); ++n)   // w / 6 in 63 bits
-        for (int count : {c.p.preSmooth, c.p.postSmooth})
-            if (n < count && !(std::fabs(smooth_weight(c, n, count)) < 2.9)) return SARAS_OK;
+    const int cpre = coarse_sweeps(c, true, true), cpost = coarse_sweeps(c, true, false);
+    for (int count : {c.p.preSmooth, c.p.postSmooth, cpre, cpost})   // w / 6 in 63 bits
+        for (int n = 0; n < count; ++n)
+            if (!(std::fabs(smooth_weight(c, n, count)) < 2.9)) return SARAS_OK;
+    // the levels below too, in units of half of level 0's, down to the tail or the coarsest
+    const int levels = cpre > 0 ? (c.tailLt > 0 ? c.tailLt : c.depth) : 1;
     MgBC bc0 = level_bc(c, 0, true);
     const int sx = (L0.n[1] + 3) * (L0.n[2] + 3), sy = L0.n[2] + 3;
     dim3 gk, bk; col_dims(L0, gk, bk);
@@ -4034,8 +4069,9 @@ static int plain_fixed(Ctx &c, const double *pp0, double mean, double bmax, doub
     unsigned long long *dmax = reinterpret_cast<unsigned long long *>(c.dscal + 34);
     const double inv2s = std::ldexp(1.0, -sc), rs = l * inv2s;
     SARAS_CUDA_TRY(cudaMemsetAsync(c.dscal + 34, 0, sizeof(double) * 2, c.stream));
-    c.hscal[36] = rs * 0.0625;
-    c.hscal[37] = (double)sc;
+    const int sl = sc + (levels > 1 ? 1 : 0);   // fx_scale: of the last level in fixed point
+    c.hscal[36] = c.lv[levels - 1].lx * std::ldexp(0.0625, -sl);
+    c.hscal[37] = (double)sl;
     SARAS_CUDA_TRY(cudaMemcpyAsync(c.dscal + 36, c.hscal + 36, 2 * sizeof(double), cudaMemcpyHostToDevice, c.stream));
     L0.cur = 0;
     k_fx_rhs<<<gk, bk, 0, c.stream>>>(fx_of(L0.r), nullptr, c.f[SARAS_FIELD_MGRHS], sx, sy, bc0, mean, std::ldexp(1.0, sc) / l, fx_flag(c));
@@ -4062,9 +4098,9 @@ static int plain_fixed(Ctx &c, const double *pp0, double mean, double bmax, doub
     if (s) return s;
     if (!bad && st) { st->guess_residual = bmax > 0 ? r / bmax : r; st->guess_source = 0; }
     while (!bad && r > target && cyc < c.mgMaxCycles) {
-        c.fxPlain = true;
+        c.fxPlain = levels;
         s = vcycle_tgt<double>(c, false);
-        c.fxPlain = false;
+        c.fxPlain = 0;
         if (s) return s;
         cyc += 1;
         if ((s = residual())) return s;
@@ -4108,8 +4144,8 @@ static int mg_solve_target_run(Ctx &c, int *cycles, double *residual, saras_step
     dim3 gk0, bk0; col_dims(L0, gk0, bk0);
     int nparts = (int)(gk0.x * gk0.y);
     if (nparts > c.redCap) { c.err = "reduction buffer too small"; return SARAS_TOO_LARGE; }
-    // the plain mode's levels are FP64 but for an isotropic level 0, in fixed point unless a
-    // guess or training reads b from level-0 r
+    // the plain mode's isotropic levels in fixed point, unless a guess or training reads b
+    // from level-0 r
     const bool fixedPlain = c.mgMode == SARAS_MG_PLAIN_TARGET && L0.lx == L0.ly && L0.ly == L0.lz && c.depth > 0 && c.tailLt != 0 && !wantGuess &&
                             !c.collecting && !c.unet && !c.ppInHist;
     k_tgt_stats<<<gk0, bk0, 0, c.stream>>>(lcview<double>(L0, rhs), fixedPath || fixedPlain ? pp0 : nullptr, bc0, c.red, c.dscal + 31, c.dscal + 32,
