@@ -4,22 +4,23 @@
 // GEMM view (channels-last activations X[z][y][x][C]):
 //   out[m][n] = sum_k A[m][k] * B[n][k],   m = output voxel, n = output channel,
 //   k = (tap, input channel), 27 taps, input channels in chunks of 16.
-// One CTA (4 warps) owns 128 consecutive output voxels (M = 128) and all N
-// output channels.  Each K step is one tcgen05.mma (K = 16): the A tile (128
-// voxels x 16 channels of one tap, gathered with cp.async, zero outside the
-// domain) and the B tile (N x 16 packed weights) sit in shared memory in the
-// canonical K-major layout without swizzle: 8x8 "core matrices" of 128 bytes,
-// K-adjacent core matrices 128 B apart (leading byte offset), M/N-adjacent
-// ones 256 B apart (stride byte offset).  A four-stage ring of three K steps a
-// stage overlaps the gathers with the MMAs (a barrier and a wait a K step bounded the
-// kernel); tcgen05.commit arrives on a per-stage mbarrier that
-// releases the stage for reuse.  The gathers' index work is a table lookup and a
-// mask a tap (each voxel's position against the faces is one set of bits), and a warp
-// gathers whole 32-byte sectors of consecutive voxels through L1, where the next
-// taps find them: 50 us for 16 -> 16 channels on 65^3 voxels (237 MB of taps), 65
-// with one K step a barrier and half-sector gathers past L1.  The accumulator (128 lanes x N FP32 columns)
-// is read back with tcgen05.ld: warp w reads lanes 32w..32w+31, i.e. thread t
-// of the CTA reads the N channels of voxel t, matching channels-last storage.
+// One CTA (4 warps) owns 128 consecutive positions (M = 128) of lines of W voxels with
+// one empty position before each, and all N output channels.  A stage is one (dz, dy) of
+// the taps: the 130 positions that the tile's three dx taps read, all input channels,
+// each once (cp.async; zero at the empty positions and outside the domain), and the
+// three taps' packed weights.  Shared memory holds a plane of 16-byte rows per 8
+// channels, a row a position: the canonical K-major layout without swizzle with
+// M-adjacent core matrices (8 rows, 128 bytes) 128 B apart and K-adjacent ones a plane
+// apart, so a tap's A tile is the stage's rows from dx on, and its 128 rows are three
+// overlapping views of one copy: 25 us for 16 -> 16 channels on 65^3 voxels, 87 for 48 ->
+// 16, where gathering each tap's tile by itself, three times the loads, took 43 and 128.
+// The descriptors are formed once (forming two in the loop cost the issuing thread 98 to
+// 175 clocks an MMA, 47 with sums; the SM takes one in 39).  The nine stages go round a ring of four (two when
+// they are too large for that): a stage's 3 x chunks tcgen05.mma (K = 16), in the taps'
+// order, overlap the loads of the next ones; tcgen05.commit arrives on a per-stage
+// mbarrier that releases the stage for reuse.  The accumulator (128 lanes x N FP32
+// columns) is read back with tcgen05.ld: warp w reads lanes 32w..32w+31, i.e. thread t
+// of the CTA reads the N channels of position t, matching channels-last storage.
 //
 // Every mbarrier wait is bounded; on timeout the kernel raises an error flag,
 // drains its own cp.async groups, frees its tensor memory and returns.
@@ -107,11 +108,8 @@ struct ConvArgs {
     int *err;
 };
 
-constexpr int kConvStages = 4, kConvK = 3;   // stages of the ring, K steps a stage (27 x channel chunks is a multiple)
-constexpr int kConvTileBytesA = 128 * 16 * 2;
-
-template <int N>
-__host__ __device__ constexpr int conv_smem_bytes() { return kConvStages * kConvK * (kConvTileBytesA + N * 32) + 128; }
+constexpr int kConvRows = 130, kConvPlane = 136 * 16;   // rows of a stage; bytes of an 8-channel plane
+__host__ __device__ constexpr int conv_stage_bytes(int N, int nch) { return 2 * nch * kConvPlane + 3 * nch * N * 32; }
 template <int N>
 __host__ __device__ constexpr uint32_t conv_tmem_cols() { return N <= 32 ? 32u : N <= 64 ? 64u : 128u; }
 
@@ -126,96 +124,102 @@ __device__ __forceinline__ int conv_crosses(int tap) {
     return 64 | (dx < 0) | (dx > 0) << 1 | (dy < 0) << 2 | (dy > 0) << 3 | (dz < 0) << 4 | (dz > 0) << 5;
 }
 
-template <int N>
+template <int N, int STAGES>
 __global__ void __launch_bounds__(128) k_conv3d_tc(ConvArgs a) {
     static_assert(N % 16 == 0 && N >= 16 && N <= 128, "N");
     extern __shared__ __align__(128) uint8_t smem[];
-    __shared__ int tapOff[27], tapMask[27];
-    constexpr int SB = kConvK * (kConvTileBytesA + N * 32);
-    uint64_t *mbar = reinterpret_cast<uint64_t *>(smem + kConvStages * SB);
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(mbar + kConvStages);
+    __shared__ int2 rows[kConvRows];   // a row's voxel and its y, z faces (64: an empty position)
+    __shared__ __align__(8) uint64_t mbar[STAGES];
+    __shared__ uint32_t tslot;
     const int tid = threadIdx.x, warp = tid >> 5;
+    const int nch0 = a.c0 >> 4, nch = (a.c0 + a.c1) >> 4, G = 2 * nch;
+    const int SA = G * kConvPlane, SB = SA + 3 * nch * N * 32;
     constexpr uint32_t NCOLS = conv_tmem_cols<N>();
     constexpr uint32_t IDESC = idesc_bf16(128, N);
 
-    if (warp == 0) { tmem_alloc(tslot, NCOLS); tmem_relinquish(); }
+    if (warp == 0) { tmem_alloc(&tslot, NCOLS); tmem_relinquish(); }
     if (tid == 0) {
-        for (int s = 0; s < kConvStages; ++s) mbar_init(&mbar[s], 1);
+        for (int s = 0; s < STAGES; ++s) mbar_init(&mbar[s], 1);
         fence_mbar_init();
     }
-    if (tid >= 32 && tid < 59) {
-        const int tap = tid - 32;
-        tapOff[tap] = ((tap / 9 - 1) * a.H + (tap / 3) % 3 - 1) * a.W + tap % 3 - 1;
-        tapMask[tap] = conv_crosses(tap);
+    for (int row = tid; row < kConvRows; row += 128) {
+        const int u = (int)blockIdx.x * 128 - 1 + row;
+        int vox = -1, face = 64;
+        if (u >= 0) {
+            const int line = u / (a.W + 1), x = u - line * (a.W + 1) - 1, y = line % a.H, z = line / a.H;
+            if (x >= 0 && z < a.D) {
+                vox = line * a.W + x;
+                face = conv_faces(1, y, z, 3, a.H, a.D);
+            }
+        }
+        rows[row] = make_int2(vox, face);
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t taddr = *tslot;
+    const uint32_t taddr = tslot;
+    const int v = rows[tid + 1].x;   // this thread's output voxel
+    const bool valid = v >= 0;
 
-    // this thread's output voxel (epilogue), and the two rows it gathers half of: a pair of
-    // neighbouring threads fetches a voxel's 32 bytes, a warp 16 consecutive voxels
-    const int v = blockIdx.x * 128 + tid;
-    const bool valid = v < a.nvox;
-    int gv[2], faces[2];
+    // a thread loads one 8-channel group of every (128 / G)-th row, a row's groups by neighbours
+    const int per = 128 / G, row0 = tid / G, g = tid - row0 * G;
+    const bool second = g >= 2 * nch0;
+    const int cs = second ? a.c1 : a.c0;
+    const __nv_bfloat16 *const src0 = second ? a.in1 + (g - 2 * nch0) * 8 : a.in0 + g * 8;
+    // one chunk (G = 2): the thread's rows, tid / 2, + 64 and (four threads) + 128, in registers
+    const int2 mine[3] = {rows[tid >> 1], rows[(tid >> 1) + 64], tid < 4 ? rows[128 + (tid >> 1)] : make_int2(0, 64)};
+    auto load_step = [&](int s, int st) {
+        const uint32_t base = su32(smem + st * SB), dst = base + g * kConvPlane;
+        const int mask = conv_crosses(3 * s + 1);
+        const __nv_bfloat16 *const src = src0 + (long)(((s / 3 - 1) * a.H + s % 3 - 1) * a.W) * cs;
+        if (G == 2) {
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-        gv[u] = blockIdx.x * 128 + (tid >> 1) + 64 * u;
-        const int x = gv[u] % a.W, t = gv[u] / a.W, y = t % a.H, z = t / a.H;
-        faces[u] = gv[u] < a.nvox ? conv_faces(x, y, z, a.W, a.H, a.D) : 64;
-    }
-    const int half = (tid & 1) * 8;
-    const uint32_t rowA = (uint32_t)(tid >> 4) * 256 + ((tid >> 1) & 7) * 16 + (tid & 1) * 128;   // row tid / 2; row + 64: 2048 further
-    const int nch0 = a.c0 >> 4, nch = (a.c0 + a.c1) >> 4;
-    const int nsteps = 27 * nch / kConvK;
-    int tap = 0, ch = 0;   // of the next K step to load
-
-    auto load_step = [&](int s, int st) {   // stages in order
-        const uint32_t base = su32(smem + st * SB);
-#pragma unroll
-        for (int e = 0; e < kConvK; ++e) {
-            const __nv_bfloat16 *src;
-            int cs, co;
-            if (ch < nch0) { src = a.in0; cs = a.c0; co = ch << 4; }
-            else { src = a.in1; cs = a.c1; co = (ch - nch0) << 4; }
-            const int off = tapOff[tap], mask = tapMask[tap];
-#pragma unroll
-            for (int u = 0; u < 2; ++u) {
-                const bool in = (faces[u] & mask) == 0;
-                cp_async16_l1(base + e * kConvTileBytesA + rowA + u * 2048, src + (in ? (long)(gv[u] + off) * cs + co + half : 0), in ? 16 : 0);
+            for (int u = 0; u < 3; ++u) {
+                const bool in = (mine[u].y & mask) == 0;
+                if (u < 2 || tid < 4) cp_async16_l1(dst + (row0 + 64 * u) * 16, in ? src + (long)mine[u].x * 16 : a.in0, in ? 16 : 0);
             }
-            if (++ch == nch) { ch = 0; ++tap; }
+        } else if (row0 < per) {
+#pragma unroll 4
+            for (int row = row0; row < kConvRows; row += per) {
+                const int2 t = rows[row];
+                const bool in = (t.y & mask) == 0;
+                cp_async16_l1(dst + row * 16, in ? src + (long)t.x * cs : a.in0, in ? 16 : 0);
+            }
         }
-        const uint8_t *wsrc = reinterpret_cast<const uint8_t *>(a.wpk) + (long)s * kConvK * N * 32;
-        const uint32_t dB = base + kConvK * kConvTileBytesA;
-        for (int q = tid; q < kConvK * N * 2; q += 128) cp_async16(dB + q * 16, wsrc + q * 16, 16);
+        const uint8_t *wsrc = reinterpret_cast<const uint8_t *>(a.wpk) + (long)s * 3 * nch * N * 32;
+        for (int q = tid; q < 3 * nch * N * 2; q += 128) cp_async16(base + SA + q * 16, wsrc + q * 16, 16);
     };
+    // stage 0's descriptors; others by adding to the start addresses (16-byte units: no
+    // carry leaves the field, shared memory ends below it)
+    const uint64_t ad0 = smem_desc(su32(smem), kConvPlane, 128), bd0 = smem_desc(su32(smem) + SA, 128, 256);
 
+    constexpr int nsteps = 9;
     bool ok = true;
 #pragma unroll 1
-    for (int s = 0; s < kConvStages - 1; ++s) {
-        if (s < nsteps) load_step(s, s);
+    for (int s = 0; s < STAGES - 1; ++s) {
+        load_step(s, s);
         cp_async_commit();
     }
 #pragma unroll 1
     for (int s = 0; s < nsteps; ++s) {
-        const int st = s % kConvStages;
-        cp_async_wait<kConvStages - 2>();
-        __syncthreads();
+        const int st = s % STAGES;
+        cp_async_wait<STAGES - 2>();
         fence_async_smem();
+        __syncthreads();
         if (tid == 0 && ok) {
             tc_fence_after();
-            const uint32_t aAddr = su32(smem + st * SB), bAddr = aAddr + kConvK * kConvTileBytesA;
+            uint64_t ad = ad0 + (uint32_t)(st * SB) / 16, bd = bd0 + (uint32_t)(st * SB) / 16;
 #pragma unroll
-            for (int e = 0; e < kConvK; ++e)
-                tc_mma_bf16(taddr, smem_desc(aAddr + e * kConvTileBytesA, 128, 256), smem_desc(bAddr + e * N * 32, 128, 256), IDESC, s + e > 0 ? 1u : 0u);
+            for (int dx = 0; dx < 3; ++dx)
+                for (int ch = 0; ch < nch; ++ch, bd += N * 2)
+                    tc_mma_bf16(taddr, ad + ch * (2 * kConvPlane / 16) + dx, bd, IDESC, s + dx + ch > 0 ? 1u : 0u);
             tc_commit(&mbar[st]);
         }
-        const int ns = s + kConvStages - 1;
+        const int ns = s + STAGES - 1;
         if (ns < nsteps) {
-            const int nst = ns % kConvStages;
-            // stage nst was last read by the MMA of step ns - kConvStages (= s - 1)
-            if (ns >= kConvStages && ok) ok = mbar_wait(&mbar[nst], (uint32_t)(((ns - kConvStages) / kConvStages) & 1), a.err);
+            const int nst = ns % STAGES;
+            // stage nst was last read by the MMAs of step ns - STAGES (= s - 1)
+            if (ns >= STAGES && ok) ok = mbar_wait(&mbar[nst], (uint32_t)(((ns - STAGES) / STAGES) & 1), a.err);
             if (ok) load_step(ns, nst);
         }
         cp_async_commit();
@@ -224,7 +228,7 @@ __global__ void __launch_bounds__(128) k_conv3d_tc(ConvArgs a) {
     // all MMAs done once the last commit has arrived
     if (ok) {
         const int last = nsteps - 1;
-        ok = mbar_wait(&mbar[last % kConvStages], (uint32_t)((last / kConvStages) & 1), a.err);
+        ok = mbar_wait(&mbar[last % STAGES], (uint32_t)((last / STAGES) & 1), a.err);
     }
     __syncthreads();
     tc_fence_after();
@@ -272,18 +276,21 @@ __global__ void __launch_bounds__(128) k_conv3d_tc(ConvArgs a) {
 }
 
 // ---- weight gradient on the tensor cores
-// dW[n][tap][c] = sum_v dY[v][n] X[v + off(tap)][c] as the GEMM
-//   D[m][n] = sum_k A[m][k] B[n][k],  m = tap * Cin + c (27 Cin rows in tiles
-//   of 128), n = output channel, k = voxel.
-// Both operands are staged MN-major, which is the order the channels-last
-// tensors already have: one 16-byte row of a core matrix is 8 consecutive
-// channels of one voxel (X at the shifted voxel for A, dY for B), so every row
-// is one 16-byte cp.async straight from global memory.  Core matrices adjacent
-// along M (or N) are 128 B apart (the stride byte offset of a no-swizzle
-// MN-major descriptor), the two 8-voxel halves of a K step of 16 voxels
-// 16 x 128 B (A) or N / 8 x 128 B (B) apart (its leading byte offset).  Each CTA reduces a chunk of voxels for one M tile
-// into its tensor-memory accumulator and adds it to the FP32 dW with atomics;
-// the CTAs of M tile 0 also add their chunk's sum of dY to db.
+// dW[n][tap][c] = sum_v dY[v][n] X[v + off(tap)][c] as GEMMs
+//   D[m][n] = sum_k A[m][k] B[n][k],  n = output channel, k = position (the lines of
+//   voxels with an empty position before each, as in the forward pass).
+// A CTA takes 16 input channels and a chunk of positions for all taps.  A stage holds,
+// for kDwK positions, nine copies of X, one a (dz, dy) of the taps, shifted by it (zero
+// outside the domain and at empty positions), as 18 planes of 16-byte rows (8 channels of
+// a position), and dY as N / 8 planes.  Both operands are MN-major, which is the order
+// the channels-last tensors already have: a core matrix is 8 consecutive rows of a plane,
+// K-adjacent ones 128 B apart (the leading byte offset), M- or N-adjacent ones a plane
+// apart (the stride byte offset).  The planes are the M dimension, m = plane * 8 +
+// channel, so the dx taps are the same planes from one row on: one accumulator a dx and
+// M tile (16 planes; the second, of 64 rows, holds planes 16, 17 and rows that nothing reads).  Each
+// copy serves three taps: 43 us for 16 -> 16 channels on 65^3 voxels, 90 for 48 -> 16,
+// where a gather a tap took 52 and 129.  The accumulators are added to the FP32 dW with atomics; the CTAs
+// of the first input channels also add their chunk's sum of dY to db.
 struct DwArgs {
     const __nv_bfloat16 *in0, *in1;   // X, channels-last, concatenated along C
     int c0, c1;
@@ -291,43 +298,45 @@ struct DwArgs {
     float *dw;                        // [N][27][c0 + c1]
     float *db;                        // [N], or null
     int D, H, W, nvox;
-    int chunk;                        // voxels a CTA reduces (a multiple of kDwK)
+    int chunk;                        // positions a CTA reduces (a multiple of kDwK)
     int *err;
 };
 
-// A stage holds kDwK voxels: kDwK / 16 K steps to a barrier.  Two neighbouring threads
-// stage one voxel's row of each of the M tile's eight pairs of channel groups (one
-// tap, 16 channels, a 32-byte sector; a warp 16 consecutive voxels), with the
-// tap's offset and face mask of each pair fixed for the whole loop and the voxel's
-// position advanced by carries.
-// (One K step of 16 voxels a barrier, two 64-bit divisions a row, half-sector gathers
-// and a serial sum for db took 162 us for 16 -> 16 channels on 65^3 voxels; this
-// takes 52, the gathers through L2 and L1 its bound.)
 constexpr int kDwStages = 4, kDwK = 64;
-constexpr int kDwTileA = 128 * 16 * 2;   // one K step
+constexpr int kDwPlaneA = (kDwK + 4) * 16, kDwPlaneB = kDwK * 16;   // bytes of a plane (66 rows are read of A's)
+constexpr int kDwPlanes = 18;
 template <int N>
-__host__ __device__ constexpr int dw_stage_bytes() { return kDwK / 16 * (kDwTileA + N * 32); }
+__host__ __device__ constexpr int dw_stage_bytes() { return kDwPlanes * kDwPlaneA + N / 8 * kDwPlaneB; }
+// (the second M tile's unused rows lie up to 6 planes past the last stage's A)
 template <int N>
-__host__ __device__ constexpr int dw_smem_bytes() { return kDwStages * dw_stage_bytes<N>() + 128; }
+__host__ __device__ constexpr int dw_smem_bytes() { return kDwStages * dw_stage_bytes<N>() + 6 * kDwPlaneA; }
+// dx taps of a CTA: all three where their accumulators (two M tiles each) fit the tensor memory
+template <int N>
+__host__ __device__ constexpr int dw_taps() { return 6 * N <= 512 ? 3 : 1; }
+template <int N>
+__host__ __device__ constexpr uint32_t dw_tmem_cols() {
+    constexpr int c = 2 * N * dw_taps<N>();
+    return c <= 32 ? 32u : c <= 64 ? 64u : c <= 128 ? 128u : c <= 256 ? 256u : 512u;
+}
 
+// Grid: chunks of positions, groups of 16 input channels, 3 / dw_taps dx taps.
 template <int N>
 __global__ void __launch_bounds__(128) k_conv_dw_tc(DwArgs a) {
     static_assert(N % 16 == 0 && N >= 16 && N <= 128, "N");
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ float sdb[N];
-    constexpr int SB = dw_stage_bytes<N>(), KS = kDwK / 16;
-    uint64_t *mbar = reinterpret_cast<uint64_t *>(smem + kDwStages * SB);
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(mbar + kDwStages);
+    __shared__ __align__(8) uint64_t mbar[kDwStages];
+    __shared__ uint32_t tslot;
+    constexpr int SB = dw_stage_bytes<N>(), SA = kDwPlanes * kDwPlaneA, KS = kDwK / 16, TAPS = dw_taps<N>();
     const int tid = threadIdx.x, warp = tid >> 5;
-    constexpr uint32_t NCOLS = conv_tmem_cols<N>();
-    constexpr uint32_t IDESC = idesc_bf16(128, N) | (1u << 15) | (1u << 16);   // A and B MN-major
-    const int cin = a.c0 + a.c1, mtot = 27 * cin;
-    const int mt = blockIdx.y;
-    const long v0 = (long)blockIdx.x * a.chunk;
-    const long v1 = min(v0 + (long)a.chunk, (long)a.nvox);
-    const int nsteps = v1 > v0 ? (int)((v1 - v0 + kDwK - 1) / kDwK) : 0;
+    constexpr uint32_t NCOLS = dw_tmem_cols<N>();
+    constexpr uint32_t MN = (1u << 15) | (1u << 16), IDESC[2] = {idesc_bf16(128, N) | MN, idesc_bf16(64, N) | MN};   // A and B MN-major
+    const int cin = a.c0 + a.c1, c = blockIdx.y * 16, dx0 = blockIdx.z;
+    const long u0 = (long)blockIdx.x * a.chunk;
+    const long u1 = min(u0 + (long)a.chunk, (long)a.D * a.H * (a.W + 1));
+    const int nsteps = u1 > u0 ? (int)((u1 - u0 + kDwK - 1) / kDwK) : 0;
 
-    if (warp == 0) { tmem_alloc(tslot, NCOLS); tmem_relinquish(); }
+    if (warp == 0) { tmem_alloc(&tslot, NCOLS); tmem_relinquish(); }
     if (tid == 0) {
         for (int s = 0; s < kDwStages; ++s) mbar_init(&mbar[s], 1);
         fence_mbar_init();
@@ -336,80 +345,93 @@ __global__ void __launch_bounds__(128) k_conv_dw_tc(DwArgs a) {
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t taddr = *tslot;
+    const uint32_t taddr = tslot;
 
-    // this thread's voxel row and its half of a pair of channel groups, eight pairs
-    const int vr = tid >> 1, r = vr & 15, half = tid & 1;
-    long v = v0 + vr;   // of the next stage to load (stages in order)
-    int x, y, z;
-    {
-        const int w = (int)min(v, (long)a.nvox - 1);   // a row past the chunk loads nothing
-        x = w % a.W;
-        const int t = w / a.W;
-        y = t % a.H;
-        z = t / a.H;
-    }
-    const int ax = kDwK % a.W, ay = (kDwK / a.W) % a.H, az = kDwK / (a.W * a.H);   // a stage's advance
-    const __nv_bfloat16 *src[8];
-    int cs[8], crosses[8];
+    const __nv_bfloat16 *const src = c < a.c0 ? a.in0 + c : a.in1 + (c - a.c0);
+    const int cs = c < a.c0 ? a.c0 : a.c1;
+    // Row q of a stage's planes is position u0 + kDwK step - 1 + q of X (A reads rows 0 ..
+    // kDwK + 1), dY's row q position u0 + kDwK step + q.  Two neighbouring threads load row
+    // tid / 2 of all nine copies, 8 channels each; the first 36 threads also rows 64 and 65.
+    struct Pos {
+        long u;
+        int x, y, z;   // x = -1: an empty position
+    };
+    auto pos_at = [&](long u) {
+        Pos p;
+        p.u = u;
+        const long w = max(u, 0L), line = w / (a.W + 1);
+        p.x = u < 0 ? -1 : (int)(w - line * (a.W + 1)) - 1;
+        p.y = (int)(line % a.H);
+        p.z = (int)(line / a.H);
+        return p;
+    };
+    const int ax = kDwK % (a.W + 1), ay = (kDwK / (a.W + 1)) % a.H, az = kDwK / ((a.W + 1) * a.H);   // a stage's advance
+    auto advance = [&](Pos &p) {
+        p.u += kDwK;
+        if (p.u - kDwK < 0) { p = pos_at(p.u); return; }
+        p.x += ax;
+        if (p.x >= a.W) { p.x -= a.W + 1; ++p.y; }
+        p.y += ay;
+        if (p.y >= a.H) { p.y -= a.H; ++p.z; }
+        p.z += az;
+    };
+    const int half = tid & 1, row = tid >> 1;
+    Pos p = pos_at(u0 - 1 + row), e = pos_at(u0 - 1 + kDwK + ((tid >> 1) & 1)), d = pos_at(u0 + row);
+    const int soy = a.W * cs, soz = a.H * soy;
+    auto face_of = [&](const Pos &q) { return q.x < 0 || q.z >= a.D ? 64 : conv_faces(1, q.y, q.z, 3, a.H, a.D); };
+    auto voxel = [&](const Pos &q) { return ((long)q.z * a.H + q.y) * a.W + q.x; };
+    auto load_x = [&](const __nv_bfloat16 *x, int face, int seg, uint32_t dst) {
+        const bool in = (face & conv_crosses(3 * seg + 1)) == 0;
+        cp_async16_l1(dst, in ? x + (seg / 3 - 1) * (long)soz + (seg % 3 - 1) * (long)soy : src, in ? 16 : 0);
+    };
+    auto load_step = [&](int st) {   // stages in order
+        const uint32_t base = su32(smem + st * SB), dst = base + half * kDwPlaneA + row * 16;
+        const __nv_bfloat16 *const x = src + voxel(p) * cs + half * 8;
+        const int face = face_of(p);
 #pragma unroll
-    for (int h = 0; h < 8; ++h) {
-        const int m0 = mt * 128 + h * 16;
-        const int tap = min(m0 / cin, 26), c = m0 - (m0 / cin) * cin;
-        const long off = (long)((tap / 9 - 1) * a.H + (tap / 3) % 3 - 1) * a.W + tap % 3 - 1;
-        crosses[h] = m0 < mtot ? conv_crosses(tap) : -1;   // -1: past the last row, always zero
-        cs[h] = c < a.c0 ? a.c0 : a.c1;
-        src[h] = (c < a.c0 ? a.in0 + c : a.in1 + (c - a.c0)) + off * cs[h] + half * 8;   // only dereferenced at voxels whose neighbour exists
-    }
-    auto load_step = [&](int, int st) {
-        const uint32_t base = su32(smem + st * SB) + (vr >> 4) * kDwTileA + (r & 7) * 16 + (r >> 3) * 2048;
-        const int faces = v < v1 ? conv_faces(x, y, z, a.W, a.H, a.D) | 128 : 64 | 128;
+        for (int seg = 0; seg < 9; ++seg) load_x(x, face, seg, dst + 2 * seg * kDwPlaneA);
+        if (tid < 36)
+            load_x(src + voxel(e) * cs + half * 8, face_of(e), tid >> 2, base + (2 * (tid >> 2) + half) * kDwPlaneA + (kDwK + ((tid >> 1) & 1)) * 16);
+        const bool ok = d.x >= 0 && d.u < u1;
+        const long w = voxel(d);
 #pragma unroll
-        for (int h = 0; h < 8; ++h) {
-            const bool in = (faces & crosses[h]) == 0;
-            cp_async16_l1(base + h * 256 + half * 128, in ? src[h] + v * cs[h] : a.in0, in ? 16 : 0);
-        }
-        const uint32_t bb = su32(smem + st * SB) + KS * kDwTileA + (vr >> 4) * (N * 32) + (r & 7) * 16 + (r >> 3) * (N / 8) * 128;
-        const bool ok = v < v1;
-#pragma unroll
-        for (int ng = half; ng < N / 8; ng += 2) cp_async16(bb + ng * 128, ok ? a.dy + v * N + ng * 8 : a.dy, ok ? 16 : 0);
-        v += kDwK;
-        x += ax;
-        if (x >= a.W) { x -= a.W; ++y; }
-        y += ay;
-        if (y >= a.H) { y -= a.H; ++z; }
-        z += az;
+        for (int g = half; g < N / 8; g += 2) cp_async16(base + SA + g * kDwPlaneB + row * 16, ok ? a.dy + w * N + g * 8 : a.dy, ok ? 16 : 0);
+        advance(p);
+        advance(e);
+        advance(d);
     };
 
+    const uint64_t ad0 = smem_desc(su32(smem) + dx0 * 16, 128, kDwPlaneA), bd0 = smem_desc(su32(smem) + SA, 128, kDwPlaneB);
     bool ok = true;
 #pragma unroll 1
     for (int s = 0; s < kDwStages - 1; ++s) {
-        if (s < nsteps) load_step(s, s);
+        if (s < nsteps) load_step(s);
         cp_async_commit();
     }
 #pragma unroll 1
     for (int s = 0; s < nsteps; ++s) {
         const int st = s % kDwStages;
         cp_async_wait<kDwStages - 2>();
-        __syncthreads();
         fence_async_smem();
+        __syncthreads();
         if (tid == 0 && ok) {
             tc_fence_after();
-            const uint32_t aAddr = su32(smem + st * SB), bAddr = aAddr + KS * kDwTileA;
-            // no-swizzle MN-major: the stride byte offset steps between core
-            // matrices along M / N, the leading byte offset along K
+            const uint64_t ad = ad0 + (uint32_t)(st * SB) / 16, bd = bd0 + (uint32_t)(st * SB) / 16;
 #pragma unroll
-            for (int e = 0; e < KS; ++e)
-                tc_mma_bf16(taddr, smem_desc(aAddr + e * kDwTileA, 2048, 128), smem_desc(bAddr + e * N * 32, (N / 8) * 128, 128), IDESC,
-                            s + e > 0 ? 1u : 0u);
+            for (int k = 0; k < KS; ++k)
+#pragma unroll
+                for (int t = 0; t < TAPS; ++t)
+#pragma unroll
+                    for (int m = 0; m < 2; ++m)
+                        tc_mma_bf16(taddr + (2 * t + m) * N, ad + (m * kDwPlaneA + t + 16 * k), bd + k * 16, IDESC[m], s + k > 0 ? 1u : 0u);
             tc_commit(&mbar[st]);
         }
         const int ns = s + kDwStages - 1;
         if (ns < nsteps) {
             const int nst = ns % kDwStages;
-            // stage nst was last read by the MMA of step ns - kDwStages (= s - 1)
+            // stage nst was last read by the MMAs of step ns - kDwStages (= s - 1)
             if (ns >= kDwStages && ok) ok = mbar_wait(&mbar[nst], (uint32_t)(((ns - kDwStages) / kDwStages) & 1), a.err);
-            if (ok) load_step(ns, nst);
+            if (ok) load_step(nst);
         }
         cp_async_commit();
     }
@@ -421,20 +443,26 @@ __global__ void __launch_bounds__(128) k_conv_dw_tc(DwArgs a) {
     __syncthreads();
     tc_fence_after();
     if (ok && nsteps > 0) {
-        const int m = mt * 128 + tid;
-        const int tap = m / cin, c = m - tap * cin;
         const uint32_t tw = taddr + ((uint32_t)(warp * 32) << 16);
 #pragma unroll
-        for (int q = 0; q < N / 16; ++q) {
-            float vals[16];
-            tc_ld16(tw + q * 16, vals);
-            if (m < mtot) {
+        for (int t = 0; t < TAPS; ++t)
 #pragma unroll
-                for (int e = 0; e < 16; ++e) atomicAdd(&a.dw[((long)(q * 16 + e) * 27 + tap) * cin + c], vals[e]);
+            for (int m = 0; m < 2; ++m) {
+                if (m == 1 && warp > 0) continue;   // rows 0 .. 15 only
+                const int plane = m * 16 + (tid >> 3), tap = 3 * (plane >> 1) + dx0 + t, ci = c + (plane & 1) * 8 + (tid & 7);
+#pragma unroll
+                for (int q = 0; q < N / 16; ++q) {
+                    float vals[16];
+                    tc_ld16(tw + (2 * t + m) * N + q * 16, vals);
+                    if (plane < kDwPlanes) {
+#pragma unroll
+                        for (int o = 0; o < 16; ++o) atomicAdd(&a.dw[((long)(q * 16 + o) * 27 + tap) * cin + ci], vals[o]);
+                    }
+                }
             }
-        }
     }
-    if (a.db && mt == 0) {   // the chunk's sum of dY: a thread 8 channels of every (1024 / N)-th voxel
+    if (a.db && c == 0 && dx0 == 0) {   // the sum of the chunk's share of dY: a thread 8 channels of every (1024 / N)-th voxel
+        const long v0 = (long)blockIdx.x * a.nvox / gridDim.x, v1 = ((long)blockIdx.x + 1) * a.nvox / gridDim.x;
         const int ng = tid % (N / 8), rows = 128 / (N / 8);
         float sum[8] = {};
         if (tid < rows * (N / 8)) {

@@ -498,13 +498,18 @@ static int ucheck(Ctx &c, const char *what) {
     return SARAS_OK;
 }
 
+template <int N, int STAGES>
+static cudaError_t launch_conv_s(const ConvArgs &a, int smem, cudaStream_t s) {
+    cudaError_t e = cudaFuncSetAttribute(k_conv3d_tc<N, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    const long rows = (long)a.D * a.H * (a.W + 1);
+    k_conv3d_tc<N, STAGES><<<(int)((rows + 127) / 128), 128, smem, s>>>(a);
+    return cudaGetLastError();
+}
 template <int N>
 static cudaError_t launch_conv_n(const ConvArgs &a, cudaStream_t s) {
-    cudaError_t e = cudaFuncSetAttribute(k_conv3d_tc<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, conv_smem_bytes<N>());
-    if (e != cudaSuccess) return e;
-    int blocks = (a.nvox + 127) / 128;
-    k_conv3d_tc<N><<<blocks, 128, conv_smem_bytes<N>(), s>>>(a);
-    return cudaGetLastError();
+    const int stage = conv_stage_bytes(N, (a.c0 + a.c1) / 16);
+    return 4 * stage <= 200 * 1024 ? launch_conv_s<N, 4>(a, 4 * stage, s) : launch_conv_s<N, 2>(a, 2 * stage, s);
 }
 
 static int launch_conv(Ctx &c, int N, const ConvArgs &a) {
@@ -705,29 +710,29 @@ static int add_mask(Ctx &c, const bf16 *a, const bf16 *b, const bf16 *mask, bf16
     return ucheck(c, "add_mask");
 }
 
-// Weight and bias gradients of layer li on the tensor cores (k_conv_dw_tc):
-// voxel chunks sized for about three CTAs an SM over all M tiles.
+// Weight and bias gradients of layer li on the tensor cores (k_conv_dw_tc): position
+// chunks for as many CTAs, over all groups of input channels, as the SMs hold
+// at once.
 template <int N>
-static cudaError_t launch_dw_n(const DwArgs &a, int mtiles, cudaStream_t st) {
+static cudaError_t launch_dw_n(DwArgs a, cudaStream_t st) {
     cudaError_t e = cudaFuncSetAttribute(k_conv_dw_tc<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, dw_smem_bytes<N>());
     if (e != cudaSuccess) return e;
-    const long nch = (a.nvox + a.chunk - 1) / a.chunk;
-    k_conv_dw_tc<N><<<dim3((unsigned)nch, (unsigned)mtiles), 128, dw_smem_bytes<N>(), st>>>(a);
+    const int groups = (a.c0 + a.c1) / 16, taps = 3 / dw_taps<N>();
+    const long rows = (long)a.D * a.H * (a.W + 1), perSM = std::min<long>(512 / dw_tmem_cols<N>(), 220 * 1024 / dw_smem_bytes<N>());
+    const long want = std::max(1L, 152 * perSM / (groups * taps));
+    a.chunk = (int)std::max((long)kDwK, ((rows + want - 1) / want + kDwK - 1) / kDwK * kDwK);
+    k_conv_dw_tc<N><<<dim3((unsigned)((rows + a.chunk - 1) / a.chunk), (unsigned)groups, (unsigned)taps), 128, dw_smem_bytes<N>(), st>>>(a);
     return cudaGetLastError();
 }
 
-static int launch_dw(Ctx &c, int N, DwArgs a) {
-    const int cin = a.c0 + a.c1;
-    const int mtiles = (27 * cin + 127) / 128;
-    const long want = std::max(1L, 3L * 152 / mtiles);   // voxel chunks
-    a.chunk = (int)std::max((long)kDwK, (((long)a.nvox + want - 1) / want + kDwK - 1) / kDwK * kDwK);
+static int launch_dw(Ctx &c, int N, const DwArgs &a) {
     cudaError_t e;
     switch (N) {
-    case 16: e = launch_dw_n<16>(a, mtiles, c.stream); break;
-    case 32: e = launch_dw_n<32>(a, mtiles, c.stream); break;
-    case 48: e = launch_dw_n<48>(a, mtiles, c.stream); break;
-    case 64: e = launch_dw_n<64>(a, mtiles, c.stream); break;
-    case 96: e = launch_dw_n<96>(a, mtiles, c.stream); break;
+    case 16: e = launch_dw_n<16>(a, c.stream); break;
+    case 32: e = launch_dw_n<32>(a, c.stream); break;
+    case 48: e = launch_dw_n<48>(a, c.stream); break;
+    case 64: e = launch_dw_n<64>(a, c.stream); break;
+    case 96: e = launch_dw_n<96>(a, c.stream); break;
     default: c.err = "unsupported convolution width"; return SARAS_BAD_ARG;
     }
     count_launch(c);
