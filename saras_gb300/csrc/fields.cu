@@ -1076,7 +1076,7 @@ __global__ void __launch_bounds__(256, 6) k_cn_delta(CnDelta a) {
 // from the current D at their sources: the boundary values of the first
 // iterate A, which the right-hand-side kernel writes on the bulk only.
 template <bool FINAL, bool COPY>
-__global__ void k_cn_delta_shell(CnDelta a) {
+__device__ __forceinline__ void cn_shell(const CnDelta &a) {
     int s = blockIdx.y, d = s >> 1;
     int lo[3], hi[3];
     for (int e = 0; e < 3; ++e) {
@@ -1094,6 +1094,15 @@ __global__ void k_cn_delta_shell(CnDelta a) {
         cn_delta_store<FINAL>(a, o, cn_delta_boundary<COPY>(a, i, j, k, o));
     }
 }
+template <bool FINAL, bool COPY>
+__global__ void k_cn_delta_shell(const __grid_constant__ CnDelta a) { cn_shell<FINAL, COPY>(a); }
+// The three components' shells in one launch (blockIdx.z): each of them is a few small
+// blocks' dependent loads, 16 us at 257^3 and 6 at 65^3 by itself.
+struct CnDelta3 {
+    CnDelta c[3];
+};
+template <bool FINAL, bool COPY>
+__global__ void k_cn_delta_shell3(const __grid_constant__ CnDelta3 a) { cn_shell<FINAL, COPY>(a.c[blockIdx.z]); }
 
 // C0 + D in FP64 over the whole padded array (in place on the field).
 __global__ void k_cn_unpack(double *V, const float *dh, const float *dl, long n) {
@@ -1156,7 +1165,7 @@ __global__ void __launch_bounds__(256) k_project_bulk(View3<double> out, View3<c
 }
 
 template <int C>
-__global__ void k_project_shell(View3<double> out, View3<const double> in, View3<const double> Pp, BcProgram prog, Box full,
+__device__ __forceinline__ void project_shell(View3<double> out, View3<const double> in, View3<const double> Pp, const BcProgram &prog, const Box &full,
                                 double fastDt) {
     int s = blockIdx.y, d = s >> 1;
     int lo[3], hi[3];
@@ -1183,6 +1192,22 @@ __global__ void k_project_shell(View3<double> out, View3<const double> in, View3
         for (int o = 0; o < prog.nops; ++o) if (in_box(prog.op[o].lo, prog.op[o].hi, i, j, k)) { targeted = true; break; }
         out(i, j, k) = targeted ? bc_resolve(prog, i, j, k, base) : base(i, j, k);
     }
+}
+// The three components' shells in one launch, as k_cn_delta_shell3's.
+struct ProjShell3 {
+    View3<double> out[3];
+    View3<const double> in[3], Pp;
+    BcProgram prog[3];
+    Box full[3];
+    double fdt[3];
+    int on[3];
+};
+__global__ void k_project_shell3(const __grid_constant__ ProjShell3 a) {
+    const int q = blockIdx.z;
+    if (!a.on[q]) return;
+    if (q == 0) project_shell<0>(a.out[0], a.in[0], a.Pp, a.prog[0], a.full[0], a.fdt[0]);
+    else if (q == 1) project_shell<1>(a.out[1], a.in[1], a.Pp, a.prog[1], a.full[1], a.fdt[1]);
+    else project_shell<2>(a.out[2], a.in[2], a.Pp, a.prog[2], a.full[2], a.fdt[2]);
 }
 
 // ------------------------------------------------------------------ diagnostics
@@ -1830,10 +1855,19 @@ int compute_trhs(Ctx &c) {
 // semantics of cn_solve: each sweep also reports the residual of its input,
 // and the input of the first sweep whose input residual is below the
 // tolerance is the answer.
-// stage 0: the whole solve; 1: its launches up to the speculative final sweep's,
-// without waiting; 2: the rest, with that sweep's residual in hscal[comp] already
-// (cn_together: the components' residuals come in one copy).
-static int cn_solve_delta(Ctx &c, int comp, int field, const CnFast &fa, double Dn, double bytes, int *iters, double *maxerr, int stage) {
+static void cn_delta_dims(const Box &full, dim3 &g, dim3 &b) {
+    g = dim3((full.ext[2] + 31) / 32, (full.ext[1] + 7) / 8, (full.ext[0] + kCnMarch - 1) / kCnMarch);
+    b = dim3(32, 8, 1);
+    if (kCnColumns) {
+        g = dim3((unsigned)(((long)full.ext[1] * full.ext[2] + 255) / 256), (full.ext[0] + kCnMarch - 1) / kCnMarch, 1);
+        b = dim3(256, 1, 1);
+    }
+}
+
+// stage 0: the whole solve; 1: N0, if it is not there yet, and the arguments of the
+// speculative final sweep (from A, its second) into *plan, for cn_together to launch;
+// 2: the rest, with that sweep's residual in hscal[comp] already.
+static int cn_solve_delta(Ctx &c, int comp, int field, const CnFast &fa, double Dn, double bytes, int *iters, double *maxerr, int stage, CnDelta *plan) {
     const FieldInfo &f = c.info[field];
     View3<double> V = mview(c, field);
     long n = V.size();
@@ -1863,7 +1897,11 @@ static int cn_solve_delta(Ctx &c, int comp, int field, const CnFast &fa, double 
     // N0): its non-bulk points from their boundary-program sources, in place.
     d.dh = d.oh = n0h;
     d.dl = d.ol = n0l;
-    if (stage != 2) {
+    if (stage == 1) {
+        *plan = d;
+        return check_launch(c, "cn pack");
+    }
+    if (stage == 0) {
         k_cn_delta_shell<false, true><<<dim3(shell_blocks(d.full), 6), 256, 0, c.stream>>>(d);
         count_launch(c);
     }
@@ -1871,11 +1909,7 @@ static int cn_solve_delta(Ctx &c, int comp, int field, const CnFast &fa, double 
     float *const bufs[3][2] = {{n0h, n0l}, {dA, dAl}, {dB, dBl}};
     int cur = 0, nxt = 1;
     auto advance = [&]() { int w = nxt; nxt = (w == 1) ? 2 : 1; cur = w; };
-    dim3 gm((fa.full.ext[2] + 31) / 32, (fa.full.ext[1] + 7) / 8, (fa.full.ext[0] + kCnMarch - 1) / kCnMarch), bm(32, 8, 1);
-    if (kCnColumns) {
-        gm = dim3((unsigned)(((long)fa.full.ext[1] * fa.full.ext[2] + 255) / 256), (fa.full.ext[0] + kCnMarch - 1) / kCnMarch, 1);
-        bm = dim3(256, 1, 1);
-    }
+    dim3 gm, bm; cn_delta_dims(fa.full, gm, bm);
     // vout: a final sweep, which writes C0 + D into vout (the field's scratch partner)
     // instead of D, the sum k_cn_unpack would form
     auto launch = [&](int withRes, double *vout) {
@@ -1924,10 +1958,9 @@ static int cn_solve_delta(Ctx &c, int comp, int field, const CnFast &fa, double 
             advance();
             sweeps += 1;
         }
-        if (stage != 2) {
+        if (stage == 0) {
             SARAS_CUDA_TRY(cudaMemsetAsync(d.resMax, 0, sizeof(double), c.stream));
             launch(1, c.scratch[slot]);
-            if (stage == 1) return check_launch(c, "cn");
             int s = read_res(res);
             if (s) return s;
         } else {
@@ -1982,7 +2015,7 @@ static int cn_solve_delta(Ctx &c, int comp, int field, const CnFast &fa, double 
     return status;
 }
 
-static int cn_solve_stage(Ctx &c, int comp, int *iters, double *maxerr, int stage) {
+static int cn_solve_stage(Ctx &c, int comp, int *iters, double *maxerr, int stage, CnDelta *plan = nullptr) {
     if (comp < 0 || comp > 3) return SARAS_BAD_ARG;
     if (comp == 3 && !c.scalar) return SARAS_BAD_ARG;
     if (comp == 1 && c.planar) { c.err = "the 2D solver has no Vy equation"; return SARAS_BAD_ARG; }
@@ -1996,7 +2029,7 @@ static int cn_solve_stage(Ctx &c, int comp, int *iters, double *maxerr, int stag
     double bytes = 3.0 * 8.0 * (double)make_view<double>(nullptr, f.n[0], f.n[1], f.n[2]).size();
     bool fast = c.p.fastKernels != 0;
     const double resScale = fast ? a.Dn : 1.0;
-    if (c.p.fastKernels == 2) return cn_solve_delta(c, comp, field, fa, a.Dn, bytes, iters, maxerr, stage);
+    if (c.p.fastKernels == 2) return cn_solve_delta(c, comp, field, fa, a.Dn, bytes, iters, maxerr, stage, plan);
     auto launch = [&](int withRes) {
         if (fast) {
             fa.in = cview(c, field);
@@ -2052,19 +2085,45 @@ static int cn_solve_stage(Ctx &c, int comp, int *iters, double *maxerr, int stag
 
 int cn_solve(Ctx &c, int comp, int *iters, double *maxerr) { return cn_solve_stage(c, comp, iters, maxerr, 0); }
 
-// fastKernels = 2: the velocity components' launches up to their speculative final
-// sweeps (each reads its own A and writes its own field's partner) with one copy of
-// the three residuals and one wait instead of three: 65^3 step 537 -> 507 us.  Only
-// when no component takes more sweeps than those two: further ones share the D buffers.
+// fastKernels = 2: the velocity components' sweeps from A, their speculative final ones
+// (each reads its own A and writes its own field's partner), with the components'
+// boundary shells in one launch before them and one after, one copy of the three
+// residuals and one wait.  Only when no component takes more sweeps than those two:
+// further ones share the D buffers.  65^3 step: one wait for three 537 -> 507 us, the
+// shells (and the projection's) together 481 -> 437 (257^3: 4.14 -> 4.09 ms).
 static int cn_together(Ctx &c, bool *begun) {
     *begun = false;
-    if (c.p.fastKernels != 2) return SARAS_OK;
+    if (c.p.fastKernels != 2 || c.planar) return SARAS_OK;
     for (int q = 0; q < 3; ++q)
         if (c.cnSweeps[q] > 2) return SARAS_OK;
+    CnDelta3 a;
+    int blocks = 0;
     for (int q = 0; q < 3; ++q) {
-        if (c.planar && q == 1) continue;
-        if (int e = cn_solve_stage(c, q, nullptr, nullptr, 1)) return e;
+        if (int e = cn_solve_stage(c, q, nullptr, nullptr, 1, &a.c[q])) return e;
+        blocks = std::max(blocks, (int)shell_blocks(a.c[q].full));
     }
+    const long N = c.cnpCount;
+    float *const dA = c.cnp + (size_t)8 * N, *const dAl = dA + N;
+    k_cn_delta_shell3<false, true><<<dim3(blocks, 6, 3), 256, 0, c.stream>>>(a);
+    count_launch(c);
+    SARAS_CUDA_TRY(cudaMemsetAsync(c.dscal, 0, 3 * sizeof(double), c.stream));
+    for (int q = 0; q < 3; ++q) {
+        CnDelta &d = a.c[q];
+        d.oh = dA; d.ol = dAl;   // not written: the sweep's output is vout
+        d.withResidual = 1;
+        d.vout = c.scratch[scratch_slot(SARAS_FIELD_VX + q)];
+        dim3 g, b; cn_delta_dims(d.full, g, b);
+        prof_begin(c, PK_CN, 0);
+        k_cn_delta<true><<<g, b, 0, c.stream>>>(d);
+        count_launch(c);
+        if (q == 2) {
+            k_cn_delta_shell3<true, false><<<dim3(blocks, 6, 3), 256, 0, c.stream>>>(a);
+            count_launch(c);
+        }
+        const int *n = c.info[SARAS_FIELD_VX + q].n;
+        prof_end(c, PK_CN, 0, 4.0 * 8.0 * (double)make_view<double>(nullptr, n[0], n[1], n[2]).size());
+    }
+    if (int e = check_launch(c, "cn")) return e;
     SARAS_CUDA_TRY(cudaMemcpyAsync(c.hscal, c.dscal, 3 * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
     SARAS_CUDA_TRY(cudaStreamSynchronize(c.stream));
     *begun = true;
@@ -2086,6 +2145,9 @@ int project(Ctx &c, bool with_bc) {
     count_launch(c);
     prof_begin(c, PK_PROJECT, 0);
     double bytes = 0;
+    ProjShell3 ps;
+    for (int &q : ps.on) q = 0;
+    int shellBlocks = 0;
     for (int q = 0; q < 3; ++q) {
         if (c.planar && q == 1) continue;   // 2D: the y gradient is 0, Vy unchanged
         int field = SARAS_FIELD_VX + q;
@@ -2101,11 +2163,11 @@ int project(Ctx &c, bool with_bc) {
             dim3 gb((unsigned)(((long)(pg.bhi[2] - pg.blo[2] + 1) * (pg.bhi[1] - pg.blo[1] + 1) + 255) / 256), 1);
             const int march = march_planes(c, gb.x, pg.bhi[0] - pg.blo[0] + 1, kProjMarch);
             gb.y = (pg.bhi[0] - pg.blo[0] + 1 + march - 1) / march;
-            dim3 gs(shell_blocks(fb), 6);
-            if (q == 0) { k_project_bulk<0><<<gb, 256, 0, c.stream>>>(out, in, Pp, pg, fdt, march); k_project_shell<0><<<gs, 256, 0, c.stream>>>(out, in, Pp, pg, fb, fdt); }
-            if (q == 1) { k_project_bulk<1><<<gb, 256, 0, c.stream>>>(out, in, Pp, pg, fdt, march); k_project_shell<1><<<gs, 256, 0, c.stream>>>(out, in, Pp, pg, fb, fdt); }
-            if (q == 2) { k_project_bulk<2><<<gb, 256, 0, c.stream>>>(out, in, Pp, pg, fdt, march); k_project_shell<2><<<gs, 256, 0, c.stream>>>(out, in, Pp, pg, fb, fdt); }
-            count_launch(c);
+            ps.out[q] = out; ps.in[q] = in; ps.Pp = Pp; ps.prog[q] = pg; ps.full[q] = fb; ps.fdt[q] = fdt; ps.on[q] = 1;
+            shellBlocks = std::max(shellBlocks, (int)shell_blocks(fb));
+            if (q == 0) k_project_bulk<0><<<gb, 256, 0, c.stream>>>(out, in, Pp, pg, fdt, march);
+            if (q == 1) k_project_bulk<1><<<gb, 256, 0, c.stream>>>(out, in, Pp, pg, fdt, march);
+            if (q == 2) k_project_bulk<2><<<gb, 256, 0, c.stream>>>(out, in, Pp, pg, fdt, march);
         } else if (c.p.fastKernels) {
             if (q == 0) k_project<0, true><<<g, bl, 0, c.stream>>>(out, in, Pp, f.full, fb, u, c.dt, wb, fdt);
             if (q == 1) k_project<1, true><<<g, bl, 0, c.stream>>>(out, in, Pp, f.full, fb, u, c.dt, wb, fdt);
@@ -2118,6 +2180,10 @@ int project(Ctx &c, bool with_bc) {
         count_launch(c);
         std::swap(c.f[field], c.scratch[q]);
         bytes += 3.0 * 8.0 * (double)out.size();
+    }
+    if (shellBlocks) {
+        k_project_shell3<<<dim3(shellBlocks, 6, 3), 256, 0, c.stream>>>(ps);
+        count_launch(c);
     }
     prof_end(c, PK_PROJECT, 0, bytes);
     return check_launch(c, "project");
