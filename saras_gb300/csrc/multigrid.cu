@@ -765,7 +765,8 @@ __device__ __forceinline__ void gs_step_sync() { asm volatile("barrier.sync 0;" 
 // set to the first sweep none of whose witness points is at or above tol.  The
 // compute warps and the witness warp run loops of the same steps; *alarm is
 // written in step 7 of 16 and read after step 15, so that all leave together.
-template <class A, bool PLANAR, bool RS, bool CHECK>
+// FULL: the steady steps run without tests (the coarsest solve's columns, GsPlan::zp).
+template <class A, bool PLANAR, bool RS, bool CHECK, bool FULL>
 __device__ __forceinline__ void gs_pipe_run(double *P, const double *R, long rsx, long rsy, double *gx, double *gy, int X, int Y, int Z,
                                             const MgBC &bc, const A &ar, const MgK &kk, int lam, int Q, int zp, int M, double tol, int *alarm) {
     const int W1 = Y + 1, nc = (X + 1) * W1;
@@ -874,7 +875,7 @@ __device__ __forceinline__ void gs_pipe_run(double *P, const double *R, long rsx
     const int fullLo = X + Y + lam * (Q - 1), fullHi = RS && period <= zp ? lam * (M - Q) + Z : 0;
     for (int t0 = 0; t0 < steps; t0 += 16) {
         const int n = min(16, steps - t0);
-        if (CHECK && t0 >= fullLo && t0 + 16 <= fullHi) {
+        if (FULL && t0 >= fullLo && t0 + 16 <= fullHi) {
 #pragma unroll 2
             for (int e = 0; e < 16; ++e) {
                 full_step();
@@ -909,7 +910,7 @@ __global__ void __launch_bounds__(1024) k_gs_pipe(View3<double> pg, View3<const 
     if (threadIdx.x == 0) alarm = -1;
     __syncthreads();
     const double *r = RS ? R : rg.p + o0;
-    gs_pipe_run<GsArith<ARITH>, PLANAR, RS, COARSE>(P, r, rg.sx, rg.sy, gx, gy, X, Y, Z, bc, ar, kk, lam, Q, zp, count, tol, &alarm);
+    gs_pipe_run<GsArith<ARITH>, PLANAR, RS, COARSE, COARSE>(P, r, rg.sx, rg.sy, gx, gy, X, Y, Z, bc, ar, kk, lam, Q, zp, count, tol, &alarm);
     if (COARSE) {
         const int stop = alarm;
         if (stop >= 0) {
@@ -917,7 +918,7 @@ __global__ void __launch_bounds__(1024) k_gs_pipe(View3<double> pg, View3<const 
             for (int t = threadIdx.x; t < n; t += blockDim.x) P[t] = 0.0;
             __syncthreads();
             if (stop > 0)
-                gs_pipe_run<GsArith<ARITH>, PLANAR, RS, false>(P, r, rg.sx, rg.sy, gx, gy, X, Y, Z, bc, ar, kk, lam, Q, zp, stop, tol, nullptr);
+                gs_pipe_run<GsArith<ARITH>, PLANAR, RS, false, true>(P, r, rg.sx, rg.sy, gx, gy, X, Y, Z, bc, ar, kk, lam, Q, zp, stop, tol, nullptr);
             const int N = (X + 3) * (Y + 3) * (Z + 3), sy = Z + 3, sx = (Y + 3) * sy;
             double *pp = R + (RS ? n : 0), *rr = pp + N;
             for (int t = threadIdx.x; t < N; t += blockDim.x) { pp[t] = 0.0; rr[t] = rg.p[t]; }
