@@ -729,6 +729,10 @@ __global__ void k_bc_apply_shell(View3<double> out, View3<const double> in, BcPr
 // residual of the incoming iterate V_in over the bulk (lines 393-407) and the
 // next iterate V_out = BCs(guess) over the whole padded box (lines 375-391),
 // where guess is the Jacobi update on the bulk and 0 elsewhere.
+__device__ __forceinline__ void zero_slots(double *slot) {
+    if ((blockIdx.x | blockIdx.y | blockIdx.z | threadIdx.x | threadIdx.y | threadIdx.z) == 0) slot[0] = slot[1] = slot[2] = 0.0;
+}
+
 struct CnArgs {
     View3<double> out;
     View3<const double> in;
@@ -741,7 +745,7 @@ struct CnArgs {
     int scalarForm;          // scalar_d3: ((A*dt)*coef)/X + rhs, Dn = 1 + (dt*coef)*B/h
     double lx, ly, lz;       // residual: metric * 1/(h*h)
     double resCoef;          // inverseRe (hydro) or nu / kappa (scalar)
-    int withResidual;
+    int withResidual;        // 1: max residual of the input into *resMax; 2: three slots there to 0
     double *resMax;
     // stretched meshes: the metrics of the component at each index (mx(i),
     // my(j), mz(k) of hydro_d3.cc:378-400), so c1..c3, B, Dn and lx..lz are
@@ -803,7 +807,8 @@ __global__ void k_cn(CnArgs a) {
             });
         }
     }
-    if (a.withResidual) block_max_to(res, a.resMax);
+    if (a.withResidual == 1) block_max_to(res, a.resMax);
+    else if (a.withResidual == 2) zero_slots(a.resMax);
 }
 
 // Fast form of the same Jacobi iteration (fastKernels = 1): the two divisions
@@ -847,7 +852,8 @@ __global__ void __launch_bounds__(256) k_cn_fast(CnFast a) {
             });
         }
     }
-    if (a.withResidual) block_max_to(res, a.resMax);
+    if (a.withResidual == 1) block_max_to(res, a.resMax);
+    else if (a.withResidual == 2) zero_slots(a.resMax);
 }
 
 // Split-FP64 form of the same Jacobi iteration (fastKernels = 2), in delta
@@ -2409,7 +2415,8 @@ int time_advance(Ctx &c, saras_step_stats *st) {
 namespace saras {
 
 constexpr long kNoAllocMaxPoints = 4L << 20;   // 4 Mi doubles (32 MiB): padded field arrays up to this size
-constexpr long kCnBatchPoints = 128L << 10;   // at most kNoAllocMaxPoints / 4
+constexpr long kCnTinyPoints = 16L << 10;
+constexpr long kCnBatchPoints = 128L << 10;   // at most kNoAllocMaxPoints / 5
 static __device__ __align__(256) double g_cn_scratch[kNoAllocMaxPoints + 32];
 // Device address of g_cn_scratch, per device ordinal.  Atomic: two host
 // threads making their first call on a device at the same time both look the
@@ -2578,45 +2585,49 @@ extern "C" int saras_cn_solve_noalloc(const saras_params *p, int component, doub
         fa.resMax = a.resMax;
     }
     const double resScale = fast ? a.Dn : 1.0;
-    // The iterates go round a ring: iterate n is in buffer n mod ring, buffer 0 being v
-    // and the others fields in the fixed array.  Sweep n + 1 writes the next iterate and,
-    // from the first on, the residual of iterate n; ring - 1 sweeps run between waits,
-    // their residuals are read in one copy and tested in order, and sweeps beyond the
-    // accepted iterate are thrown away.  A wait costs as much as several sweeps of a
-    // small field (33^3: a solve 106 -> 81 us), but less than one of a large field, which
-    // waits after each sweep.
+    // Sweep n + 1 writes iterate n + 1 and, from the second on, the residual of iterate n.
+    // A wait costs as much as several sweeps of a small field, so there three sweeps (two
+    // on a tiny one), then four at a time, run between waits (33^3, 1 / 2 / 4 / 10 sweeps:
+    // 55 / 70 / 123 / 278 us with a wait each, 53 / 63 / 110 / 156; 17^3, 1 / 2 / 3 / 7:
+    // 44 / 60 / 96 / 199, 39 / 50 / 95 / 138, with three first 51 / 62 / 61 / 105); their residuals are read in one copy and tested
+    // in order, and sweeps beyond the accepted iterate are thrown away. Iterates 1, 2, ...
+    // go round five fields of the fixed array, and iterate 1, often the answer, is in v
+    // by the first wait. A large field waits after each sweep, between s1 and v.
     constexpr int kRing = 5;
-    const int ring = points <= kCnBatchPoints ? kRing : 2;
-    const int batch = ring - 1;
-    auto buf = [&](int n) { return n % ring == 0 ? v : scratch + (long)(n % ring - 1) * points; };
+    const bool batched = points <= kCnBatchPoints;
+    auto buf = [&](int n) {
+        if (!batched) return n % 2 ? scratch : v;
+        return n == 0 ? v : scratch + (long)((n - 1) % kRing) * points;
+    };
     auto view_of = [&](double *ptr) { return make_view<double>(ptr, f.n[0], f.n[1], f.n[2]); };
-    auto launch = [&](int n, double *slot) {   // iterate n -> n + 1; slot: iterate n's residual
+    auto launch = [&](int n, double *slot) {   // iterate n -> n + 1; slot: iterate n's residual (n = 0: slots to 0)
         View3<double> in = view_of(buf(n)), out = view_of(buf(n + 1));
         View3<const double> cin;
         cin.p = in.p; cin.n[0] = in.n[0]; cin.n[1] = in.n[1]; cin.n[2] = in.n[2]; cin.sx = in.sx; cin.sy = in.sy;
         if (fast) {
-            fa.in = cin; fa.out = out; fa.withResidual = slot ? 1 : 0; fa.resMax = slot;
+            fa.in = cin; fa.out = out; fa.withResidual = n ? 1 : 2; fa.resMax = slot;
             // fastKernels 1 and 2 both run this fused multiply-add form: the
             // split-FP64 form of fastKernels = 2 keeps N0 and the correction
             // as float pairs, 12 more floats a point than the fixed array holds
             k_cn_fast<<<g, bl, 0, st>>>(fa);
         } else {
-            a.in = cin; a.out = out; a.withResidual = slot ? 1 : 0; a.resMax = slot;
+            a.in = cin; a.out = out; a.withResidual = n ? 1 : 2; a.resMax = slot;
             k_cn<<<g, bl, 0, st>>>(a);
         }
         return cudaGetLastError();
     };
-    cudaError_t e = launch(0, nullptr);
+    cudaError_t e = launch(0, resSlots);
     if (e != cudaSuccess) { set_error(cudaGetErrorString(e)); return SARAS_CUDA_ERROR; }
     int sweeps = 1, failed = 0, done = 1;   // iterate under test; iterates computed
     double res = 0.0, got[kRing];
     int status = SARAS_OK;
     bool more = true;
     while (more) {
-        const int n = batch;
-        if ((e = cudaMemsetAsync(resSlots, 0, sizeof(double) * n, st)) != cudaSuccess) break;
+        const int n = !batched ? 1 : done > 1 ? kRing - 1 : points <= kCnTinyPoints ? 2 : 3, first = done;
+        if (done > 1 && (e = cudaMemsetAsync(resSlots, 0, sizeof(double) * n, st)) != cudaSuccess) break;
         for (int q = 0; q < n && e == cudaSuccess; ++q) e = launch(done++, resSlots + q);
         if (e != cudaSuccess) break;
+        if (batched && first == 1 && (e = cudaMemcpyAsync(v, buf(1), sizeof(double) * points, cudaMemcpyDeviceToDevice, st)) != cudaSuccess) break;
         if ((e = cudaMemcpyAsync(got, resSlots, sizeof(double) * n, cudaMemcpyDeviceToHost, st)) != cudaSuccess) break;
         if ((e = cudaStreamSynchronize(st)) != cudaSuccess) break;
         for (int q = 0; q < n; ++q) {
@@ -2633,7 +2644,7 @@ extern "C" int saras_cn_solve_noalloc(const saras_params *p, int component, doub
     if (e != cudaSuccess) { set_error(cudaGetErrorString(e)); return SARAS_CUDA_ERROR; }
     // the answer is iterate `sweeps`; bring it into the caller's array if it sits in the scratch
     const double *cur = buf(sweeps);
-    if (cur != v) {
+    if (cur != v && !(batched && sweeps == 1)) {
         if ((e = cudaMemcpyAsync(v, cur, sizeof(double) * points, cudaMemcpyDeviceToDevice, st)) != cudaSuccess ||
             (e = cudaStreamSynchronize(st)) != cudaSuccess) {
             set_error(cudaGetErrorString(e));
