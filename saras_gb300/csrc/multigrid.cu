@@ -734,7 +734,7 @@ __global__ void k_mg_gs_block(View3<double> pg, View3<const double> rg, MgK kk, 
 // Arith forms below save (exact folding of powers of two: 9 operations on
 // equal power-of-two spacings and metrics, 12 otherwise, 16 as the expression is written).
 // Measured, one sweep at a time -> pipelined: 217 sweeps of a 5^3 level 2.65 ms ->
-// 0.20 (mirror, lam 2) and 0.46 (periodic, general metrics, lam 4); 1001 of a 9^3
+// 0.19 (mirror, lam 2) and 0.46 (periodic, general metrics, lam 4); 1001 of a 9^3
 // periodic level 24.9 -> 3.66 ms; four sweeps of a 17^3 level 0.27 -> 0.11 ms and of
 // a 65 x 65 2D level 1.66 -> 0.15 ms.
 //

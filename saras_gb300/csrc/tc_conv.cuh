@@ -13,7 +13,7 @@
 // M-adjacent core matrices (8 rows, 128 bytes) 128 B apart and K-adjacent ones a plane
 // apart, so a tap's A tile is the stage's rows from dx on, and its 128 rows are three
 // overlapping views of one copy: 25 us for 16 -> 16 channels on 65^3 voxels, 87 for 48 ->
-// 16, where gathering each tap's tile by itself, three times the loads, took 43 and 128.
+// 16, where gathering each tap's tile by itself, three times the loads, took 40 and 121.
 // The descriptors are formed once (forming two in the loop cost the issuing thread 98 to
 // 175 clocks an MMA, 47 with sums; the SM takes one in 39).  The nine stages go round a ring of four (two when
 // they are too large for that): a stage's 3 x chunks tcgen05.mma (K = 16), in the taps'
