@@ -1892,9 +1892,9 @@ __global__ void __launch_bounds__(256, 3) k_fx_refine(const long long *__restric
 // last bit.  With 2^57 <= max|P| < 2^58 that bit is finer than FP64's for every value
 // above max|P| / 32; what the solve returns is rounded to FP64 by its last sweep.  The
 // exact residual left after 25 cycles, relative to max|b| (Taylor-Green 33^3 / 65^3 /
-// 129^3): 2.0e-15 / 8.7e-15 / 3.8e-14, with FP64 levels 4.2e-15 / 2.8e-14 / 9.9e-14.  An FP64 sweep is bound by the FP64 pipe (one warp instruction in
-// 64 clocks on an SM quarter), the integer one by HBM: at
-// 257^3 a sweep 265 -> 76 us, residual 265 -> 70, its maximum 298 -> 62, restriction
+// 129^3): 2.0e-15 / 8.7e-15 / 3.8e-14, with FP64 levels 4.2e-15 / 2.8e-14 / 9.9e-14.  An
+// FP64 sweep is bound by the FP64 pipe (one warp instruction in 64 clocks on an SM
+// quarter), the integer one by HBM: at 257^3 a sweep 265 -> 76 us, residual 265 -> 70, its maximum 298 -> 62, restriction
 // 134 -> 32, prolongation 182 -> 55; a step 14.6 -> 9.0 ms with level 0 alone, 6.2 with
 // every level above the tail (129^3: sweep 37 -> 13 us).
 // The levels' arrays hold the integers themselves (pa, pb, r), so the mode takes no more
@@ -2695,8 +2695,9 @@ static int chk(Ctx &c, const char *what) {
     return SARAS_OK;
 }
 
-// First level of the fused coarse tail (k_mg_tail), or -1: all axes at most 16
-// intervals, at least two levels, and every tail level in shared memory.
+// First level of the fused coarse tail (k_mg_tail), or -1: all axes at most
+// kTailIntervals, at least two levels, and every tail level in shared memory (FP32 tails
+// start a level above where Ctx::tailBig says so).
 static int tail_level(const Ctx &c) {
     if (c.p.preSmooth > kTailMaxSweeps || c.p.postSmooth > kTailMaxSweeps || c.p.coarseSmooth > kTailMaxSweeps) return -1;
     for (int l = 1; l < c.depth; ++l) {
