@@ -3211,7 +3211,8 @@ static int gs_smooth(Ctx &c, int l, int count, bool zero_first) {
     GsArith<2> a = {};
     const int form = bc.dirichlet && c.planar ? -1 : gs_arith(c, L, a);
     cudaError_t e = cudaSuccess;
-    for (int st = 0; st < g.stages + g.lam * (count - 1) && e == cudaSuccess; ++st) {
+    const int last = count > 0 ? g.stages + g.lam * (count - 1) : 0;   // a phase of no sweeps leaves the ghosts alone to fill
+    for (int st = 0; st < last && e == cudaSuccess; ++st) {
         const dim3 grid(g.nb[0] * g.nb[1], count, 1);
         auto go = [&](auto k, auto ar) {
             ar.cx2 = a.cx2; ar.cy2 = a.cy2; ar.cz2 = a.cz2; ar.c7 = a.c7; ar.den = a.den; ar.iden = a.iden;
