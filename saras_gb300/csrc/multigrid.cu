@@ -2529,6 +2529,10 @@ __global__ void __launch_bounds__(BIG ? kTailBigThreads : kTailThreads) k_mg_tai
             if (p.on) out[p.o] = v;
             __syncthreads();
         }
+        if (a.pre == 0) {   // the 0 start that no sweep writes
+            if (p.on) arr(l, 0)[p.o] = (T)0;
+            __syncthreads();
+        }
         // residual into the other array, then the restriction
         const TgK<T> &c = a.tr[l];
         const T *in = arr(l, a.pre & 1);
@@ -3277,6 +3281,7 @@ static int smooth(Ctx &c, int l, int count, bool zero_first, bool tgt) {
             return launch_pdl(k_tgt_sweep<T, decltype(zero)::value, decltype(m)::value>, gm, bm, 0, c.stream, B_<T>(L), A_<T>(L), R_<T>(L), sx, sy, bc, tk);
         });
     };
+    if (zero_first && count <= 0) SARAS_CUDA_TRY(cudaMemsetAsync(A_<T>(L), 0, sizeof(T) * (size_t)L.count, c.stream));   // no sweep writes the 0 start
     for (int n = 0; n < count; ++n) {
         TgK<T> tk = make_tgk<T>(L, tgt ? smooth_weight(c, n, count) : c.p.jacobiWeight);
         prof_begin(c, pk, l);

@@ -59,3 +59,33 @@ def test_gauss_seidel_phase_of_no_sweeps(ind, depth):
 @pytest.mark.parametrize("pre,post", [(0, 3), (3, 0), (0, 1)])
 def test_gauss_seidel_cycle(ind, depth, pre, post):
     two_steps(cavity(ind, depth, 1, pre, post))
+
+
+@pytest.mark.parametrize("pre,post", [(0, 3), (0, 1), (3, 0)])
+def test_jacobi_cycle(pre, post):
+    two_steps(cavity((5, 5, 5), 2, 0, pre, post))
+
+
+@pytest.mark.parametrize("depth", [2, 4])    # levels of their own, and a tail from 9^3 down
+def test_target_cycle(depth):
+    """V(0, 3) cycles of the target modes: each one starts the coarse levels from 0, so the FP32
+    and the FP64 cycles leave the same residual, up to FP32's rounding of a correction (1e-5 of the
+    residual before it, and a cycle reduces that by 100 at most), and reduce it each time."""
+    left = {}
+    for mode in (F.MG_PLAIN_TARGET, F.MG_MIXED):
+        for cycles in (1, 2, 3):
+            p = cavity((5, 5, 5), depth, 0, 0, 3)
+            p.mgMode, p.mgTarget, p.mgMaxCycles, p.mixedCycles = mode, 1e-13, cycles, 1
+            p.smoother, p.jacobiWeight = F.SMOOTHER_JACOBI, 6.0 / 7.0
+            g = Solver(p)
+            rng = np.random.default_rng(3)
+            for f in (F.FIELD_VX, F.FIELD_VZ):
+                g.set(f, 0.1 * rng.standard_normal(g.dims(f)))
+                g.apply_bc(f)
+            status, st = g.time_advance()
+            assert status == F.NOT_CONVERGED and st.vcycles == cycles
+            left[mode, cycles] = st.fine_residual
+    for cycles in (1, 2, 3):
+        a, b = left[F.MG_PLAIN_TARGET, cycles], left[F.MG_MIXED, cycles]
+        assert abs(a - b) <= 1e-3 * a, left
+        assert cycles == 1 or a < 0.5 * left[F.MG_PLAIN_TARGET, cycles - 1], left
