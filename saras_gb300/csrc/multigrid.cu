@@ -1898,7 +1898,9 @@ __global__ void __launch_bounds__(256, 3) k_fx_refine(const long long *__restric
 // 134 -> 32, prolongation 182 -> 55; a step 14.6 -> 9.0 ms with level 0 alone, 6.2 with
 // every level above the tail (129^3: sweep 37 -> 13 us).
 // The levels' arrays hold the integers themselves (pa, pb, r), so the mode takes no more
-// memory.  flag: P beyond +-2^59 or B beyond +-2^60, above which a sum could pass 2^63.
+// memory.  flag: P beyond +-2^59, B beyond +-2^60 or a residual on its way down beyond
+// +-2^58, above which a stencil sum (14 x 2^59) or a plane sum of the restriction (16 x
+// 2^58) could pass 2^63: the solve then starts over on the FP64 levels.
 __device__ __forceinline__ bool fx_far(long long p) { return p > (1LL << 59) || p < -(1LL << 59); }
 
 // ROUND: the sweep whose output the solve may return (round53).  ZERO: from P = 0.
@@ -1926,18 +1928,24 @@ __global__ void __launch_bounds__(256, 3) k_fx_sweep(long long *__restrict__ out
     if (bad) atomicExch(flag, 1);
 }
 
-// -d over the core: the residual in units of l 2^-s.
+// -d over the core: the residual in units of l 2^-s.  A smooth one below level 0 keeps its
+// level's B's size, up to 2^60, which the 16 of a plane sum would carry past 2^63.
 template <int CH>
 __global__ void __launch_bounds__(256, 3) k_fx_residual(long long *__restrict__ out, const long long *__restrict__ in, const long long *__restrict__ bfx,
-                                                        int sx, int sy, MgBC bc) {
+                                                        int sx, int sy, MgBC bc, int *flag) {
     pdl_wait();
     int j, k, seg;
     if (!col_of<true>(bc, j, k, seg)) return;
-    fx_column<CH>(in, bfx, sx, sy, bc, j, k, seg, [&](long o, long long, long long d) { out[o] = -d; });
+    bool bad = false;
+    fx_column<CH>(in, bfx, sx, sy, bc, j, k, seg, [&](long o, long long, long long d) {
+        bad |= d > (1LL << 58) || d < -(1LL << 58);
+        out[o] = -d;
+    });
+    if (bad) atomicExch(flag, 1);
 }
 
 // Full weighting of the integer residual (k_tgt_restrict's stencil): exact sums in a
-// plane, the planes' sum in units of four (residuals up to 2^58 stay inside 63 bits),
+// plane, the planes' sum in units of four (residuals up to 2^58, k_fx_residual's bound, stay inside 63 bits),
 // then one conversion (scale[0] = l 2^-s / 16), or, to a level in fixed point, the
 // shift sh: B = 4 R there (a quarter of l), and twice that below level 0, whose unit is
 // two of the others'.
@@ -3516,7 +3524,8 @@ static int fx_restrict(Ctx &c, int l) {
     const int ch = level_dims<double>(c, L, g, b);
     prof_begin(c, PK_MG_RESID64, l);
     SARAS_CUDA_TRY(with_march<double>(ch, [&](auto m) {
-        return launch_pdl(k_fx_residual<decltype(m)::value>, g, b, 0, c.stream, fx_of(L.pb()), fx_of(L.pa()), fx_of(L.r), sx, sy, bc);
+        return launch_pdl(k_fx_residual<decltype(m)::value>, g, b, 0, c.stream, fx_of(L.pb()), fx_of(L.pa()), fx_of(L.r), sx, sy, bc,
+                          fx_flag(c));
     }));
     prof_end(c, PK_MG_RESID64, l, 3.0 * 8.0 * pts);
     const long ccols = (long)(C.n[1] + 1) * (C.n[2] + 1);
@@ -4098,7 +4107,7 @@ static int plain_fixed(Ctx &c, const double *pp0, double mean, double bmax, doub
         int fl;
         std::memcpy(&mx, &c.hscal[34], sizeof mx);
         std::memcpy(&fl, &c.hscal[35], sizeof fl);
-        bad = fl != 0 || mx > (1ull << 58);   // k_fx_restrict sums 16 of them in a plane
+        bad = fl != 0 || mx > (1ull << 58);   // k_fx_residual's bound, before a cycle runs for nothing
         r = (double)mx * rs;
         return SARAS_OK;
     };
