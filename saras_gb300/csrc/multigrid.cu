@@ -1899,8 +1899,8 @@ __global__ void __launch_bounds__(256, 3) k_fx_refine(const long long *__restric
 // every level above the tail (129^3: sweep 37 -> 13 us).
 // The levels' arrays hold the integers themselves (pa, pb, r), so the mode takes no more
 // memory.  flag: P beyond +-2^59, B beyond +-2^60 or a residual on its way down beyond
-// +-2^58, above which a stencil sum (14 x 2^59) or a plane sum of the restriction (16 x
-// 2^58) could pass 2^63: the solve then starts over on the FP64 levels.
+// +-(2^59 - 4), above which a stencil sum (14 x 2^59) or a plane sum of the restriction
+// (16 residuals) could pass 2^63: the solve then starts over on the FP64 levels.
 __device__ __forceinline__ bool fx_far(long long p) { return p > (1LL << 59) || p < -(1LL << 59); }
 
 // ROUND: the sweep whose output the solve may return (round53).  ZERO: from P = 0.
@@ -1938,14 +1938,14 @@ __global__ void __launch_bounds__(256, 3) k_fx_residual(long long *__restrict__ 
     if (!col_of<true>(bc, j, k, seg)) return;
     bool bad = false;
     fx_column<CH>(in, bfx, sx, sy, bc, j, k, seg, [&](long o, long long, long long d) {
-        bad |= d > (1LL << 58) || d < -(1LL << 58);
+        bad |= d > (1LL << 59) - 4 || d < 4 - (1LL << 59);
         out[o] = -d;
     });
     if (bad) atomicExch(flag, 1);
 }
 
 // Full weighting of the integer residual (k_tgt_restrict's stencil): exact sums in a
-// plane, the planes' sum in units of four (residuals up to 2^58, k_fx_residual's bound, stay inside 63 bits),
+// plane, the planes' sum in units of four (residuals up to 2^59 - 4, k_fx_residual's bound, stay inside 63 bits),
 // then one conversion (scale[0] = l 2^-s / 16), or, to a level in fixed point, the
 // shift sh: B = 4 R there (a quarter of l), and twice that below level 0, whose unit is
 // two of the others'.
@@ -4107,7 +4107,7 @@ static int plain_fixed(Ctx &c, const double *pp0, double mean, double bmax, doub
         int fl;
         std::memcpy(&mx, &c.hscal[34], sizeof mx);
         std::memcpy(&fl, &c.hscal[35], sizeof fl);
-        bad = fl != 0 || mx > (1ull << 58);   // k_fx_residual's bound, before a cycle runs for nothing
+        bad = fl != 0 || mx > (1ull << 58);   // no cycle from the edge of k_fx_residual's range
         r = (double)mx * rs;
         return SARAS_OK;
     };
