@@ -1944,6 +1944,19 @@ __global__ void __launch_bounds__(256, 3) k_fx_residual(long long *__restrict__ 
     if (bad) atomicExch(flag, 1);
 }
 
+// max |P| over the core.
+__global__ void __launch_bounds__(256) k_fx_maxabs(const long long *__restrict__ pin, int sx, int sy, MgBC bc, unsigned long long *maxp) {
+    int j, k, seg;
+    const bool on = col_of<true>(bc, j, k, seg);
+    unsigned long long m = 0;
+    for (int i = seg * kIch; on && i <= min(seg * kIch + kIch - 1, bc.E[0]); ++i) {
+        const long long p = pin[(long)(i + 1) * sx + (long)(j + 1) * sy + (k + 1)];
+        const unsigned long long a = (unsigned long long)(p < 0 ? -p : p);
+        m = a > m ? a : m;
+    }
+    block_max_bits_to(m, reinterpret_cast<double *>(maxp));
+}
+
 // Full weighting of the integer residual (k_tgt_restrict's stencil): exact sums in a
 // plane, the planes' sum in units of four (residuals up to 2^59 - 4, k_fx_residual's bound, stay inside 63 bits),
 // then one conversion (scale[0] = l 2^-s / 16), or, to a level in fixed point, the
@@ -4062,8 +4075,16 @@ static int mixed_fixed(Ctx &c, const double *pp0, double mean, double bmax, doub
 }
 
 // The plain mode's solve in fixed point (k_fx_sweep): V-cycles until the
-// exact residual meets the target.  done: the result is in Pp; otherwise (no scale to
-// take from the previous Pp, or values out of range) nothing the FP64 path reads has changed.
+// exact residual meets the target.  done: the result is in Pp; otherwise nothing the FP64
+// path reads has changed.  That path takes the solve when
+//   the previous Pp gives no scale, or values leave the range;
+//   the iterate has shrunk far below the previous Pp (a start far off, a changed time
+//   step) and its residual stalls: the unit stays that of the largest value, where FP64's
+//   rounding follows the iterate.  Asked for where a cycle below kFxStall units, far above
+//   what rounding leaves (a few hundred), does not halve the residual, or is the last one;
+//   below 2^53 units an FP64 iterate's last bit is finer than the unit;
+//   the residual meets the target by less than B's own rounding.
+constexpr unsigned long long kFxStall = 1ull << 16;
 static int plain_fixed(Ctx &c, const double *pp0, double mean, double bmax, double pmax, double target, double &r, int &cyc, bool &done,
                        saras_step_stats *st) {
     done = false;
@@ -4095,6 +4116,7 @@ static int plain_fixed(Ctx &c, const double *pp0, double mean, double bmax, doub
     k_fx_init<<<gc, bcd, 0, c.stream>>>(fx_of(L0.pa()), lcview<double>(L0, pp0), bc0, sc, fx_flag(c));
     count_launch(c, 2);
     bool bad = false;
+    unsigned long long mx = 0;
     auto residual = [&]() -> int {
         SARAS_CUDA_TRY(cudaMemsetAsync(c.dscal + 34, 0, sizeof(double), c.stream));
         prof_begin(c, PK_REFINE_RESID, 0);
@@ -4103,7 +4125,6 @@ static int plain_fixed(Ctx &c, const double *pp0, double mean, double bmax, doub
         count_launch(c);
         if (int e = chk(c, "fixed-point residual")) return e;
         if (int e = read_scalars(c, 34, 2)) return e;
-        unsigned long long mx;
         int fl;
         std::memcpy(&mx, &c.hscal[34], sizeof mx);
         std::memcpy(&fl, &c.hscal[35], sizeof fl);
@@ -4120,8 +4141,20 @@ static int plain_fixed(Ctx &c, const double *pp0, double mean, double bmax, doub
         c.fxPlain = 0;
         if (s) return s;
         cyc += 1;
+        const unsigned long long before = mx;
         if ((s = residual())) return s;
+        if (!bad && r > target && mx < kFxStall && (mx > before / 2 || cyc == c.mgMaxCycles)) {
+            unsigned long long pm;
+            SARAS_CUDA_TRY(cudaMemsetAsync(c.dscal + 34, 0, sizeof(double), c.stream));
+            k_fx_maxabs<<<gk, bk, 0, c.stream>>>(fx_of(L0.pa()), sx, sy, bc0, dmax);
+            count_launch(c);
+            if ((s = chk(c, "fixed-point maximum"))) return s;
+            if ((s = read_scalars(c, 34, 1))) return s;
+            std::memcpy(&pm, &c.hscal[34], sizeof pm);
+            bad = pm < (1ull << 53);
+        }
     }
+    if (!bad && r <= target && r + rs > target) bad = true;
     if (bad) {
         cyc = 0;
         L0.cur = 0;

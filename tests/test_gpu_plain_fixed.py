@@ -57,3 +57,38 @@ def test_residual_too_large_for_a_plane_sum(k, amplitude):
         out = [solve(solver(fp64, pre=1, post=2, smoother=F.SMOOTHER_JACOBI, cycles=cycles), P, b) for fp64 in (0, 1)]
         assert out[0][:2] == out[1][:2] and (out[0][0] == 0) == (cycles == 100)
         assert np.array_equal(out[0][2], out[1][2]), cycles
+
+
+def smooth(n, seed):
+    """A few of the first waves, without a mean."""
+    rng = np.random.default_rng(seed)
+    x = 2 * np.pi * np.arange(n) / n
+    b = np.zeros((n, n, n))
+    for _ in range(6):
+        k = rng.integers(0, 5, 3) + np.array([1, 0, 0])
+        b += rng.standard_normal() * np.cos(k[0] * x[:, None, None] + k[1] * x[None, :, None] + k[2] * x[None, None, :] + 6 * rng.random())
+    return b - b.mean()
+
+
+@pytest.mark.parametrize("scale,target,fp64", [(0, 1e-8, False), (0, 1e-12, False), (10, 1e-12, False), (20, 1e-8, False), (20, 1e-12, True),
+                                               (30, 1e-8, True), (40, 1e-8, True), (60, 1e-8, True)])
+def test_start_far_above_the_solution(scale, target, fp64):
+    """A start 2^scale times the solution's size: the solve meets its target (the exact residual of the
+    returned Pp, in extended precision), on the FP64 levels where the start's unit is too coarse for it."""
+    n = 32
+    b, P = smooth(n, 2), 2.0 ** scale * 3.0 / n ** 2 * smooth(n, 3)
+    out = [solve(solver(a, target=target), P, b) for a in (0, 1)]
+    assert out[0][0] == out[1][0] == 0
+    assert np.array_equal(out[0][2], out[1][2]) == fp64
+    c = b.astype(np.longdouble) - b.astype(np.longdouble).mean()
+    r = c - n * n * lap(out[0][2].astype(np.longdouble))
+    assert np.max(np.abs(r)) <= target * np.max(np.abs(c)) * (1 + 1e-6)
+
+
+def test_right_hand_side_below_the_unit():
+    """Pp all one value, 2^70 times the right-hand side: in its unit the right-hand side is 0 and the
+    residual too, which says nothing; FP64 levels cannot reduce it and say so."""
+    b = smooth(32, 2)
+    out = [solve(solver(a, cycles=20), np.full(b.shape, 2.0 ** 70), b) for a in (0, 1)]
+    assert out[0][0] == out[1][0] == F.NOT_CONVERGED
+    assert np.array_equal(out[0][2], out[1][2])
