@@ -68,6 +68,8 @@ struct Level {
     double hx2 = 0, hz2 = 0;         // 2D: pow(2^l dXi, 2), pow(2^l dZt, 2) (poisson.cc:426-428)
     int planar = 0;
     const double *xix2 = nullptr, *xixx = nullptr, *ety2 = nullptr, *etyy = nullptr, *ztz2 = nullptr, *ztzz = nullptr;
+    bool fxHeld = false;   // pa and r hold integers in units of 2^-fxUnit (plain_fixed), until mg_release_levels
+    int fxUnit = 0;
     double *pa() const { return cur == 0 ? a : b; }
     double *pb() const { return cur == 0 ? b : a; }
     float *pa32() const { return cur32 == 0 ? a32 : b32; }
@@ -218,6 +220,7 @@ int mg_smooth_level(Ctx &c, int level, int count);
 int mg_restrict_level(Ctx &c, int level);
 int mg_prolong_level(Ctx &c, int level);
 int mg_compute_error(Ctx &c, int norm, double *err);
+int mg_release_levels(Ctx &c);
 int mg_set_level(Ctx &c, int level, int which, const double *host);
 int mg_get_level(Ctx &c, int level, int which, double *host);
 int mg_test_prolong(Ctx &c, double *err);

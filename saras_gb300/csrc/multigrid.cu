@@ -2256,6 +2256,15 @@ __global__ void __launch_bounds__(256) k_fx_rhs(long long *__restrict__ dst, dou
 }
 
 
+// The FP64 values of a level's integers: P with its face ghosts into dst, B in place.
+__global__ void k_fx_release(View3<double> dst, View3<const double> p, double *r, MgBC bc, double unit, double l) {
+    int i, j, k;
+    if (!core_pt(bc.E, i, j, k)) return;
+    put_scatter(dst, i, j, k, __ll2double_rn(__double_as_longlong(p(i, j, k))) * unit, bc);
+    const long o = p.off(i, j, k);
+    r[o] = __ll2double_rn(__double_as_longlong(r[o])) * unit * l;
+}
+
 // ---- target modes (FP64 / mixed)
 // Order-preserving key of a double (unsigned comparison of keys = numeric
 // comparison of values, NaN above +Inf), and its inverse on the host.
@@ -3787,6 +3796,7 @@ static double error_value(const Ctx &c, int norm) {
 
 int mg_compute_error(Ctx &c, int norm, double *err) {
     int s;
+    if ((s = mg_release_levels(c))) return s;
     if (norm == 1 && (s = error_denominator(c))) return s;
     if ((s = error_launches(c, norm))) return s;
     SARAS_CUDA_TRY(cudaStreamSynchronize(c.stream));
@@ -3797,6 +3807,7 @@ int mg_compute_error(Ctx &c, int norm, double *err) {
 // poisson::mgSolve (poisson.cc:100-205), reference mode.
 static int mg_solve_reference(Ctx &c, int *cycles, double *residual) {
     int s;
+    if ((s = mg_release_levels(c))) return s;
     Level &L0 = c.lv[0];
     MgBC bc0 = level_bc(c, 0, false);
     // zero scalars used for the |r| denominator and the mean offset trick
@@ -4074,6 +4085,26 @@ static int mixed_fixed(Ctx &c, const double *pp0, double mean, double bmax, doub
     return fp64_start();
 }
 
+// The level arrays as FP64 values again after plain_fixed, for whatever else reads them
+// (the other solves, the level calls below, the network's guess of the current b).  The
+// solves themselves leave the integers: nothing in a time step reads them.
+int mg_release_levels(Ctx &c) {
+    for (int l = 0; l <= c.depth; ++l) {
+        Level &L = c.lv[l];
+        if (!L.fxHeld) continue;
+        const size_t bytes = sizeof(double) * (size_t)L.count;
+        dim3 g, b; core_dims(L, g, b);
+        SARAS_CUDA_TRY(cudaMemsetAsync(L.pb(), 0, bytes, c.stream));   // the padding off the faces
+        k_fx_release<<<g, b, 0, c.stream>>>(lview<double>(L, L.pb()), lcview<double>(L, L.pa()), L.r, level_bc(c, l, true), std::ldexp(1.0, -L.fxUnit),
+                                            L.lx);
+        count_launch(c);
+        L.cur ^= 1;
+        SARAS_CUDA_TRY(cudaMemsetAsync(L.pb(), 0, bytes, c.stream));
+        L.fxHeld = false;
+    }
+    return chk(c, "release levels");
+}
+
 // The plain mode's solve in fixed point (k_fx_sweep): V-cycles until the
 // exact residual meets the target.  done: the result is in Pp; otherwise nothing the FP64
 // path reads has changed.  That path takes the solve when
@@ -4115,6 +4146,8 @@ static int plain_fixed(Ctx &c, const double *pp0, double mean, double bmax, doub
     k_fx_rhs<<<gk, bk, 0, c.stream>>>(fx_of(L0.r), nullptr, c.f[SARAS_FIELD_MGRHS], sx, sy, bc0, mean, std::ldexp(1.0, sc) / l, fx_flag(c));
     k_fx_init<<<gc, bcd, 0, c.stream>>>(fx_of(L0.pa()), lcview<double>(L0, pp0), bc0, sc, fx_flag(c));
     count_launch(c, 2);
+    L0.fxHeld = true;
+    L0.fxUnit = sc;
     bool bad = false;
     unsigned long long mx = 0;
     auto residual = [&]() -> int {
@@ -4140,6 +4173,7 @@ static int plain_fixed(Ctx &c, const double *pp0, double mean, double bmax, doub
         s = vcycle_tgt<double>(c, false);
         c.fxPlain = 0;
         if (s) return s;
+        for (int q = 1; q < levels; ++q) { c.lv[q].fxHeld = true; c.lv[q].fxUnit = sl; }
         cyc += 1;
         const unsigned long long before = mx;
         if ((s = residual())) return s;
@@ -4198,6 +4232,7 @@ static int mg_solve_target_run(Ctx &c, int *cycles, double *residual, saras_step
     // from level-0 r
     const bool fixedPlain = c.mgMode == SARAS_MG_PLAIN_TARGET && L0.lx == L0.ly && L0.ly == L0.lz && c.depth > 0 && c.tailLt != 0 && !wantGuess &&
                             !c.collecting && !c.unet && !c.ppInHist;
+    if (!fixedPlain && (s = mg_release_levels(c))) return s;
     k_tgt_stats<<<gk0, bk0, 0, c.stream>>>(lcview<double>(L0, rhs), fixedPath || fixedPlain ? pp0 : nullptr, bc0, c.red, c.dscal + 31, c.dscal + 32,
                                            c.dscal + 33);
     k_final_reduce<<<1, 256, 0, c.stream>>>(c.red, nparts, 0, c.dscal + 30);
@@ -4221,6 +4256,10 @@ static int mg_solve_target_run(Ctx &c, int *cycles, double *residual, saras_step
     bool fixedDone = false;
     if (fixedPlain) {
         if ((s = plain_fixed(c, pp0, mean, bmax, pmax, c.mgTarget * bmax, r, cyc, fixedDone, st))) return s;
+        if (!fixedDone) {
+            L0.fxHeld = false;   // its arrays are written below
+            if ((s = mg_release_levels(c))) return s;
+        }
     }
     if (!fixedPath && !fixedDone) {
         dim3 g, b; core_dims(L0, g, b);
@@ -4351,6 +4390,7 @@ int mg_solve(Ctx &c, int *cycles, double *residual, saras_step_stats *st) {
 // ---- test hooks mirroring the protected multigrid_d3 methods
 int mg_set_level(Ctx &c, int level, int which, const double *host) {
     if (level < 0 || level > c.depth || (which != 0 && which != 1)) return SARAS_BAD_ARG;
+    if (int e = mg_release_levels(c)) return e;
     Level &L = c.lv[level];
     double *dst = which == 0 ? L.pa() : L.r;
     SARAS_CUDA_TRY(cudaMemcpyAsync(dst, host, sizeof(double) * L.count, cudaMemcpyHostToDevice, c.stream));
@@ -4367,6 +4407,7 @@ int mg_set_level(Ctx &c, int level, int which, const double *host) {
 
 int mg_get_level(Ctx &c, int level, int which, double *host) {
     if (level < 0 || level > c.depth || (which != 0 && which != 1)) return SARAS_BAD_ARG;
+    if (int e = mg_release_levels(c)) return e;
     Level &L = c.lv[level];
     const double *src = which == 0 ? L.pa() : L.r;
     SARAS_CUDA_TRY(cudaMemcpyAsync(host, src, sizeof(double) * L.count, cudaMemcpyDeviceToHost, c.stream));
@@ -4376,23 +4417,27 @@ int mg_get_level(Ctx &c, int level, int which, double *host) {
 
 int mg_smooth_level(Ctx &c, int level, int count) {
     if (level < 0 || level > c.depth) return SARAS_BAD_ARG;
+    if (int e = mg_release_levels(c)) return e;
     if (level == c.depth && count < 0) return coarse_solve<double>(c, false);
     return smooth<double>(c, level, count, false, false);
 }
 
 int mg_restrict_level(Ctx &c, int level) {
     if (level < 0 || level >= c.depth) return SARAS_BAD_ARG;
+    if (int e = mg_release_levels(c)) return e;
     return restrict_level<double>(c, level, false);
 }
 
 int mg_prolong_level(Ctx &c, int level) {
     if (level < 0 || level >= c.depth) return SARAS_BAD_ARG;
+    if (int e = mg_release_levels(c)) return e;
     return prolong_level<double>(c, level, false, true);
 }
 
 // multigrid_d3::testProlong (poisson_d3.cc:689-719)
 int mg_test_prolong(Ctx &c, double *err) {
     if (c.depth < 1) return SARAS_BAD_ARG;
+    if (int e = mg_release_levels(c)) return e;
     Level &L0 = c.lv[0], &L1 = c.lv[1];
     std::vector<double> h1(L1.count, 0.0), h0(L0.count, 0.0);
     View3<double> v1 = lview<double>(L1, nullptr), v0 = lview<double>(L0, nullptr);
@@ -4420,6 +4465,7 @@ int mg_test_prolong(Ctx &c, double *err) {
 // multigrid_d3::testTransfer (poisson_d3.cc:722-777) at level 0: face pads
 // after updatePads, for periodic x and y.
 int mg_test_transfer(Ctx &c, double *err) {
+    if (int e = mg_release_levels(c)) return e;
     Level &L0 = c.lv[0];
     View3<double> v0 = lview<double>(L0, nullptr);
     std::vector<double> h(L0.count, 0.0), e(L0.count, 0.0);
@@ -4455,6 +4501,7 @@ int mg_test_transfer(Ctx &c, double *err) {
 // multigrid_d3::testPeriodic (poisson_d3.cc:780-857) at level 0: face ghosts
 // of sin*cos*cos after imposeBC.
 int mg_test_periodic(Ctx &c, double *err) {
+    if (int e = mg_release_levels(c)) return e;
     Level &L0 = c.lv[0];
     View3<double> v0 = lview<double>(L0, nullptr);
     int X = L0.n[0], Y = L0.n[1], Z = L0.n[2];

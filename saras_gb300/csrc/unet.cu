@@ -1190,6 +1190,7 @@ int unet_grad_check(Ctx &c, const float *feat, const float *target, const float 
 // The learned guess for the current right-hand side into `out` (history and
 // the level-lb rings as the next solve would see them; no rotation).
 int unet_infer(Ctx &c, double *out) {
+    if (int e = mg_release_levels(c)) return e;
     return unet_guess(c, c.lv[0].r, out, SARAS_GUESS_LEARNED);
 }
 

@@ -30,17 +30,17 @@ def lap(P):
 
 
 def solve(g, P, b):
-    """(status, V-cycles, Pp) of the solve of l lap(Pp) = b from P, l = N^2."""
+    """(status, V-cycles, Pp, reported residual) of the solve of l lap(Pp) = b from P, l = N^2."""
     n = b.shape[0]
     i = np.arange(-1, n + 2) % n
     g.set(F.FIELD_PP, P[np.ix_(i, i, i)])
     g.set(F.FIELD_MGRHS, b[np.ix_(i, i, i)])
-    status, cycles = 0, None
+    status, cycles, res = 0, None, None
     try:
-        cycles, _ = g.mg_solve()
+        cycles, res = g.mg_solve()
     except S.SarasError as e:
         status = e.status
-    return status, cycles, g.get(F.FIELD_PP)[1:n + 1, 1:n + 1, 1:n + 1]
+    return status, cycles, g.get(F.FIELD_PP)[1:n + 1, 1:n + 1, 1:n + 1], res
 
 
 @pytest.mark.parametrize("k,amplitude", [((2, 2, 2), 57.25), ((1, 2, 2), 57.0)])
@@ -92,3 +92,36 @@ def test_right_hand_side_below_the_unit():
     out = [solve(solver(a, cycles=20), np.full(b.shape, 2.0 ** 70), b) for a in (0, 1)]
     assert out[0][0] == out[1][0] == F.NOT_CONVERGED
     assert np.array_equal(out[0][2], out[1][2])
+
+
+@pytest.mark.parametrize("depth", [1, 4])
+def test_level_arrays_after_a_solve(depth):
+    """The level calls read the FP64 values of what the fixed-point cycles left: level 0's right-hand
+    side and solution exactly as given and returned, the residual they leave, and the levels below up
+    to the FP64 residual's rounding (12 terms of the iterate's size).  A solve of the same problem
+    after them has the same bits."""
+    n = 32
+    b, P = smooth(n, 2), 3.0 / n ** 2 * smooth(n, 3)
+    g, h = solver(0, depth=depth), solver(1, depth=depth)
+    (s, cycles, p, res), (t, _, q, _) = solve(g, P, b), solve(h, P, b)
+    assert s == t == 0 and not np.array_equal(p, q)
+    core = slice(1, n + 1)
+    c = b - b.mean()
+    unit = 2.0 ** -57 * np.max(np.abs(P)) * n * n                  # B's, at most
+    assert np.max(np.abs(g.get_level(0, 1)[core, core, core] - c)) <= unit + 2.0 ** -52 * np.max(np.abs(c))
+    assert np.array_equal(g.get_level(0, 0)[core, core, core], p)
+    # (the reported residual is over both copies of a periodic plane, which a Gauss-Seidel coarse solve leaves unequal)
+    assert abs(g.mg_compute_error(1) - res) <= 14 * 2.0 ** -53 * n * n * np.max(np.abs(p)) / np.max(np.abs(c))
+    for level in range(1, depth + 1):
+        for which in (0, 1):
+            a, e = g.get_level(level, which), h.get_level(level, which)
+            a, e = (v[1:-1, 1:-1, 1:-1] for v in (a, e))
+            if which == 1:
+                assert np.max(np.abs(a - e)) <= 14 * 2.0 ** -53 * n * n * np.max(np.abs(P) + np.abs(p)), level
+            else:
+                assert np.all(np.isfinite(a)) and np.max(np.abs(a)) <= 2 * np.max(np.abs(e)), level
+    again = solve(g, P, b)
+    assert again[:2] == (s, cycles) and np.array_equal(again[2], p)
+    g.mg_set_mode(F.MG_REFERENCE)                                  # and another solver on the same arrays
+    h.mg_set_mode(F.MG_REFERENCE)
+    assert np.array_equal(solve(g, P, b)[2], solve(h, P, b)[2])
