@@ -3100,6 +3100,10 @@ static double smooth_weight(const Ctx &c, int n, int count) {
 }
 
 // ---- the pipelined Gauss-Seidel kernel's launches
+// Dynamic shared memory of any of its launches, and the limit set on the kernel: the limit is the
+// kernel's on the device, for all contexts and threads, so it never follows a launch's own size.
+constexpr int kGsPipeSmem = 220 * 1024;
+
 static bool is_pow2(double x) {
     int e;
     return std::isfinite(x) && std::frexp(x, &e) == 0.5;
@@ -3141,7 +3145,7 @@ static bool gs_plan(const Ctx &c, const Level &L, const MgBC &bc, int form, int 
     if (bc.dirichlet || form < 0) return false;
     const int X = L.n[0], Y = c.planar ? 0 : L.n[1], Z = L.n[2];
     const long nc = (long)(X + 1) * (Y + 1);
-    const size_t cap = 220 * 1024;
+    const size_t cap = kGsPipeSmem;
     if (nc > 992) return false;
     int lmin = 2;
     for (int d = 0; d < 3; ++d)
@@ -3179,7 +3183,7 @@ static cudaError_t gs_pipe_launch(Ctx &c, Level &L, const MgBC &bc, const GsArit
     void (*k)(View3<double>, View3<const double>, MgK, MgBC, GsArith<ARITH>, int, int, int, int, int, double, int, long long *);
     if (COARSE || g.rsmem) k = c.planar ? k_gs_pipe<ARITH, true, true, COARSE> : k_gs_pipe<ARITH, false, true, COARSE>;
     else k = c.planar ? k_gs_pipe<ARITH, true, false, false> : k_gs_pipe<ARITH, false, false, false>;
-    cudaError_t e = cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g.smem);
+    cudaError_t e = cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, kGsPipeSmem);
     if (e != cudaSuccess) return e;
     return launch_pdl(k, dim3(1), dim3(g.threads + (COARSE ? 32 : 0)), g.smem, c.stream, lview<double>(L, L.pa()), lcview<double>(L, L.r), make_k(L), bc,
                       ar, g.lam, g.Q, g.zp, count, zero ? 1 : 0, c.p.mgTolerance, c.maxCount, (long long *)(c.dscal + 40));
