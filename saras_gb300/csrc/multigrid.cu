@@ -683,6 +683,7 @@ __global__ void k_mg_coarse(View3<T> pg, View3<const T> rg, MgK kk, MgBC bc, T t
 // kGsBlockSmem bytes together): one CTA, the stages separated by
 // __syncthreads.  zero: pressureData = 0 on entry.
 constexpr size_t kGsBlockSmem = 200 * 1024;
+constexpr size_t kCoarseSmem = 220 * 1024;   // the coarsest level's two arrays
 __global__ void k_mg_gs_block(View3<double> pg, View3<const double> rg, MgK kk, MgBC bc, int count, int zero,
                               const double *wx, const double *wy, const double *wz) {
     pdl_wait();
@@ -1593,6 +1594,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 6 : 5) k_tgt_residual(OT
 // operand, so the results are the same bits.
 constexpr int kPlaneRows = 8;
 constexpr int kPlaneRing = 4;
+constexpr size_t kPlaneSmem = 200 * 1024;   // dynamic shared memory at most
 constexpr int kPlaneVec = 64;        // floats a tensor-map row (256 bytes)
 constexpr int kPlaneThreads = 512;
 
@@ -2852,7 +2854,7 @@ static int plane_setup(Ctx &c) {
     const int sideOff = (int)mainRows * kPlaneVec, rOff = sideOff + (int)sideRows * kPlaneVec;
     const int slot = rOff + (int)rRows * kPlaneVec;
     const size_t smem = (size_t)kPlaneRing * slot * sizeof(float) + 128;   // + alignment of the first slot
-    if (smem > 200 * 1024) return SARAS_OK;
+    if (smem > kPlaneSmem) return SARAS_OK;
     cuuint64_t dims[2] = {(cuuint64_t)kPlaneVec, (cuuint64_t)(L.count / kPlaneVec)};
     cuuint64_t strides[1] = {(cuuint64_t)kPlaneVec * sizeof(float)};
     cuuint32_t box[2] = {(cuuint32_t)kPlaneVec, (cuuint32_t)mainRows}, sbox[2] = {(cuuint32_t)kPlaneVec, (cuuint32_t)sideRows},
@@ -2870,7 +2872,7 @@ static int plane_setup(Ctx &c) {
     c.planeMaxQ = maxq <= 5 ? 5 : 11;
     const void *fns[2] = {c.planeMaxQ == 5 ? (const void *)k_tgt_plane_tma<0, 5> : (const void *)k_tgt_plane_tma<0, 11>,
                           c.planeMaxQ == 5 ? (const void *)k_tgt_plane_tma<1, 5> : (const void *)k_tgt_plane_tma<1, 11>};
-    for (const void *f : fns) SARAS_CUDA_TRY(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    for (const void *f : fns) SARAS_CUDA_TRY(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPlaneSmem));   // (all contexts')
     // one wave: as many CTAs as fit (shared memory bounds them), tiles x segments of planes
     int perSM = 0;
     SARAS_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, fns[0], kPlaneThreads, smem));
@@ -2984,9 +2986,10 @@ int mg_setup(Ctx &c) {
     const Level &C = c.lv[c.depth];
     c.maxCount = (C.n[0] + 2) * (C.n[1] + 2) * (C.n[2] + 2);                            // poisson.cc:360-361
     size_t smem = 2 * sizeof(double) * C.count;
-    if (smem > 220 * 1024) { c.err = "coarsest multigrid level too large for one CTA; increase V-Cycle Depth"; return SARAS_BAD_CONFIG; }
-    SARAS_CUDA_TRY(cudaFuncSetAttribute(k_mg_coarse<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    SARAS_CUDA_TRY(cudaFuncSetAttribute(k_mg_coarse<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > kCoarseSmem) { c.err = "coarsest multigrid level too large for one CTA; increase V-Cycle Depth"; return SARAS_BAD_CONFIG; }
+    // the limit is the kernel's on the device, for every context: the most any of them takes
+    SARAS_CUDA_TRY(cudaFuncSetAttribute(k_mg_coarse<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCoarseSmem));
+    SARAS_CUDA_TRY(cudaFuncSetAttribute(k_mg_coarse<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCoarseSmem));
     SARAS_CUDA_TRY(cudaDeviceGetAttribute(&c.numSMs, cudaDevAttrMultiProcessorCount, c.dev));
     SARAS_CUDA_TRY(cudaFuncSetAttribute(k_mg_gs_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGsBlockSmem));
     SARAS_CUDA_TRY(cudaMemsetAsync(c.dflag, 0, 3 * sizeof(int), c.stream));

@@ -1,12 +1,13 @@
-"""GPU check of two solvers in two host threads whose launches of one kernel ask for
-different amounts of dynamic shared memory: the kernel's limit on the device is shared
-by all of them."""
+"""GPU check of solvers, in one host thread or in two, whose launches of one kernel ask
+for different amounts of dynamic shared memory: the kernel's limit on the device is
+shared by all of them."""
 import threading
 
 import numpy as np
 import pytest
 
 import saras_gb300 as S
+from saras_gb300 import _abi as F
 from tests import _cases as C
 
 pytestmark = pytest.mark.gpu
@@ -42,3 +43,15 @@ def test_gauss_seidel_levels_of_two_solvers():
         g.close()
 
     together(lambda: sweeps(4, 1), lambda: sweeps(5, 1))          # 9^3 and 17^3
+
+
+def test_coarsest_level_of_an_earlier_solver():
+    """A coarsest level of 17^3 points (110 KB), then a solver with one of 5^3, then the first one's step."""
+    p = C.tgv(ind=5, depth=1)
+    p.mgMode, p.mgTarget, p.mgMaxCycles = F.MG_PLAIN_TARGET, 1e-8, 50
+    first = S.Solver(p)
+    C.initialise(first, p, "tgv")
+    other = S.Solver(C.tgv(ind=4, depth=2))
+    assert first.time_advance()[0] == 0
+    other.close()
+    first.close()
