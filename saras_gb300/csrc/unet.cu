@@ -498,9 +498,12 @@ static int ucheck(Ctx &c, const char *what) {
     return SARAS_OK;
 }
 
+// Dynamic shared memory of a launch at most, and the limit set on the kernel: the limit is the
+// kernel's on the device, for all contexts and threads, so it never follows a layer's own size.
+constexpr int kConvSmem = 200 * 1024;
 template <int N, int STAGES>
 static cudaError_t launch_conv_s(const ConvArgs &a, int smem, cudaStream_t s) {
-    cudaError_t e = cudaFuncSetAttribute(k_conv3d_tc<N, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(k_conv3d_tc<N, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, kConvSmem);
     if (e != cudaSuccess) return e;
     const long rows = (long)a.D * a.H * (a.W + 1);
     k_conv3d_tc<N, STAGES><<<(int)((rows + 127) / 128), 128, smem, s>>>(a);
@@ -509,7 +512,7 @@ static cudaError_t launch_conv_s(const ConvArgs &a, int smem, cudaStream_t s) {
 template <int N>
 static cudaError_t launch_conv_n(const ConvArgs &a, cudaStream_t s) {
     const int stage = conv_stage_bytes(N, (a.c0 + a.c1) / 16);
-    return 4 * stage <= 200 * 1024 ? launch_conv_s<N, 4>(a, 4 * stage, s) : launch_conv_s<N, 2>(a, 2 * stage, s);
+    return 4 * stage <= kConvSmem ? launch_conv_s<N, 4>(a, 4 * stage, s) : launch_conv_s<N, 2>(a, 2 * stage, s);
 }
 
 static int launch_conv(Ctx &c, int N, const ConvArgs &a) {

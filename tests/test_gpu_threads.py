@@ -55,3 +55,15 @@ def test_coarsest_level_of_an_earlier_solver():
     assert first.time_advance()[0] == 0
     other.close()
     first.close()
+
+
+def test_convolutions_of_two_threads():
+    def passes(cin, value):
+        x = np.full((3, 3, 3, cin), value, dtype=np.float32)
+        w = np.full((16, 27, cin), 0.125, dtype=np.float32)
+        bits = S.to_bf16_bits(x)
+        for _ in range(1500):
+            y = S.conv3d_check(0, bits, None, w, None, 0, (3, 3, 3), cin, 16)
+        assert np.all(y.reshape(3, 3, 3, 16)[1, 1, 1] == 0.125 * value * 27 * cin)   # exact: small integers over 8
+
+    together(lambda: passes(16, 1.0), lambda: passes(96, 2.0))     # 24 and 140 KB
