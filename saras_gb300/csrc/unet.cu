@@ -535,10 +535,7 @@ enum { A_X0 = 0, A_0, A_E1, A_P1, A_2, A_E2, A_P2, A_4, A_E3, A_U2, A_6, A_F2, A
 
 static UNet *U(Ctx &c) { return reinterpret_cast<UNet *>(c.unet); }
 
-static int unet_alloc(Ctx &c) {
-    if (c.unet) return SARAS_OK;
-    UNet *u = new UNet();
-    c.unet = u;
+static int unet_build(Ctx &c, UNet *u) {
     if (c.depth < 3) { c.err = "the U-Net needs a multigrid depth of at least 3"; return SARAS_BAD_CONFIG; }
     // finest network level: the first with at most 64 intervals per axis (at
     // least level 1), keeping two coarser levels for the U-Net's depth
@@ -637,6 +634,17 @@ void unet_free(Ctx &c) {
     cudaFree(u->rpnew); cudaFree(u->tmp[0]); cudaFree(u->tmp[1]);
     delete u;
     c.unet = nullptr;
+}
+
+// The context's network, made at its first use; none is left behind where that fails (a
+// half-made one has null buffers).
+static int unet_alloc(Ctx &c) {
+    if (c.unet) return SARAS_OK;
+    UNet *u = new UNet();
+    c.unet = u;
+    const int s = unet_build(c, u);
+    if (s) unet_free(c);
+    return s;
 }
 
 int unet_create(Ctx &c) { return unet_alloc(c); }

@@ -125,3 +125,15 @@ def test_level_arrays_after_a_solve(depth):
     g.mg_set_mode(F.MG_REFERENCE)                                  # and another solver on the same arrays
     h.mg_set_mode(F.MG_REFERENCE)
     assert np.array_equal(solve(g, P, b)[2], solve(h, P, b)[2])
+
+
+def test_network_that_does_not_fit():
+    """A grid too shallow for the network: every call that needs it says so, and solves are as before."""
+    b, P = smooth(32, 2), 3.0 / 32 ** 2 * smooth(32, 3)
+    g, h = solver(0, depth=2), solver(0, depth=2)
+    for call in (g.unet_shape, g.unet_shape, g.unet_collect, g.unet_collect, lambda: g.unet_train(1, 1e-3)):
+        with pytest.raises(S.SarasError) as e:
+            call()
+        assert e.value.status == F.BAD_CONFIG
+    p, q = solve(g, P, b), solve(h, P, b)
+    assert p[:2] == q[:2] and np.array_equal(p[2], q[2])
