@@ -2,6 +2,8 @@
 solves of given right-hand sides and starts against the FP64 levels.  A context that
 asks for an extrapolated guess runs the FP64 levels; its first solve has no history, so
 it starts from the given Pp too."""
+import math
+
 import numpy as np
 import pytest
 
@@ -137,3 +139,84 @@ def test_network_that_does_not_fit():
         assert e.value.status == F.BAD_CONFIG
     p, q = solve(g, P, b), solve(h, P, b)
     assert p[:2] == q[:2] and np.array_equal(p[2], q[2])
+
+
+def waves(p, seed):
+    """A few of the first waves of the box on its padded points (whole waves on periodic axes, half waves between walls)."""
+    rng = np.random.default_rng(seed)
+    out = 0.0
+    for _ in range(6):
+        f = rng.standard_normal()
+        for e, per, d in ((p.xInd, p.xPer, 0), (p.yInd, p.yPer, 1), (p.zInd, p.zPer, 2)):
+            k = rng.integers(1, 4) * (2 if per else 1)
+            f = f * np.cos(math.pi * k * np.arange(-1, 2 ** e + 2) / 2 ** e).reshape([-1 if q == d else 1 for q in range(3)])
+        out = out + f
+    return out
+
+
+def problem(p):
+    """A start and a right-hand side whose solution differs from it by a few hundredths (its residual, in
+    units of 2^-57 of its maximum and less, stays where a level below can hold eight times as much)."""
+    P, d = waves(p, 3), 0.03 * waves(p, 2)
+    c = slice(1, -1)
+    b = np.zeros(P.shape)
+    b[c, c, c] = (2 ** p.xInd / p.Lx) ** 2 * sum(Q[2:, c, c] + Q[:-2, c, c] + Q[c, 2:, c] + Q[c, :-2, c] + Q[c, c, 2:] + Q[c, c, :-2] - 6 * Q[c, c, c]
+                                               for Q in (P, d))
+    return P, b
+
+
+def one_cycle(make, fp64, pre, post, smoother):
+    """(Pp before, Pp after) one V-cycle."""
+    p = make()
+    p.mgMode, p.mgTarget, p.mgMaxCycles = F.MG_PLAIN_TARGET, 1e-30, 1
+    p.smoother, p.coarseCycles = smoother, 2
+    p.preSmooth, p.postSmooth = pre, post
+    g = S.Solver(p)
+    if fp64:
+        g.set_guess_mode(F.GUESS_EXTRAPOLATE)
+    start, b = problem(p)
+    g.set(F.FIELD_PP, start)
+    g.set(F.FIELD_MGRHS, b)
+    with pytest.raises(S.SarasError) as e:
+        g.mg_solve()
+    assert e.value.status == F.NOT_CONVERGED
+    out = g.get(F.FIELD_PP)
+    g.close()
+    return start, out
+
+
+@pytest.mark.parametrize("make,pre,post,smoother", [
+    (lambda: C.tgv(ind=4, depth=1), 2, 1, 0),      # one 17^3 level above the coarsest, an odd sweep count
+    (lambda: C.tgv(ind=5, depth=2), 2, 2, 1),      # two of them
+    (lambda: C.ldc(ind=5, depth=3), 2, 2, 1),      # walls
+    (lambda: C.rbc(ind=(5, 5, 4), depth=2), 1, 2, 1),
+    (lambda: C.rbc(ind=(5, 5, 4), depth=2), 3, 0, 0),   # no sweep after the correction
+    (lambda: C.tgv(ind=7, depth=5), 3, 3, 1),      # marches of eight planes
+])
+def test_cycle_runs_on_integers(make, pre, post, smoother):
+    """The two arms run different levels (their last bits differ), and leave the same Pp up to the FP64
+    arm's rounding: 12 terms of the iterate's size in the residual, which the coarse levels' inverse
+    Laplacian amplifies by (N / pi)^2 at most, and a few more terms a sweep, not amplified; twice
+    their sum, of the largest value on the way."""
+    sa, a = one_cycle(make, False, pre, post, smoother)
+    sb, b = one_cycle(make, True, pre, post, smoother)
+    assert np.array_equal(sa, sb) and not np.array_equal(a, b)
+    n = 2 ** make().xInd
+    tol = 2.0 * (12.0 * (n / math.pi) ** 2 + 8.0 * (pre + post + 1)) * 2.0 ** -53
+    assert np.max(np.abs(a - b)) <= tol * max(np.max(np.abs(sa)), np.max(np.abs(a)))
+
+
+@pytest.mark.parametrize("bad", [math.nan, math.inf, -math.inf, None])
+def test_values_out_of_range(bad):
+    """Not a number or an infinity in the right-hand side, or (None) a solution a hundred times the
+    start: the FP64 levels' result, bit for bit."""
+    n = 32
+    x = 2 * np.pi * np.arange(n) / n
+    P = np.cos(x)[:, None, None] * np.ones((n, n, n))
+    b = 100 * n * n * lap(P)
+    assert np.max(np.abs(b)) / n ** 2 <= 4 * np.max(np.abs(P))     # a scale is taken
+    if bad is not None:
+        b[3, 4, 5] = bad
+    out = [solve(solver(a, cycles=30), P, b) for a in (0, 1)]
+    assert out[0][:2] == out[1][:2]
+    assert np.array_equal(out[0][2], out[1][2], equal_nan=True)
