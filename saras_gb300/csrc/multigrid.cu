@@ -3915,6 +3915,27 @@ static void note_contraction(Ctx &c, double r0, double r, int n) {
 // by a cycle at most.
 constexpr double kGuessTrusted = 1e-4;
 
+// Fixed-point solves keep the unit of the largest value they started from, where FP64's
+// rounding follows the iterate: one whose iterate has shrunk far below its start (a start
+// far off, a changed time step) stalls at a few units. Asked for where the residual is
+// below kFxStall units, far above what rounding leaves (a few hundred), and the cycles
+// do not halve it any more or have run out; below 2^53 units an FP64 iterate's last bit is
+// finer than the unit, and the FP64 levels take the solve over.
+constexpr unsigned long long kFxStall = 1ull << 16;
+static int fx_outgrown(Ctx &c, const long long *p, bool &yes) {
+    const Level &L0 = c.lv[0];
+    dim3 g, b; col_dims(L0, g, b);
+    SARAS_CUDA_TRY(cudaMemsetAsync(c.dscal + 34, 0, sizeof(double), c.stream));
+    k_fx_maxabs<<<g, b, 0, c.stream>>>(p, (L0.n[1] + 3) * (L0.n[2] + 3), L0.n[2] + 3, level_bc(c, 0, true), reinterpret_cast<unsigned long long *>(c.dscal + 34));
+    count_launch(c);
+    if (int s = chk(c, "fixed-point maximum")) return s;
+    if (int s = read_scalars(c, 34, 1)) return s;
+    unsigned long long m;
+    std::memcpy(&m, &c.hscal[34], sizeof m);
+    yes = m < (1ull << 53);
+    return SARAS_OK;
+}
+
 static int mixed_fixed(Ctx &c, const double *pp0, double mean, double bmax, double pmax, double target, bool wantGuess, double &r, int &source,
                        int &cyc, int &steps, bool &done, saras_step_stats *st) {
     int s;
@@ -3960,6 +3981,7 @@ static int mixed_fixed(Ctx &c, const double *pp0, double mean, double bmax, doub
     // refinement update writes its FP64 iterate into Pp's core as it goes.
     double *outp = c.ppInHist ? c.f[SARAS_FIELD_PP] : nullptr;
     // residual of fixed iterate q (with e: advanced into q ^ 1 first); returns the max in value units
+    unsigned long long mx = 0;   // the last one's maximum in units
     auto refine = [&](int q, bool withE, double &out, bool &bad, bool fill32 = true) -> int {
         SARAS_CUDA_TRY(cudaMemsetAsync(c.dscal + 34, 0, sizeof(double), c.stream));
         if (withE) {
@@ -3979,7 +4001,6 @@ static int mixed_fixed(Ctx &c, const double *pp0, double mean, double bmax, doub
         count_launch(c);
         int e = chk(c, "fixed-point refinement");
         if (e) return e;
-        unsigned long long mx = 0;
         int fl = 0, tmaErr = 0;
         SARAS_CUDA_TRY(cudaMemcpyAsync(&mx, dmax, sizeof(mx), cudaMemcpyDeviceToHost, c.stream));
         SARAS_CUDA_TRY(cudaMemcpyAsync(&fl, dflag, sizeof(fl), cudaMemcpyDeviceToHost, c.stream));
@@ -4060,6 +4081,7 @@ static int mixed_fixed(Ctx &c, const double *pp0, double mean, double bmax, doub
         if (!std::isfinite(r)) { c.err = "multigrid residual is not finite"; return SARAS_NOT_FINITE; }
         int n = refine_cycles(c, r, target, cyc, steps == 0);
         double r0 = r;
+        const unsigned long long before = mx;
         for (int q = 0; q < n; ++q) {
             if ((s = vcycle_tgt<float>(c, q == 0))) return s;
             cyc += 1;
@@ -4069,8 +4091,13 @@ static int mixed_fixed(Ctx &c, const double *pp0, double mean, double bmax, doub
         if (bad) break;
         cur ^= 1;
         updated = true;
+        if (r > target && mx < kFxStall && (mx > before / 2 || cyc >= c.mgMaxCycles)) {
+            if ((s = fx_outgrown(c, c.fx[cur], bad))) return s;
+            if (bad) break;
+        }
         note_contraction(c, r0, r, n);
     }
+    if (bmax > 0 && r <= target && r + rs > target) bad = true;   // it meets the target by less than B's own rounding
     if (!bad) {
         // the FP64 result P 2^-s (exact), whose exact residual is r
         if (updated && outp) {   // the core is written: the ghost positions
@@ -4086,7 +4113,7 @@ static int mixed_fixed(Ctx &c, const double *pp0, double mean, double bmax, doub
         done = true;
         return chk(c, "fixed-point output");
     }
-    // out of range: restart from the previous Pp in FP64
+    // out of range, or below the unit: restart from the previous Pp in FP64
     L0.cur = 0;
     r = 0; source = 0; cyc = 0; steps = 0;
     return fp64_start();
@@ -4116,13 +4143,8 @@ int mg_release_levels(Ctx &c) {
 // exact residual meets the target.  done: the result is in Pp; otherwise nothing the FP64
 // path reads has changed.  That path takes the solve when
 //   the previous Pp gives no scale, or values leave the range;
-//   the iterate has shrunk far below the previous Pp (a start far off, a changed time
-//   step) and its residual stalls: the unit stays that of the largest value, where FP64's
-//   rounding follows the iterate.  Asked for where a cycle below kFxStall units, far above
-//   what rounding leaves (a few hundred), does not halve the residual, or is the last one;
-//   below 2^53 units an FP64 iterate's last bit is finer than the unit;
+//   the iterate has shrunk below the unit's use (fx_outgrown);
 //   the residual meets the target by less than B's own rounding.
-constexpr unsigned long long kFxStall = 1ull << 16;
 static int plain_fixed(Ctx &c, const double *pp0, double mean, double bmax, double pmax, double target, double &r, int &cyc, bool &done,
                        saras_step_stats *st) {
     done = false;
@@ -4185,17 +4207,10 @@ static int plain_fixed(Ctx &c, const double *pp0, double mean, double bmax, doub
         const unsigned long long before = mx;
         if ((s = residual())) return s;
         if (!bad && r > target && mx < kFxStall && (mx > before / 2 || cyc == c.mgMaxCycles)) {
-            unsigned long long pm;
-            SARAS_CUDA_TRY(cudaMemsetAsync(c.dscal + 34, 0, sizeof(double), c.stream));
-            k_fx_maxabs<<<gk, bk, 0, c.stream>>>(fx_of(L0.pa()), sx, sy, bc0, dmax);
-            count_launch(c);
-            if ((s = chk(c, "fixed-point maximum"))) return s;
-            if ((s = read_scalars(c, 34, 1))) return s;
-            std::memcpy(&pm, &c.hscal[34], sizeof pm);
-            bad = pm < (1ull << 53);
+            if ((s = fx_outgrown(c, fx_of(L0.pa()), bad))) return s;
         }
     }
-    if (!bad && r <= target && r + rs > target) bad = true;
+    if (!bad && bmax > 0 && r <= target && r + rs > target) bad = true;
     if (bad) {
         cyc = 0;
         L0.cur = 0;

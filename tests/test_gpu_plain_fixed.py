@@ -87,6 +87,31 @@ def test_start_far_above_the_solution(scale, target, fp64):
     assert np.max(np.abs(r)) <= target * np.max(np.abs(c)) * (1 + 1e-6)
 
 
+@pytest.mark.parametrize("scale,target", [(0, 1e-12), (10, 1e-12), (20, 1e-8), (20, 1e-12), (30, 1e-8), (40, 1e-8)])
+def test_start_far_above_the_solution_mixed(scale, target):
+    """The same for the mixed mode's fixed-point refinement, which FP64 refinement takes over."""
+    n = 32
+    b, P = smooth(n, 2), 2.0 ** scale * 3.0 / n ** 2 * smooth(n, 3)
+    g = solver(0)
+    g.mg_set_mode(F.MG_MIXED, target, 100)
+    status, _, p, _ = solve(g, P, b)
+    c = b.astype(np.longdouble) - b.astype(np.longdouble).mean()
+    r = c - n * n * lap(p.astype(np.longdouble))
+    # FP64's own rounding of the residual it stops on: 14 terms of the solution's size
+    slack = 14 * 2.0 ** -53 * n * n * np.max(np.abs(p))
+    assert status == 0 and np.max(np.abs(r)) <= target * np.max(np.abs(c)) * (1 + 1e-6) + slack
+
+
+@pytest.mark.parametrize("mode", [F.MG_PLAIN_TARGET, F.MG_MIXED])
+def test_no_right_hand_side(mode):
+    """0 on the right-hand side is exact in any unit: a constant Pp is its solution as it is."""
+    g = solver(0)
+    g.mg_set_mode(mode, 1e-8, 20)
+    P = np.full((32, 32, 32), 0.7)
+    status, cycles, p, res = solve(g, P, np.zeros(P.shape))
+    assert (status, cycles, res) == (0, 0, 0.0) and np.array_equal(p, P)
+
+
 def test_right_hand_side_below_the_unit():
     """Pp all one value, 2^70 times the right-hand side: in its unit the right-hand side is 0 and the
     residual too, which says nothing; FP64 levels cannot reduce it and say so."""
