@@ -9,7 +9,8 @@ max|b - Ap| / max|b| <= 1e-8, projection and boundary fills.
 
 Our arm runs the pressure solve as FP32 V-cycles inside FP64 iterative
 refinement (optionally warm-started by the U-Net); the same run also times the
-plain FP64 V-cycle solve to the same residual target and reports both.
+plain 64-bit V-cycle solve (its levels in 64-bit fixed point on this grid, the
+coarse tail in FP64) to the same residual target and reports both.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
 
@@ -50,8 +51,8 @@ def tgv_params(mode, guess=0, ind=GRID_INDEX, depth=DEPTH):
     p.cnTolerance = 1.0e-8
     p.mgTolerance = 1.0e-8
     # both target-mode arms with the cycle each is fastest with at 257^3
-    # (ms a step): plain FP64 -- Chebyshev (2,2) cycles with three cycles at
-    # the second level a visit, 15.5 (4 cycles; with two 16.6, four 17.1,
+    # (ms a step): plain -- Chebyshev (2,2) cycles with three cycles at the
+    # second level a visit (measured with FP64 levels: 15.5 with 4 cycles; with two 16.6, four 17.1,
     # Chebyshev (3,3) with three 19.0, damped-Jacobi (2,2) with three 21.7,
     # Chebyshev V(3,3) 23.9); mixed -- Chebyshev V(3,3) 4.61 (3 cycles in one
     # refinement step; V(2,2) 4.68 with 4, (2,2) with two cycles at the second
@@ -237,7 +238,7 @@ def time_steps(g, n):
 
 
 def plain_arm(args, fast, before):
-    """Plain FP64 multigrid (FP64 V-cycles to the same residual target) over the
+    """Plain multigrid (64-bit V-cycles to the same residual target) over the
     headline arm's step window: `before` untimed steps, then args.steps timed."""
     import saras_gb300 as S
     from saras_gb300 import _abi as F
@@ -293,7 +294,7 @@ def tma_arm(args, before):
 
 def accuracy_run(args):
     """Config 3's accuracy figures: the headline arm (its guess mode, mixed
-    refinement, fastKernels = 2) and the plain FP64 arm with the reference's
+    refinement, fastKernels = 2) and the plain 64-bit arm with the reference's
     arithmetic (fastKernels = 0) both run args.accuracy_steps steps from the
     initial condition; the energy series (tseries.cc:137-178) every step and
     the fields at the end are compared."""
@@ -304,7 +305,7 @@ def accuracy_run(args):
     series = {}
     fields = {}
     sec = {}
-    for arm in ("headline", "plain_fp64"):
+    for arm in ("headline", "plain_64bit"):
         t0 = time.perf_counter()
         if arm == "headline":
             p = tgv_params(F.MG_MIXED, F.GUESS_PREVIOUS)
@@ -328,12 +329,12 @@ def accuracy_run(args):
         fields[arm] = {nm: g.get(f) for f, nm in ((F.FIELD_VX, "Vx"), (F.FIELD_VY, "Vy"), (F.FIELD_VZ, "Vz"), (F.FIELD_P, "P"))}
         sec[arm] = round(time.perf_counter() - t0, 2)
         g.close()
-    a, b = fields["headline"], fields["plain_fp64"]
+    a, b = fields["headline"], fields["plain_64bit"]
     err = {nm: float(np.max(np.abs(a[nm] - b[nm])) / max(np.max(np.abs(b[nm])), 1e-300)) for nm in a}
     first = len(series["headline"]) - sum(x is not None for x in series["headline"])
-    eh, ep = np.array(series["headline"][first:], dtype=float), np.array(series["plain_fp64"][first:], dtype=float)
+    eh, ep = np.array(series["headline"][first:], dtype=float), np.array(series["plain_64bit"][first:], dtype=float)
     ke = float(np.max(np.abs(eh - ep) / np.abs(ep)))
-    return {"steps": n, "dt": DT, "reference": "plain FP64 V-cycles to 1e-8, fastKernels 0 (FP64 throughout)",
+    return {"steps": n, "dt": DT, "reference": "plain V-cycles to 1e-8 (levels in 64-bit fixed point, tail FP64), fastKernels 0 (the rest of the step FP64)",
             "max_pointwise_rel_err": err, "kinetic_energy_max_rel_err": ke,
             "kinetic_energy_compared_steps": [first + 1, n],
             "kinetic_energy_final": [float(eh[-1]), float(ep[-1])], "seconds": sec}
@@ -392,7 +393,7 @@ def run_ours(args, dist):
     g.profile_sample(1)
     ms_max = dist.max(ms)
     value = dist.world * args.steps / (ms_max / 1e3)
-    # --- plain FP64 multigrid over the same step window
+    # --- plain multigrid over the same step window
     plain = plain_strict = None
     if not args.no_plain and dist.rank == 0:
         plain = plain_arm(args, 2, done)
@@ -460,7 +461,8 @@ def run_ours(args, dist):
                         "pressure solve: FP32 V(3,3) cycles (Chebyshev-weighted Jacobi smoothing) inside iterative refinement with an "
                         "exact fixed-point residual, refinement steps sized by the measured contraction per cycle, to "
                         "max|b-Ap|/max|b| <= 1e-8; Crank-Nicolson and right-hand side in split-FP64 (fastKernels 2); "
-                        "plain arms: FP64 Chebyshev (2,2) cycles with three cycles at the second level a visit, same residual, "
+                        "plain arms: Chebyshev (2,2) cycles with three cycles at the second level a visit, levels in 64-bit fixed point "
+                        "(tail FP64), same residual, "
                         "over the same step window",
             "grid": [257, 257, 257], "vcycle_depth": DEPTH, "mg_mode": "mixed_fp32_in_fp64", "fastKernels": p.fastKernels,
             "warm_start": "unet (3-level 16/32/64, tcgen05 BF16 convs) correcting 2 Pp(n-1) - Pp(n-2), "
@@ -472,11 +474,11 @@ def run_ours(args, dist):
             "steps_before_timed": done,
             "residual_target": TARGET, "vcycles_per_step": sum(vc) / len(vc),
             "refine_steps_per_step": sum(rs) / len(rs), "max_fine_residual": max(fine),
-            "plain_fp64": plain,
-            "plain_fp64_strict": plain_strict,
-            "speedup_vs_plain_fp64": round(value / dist.world / plain["steps_per_s"], 3) if plain else None,
-            "speedup_vs_plain_fp64_strict": round(value / dist.world / plain_strict["steps_per_s"], 3) if plain_strict else None,
-            "accuracy_vs_plain_fp64": acc,
+            "plain_64bit": plain,
+            "plain_64bit_strict": plain_strict,
+            "speedup_vs_plain_64bit": round(value / dist.world / plain["steps_per_s"], 3) if plain else None,
+            "speedup_vs_plain_64bit_strict": round(value / dist.world / plain_strict["steps_per_s"], 3) if plain_strict else None,
+            "accuracy_vs_plain_64bit": acc,
             "plane_tma_variant": tma,
             "l2": "inputs larger than L2: every FP64 field is 259^3*8 B = 139 MB > 129 MB L2",
             "parallelism": "replicas" if dist.world > 1 else "single GPU",
@@ -651,13 +653,13 @@ def study_rbc_learned(args):
 
 def study_tgv513(args):
     """Taylor-Green 513^3, dt 2.5e-4, 200 steps: the learned + mixed solve
-    against the plain FP64 solve to the same 1e-8 residual, with the HBM rate of
+    against the plain 64-bit solve to the same 1e-8 residual, with the HBM rate of
     the kernels with the largest shares of the mixed arm."""
     import saras_gb300 as S
     from saras_gb300 import _abi as F
     steps = args.study_steps or 200
     out = {}
-    for arm in ("learned_mixed", "plain_fp64"):
+    for arm in ("learned_mixed", "plain_64bit"):
         mode = F.MG_MIXED if arm == "learned_mixed" else F.MG_PLAIN_TARGET
         p = tgv_params(mode, F.GUESS_PREVIOUS, ind=9, depth=7)
         p.tStp = 2.5e-4
@@ -699,9 +701,9 @@ def study_tgv513(args):
                     "max_fine_residual": max(x[2] for x in sts), "learned": info, "kernels": kern[:8],
                     "timing": "profiling events on (one V-cycle in %d timed)" % PROF_EVERY}
         g.close()
-    return {"study": "combined at scale", "metric": "steps/s at 513^3, learned+mixed vs plain FP64 at equal 1e-8 residual",
+    return {"study": "combined at scale", "metric": "steps/s at 513^3, learned+mixed vs plain 64-bit at equal 1e-8 residual",
             "workload": "Taylor-Green 513^3, [0,2pi]^3 PPP, Re 1600, dt 2.5e-4, %d steps" % steps,
-            "arms": out, "speedup": round(out["learned_mixed"]["steps_per_s"] / out["plain_fp64"]["steps_per_s"], 3),
+            "arms": out, "speedup": round(out["learned_mixed"]["steps_per_s"] / out["plain_64bit"]["steps_per_s"], 3),
             "data": "synthetic (Taylor-Green initial condition)"}
 
 

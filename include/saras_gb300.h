@@ -56,7 +56,13 @@ enum saras_field {
 /* Multigrid modes (GB300 extension; SARAS_MG_REFERENCE is the drop-in). */
 enum saras_mg_mode {
     SARAS_MG_REFERENCE = 0,  /* FP64 V-cycles, stop on |delta residual| < tol  poisson.cc:132-148 */
-    SARAS_MG_PLAIN_TARGET = 1, /* FP64 V-cycles until max|b-Ap|/max|b| <= target              */
+    SARAS_MG_PLAIN_TARGET = 1, /* 64-bit V-cycles until max|b-Ap|/max|b| <= target: with equal
+                                spacings the levels above the coarse tail hold P and b as
+                                64-bit fixed point in units set by the previous Pp (max|Pp| is
+                                2^57 to 2^58 of them; the residual exact, Pp returned in FP64),
+                                FP64 on other grids, at the first solve, with a guess other than
+                                the previous Pp or a network in the context, where values leave
+                                that range, and where the solution shrinks below its unit      */
     SARAS_MG_MIXED = 2       /* FP32 V-cycles inside FP64 iterative refinement to the target   */
 };
 
@@ -141,12 +147,12 @@ typedef struct saras_params {
 
 typedef struct saras_step_stats {
     int cn_iters[4];          /* Jacobi iterations for Vx, Vy, Vz, T */
-    int vcycles;              /* V-cycles in this step (FP64 or FP32) */
+    int vcycles;              /* V-cycles in this step (FP64, 64-bit fixed point or FP32) */
     int refine_steps;         /* FP64 refinement steps (mixed mode)  */
     int coarse_iters;         /* coarsest-level Gauss-Seidel iterations */
     double mg_residual;       /* last value of computeError (poisson_d3.cc:391-459) */
-    double fine_residual;     /* FP64 max|b-Ap|/max|b| after the solve (target modes) */
-    double guess_residual;    /* FP64 residual of the chosen initial guess */
+    double fine_residual;     /* max|b-Ap|/max|b| after the solve (target modes; FP64, exact in fixed point) */
+    double guess_residual;    /* the same of the chosen initial guess */
     int guess_source;         /* guess used: 0 previous Pp, else the saras_guess mode that won */
     int status;
 } saras_step_stats;

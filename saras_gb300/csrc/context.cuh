@@ -141,7 +141,7 @@ struct Ctx {
     void *probeBuf = nullptr;       // probe indices and values (grown on demand)
     size_t probeBytes = 0;
     double *hscal = nullptr;        // pinned host mirror
-    int *dflag = nullptr;
+    int *dflag = nullptr;           // error flag of the plane-streaming kernels
     double *gsFace = nullptr;       // planes kept by the wavefront of blocks (Gauss-Seidel on large levels)
     // stats
     long long launches = 0;

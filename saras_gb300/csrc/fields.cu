@@ -685,8 +685,8 @@ __global__ void k_bc_apply(View3<double> out, View3<const double> in, BcProgram 
     out(i, j, k) = bc_resolve(prog, i, j, k, [&](int a, int b, int c) -> double { return in(a, b, c); });
 }
 
-// Blocks a slab of the shell kernels (k_bc_apply_shell, k_cn_delta_shell,
-// k_project_shell): each thread resolves boundary programs with dependent
+// Blocks a slab of the shell kernels (k_bc_apply_shell, k_cn_delta_shell and its form
+// for three components, k_project_shell3): each thread resolves boundary programs with dependent
 // loads, so the slabs want many threads in flight (257^3: 256 blocks a slab
 // took 0.187 ms a Jacobi solve and 0.279 ms a projection, against 0.191 and
 // 0.289 with 64 and 0.192 and 0.289 with 1024).
@@ -1144,8 +1144,8 @@ __global__ void k_project(View3<double> out, View3<const double> in, View3<const
 // The fused-form projection with its boundary program split in two launches
 // (as the split Jacobi sweep): k_project_bulk marches the bulk box (the points
 // no boundary op targets: V - fastDt (Pp(+1) - Pp), no device calls, Pp along
-// the component's own axis carried in registers for Vx), k_project_shell
-// resolves the program on the remaining points of the full box.
+// the component's own axis carried in registers for Vx), k_project_shell3
+// resolves the program on the remaining points of the full box, all components in one.
 template <int C>
 __global__ void __launch_bounds__(256) k_project_bulk(View3<double> out, View3<const double> in, View3<const double> Pp, BcProgram prog,
                                                       double fastDt, int march) {

@@ -5,10 +5,10 @@
 //   SARAS_MG_REFERENCE     FP64, the reference V-cycle loop bit for bit
 //                          (padded-array mean removal, |delta residual| stop,
 //                          coarsest Gauss-Seidel to mgTolerance / maxCount).
-//   SARAS_MG_PLAIN_TARGET  FP64 V-cycles on the compatible system until
-//                          max|b-Ap| <= target * max|b|.
-//                          (levels above the tail in 64-bit fixed point when
-//                          the stencil is isotropic, k_fx_sweep).
+//   SARAS_MG_PLAIN_TARGET  64-bit V-cycles on the compatible system until
+//                          max|b-Ap| <= target * max|b|: the levels above the
+//                          tail in fixed point when the stencil is isotropic
+//                          (k_fx_sweep), else FP64.
 //   SARAS_MG_MIXED         FP32 V-cycles as the inner solver of an
 //                          iterative-refinement loop to the same target; the
 //                          outer residual is FP64, or exact 64-bit fixed point
@@ -1892,9 +1892,15 @@ __global__ void __launch_bounds__(256, 3) k_fx_refine(const long long *__restric
 // residual for the level below is -d, exact, where an FP64 residual loses the
 // digits that the stencil cancels; the correction comes back rounded to P's
 // last bit.  With 2^57 <= max|P| < 2^58 that bit is finer than FP64's for every value
-// above max|P| / 32; what the solve returns is rounded to FP64 by its last sweep.  The
-// exact residual left after 25 cycles, relative to max|b| (Taylor-Green 33^3 / 65^3 /
-// 129^3): 2.0e-15 / 8.7e-15 / 3.8e-14, with FP64 levels 4.2e-15 / 2.8e-14 / 9.9e-14.  An
+// above max|P| / 32; what the solve returns is rounded to FP64 by its last sweep.
+// Coarser than FP64 are: B where max|b| / l is below max|P| / 32 (2^-8 of it on the smooth
+// 257^3 flow: 50 bits), P below max|P| / 32, the levels below in the same absolute unit
+// (half of it), and a plane sum's two last bits in the restriction.  None of them is above
+// the rounding an FP64 cycle adds: its stencil sums lose six times max|P| 2^-53, that is
+// 100 to 400 of these units, at every point.  After 25 cycles (Taylor-Green 33^3 / 65^3 /
+// 129^3 / 257^3) the exact residual over max|b| is 3.2e-15 / 1.2e-14 / 5.1e-14 / 2.2e-13,
+// with FP64 levels 8.2e-15 / 4.0e-14 / 2.2e-13 / 8.8e-13; the error of P over max|P| 2.5e-16
+// / 2.9e-16 / 1.6e-16 / 2.2e-16, with FP64 levels 1.8e-15 / 6.2e-15 / 2.6e-14 / 1.0e-13.  An
 // FP64 sweep is bound by the FP64 pipe (one warp instruction in 64 clocks on an SM
 // quarter), the integer one by HBM: at 257^3 a sweep 265 -> 76 us, residual 265 -> 70, its maximum 298 -> 62, restriction
 // 134 -> 32, prolongation 182 -> 55; a step 14.6 -> 9.0 ms with level 0 alone, 6.2 with
@@ -2908,7 +2914,7 @@ static void plane_launch(Ctx &c, int mode, float *out, const float *in, const fl
     a.rOff = c.planeROff;
     a.slotFloats = c.planeSlotFloats;
     a.planesPerSeg = c.planeSegPlanes;
-    a.err = c.dflag + 2;
+    a.err = c.dflag;
     const int b = in == L.a32 ? 0 : 1;
     dim3 g((L.n[1] + 1) / kPlaneRows, c.planeSegs, 1);
     if (c.planeMaxQ == 5) {
@@ -2992,7 +2998,7 @@ int mg_setup(Ctx &c) {
     SARAS_CUDA_TRY(cudaFuncSetAttribute(k_mg_coarse<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCoarseSmem));
     SARAS_CUDA_TRY(cudaDeviceGetAttribute(&c.numSMs, cudaDevAttrMultiProcessorCount, c.dev));
     SARAS_CUDA_TRY(cudaFuncSetAttribute(k_mg_gs_block, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGsBlockSmem));
-    SARAS_CUDA_TRY(cudaMemsetAsync(c.dflag, 0, 3 * sizeof(int), c.stream));
+    SARAS_CUDA_TRY(cudaMemsetAsync(c.dflag, 0, sizeof(int), c.stream));
     if (p.gsSmooth) SARAS_CUDA_TRY(cudaMalloc(&c.gsFace, sizeof(double) * gs_face_count(c.lv[0])));
     if (int e = plane_setup(c)) return e;
     c.tailLt = c.planar ? 0 : tail_level(c);   // target modes only (3D)
@@ -4004,7 +4010,7 @@ static int mixed_fixed(Ctx &c, const double *pp0, double mean, double bmax, doub
         int fl = 0, tmaErr = 0;
         SARAS_CUDA_TRY(cudaMemcpyAsync(&mx, dmax, sizeof(mx), cudaMemcpyDeviceToHost, c.stream));
         SARAS_CUDA_TRY(cudaMemcpyAsync(&fl, dflag, sizeof(fl), cudaMemcpyDeviceToHost, c.stream));
-        if (c.planeOk) SARAS_CUDA_TRY(cudaMemcpyAsync(&tmaErr, c.dflag + 2, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
+        if (c.planeOk) SARAS_CUDA_TRY(cudaMemcpyAsync(&tmaErr, c.dflag, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
         SARAS_CUDA_TRY(cudaStreamSynchronize(c.stream));
         if (tmaErr) { c.err = "plane-streaming stencil: an mbarrier wait timed out"; return SARAS_CUDA_ERROR; }
         out = (double)mx * rs;
